@@ -408,7 +408,8 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
     kern_ms = stages.get("trace", {}).get("ms", float("nan")) / K
     trace_bytes = n_rays * BYTES_PER_RAY + int(info.device_bytes)
     prof = trace_profile()
-    kname = (f"k_trace_ww<{width},false,{topts['stack_depth']}>" if topts["persistent"] == 2 else
+    kname = ("k_trace4<false>" if width == 4 else
+             f"k_trace_ww<{width},false,{topts['stack_depth']}>" if topts["persistent"] == 2 else
              f"k_trace_persistent<{width},false,{topts['stack_depth']}>" if topts["persistent"] else
              f"k_trace_wide<{width},false,{topts['stack_depth']}>") if width > 2 else "k_trace_bvh2<false>"
     prof_ok = bool(prof) and not prof["stale"] and prof.get("kernel") == kname

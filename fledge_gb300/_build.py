@@ -21,6 +21,7 @@ LIB = os.path.join(HERE, "libflg.so")
 SOURCES = ["api.cu", "build.cu", "sort.cu", "collapse.cu", "trace.cu", "volume.cu",
            "adjoint.cu", "gen.cu", "pathtrace.cu", "ploc.cu", "sah.cu", "treelet.cu", "ply.cpp"]
 HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "internal.h"), os.path.join(CSRC, "volume.cuh"),
+           os.path.join(CSRC, "wide.cuh"),
            os.path.join(ROOT, "include", "flg.h")]
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

@@ -104,8 +104,7 @@ FLG_API int flg_ctx_destroy(flg_ctx c) {
   cudaFree(c->d_err);
   if (c->h_err) cudaFreeHost(c->h_err);
   cudaFree(c->d_ovf);
-  cudaFree(c->d_ovf_count);
-  cudaFree(c->d_work);
+  cudaFree(c->d_trace_ctr);
   cudaFree(c->d_ray_off);
   cudaFree(c->stage);
   cudaFree(c->pt_buf);

@@ -9,9 +9,11 @@
 // The Karras topology itself (the parity object) is unchanged.
 #include <algorithm>
 #include <climits>
+#include <vector>
 
 #include "common.cuh"
 #include "internal.h"
+#include "wide.cuh"
 
 namespace flg {
 
@@ -20,54 +22,6 @@ constexpr int kMaxLevels = 64;
 // [kMaxLevels + 2 .. + 3] the one-launch collapse's barrier; the initial
 // values of these kCtrLive words follow as a static copy.
 constexpr int kCtrLive = kMaxLevels + 4;
-
-struct Cand {
-  int32_t ref;     // BVH2 ref (>=0 internal, <0 ~leaf position)
-  int32_t first;   // first sorted triangle of the subtree
-  int32_t count;   // triangles in the subtree
-  float lo[3], hi[3];
-};
-
-__device__ __forceinline__ float half_area(const Cand &c) {
-  float dx = c.hi[0] - c.lo[0], dy = c.hi[1] - c.lo[1], dz = c.hi[2] - c.lo[2];
-  return dx * dy + dy * dz + dz * dx;
-}
-
-// Leaf ranges of internal nodes.  LBVH records carry their own range
-// (d.z, d.w: first and last sorted triangle) and split (the left child ref
-// names it, node slots being numbered by sorted position), so both children's
-// ranges come from the parent's record; PLOC trees keep explicit depth-first
-// ranges (rfirst / rcount) per node.
-struct Ranges {
-  const int32_t *rfirst, *rcount;
-};
-
-__device__ __forceinline__ void child_cands(const Node2 &nd, const Ranges &R, Cand &c0, Cand &c1) {
-  int32_t r[2] = {nd.d.x, nd.d.y};
-  Cand *o[2] = {&c0, &c1};
-  const float lo[2][3] = {{nd.a.x, nd.a.z, nd.c.x}, {nd.b.x, nd.b.z, nd.c.z}};
-  const float hi[2][3] = {{nd.a.y, nd.a.w, nd.c.y}, {nd.b.y, nd.b.w, nd.c.w}};
-  const int32_t split = r[0] >= 0 ? r[0] : ~r[0];
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    Cand &c = *o[k];
-    c.ref = r[k];
-    for (int a = 0; a < 3; ++a) {
-      c.lo[a] = lo[k][a];
-      c.hi[a] = hi[k][a];
-    }
-    if (!R.rfirst) {
-      c.first = k == 0 ? nd.d.z : split + 1;
-      c.count = k == 0 ? split - nd.d.z + 1 : nd.d.w - split;
-    } else if (r[k] < 0) {
-      c.first = ~r[k];
-      c.count = 1;
-    } else {
-      c.first = R.rfirst[r[k]];
-      c.count = R.rcount[r[k]];
-    }
-  }
-}
 
 // One wide node per queued BVH2 node of a level (cnt items in q_in).  The
 // new wide slots and queue entries of a warp are claimed with one atomic per
@@ -79,7 +33,7 @@ template <int W>
 __device__ __forceinline__ void collapse_level(const Node2 *__restrict__ nodes2, const Ranges &R, int leaf_size,
                                                const int2 *__restrict__ q_in, int cnt, int2 *__restrict__ q_out,
                                                int32_t *q_out_count, int32_t *node_ctr, int64_t cap,
-                                               NodeW<W> *__restrict__ wide, uint32_t *err) {
+                                               typename WideRec<W>::T *__restrict__ wide, uint32_t *err) {
   const int lane = threadIdx.x & 31;
   // Warp-uniform loop: all lanes of a warp share it0.
   for (int it0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) & ~31u); it0 < cnt;
@@ -92,49 +46,10 @@ __device__ __forceinline__ void collapse_level(const Node2 *__restrict__ nodes2,
     if (valid) {
       item = __ldcg(q_in + it);
       // cap = BVH2 node count + 1: item.x names a BVH2 node, item.y a wide slot.
-      if (item.x < 0 || item.y < 0 || item.x >= cap - 1 || item.y >= cap) {
+      if (item.x < 0 || item.y < 0 || item.x >= cap - 1 || item.y >= cap)
         atomicOr(err, kErrQueue);  // a hole left by an overflowing level
-      } else {
-        nc = 2;
-        child_cands(nodes2[item.x], R, c[0], c[1]);
-      }
-    }
-    // The records of both children that may be opened are fetched together:
-    // the first opening takes one of them and the second usually the other,
-    // so most wide nodes wait on two dependent loads instead of three.
-    Node2 pf0, pf1;
-    const int32_t pf0_ref = nc == 2 && c[0].ref >= 0 && c[0].count > leaf_size ? c[0].ref : -1;
-    const int32_t pf1_ref = nc == 2 && c[1].ref >= 0 && c[1].count > leaf_size ? c[1].ref : -1;
-    if (pf0_ref >= 0) pf0 = nodes2[pf0_ref];
-    if (pf1_ref >= 0) pf1 = nodes2[pf1_ref];
-    while (nc >= 2 && nc < W) {
-      int best = -1;
-      float ba = -1.0f;
-#pragma unroll
-      for (int k = 0; k < W; ++k) {
-        if (k < nc && c[k].ref >= 0 && c[k].count > leaf_size) {
-          float a = half_area(c[k]);
-          if (a > ba) {
-            ba = a;
-            best = k;
-          }
-        }
-      }
-      if (best < 0) break;
-      Cand a, b;
-      int32_t r = 0;
-#pragma unroll
-      for (int k = 0; k < W; ++k)
-        if (k == best) r = c[k].ref;
-      if (r == pf0_ref) child_cands(pf0, R, a, b);
-      else if (r == pf1_ref) child_cands(pf1, R, a, b);
-      else child_cands(nodes2[r], R, a, b);
-#pragma unroll
-      for (int k = 0; k < W; ++k) {
-        if (k == best) c[k] = a;
-        if (k == nc) c[k] = b;
-      }
-      ++nc;
+      else
+        open_wide<W>(nodes2, R, leaf_size, item.x, c, nc);
     }
     // Children that become wide nodes of the next level.
     int need = 0;
@@ -156,35 +71,54 @@ __device__ __forceinline__ void collapse_level(const Node2 *__restrict__ nodes2,
     slot0 = __shfl_sync(0xFFFFFFFFu, slot0, 31) + incl - need;
     q0 = __shfl_sync(0xFFFFFFFFu, q0, 31) + incl - need;
     if (!valid || nc == 0) continue;
-    NodeW<W> out;
+    int32_t child[W];
 #pragma unroll
     for (int k = 0; k < W; ++k) {
+      child[k] = kEmptyChild;
       if (k < nc) {
-        out.lox[k] = c[k].lo[0];
-        out.loy[k] = c[k].lo[1];
-        out.loz[k] = c[k].lo[2];
-        out.hix[k] = c[k].hi[0];
-        out.hiy[k] = c[k].hi[1];
-        out.hiz[k] = c[k].hi[2];
         if (c[k].ref < 0 || c[k].count <= leaf_size) {
-          out.child[k] = ~((c[k].first << 3) | (c[k].count - 1));
+          child[k] = ~((c[k].first << 3) | (c[k].count - 1));
         } else {
           const int slot = slot0++;
           if (slot >= cap) {
             atomicOr(err, kErrQueue);
             if (q0 < cap) q_out[q0] = make_int2(-1, -1);  // the next level skips it
             ++q0;
-            out.child[k] = kEmptyChild;
           } else {
             q_out[q0++] = make_int2(c[k].ref, slot);
-            out.child[k] = slot;
+            child[k] = slot;
           }
         }
-      } else {
-        const float inf = __int_as_float(0x7f800000);
-        out.lox[k] = out.loy[k] = out.loz[k] = inf;
-        out.hix[k] = out.hiy[k] = out.hiz[k] = inf;
-        out.child[k] = kEmptyChild;
+      }
+    }
+    typename WideRec<W>::T out;
+    if constexpr (W == 4) {
+      quantise(c, nc, out);
+      // This lane's inner children took consecutive slots.
+      out.base = 0;
+      out.kind = 0u;
+      uint32_t rank = 0u;
+#pragma unroll
+      for (int k = 3; k >= 0; --k)
+        if (child[k] >= 0 && child[k] != kEmptyChild) out.base = child[k];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const bool inner = child[k] >= 0 && child[k] != kEmptyChild;
+        out.kind |= (inner ? rank : 0x80u | (uint32_t)k) << (8 * k);
+        rank += inner ? 1u : 0u;
+        out.leaf[k] = inner ? kEmptyChild : child[k];
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < W; ++k) {
+        const float inf = __int_as_float(0x7f800000);  // unused slots: +inf boxes, which no ray enters
+        out.lox[k] = k < nc ? c[k].lo[0] : inf;
+        out.loy[k] = k < nc ? c[k].lo[1] : inf;
+        out.loz[k] = k < nc ? c[k].lo[2] : inf;
+        out.hix[k] = k < nc ? c[k].hi[0] : inf;
+        out.hiy[k] = k < nc ? c[k].hi[1] : inf;
+        out.hiz[k] = k < nc ? c[k].hi[2] : inf;
+        out.child[k] = child[k];
       }
     }
     wide[item.y] = out;
@@ -195,7 +129,7 @@ template <int W>
 __global__ void __launch_bounds__(128)
     k_collapse_level(const Node2 *__restrict__ nodes2, Ranges R, int leaf_size,
                      const int2 *__restrict__ q_in, const int32_t *__restrict__ q_in_count, int2 *__restrict__ q_out,
-                     int32_t *q_out_count, int32_t *node_ctr, int64_t cap, NodeW<W> *__restrict__ wide,
+                     int32_t *q_out_count, int32_t *node_ctr, int64_t cap, typename WideRec<W>::T *__restrict__ wide,
                      uint32_t *err) {
   // Counts beyond the queue capacity only arise from a corrupted tree.
   const int cnt = (int)min((int64_t)*q_in_count, cap);
@@ -236,7 +170,7 @@ __device__ __forceinline__ void grid_barrier(uint32_t *bar, uint32_t limit, uint
 template <int W>
 __global__ void __launch_bounds__(128)
     k_collapse_all(const Node2 *__restrict__ nodes2, Ranges R, int leaf_size, int2 *q0, int2 *q1, int32_t *ctr,
-                   uint32_t *bar, int64_t cap, NodeW<W> *__restrict__ wide, uint32_t spin_limit, uint32_t *err) {
+                   uint32_t *bar, int64_t cap, typename WideRec<W>::T *__restrict__ wide, uint32_t spin_limit, uint32_t *err) {
   for (int L = 0; L < kMaxLevels; ++L) {
     // Counts beyond the queue capacity only arise from a corrupted tree.
     const int cnt = (int)min((int64_t)(int32_t)ld_volatile((const uint32_t *)(ctr + 1 + L)), cap);
@@ -254,7 +188,7 @@ __global__ void k_collapse_check(const int32_t *last_count, uint32_t *err) {
 int collapse_reserve(flg_ctx ctx, flg_bvh b) {
   // Every wide node corresponds to a distinct BVH2 internal node.
   const int64_t cap = b->n_nodes + 1;
-  const size_t rec = b->width == 4 ? sizeof(NodeW<4>) : sizeof(NodeW<8>);
+  const size_t rec = b->width == 4 ? sizeof(NodeQ) : sizeof(NodeW<8>);
   int rc = FLG_OK;
   if (b->d_wide) {
     cudaFree(b->d_wide);
@@ -274,42 +208,57 @@ int collapse_reserve(flg_ctx ctx, flg_bvh b) {
     if ((rc = halloc(b, &b->d_queue[0], cap))) return rc;
     if ((rc = halloc(b, &b->d_queue[1], cap))) return rc;
     if ((rc = halloc(b, &b->d_queue_init, b->n_scenes))) return rc;
-    std::vector<int32_t> roots(b->n_scenes);
-    std::vector<int2> q;
-    for (int s = 0; s < b->n_scenes; ++s) {
-      int64_t c = b->tri_off_h[s + 1] - b->tri_off_h[s];
-      if (c >= 2) {
-        roots[s] = (int32_t)q.size();
-        q.push_back(make_int2((int)b->node_off_h[s], (int)q.size()));
-      } else if (c == 1) {
-        roots[s] = ~(int32_t)(b->tri_off_h[s] << 3);
-      } else {
-        roots[s] = kEmptyChild;
-      }
-    }
-    b->n_wide_roots = (int32_t)q.size();
-    std::vector<int32_t> ctr(2 * kCtrLive, 0);
-    ctr[0] = b->n_wide_roots;
-    ctr[1] = b->n_wide_roots;
-    ctr[kCtrLive] = b->n_wide_roots;
-    ctr[kCtrLive + 1] = b->n_wide_roots;
-    cudaStream_t st = ctx->stream;
-    cudaError_t e = cudaMemcpyAsync(b->d_wide_root, roots.data(), sizeof(int32_t) * b->n_scenes,
-                                    cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && !q.empty())
-      e = cudaMemcpyAsync(b->d_queue_init, q.data(), sizeof(int2) * q.size(), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(b->d_wide_ctr, ctr.data(), sizeof(int32_t) * ctr.size(), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "collapse upload");
   }
+  // Scenes of one triangle: their root is the leaf in the 8-wide layout; in
+  // the 4-wide one a node, written here once, whose one box constrains
+  // nothing.
+  std::vector<int32_t> roots(b->n_scenes);
+  std::vector<int2> q;
+  std::vector<NodeQ> lone;  // records of slots [0, lone.size())
+  int32_t slots = 0;
+  for (int s = 0; s < b->n_scenes; ++s) {
+    int64_t c = b->tri_off_h[s + 1] - b->tri_off_h[s];
+    if (c >= 2) {
+      roots[s] = slots;
+      q.push_back(make_int2((int)b->node_off_h[s], slots++));
+    } else if (c == 1 && b->width == 4) {
+      NodeQ nd = {};
+      nd.step = kLoneStep;
+      nd.kind = 0x83828180u;
+      nd.leaf[0] = ~(int32_t)(b->tri_off_h[s] << 3);
+      nd.leaf[1] = nd.leaf[2] = nd.leaf[3] = kEmptyChild;
+      roots[s] = slots++;
+      lone.resize(slots);  // the ones between are written by every collapse
+      lone.back() = nd;
+    } else if (c == 1) {
+      roots[s] = ~(int32_t)(b->tri_off_h[s] << 3);
+    } else {
+      roots[s] = kEmptyChild;
+    }
+  }
+  b->n_wide_roots = (int32_t)q.size();
+  std::vector<int32_t> ctr(2 * kCtrLive, 0);
+  ctr[0] = ctr[kCtrLive] = slots;
+  ctr[1] = ctr[kCtrLive + 1] = b->n_wide_roots;
+  cudaStream_t st = ctx->stream;
+  cudaError_t e = cudaMemcpyAsync(b->d_wide_root, roots.data(), sizeof(int32_t) * b->n_scenes,
+                                  cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && !q.empty())
+    e = cudaMemcpyAsync(b->d_queue_init, q.data(), sizeof(int2) * q.size(), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(b->d_wide_ctr, ctr.data(), sizeof(int32_t) * ctr.size(), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && !lone.empty())
+    e = cudaMemcpyAsync(b->d_wide, lone.data(), sizeof(NodeQ) * lone.size(), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "collapse upload");
   return FLG_OK;
 }
 
 template <int W>
 static int collapse_levels(flg_ctx ctx, flg_bvh b) {
   cudaStream_t st = ctx->stream;
-  NodeW<W> *wide = (NodeW<W> *)b->d_wide;
+  using Rec = typename WideRec<W>::T;
+  Rec *wide = (Rec *)b->d_wide;
   const Ranges R{b->d_rfirst, b->d_rcount};
   // Level sizes are only known on the device.  Default: one cooperative
   // launch of one resident wave that walks the levels with a grid barrier in

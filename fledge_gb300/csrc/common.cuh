@@ -172,19 +172,9 @@ __device__ __forceinline__ float3 f3cross(float3 a, float3 b) {
   return make_float3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
 }
 
-// Hit test and t only; U, V and U+V+W are returned for the barycentrics.
-__device__ __forceinline__ bool pluecker_core(float3 a, float3 b, float3 c, float3 O, float3 D, float &t, float &U,
-                                              float &V, float &UVW) {
-  float3 v0 = f3sub(a, O), v1 = f3sub(b, O), v2 = f3sub(c, O);
-  float3 e0 = f3sub(v2, v0), e1 = f3sub(v0, v1), e2 = f3sub(v1, v2);
-  U = f3dot(f3cross(e0, f3add(v2, v0)), D);
-  V = f3dot(f3cross(e1, f3add(v0, v1)), D);
-  float W = f3dot(f3cross(e2, f3add(v1, v2)), D);
-  UVW = U + V + W;
-  float eps = 1.1920928955078125e-07f * fabsf(UVW);
-  bool valid = fminf(U, fminf(V, W)) >= -eps || fmaxf(U, fmaxf(V, W)) <= eps;
-  if (!valid) return false;
-  // StableTriangleNormal (intersector.hpp:45-60)
+// The distance of the plane hit, from StableTriangleNormal (intersector.hpp:
+// 45-60); false if it is not in front or the ray is parallel.
+__device__ __forceinline__ bool pluecker_dist(float3 v0, float3 e0, float3 e1, float3 e2, float3 D, float &t) {
   float ab_x = e0.z * e1.y, ab_y = e0.x * e1.z, ab_z = e0.y * e1.x;
   float bc_x = e1.z * e2.y, bc_y = e1.x * e2.z, bc_z = e1.y * e2.x;
   float3 N;
@@ -198,6 +188,21 @@ __device__ __forceinline__ bool pluecker_core(float3 a, float3 b, float3 c, floa
   if (!(den != 0.0f)) return false;
   t = tt;
   return true;
+}
+
+// Hit test and t only; U, V and U+V+W are returned for the barycentrics.
+__device__ __forceinline__ bool pluecker_core(float3 a, float3 b, float3 c, float3 O, float3 D, float &t, float &U,
+                                              float &V, float &UVW) {
+  float3 v0 = f3sub(a, O), v1 = f3sub(b, O), v2 = f3sub(c, O);
+  float3 e0 = f3sub(v2, v0), e1 = f3sub(v0, v1), e2 = f3sub(v1, v2);
+  U = f3dot(f3cross(e0, f3add(v2, v0)), D);
+  V = f3dot(f3cross(e1, f3add(v0, v1)), D);
+  float W = f3dot(f3cross(e2, f3add(v1, v2)), D);
+  UVW = U + V + W;
+  float eps = 1.1920928955078125e-07f * fabsf(UVW);
+  bool valid = fminf(U, fminf(V, W)) >= -eps || fmaxf(U, fmaxf(V, W)) <= eps;
+  if (!valid) return false;
+  return pluecker_dist(v0, e0, e1, e2, D, t);
 }
 
 // Triangle::intersect of the live renderer (shape.cpp:100-148): Moller-

@@ -29,20 +29,49 @@ struct alignas(16) Node2 {
 // or the canonical NaN).
 constexpr int32_t kBoxUnset = (int32_t)0xFFC0DEADu;
 
-// Wide node of width W, structure of arrays inside the record (7 / 14
-// 16-byte loads per visit).  Child refs: >= 0 wide node index; < 0 leaf range
-// ~(first << 3 | (count - 1)) over sorted triangles; kEmptyChild = unused
-// slot.  (8-bit quantised child boxes, 64 / 96 bytes, were measured too: no
-// gain on incoherent rays, 35 % slower on coherent camera rays, where the
-// decode's integer work dominates.)
+// Wide nodes: child refs >= 0 are wide node indices; < 0 leaf ranges
+// ~(first << 3 | (count - 1)) over sorted triangles; kEmptyChild = unused slot.
 constexpr int32_t kEmptyChild = 0x7FFFFFFF;
+
+// 4-wide node: the children's boxes in 8 bits per plane, as (origin + byte x
+// 2^(e - 127)) per axis, conservative (quantise, wide.cuh).  The traversal is
+// bound by its divergent 16-byte loads, one L1 wavefront per lane and load:
+// this record takes 3 per visit against 6 and the refs for the same boxes in
+// fp32.  Inner children sit in consecutive slots; a leaf child's range is read
+// when the leaf is tested.  What the exact boxes decide beyond that is
+// re-decided per hit (k_trace4, k_trace_finish4).
+struct alignas(16) NodeQ {
+  float org[3];
+  uint32_t step;    // exponents: y << 23 | z << 15 | x << 7
+  uint32_t qlo[3];  // per axis, byte k: child k's lower plane
+  uint32_t qhi[3];
+  int32_t base;     // slot of the first inner child
+  uint32_t kind;    // byte k: child k's rank among the inner children, or 0x80 | k (leaf, unused)
+  int32_t leaf[4];  // leaf children: ~range
+};
+static_assert(sizeof(NodeQ) == 64, "NodeQ layout");
+// Step word of the node of a one-triangle scene: infinite on every axis (a
+// word that quantise gives to no node with a finite box).
+constexpr uint32_t kLoneStep = 255u << 23 | 255u << 15 | 255u << 7;
+
+// 8-wide node, structure of arrays inside the record (14 16-byte loads per
+// visit).
 template <int W>
 struct alignas(16) NodeW {
   float lox[W], hix[W], loy[W], hiy[W], loz[W], hiz[W];
   int32_t child[W];
 };
-static_assert(sizeof(NodeW<4>) == 112, "NodeW<4> layout");
 static_assert(sizeof(NodeW<8>) == 224, "NodeW<8> layout");
+
+// The record of a layout of width W.
+template <int W>
+struct WideRec {
+  using T = NodeW<W>;
+};
+template <>
+struct WideRec<4> {
+  using T = NodeQ;
+};
 
 // Sorted triangle record: v0.xyz + original (scene-local) id, v1, v2.
 struct alignas(16) TriRec {
@@ -63,12 +92,13 @@ struct flg_ctx_t {
   int num_sms = 0;
   int64_t launches = 0;  // kernels launched through this context
   std::string last_error;
-  // Traversal scratch: rays whose stack overflowed (retried with a deep
-  // stack), the persistent kernels' work counter, per-call ray offsets.
+  // Traversal scratch, two sets: rays to trace again (stack overflow, and for
+  // the 4-wide layout hits that the exact boxes have to settle).  Counters, in
+  // pairs: rays taken by persistent kernels, entries of that list.
   int64_t *d_ovf = nullptr;
-  uint32_t *d_ovf_count = nullptr;
   int64_t ovf_cap = 0;
-  unsigned long long *d_work = nullptr;  // [0] persistent ray counter
+  unsigned long long *d_trace_ctr = nullptr;
+  bool trace4_open = false;              // a 4-wide trace's launches were cut short: clear its counters
   int64_t *d_ray_off = nullptr;          // device copy of batched ray offsets
   int64_t ray_off_cap = 0;
   std::vector<int64_t> ray_off_h;        // host copy of what d_ray_off holds

@@ -3,17 +3,19 @@
 // watertight Pluecker test of intersector.hpp:63-101).
 //
 // Layouts: BVH2 nodes carry both children's boxes (one 64-byte record per
-// visit); wide nodes (4 or 8 children) store their child boxes as structure
-// of arrays inside a 112/224-byte record read with 16-byte loads; triangles
-// are gathered in sorted (leaf) order, 48 bytes each.
+// visit); 4-wide nodes hold their child boxes in 8 bits per plane (64 bytes);
+// 8-wide nodes as structure of arrays in fp32 (224 bytes); triangles are
+// gathered in sorted (leaf) order, 48 bytes each.
 //
 // Kernels:
+//   k_trace4            4-wide: while-while traversal with parked leaves, one
+//                       ray per thread or persistent warps that refill idle
+//                       lanes from a global ray counter (work stealing across
+//                       scenes of a batch); k_trace_finish4 after it
 //   k_trace_bvh2        one ray per thread over BVH2, leaf triangles tested
 //                       directly as the reference does (no leaf box test)
-//   k_trace_wide        one ray per thread over 4/8-wide nodes, children
-//                       visited nearest first (sorting network on t|ref keys)
-//   k_trace_persistent  persistent warps that refill idle lanes from a global
-//                       ray counter (work stealing across scenes of a batch)
+//   k_trace_wide, k_trace_persistent, k_trace_ww   the same three schedules
+//                       over 8-wide nodes
 //   k_trace_retry       rays whose short stack overflowed, with a deep stack
 #include <algorithm>
 #include <chrono>
@@ -24,6 +26,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "wide.cuh"
 
 namespace flg {
 
@@ -490,12 +493,848 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// ----------------------------------------------------------------------------
+// 4-wide traversal over quantised nodes (NodeQ).
+//
+// The results are those of a traversal over the exact child boxes (fp32, the
+// reference's slab test, children nearest first, first found kept among equal
+// t), although the boxes the traversal reads are a little larger:
+//   * A quantised box contains the exact one with room for every rounding of
+//     visit_q, so the leaves visited are a superset of the exact ones.
+//   * Closest hit: a finished ray's winner stands if its own box, which its
+//     leaf range's and every ancestor's box contain, passes the exact slab
+//     test with tnear <= t: then the exact traversal reaches it, whatever it
+//     found before.  (tnear > t is a matter of rounding, for flat boxes; it
+//     counts only if another candidate, or tmax, lay within kNear.)  Among
+//     equal t the first in the exact order of visits wins.  The rays that this
+//     does not settle go on a list, and k_settle4 settles the equal pairs
+//     (first_of_two) and traces the others again over the exact boxes
+//     (retrace4): about one ray per million on random soups.
+//   * Any hit: an accepted triangle counts if its own box, or else the box of
+//     its leaf range, passes the exact slab test.
+// ----------------------------------------------------------------------------
+constexpr float kNear = 4.76837158203125e-07f;  // 2^-21
+// prim between k_trace4 and the kernels after it: a sorted position (< 2^28) with
+// kPending, -1, or kListed for a listed ray.  A listed ray's u and v hold two
+// positions at the same t, or v = -1: trace it again.
+constexpr int32_t kPending = 1 << 30;
+constexpr int32_t kListed = INT32_MIN;
+
+__device__ __forceinline__ float max3f(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float min3f(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// Inverse direction for the quantised slab test: the infinite inverse of a
+// zero component becomes +-2^90, so that plane distances stay finite (an
+// infinite one would be NaN after the multiply-add and drop the axis).
+__device__ __forceinline__ float inv_q(float inv) {
+  return fabsf(inv) <= 3.402823466e+38f ? inv : copysignf(1.2379400392853803e27f, inv);
+}
+
+// Two fp32 values in one 64-bit register: sm_103a's packed add, multiply and
+// fused multiply-add do both in one issue slot, with the scalar roundings.
+// The traversal is bound by issue slots once its loads are few.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &a, float &b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// Byte k of w as the float 2^15 + byte: one byte permute puts it above the
+// last mantissa byte of 2^15.
+template <int K>
+__device__ __forceinline__ float byte_f(uint32_t w) {
+  return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7404 | (K << 4)));
+}
+
+// Tests the children of a quantised node.  key[k]: tnear with child k's kind
+// byte in place of its low byte (masked off again, i.e. rounded down, when a
+// stack entry is culled); a miss is ~0.  Per axis the plane distance
+// of byte q is fma(2^15 + q, step inv, (origin - o) inv - 2^15 step inv).  Its
+// error is below 1/64 step (the boxes' slack) plus 2^-22 of itself, and the
+// exact test's own below 2^-23: with tnear scaled by 1 - 2^-20 the test passes
+// whenever the exact one does.
+__device__ __forceinline__ void visit_q(const NodeQ *__restrict__ node, const float3 &o, const float3 &inv, float lim,
+                                        uint32_t (&key)[4], int32_t &base) {
+  const uint4 *np = (const uint4 *)node;
+  const uint4 A = __ldg(np), B = __ldg(np + 1), C = __ldg(np + 2);
+  base = (int32_t)C.z;
+  const float ex = __uint_as_float((A.w << 16) & 0x7F800000u);
+  const float ey = __uint_as_float(A.w & 0x7F800000u);
+  const float ez = __uint_as_float((A.w << 8) & 0x7F800000u);
+  const float sx = ex * inv.x, sy = ey * inv.y, sz = ez * inv.z;
+  const float bx = fmaf(-32768.0f, sx, (__uint_as_float(A.x) - o.x) * inv.x);
+  const float by = fmaf(-32768.0f, sy, (__uint_as_float(A.y) - o.y) * inv.y);
+  const float bz = fmaf(-32768.0f, sz, (__uint_as_float(A.z) - o.z) * inv.z);
+  // (near, far) pairs, the near one scaled
+  constexpr float k = 0.99999905f;  // 1 - 2^-20
+  const f32x2 sx2 = pack2(sx * k, sx), sy2 = pack2(sy * k, sy), sz2 = pack2(sz * k, sz);
+  const f32x2 bx2 = pack2(bx * k, bx), by2 = pack2(by * k, by), bz2 = pack2(bz * k, bz);
+  const bool gx = __float_as_int(inv.x) < 0, gy = __float_as_int(inv.y) < 0, gz = __float_as_int(inv.z) < 0;
+  const uint32_t nx = gx ? B.w : B.x, fx = gx ? B.x : B.w;
+  const uint32_t ny = gy ? C.x : B.y, fy = gy ? B.y : C.x;
+  const uint32_t nz = gz ? C.y : B.z, fz = gz ? B.z : C.y;
+  const float t1c = fminf(lim, 3.402823466e+38f);
+  auto child = [&](auto kc) {
+    constexpr int K = decltype(kc)::value;
+    float ax, ay, az, cx, cy, cz;
+    unpack2(fma2(pack2(byte_f<K>(nx), byte_f<K>(fx)), sx2, bx2), ax, cx);
+    unpack2(fma2(pack2(byte_f<K>(ny), byte_f<K>(fy)), sy2, by2), ay, cy);
+    unpack2(fma2(pack2(byte_f<K>(nz), byte_f<K>(fz)), sz2, bz2), az, cz);
+    const float t0 = fmaxf(max3f(ax, ay, az), 0.0f);
+    const float t1 = fminf(min3f(cx, cy, cz), t1c);
+    key[K] = t0 <= t1 ? __byte_perm(__float_as_uint(t0), C.w, 0x3214 + K) : ~0u;
+  };
+  child(std::integral_constant<int, 0>{});
+  child(std::integral_constant<int, 1>{});
+  child(std::integral_constant<int, 2>{});
+  child(std::integral_constant<int, 3>{});
+}
+
+// The child of node `cur` that a key names: an inner child's slot, or, with
+// the sign bit set, 4 cur + its slot in the node for a leaf, whose range is
+// read when it is tested.
+__device__ __forceinline__ int32_t child_ref(uint32_t key, int32_t cur, int32_t base) {
+  const uint32_t code = key & 0xFFu;
+  const uint32_t from = code & 0x80u ? 0x7FFFFF80u + 4u * (uint32_t)cur : (uint32_t)base;
+  return (int32_t)(from + code);
+}
+
+// pluecker_t with the U and V sides in packed arithmetic: the same operations
+// in the same order.  ptxas contracts a packed multiplication and addition
+// whatever their rounding modifiers and -fmad say, so sums of products are
+// formed as fma(p, one, q) with a `one` that it cannot see through (the two
+// are equal: p x 1 is exact), and differences as sums with a negated edge.
+__device__ __forceinline__ bool pluecker_t2(float3 a, float3 b, float3 c, float3 O, float3 D, f32x2 one, float &t) {
+  const float3 v0 = f3sub(a, O), v1 = f3sub(b, O), v2 = f3sub(c, O);
+  // lower half: edge e0 = v2 - v0 with v2 + v0, upper half: e1 = v0 - v1 with v0 + v1
+  const f32x2 px = pack2(v2.x, v0.x), py = pack2(v2.y, v0.y), pz = pack2(v2.z, v0.z);
+  const f32x2 qx = pack2(v0.x, v1.x), qy = pack2(v0.y, v1.y), qz = pack2(v0.z, v1.z);
+  const f32x2 ex = sub2(px, qx), ey = sub2(py, qy), ez = sub2(pz, qz);
+  const f32x2 mx = sub2(qx, px), my = sub2(qy, py), mz = sub2(qz, pz);
+  const f32x2 sx = add2(px, qx), sy = add2(py, qy), sz = add2(pz, qz);
+  const f32x2 kx = fma2(mul2(mz, sy), one, mul2(ey, sz)), ky = fma2(mul2(mx, sz), one, mul2(ez, sx)),
+              kz = fma2(mul2(my, sx), one, mul2(ex, sy));
+  float U, V;
+  unpack2(fma2(fma2(mul2(kx, pack2(D.x, D.x)), one, mul2(ky, pack2(D.y, D.y))), one, mul2(kz, pack2(D.z, D.z))), U, V);
+  const float3 e2 = f3sub(v1, v2);
+  const float W = f3dot(f3cross(e2, f3add(v1, v2)), D);
+  const float UVW = U + V + W;
+  const float eps = 1.1920928955078125e-07f * fabsf(UVW);
+  if (!(min3f(U, V, W) >= -eps || max3f(U, V, W) <= eps)) return false;
+  float3 e0, e1;
+  unpack2(ex, e0.x, e1.x);
+  unpack2(ey, e0.y, e1.y);
+  unpack2(ez, e0.z, e1.z);
+  return pluecker_dist(v0, e0, e1, e2, D, t);
+}
+
+// The exact slab test of a box against (o, inv), limit lim: tnear, or NaN on
+// a miss — the same operations as the fp32 wide nodes' visit_node.
+__device__ __forceinline__ float slab_exact(const float *lo, const float *hi, const float3 &o, const float3 &inv,
+                                            float lim) {
+  const float oo[3] = {o.x, o.y, o.z}, ii[3] = {inv.x, inv.y, inv.z};
+  float t0 = 0.0f, t1 = fminf(lim, 3.402823466e+38f);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const bool g = (__float_as_uint(ii[a]) >> 31) != 0u;
+    const float tn = ((g ? hi[a] : lo[a]) - oo[a]) * ii[a], tf = ((g ? lo[a] : hi[a]) - oo[a]) * ii[a];
+    t0 = fmaxf(tn, t0);
+    t1 = fminf(tf, t1);
+  }
+  return t0 <= t1 ? t0 : __int_as_float(0x7fffffff);
+}
+
+// The exact-box tree of a 4-wide handle.
+struct Exact4 {
+  const Node2 *nodes2;
+  const TriRec *tris;
+  Ranges R;
+  int32_t leaf_size;
+  const int32_t *roots;  // BVH2 roots per scene
+  const int64_t *ray_off;
+  int32_t n_scenes;
+};
+
+// Ray `ray` over the exact boxes, in the exact order: the children of a wide
+// node are formed from the BVH2 records as the collapse forms them, and
+// visited nearest first with a deep stack.  Returns the sorted position and t
+// of the closest hit (any hit: any position), or -1 and tmax.
+struct ExactHit {
+  int32_t prim;
+  float t;
+};
+template <bool ANY>
+__device__ __forceinline__ ExactHit retrace4(const Exact4 &X, const RaySoA &RS, int64_t ray,
+                                             uint32_t *err) {
+  // Entries: (tnear rounded down | BVH2 ref, or ~(first << 3 | count - 1)).
+  uint64_t stk[kRetryStack];
+  float3 o, d, inv;
+  float tmin, tmax;
+  load_ray(RS, ray, o, d, inv, tmin, tmax);
+  const int32_t root = scene_root(X.roots, X.ray_off, X.n_scenes, ray);
+  ExactHit h{-1, tmax};
+  if (root == INT32_MIN) return h;
+  float best = tmax;
+  bool have = false;
+  int sp = 0;
+  stk[sp++] = (uint32_t)(root < 0 ? ~((~root) << 3) : root);
+  // (a ray visits far fewer nodes; the bound ends a walk over a broken tree)
+  for (int visits = 0; sp > 0 && visits < (1 << 22); ++visits) {
+    const uint64_t e = stk[--sp];
+    if (__uint_as_float((uint32_t)(e >> 32)) > best) continue;
+    const int32_t cur = (int32_t)(uint32_t)e;
+    if (cur >= 0) {
+      Cand c[4];
+      int nc;
+      open_wide<4>(X.nodes2, X.R, X.leaf_size, cur, c, nc);
+      uint32_t key[4];
+      int32_t ref[4];
+      int nh = 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        key[k] = ~0u;
+        ref[k] = 0;
+        if (k < nc) {
+          const float t0 = slab_exact(c[k].lo, c[k].hi, o, inv, best);
+          if (t0 == t0) {
+            key[k] = (__float_as_uint(t0) & 0x7FFFFFFCu) | (uint32_t)k;
+            ++nh;
+          }
+          ref[k] = c[k].ref < 0 || c[k].count <= X.leaf_size ? ~((c[k].first << 3) | (c[k].count - 1)) : c[k].ref;
+        }
+      }
+      sort_keys<4>(key);
+      if (sp + nh > kRetryStack) {
+        atomicOr(err, kErrStack);
+        return h;
+      }
+#pragma unroll
+      for (int k = 3; k >= 0; --k)
+        if (k < nh) stk[sp++] = key_entry<4>(key[k], ref);
+    } else {
+      const int32_t enc = ~cur;
+      const int64_t first = (int64_t)((uint32_t)enc >> 3);
+      const int count = (enc & 7) + 1;
+      for (int j = 0; j < count; ++j) {
+        if (ANY) {
+          if (test_tri_any(X.tris, first + j, o, d, tmin, tmax)) return ExactHit{(int32_t)(first + j), tmax};
+        } else {
+          test_tri(X.tris, first + j, o, d, tmin, best, have, h.prim);
+        }
+      }
+    }
+  }
+  if (have) h.t = best;
+  return h;
+}
+
+__device__ __forceinline__ void tri_rec_box(const TriRec *__restrict__ tris, int64_t g, float *lo, float *hi) {
+  const float4 *p = (const float4 *)(tris + g);
+  const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+  tri_box(make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z), make_float3(c.x, c.y, c.z), lo, hi);
+}
+
+// A child of a wide node on the walk of first_of_two: as Cand, but with the
+// record that holds its box (4-wide: BVH2 node x 2 + side) for the box.
+struct WalkCand {
+  int32_t ref, first, count, box;
+  float area;
+};
+__device__ __forceinline__ void walk_cands(const Exact4 &X, int32_t node, WalkCand &a, WalkCand &b) {
+  const float4 *np = (const float4 *)(X.nodes2 + node);
+  Node2 nd;
+  nd.a = __ldg(np);
+  nd.b = __ldg(np + 1);
+  nd.c = __ldg(np + 2);
+  nd.d = __ldg((const int4 *)(np + 3));
+  Cand c, e;
+  child_cands(nd, X.R, c, e);
+  a = WalkCand{c.ref, c.first, c.count, 2 * node, half_area(c)};
+  b = WalkCand{e.ref, e.first, e.count, 2 * node + 1, half_area(e)};
+}
+
+// Which of two sorted positions of a scene the exact traversal of a ray tests
+// first: at the wide node where their paths part, the child that is entered
+// first; within a leaf range, the lower one.  Walks down from the root,
+// forming each wide node's children as open_wide does.
+__device__ __noinline__ int32_t first_of_two(const Exact4 &X, const RaySoA &RS, int64_t ray, int32_t p, int32_t q) {
+  int32_t cur = scene_root(X.roots, X.ray_off, X.n_scenes, ray);
+  for (int level = 0; cur >= 0 && level < 4096; ++level) {
+    WalkCand c[4];
+    int nc = 2;
+    walk_cands(X, cur, c[0], c[1]);
+    while (nc < 4) {
+      int best = -1;
+      float ba = -1.0f;
+      int32_t r = 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (k < nc && c[k].ref >= 0 && c[k].count > X.leaf_size && c[k].area > ba) {
+          ba = c[k].area;
+          best = k;
+          r = c[k].ref;
+        }
+      }
+      if (best < 0) break;
+      WalkCand a, b;
+      walk_cands(X, r, a, b);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (k == best) c[k] = a;
+        if (k == nc) c[k] = b;
+      }
+      ++nc;
+    }
+    int32_t next = INT32_MIN, bp = -1, bq = -1, sp = 0, sq = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k < nc) {
+        if ((uint32_t)(p - c[k].first) < (uint32_t)c[k].count) {
+          bp = c[k].box;
+          sp = k;
+          if (c[k].ref >= 0 && c[k].count > X.leaf_size) next = c[k].ref;
+        }
+        if ((uint32_t)(q - c[k].first) < (uint32_t)c[k].count) {
+          bq = c[k].box;
+          sq = k;
+        }
+      }
+    }
+    if (bp < 0 || bq < 0) break;  // a broken tree
+    if (bp != bq) {
+      float3 o, d, inv;
+      float tmin, tmax;
+      load_ray(RS, ray, o, d, inv, tmin, tmax);
+      auto key = [&](int32_t box, int slot) {
+        const Node2 &nd = X.nodes2[box >> 1];
+        const float4 ab = (box & 1) ? nd.b : nd.a;
+        const float lo[3] = {ab.x, ab.z, (box & 1) ? nd.c.z : nd.c.x}, hi[3] = {ab.y, ab.w, (box & 1) ? nd.c.w : nd.c.y};
+        return (__float_as_uint(slab_exact(lo, hi, o, inv, 3.402823466e+38f)) & 0x7FFFFFFCu) | (uint32_t)slot;
+      };
+      return key(bp, sp) < key(bq, sq) ? p : q;
+    }
+    cur = next;
+  }
+  return min(p, q);
+}
+
+// Whether an any-hit candidate counts: its box, or that of its leaf range
+// (enc), passes the exact slab test.  Both only fail where the quantised
+// boxes let a ray in that the exact ones keep out.
+__device__ __forceinline__ bool hit_any_box(const TriRec *__restrict__ tris, int64_t g, int32_t enc, const float3 &o,
+                                            const float3 &inv, float tmax) {
+  float lo[3], hi[3];
+  tri_rec_box(tris, g, lo, hi);
+  float t0 = slab_exact(lo, hi, o, inv, tmax);
+  if (t0 == t0) return true;
+  const int64_t first = (int64_t)((uint32_t)enc >> 3);
+  const int count = (enc & 7) + 1;
+  for (int j = 0; j < count; ++j) {
+    float l[3], h[3];
+    tri_rec_box(tris, first + j, l, h);
+    for (int a = 0; a < 3; ++a) {
+      lo[a] = fminf(lo[a], l[a]);
+      hi[a] = fmaxf(hi[a], h[a]);
+    }
+  }
+  t0 = slab_exact(lo, hi, o, inv, tmax);
+  return t0 == t0;
+}
+
+// Final values of a closest hit: sorted position g, fp32 t.
+__device__ __forceinline__ void finish_hit(const RaySoA &R, const Out &O, const TriRec *__restrict__ tris, int64_t i,
+                                           int32_t g, float best) {
+  const float3 o = make_float3(__ldg(R.ox + i), __ldg(R.oy + i), __ldg(R.oz + i));
+  const float3 d = make_float3(__ldg(R.dx + i), __ldg(R.dy + i), __ldg(R.dz + i));
+  const float4 *p = (const float4 *)(tris + g);
+  const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+  const float3 pa = make_float3(a.x, a.y, a.z), pb = make_float3(b.x, b.y, b.z), pc = make_float3(c.x, c.y, c.z);
+  float u = 0.0f, v = 0.0f;
+  if (!refine_tuv(pa, pb, pc, o, d, best, u, v)) {
+    // N.D == 0: the fp32 barycentrics of the test stand (t stays the test's)
+    float tf;
+    pluecker(pa, pb, pc, o, d, tf, u, v);
+  }
+  O.prim[i] = __float_as_int(a.w);
+  O.t[i] = best;
+  O.u[i] = u;
+  O.v[i] = v;
+}
+
+__device__ __noinline__ ExactHit retrace_closest(const Exact4 &X, const RaySoA &R, int64_t i, uint32_t *err) {
+  return retrace4<false>(X, R, i, err);
+}
+
+// Settles the rays that k_trace4 left open and writes their final values.
+// k_trace_finish4 may start at once: the two work on different rays.
+__global__ void __launch_bounds__(128)
+    k_settle4(const __grid_constant__ RaySoA R, int64_t n, Out O, const __grid_constant__ Exact4 X, Scratch S) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const uint32_t cnt = *S.ovf_count;
+  const bool listed = cnt <= S.ovf_cap;  // else look for the marks
+  const int64_t end = listed ? (int64_t)cnt : n;
+  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < end; j += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = listed ? S.ovf[j] : j;
+    if (O.prim[i] != kListed) continue;
+    const int32_t q = __float_as_int(O.v[i]);
+    ExactHit h{__float_as_int(O.u[i]), O.t[i]};
+    if (q >= 0) h.prim = first_of_two(X, R, i, h.prim, q);
+    else h = retrace_closest(X, R, i, S.err);
+    if (h.prim >= 0) {
+      finish_hit(R, O, X.tris, i, h.prim, h.t);
+    } else {
+      O.prim[i] = -1;
+      O.t[i] = h.t;
+      O.u[i] = 0.0f;
+      O.v[i] = 0.0f;
+    }
+  }
+}
+
+// Hit values of every closest hit of k_trace4, one ray per thread (as
+// k_trace_finish), beside k_settle4, whose latency it hides; the rays of that
+// are left alone: neither kListed nor a finished id has kPending.  Then clears
+// the trace's counters for the next one.
+__global__ void __launch_bounds__(256, 4)
+    k_trace_finish4(RaySoA R, int64_t n, Out O, const TriRec *__restrict__ tris, Scratch S) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t g = O.prim[i];
+    if (g < 0 || !(g & kPending)) continue;
+    finish_hit(R, O, tris, i, g & ~kPending, O.t[i]);
+  }
+  // k_settle4 has ended and its writes are visible: so they are to what
+  // follows this kernel
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *S.work = 0ull;
+    *S.ovf_count = 0u;
+  }
+}
+
+// Any-hit rays whose stack overflowed.
+__global__ void __launch_bounds__(128)
+    k_trace_retry4(const __grid_constant__ RaySoA R, Out O, const __grid_constant__ Exact4 X, Scratch S) {
+  const uint32_t cnt = min((int64_t)*S.ovf_count, S.ovf_cap);
+  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
+    const int64_t i = S.ovf[j];
+    O.occ[i] = retrace4<true>(X, R, i, S.err).prim >= 0 ? 1 : 0;
+  }
+}
+
+// The traversal: while-while with speculative leaf postponing (Aila & Laine,
+// "Understanding the efficiency of ray traversal on GPUs", HPG 2009).  Each
+// lane walks inner nodes; a lane that reaches a leaf parks it (up to two) and
+// keeps walking until at most kLeafWait lanes of the warp still look for
+// their first leaf; then the warp tests the parked leaves together, so node
+// and leaf code run with most lanes active.  One wave of resident blocks at
+// most; warps refill idle lanes from the ray counter once `refill` of them
+// are idle.
+//
+// Stack: entries (key | ref) in shared memory, [slot][thread], over a sentinel
+// that no culling removes and that names the end of the ray.  When it is full
+// its lower half moves to the per-thread local array, and back when the
+// sentinel is reached; a ray that overflows both is traced again with a deep
+// stack (closest: k_settle4, any: k_trace_retry4).
+//
+// A ray is a chain of dependent steps, and a few rays visit ten times as many
+// nodes as the average, so without more the last of them set the time of a
+// launch (of half of it on camera rays of a surface), and the longest that of
+// a small batch.  Once the counter is exhausted, idle lanes of a warp
+// therefore help the others: each takes the lowest stack entry (the farthest,
+// and mostly the largest, subtree) of a lane that has one, with a copy of its
+// ray, and walks it as a ray of its own.  The lane that took the ray from the
+// counter leads: it collects its helpers' hits under the rules for a second
+// candidate of the same ray, and retires once they are done.  Lanes of one
+// ray share the closest t at every turn of the outer loop.
+constexpr int kLeafWait = 8;
+// Slots, the sentinel's included.  With the ray indices 32 KB per 256-thread
+// block: four blocks leave 124 KB of an SM for L1, a byte more only 92.
+constexpr int kStackSlots = 15;
+constexpr int kStackMove = 8;    // entries moved at a time
+constexpr int kStackLocal = 64;
+constexpr int kHelpAfter = 32;  // turns after the counter's end before lanes help
+constexpr int kHelpTurns = 8;
+
+__device__ __forceinline__ void stack_store(uint32_t at, uint32_t key, int32_t ref) {
+  asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at), "r"(key), "r"(ref) : "memory");
+}
+__device__ __forceinline__ void stack_load(uint32_t at, uint32_t &key, int32_t &ref) {
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(key), "=r"(ref) : "r"(at) : "memory");
+}
+
+template <bool ANY>
+__global__ void __launch_bounds__(256, 4)
+    k_trace4(const NodeQ *__restrict__ nodes, const TriRec *__restrict__ tris, const int32_t *__restrict__ roots,
+             const int64_t *__restrict__ ray_off, int n_scenes, RaySoA R, int64_t n, Out O, Scratch S, int refill,
+             int lanes, float one) {
+  // What a lane does next: a node (0 .. kPop - 1), a leaf (< 0), a pop, nothing
+  // more for its ray, or nothing.  No parked leaf: 0.
+  constexpr int32_t kPop = 0x7FFFFFFD, kDone = 0x7FFFFFFE, kIdle = 0x7FFFFFFF;
+  constexpr uint32_t kSlot = 256 * sizeof(uint64_t);  // bytes between a thread's slots
+  constexpr unsigned kAll = 0xFFFFFFFFu;
+  constexpr int64_t kOverflow = INT64_MIN;  // on a ray's index: its stack overflowed
+  // A second candidate near the closest hit: none, one within kNear but not
+  // equal, two or more equal, or (>= 0) the one that is equal.
+  constexpr int32_t kNone = -1, kSome = -2, kMany = -3;
+  __shared__ uint64_t s_stk[kStackSlots][256];
+  __shared__ int64_t s_ray[256];
+  const uint32_t s_base = (uint32_t)__cvta_generic_to_shared(&s_stk[0][0]);
+  const uint32_t bottom = s_base + threadIdx.x * (uint32_t)sizeof(uint64_t);
+  stack_store(bottom, 0xFF800000u, kDone);  // the sentinel: -inf
+  uint64_t stk[kStackLocal];
+  float3 o = make_float3(0.f, 0.f, 0.f), d = o, inv = o;
+  float tmin = 0.f;
+  float best = 0.f;  // the ray's limit: tmax, and the closest t so far
+  int32_t prim = -1, tie = kNone, cur = kIdle, leaf = 0, leaf2 = 0;
+  uint32_t low = bottom;          // the lane's sentinel: entries given away lie below it
+  uint32_t top = bottom + kSlot;  // the next free slot
+  int moved = 0;                  // entries in the local array
+  int scene = -1;
+  int lead = 0;                   // the lane that leads this ray | its helpers at work << 8
+  int phase = 0;                  // 0 at the start; 1 the counter has rays; then 2 + turns since it has none
+  // The first `lanes` rays of every warp by its index, the others from the
+  // counter, which starts behind them.
+  const int64_t taken = (int64_t)gridDim.x * (blockDim.x >> 5) * lanes;
+
+  while (true) {
+    const int lane = threadIdx.x & 31;
+    // Lanes that help: shared limits, finished helpers.
+    if (phase > kHelpAfter && __any_sync(kAll, cur != kIdle && (lead & 0xFF) != lane)) {
+      const unsigned group = __match_any_sync(kAll, cur != kIdle ? lead & 0xFF : 32 + lane);
+      if (ANY) {
+        if (__reduce_or_sync(group, prim >= 0 ? 1u : 0u) && cur != kIdle) {
+          cur = kDone;
+          leaf = leaf2 = 0;
+        }
+      } else {
+        const float m = __uint_as_float(__reduce_min_sync(group, __float_as_uint(best)));
+        if (m < best) {
+          tie = prim >= 0 && best <= m * (1.0f + kNear) ? kSome : kNone;
+          prim = -1;
+          best = m;
+        }
+      }
+      for (unsigned done = __ballot_sync(kAll, cur == kDone && leaf == 0 && (lead & 0xFF) != lane); done != 0u;
+           done &= done - 1u) {
+        const int h = __ffs(done) - 1;
+        const int to = __shfl_sync(kAll, lead & 0xFF, h);
+        const float h_best = __shfl_sync(kAll, best, h);
+        const int32_t h_prim = __shfl_sync(kAll, prim, h), h_tie = __shfl_sync(kAll, tie, h);
+        if (lane == h) cur = kIdle;
+        if (lane == to) {
+          lead -= 1 << 8;
+          if (ANY) {
+            prim = max(prim, h_prim);
+          } else if (h_prim < 0) {
+            if (h_tie != kNone && tie == kNone) tie = kSome;
+          } else if (h_best < best || (prim < 0 && h_best == best)) {
+            tie = h_tie != kNone ? h_tie : best <= h_best * (1.0f + kNear) ? kSome : kNone;
+            best = h_best;
+            prim = h_prim;
+          } else if (h_best == best) {
+            tie = tie < 0 && tie != kMany && h_tie < 0 && h_tie != kMany ? h_prim : kMany;
+          } else if (h_best <= best * (1.0f + kNear) && tie == kNone) {
+            tie = kSome;
+          }
+        }
+      }
+    }
+    // Retire finished rays.
+    if (cur == kDone && leaf == 0 && lead == lane) {
+      const int64_t ray = s_ray[threadIdx.x];
+      if (ANY) {
+        if (ray < 0 && prim < 0) record_overflow(S, ray - kOverflow);
+        else O.occ[ray < 0 ? ray - kOverflow : ray] = prim >= 0 ? 1 : 0;
+      } else {
+        const int64_t at = ray < 0 ? ray - kOverflow : ray;
+        bool listed = ray < 0;
+        int32_t other = -1;
+        if (prim >= 0 && !listed) {
+          // the winner's box, and that of a second triangle at the same t
+          const float3 ie = make_float3(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z));
+          float lo[3], hi[3];
+          tri_rec_box(tris, prim, lo, hi);
+          float t0 = slab_exact(lo, hi, o, ie, 3.402823466e+38f);
+          listed = !(t0 == t0) || (tie == kSome ? t0 > best : tie != kNone);
+          if (tie >= 0 && t0 <= best) {
+            tri_rec_box(tris, tie, lo, hi);
+            t0 = slab_exact(lo, hi, o, ie, 3.402823466e+38f);
+            if (t0 <= best) other = tie;
+          }
+        }
+        O.t[at] = best;  // of a miss, tmax
+        O.prim[at] = listed ? kListed : prim >= 0 ? prim | kPending : -1;
+        if (listed) {
+          O.u[at] = __int_as_float(prim);
+          O.v[at] = __int_as_float(other);
+          const uint32_t k = atomicAdd(S.ovf_count, 1u);
+          if (k < S.ovf_cap) S.ovf[k] = at;  // past the end the mark is looked for
+        } else if (prim < 0) {
+          O.u[at] = 0.0f;
+          O.v[at] = 0.0f;
+        }
+      }
+      cur = kIdle;
+    }
+    // Take new rays.
+    const unsigned idle = __ballot_sync(kAll, cur == kIdle);
+    const int nidle = __popc(idle);
+    if (phase < 2 && nidle >= refill) {
+      int64_t my;
+      if (phase == 0) {
+        my = lane < lanes ? ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * lanes + lane : n;
+        phase = taken >= n ? 2 : 1;
+      } else {
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(S.work, (unsigned long long)nidle);
+        base = __shfl_sync(kAll, base, 0) + (unsigned long long)taken;
+        my = (int64_t)base + __popc(idle & ((1u << lane) - 1u));
+        if ((int64_t)base + nidle >= n) phase = 2;
+      }
+      if (cur == kIdle && my < n) {
+        s_ray[threadIdx.x] = my;
+        load_ray(R, my, o, d, inv, tmin, best);
+        inv = make_float3(inv_q(inv.x), inv_q(inv.y), inv_q(inv.z));
+        tie = kNone;
+        prim = -1;
+        cur = scene_root_walk(roots, ray_off, n_scenes, my, scene);
+        if (cur == kEmptyChild) cur = kDone;
+        low = bottom;
+        top = bottom + kSlot;
+        moved = 0;
+        lead = lane;
+      }
+    } else if (phase >= 2 && idle != 0u) {
+      if (idle == kAll) break;
+      // Help: the r-th idle lane takes the lowest entry of the r-th lane that
+      // has one to give.
+      const unsigned donors =
+          phase > kHelpAfter ? __ballot_sync(kAll, cur < kDone && moved == 0 && top - low > kSlot) : 0u;
+      if (donors != 0u) {
+        const unsigned lt = (1u << lane) - 1u;
+        const int k = min(nidle, __popc(donors));
+        const bool give = (donors >> lane & 1u) && __popc(donors & lt) < k;
+        const bool take = cur == kIdle && __popc(idle & lt) < k;
+        int from = lane;
+        if (take) {  // the donors' r-th bit
+          int r = __popc(idle & lt);
+          from = 0;
+#pragma unroll
+          for (int w = 16; w >= 1; w >>= 1) {
+            const int c = __popc(donors >> from & ((1u << w) - 1u));
+            if (r >= c) {
+              r -= c;
+              from += w;
+            }
+          }
+        }
+        o.x = __shfl_sync(kAll, o.x, from);
+        o.y = __shfl_sync(kAll, o.y, from);
+        o.z = __shfl_sync(kAll, o.z, from);
+        d.x = __shfl_sync(kAll, d.x, from);
+        d.y = __shfl_sync(kAll, d.y, from);
+        d.z = __shfl_sync(kAll, d.z, from);
+        inv.x = __shfl_sync(kAll, inv.x, from);
+        inv.y = __shfl_sync(kAll, inv.y, from);
+        inv.z = __shfl_sync(kAll, inv.z, from);
+        tmin = __shfl_sync(kAll, tmin, from);
+        best = __shfl_sync(kAll, best, from);
+        const int to = __shfl_sync(kAll, lead & 0xFF, from);
+        const uint32_t at = __shfl_sync(kAll, low, from) + kSlot;
+        if (take) {
+          uint32_t key;
+          stack_load(at, key, cur);
+          tie = kNone;
+          prim = -1;
+          low = bottom;
+          top = bottom + kSlot;
+          moved = 0;
+          lead = to;
+        }
+        __syncwarp();  // the entries are read before their slots become sentinels
+        for (unsigned m = __ballot_sync(kAll, take); m != 0u; m &= m - 1u)
+          if (__shfl_sync(kAll, to, __ffs(m) - 1) == lane) lead += 1 << 8;
+        if (give) {
+          low += kSlot;  // the slot given away becomes the sentinel
+          stack_store(low, 0xFF800000u, kDone);
+        }
+      }
+    }
+
+    // Inner nodes, parking the first two leaves found.  Ends once at most
+    // kLeafWait lanes are still looking for their first leaf (waiting for the
+    // last few cost more idle node iterations than the leaf tests they would
+    // have joined), unless there is neither a leaf to test nor a ray to take;
+    // with idle lanes that can only help, after kHelpTurns at the latest.
+    unsigned seeking;
+    int turns = 0;
+    do {
+      if (cur == kPop) {
+        uint32_t key;
+        do {
+          top -= kSlot;
+          stack_load(top, key, cur);
+        } while (__uint_as_float(key & ~0xFFu) > best);
+        if (cur == kDone && moved > 0) {
+          moved -= kStackMove;
+          for (int k = 0; k < kStackMove; ++k) {
+            top += kSlot;
+            stack_store(top, (uint32_t)(stk[moved + k] >> 32), (int32_t)(uint32_t)stk[moved + k]);
+          }
+          top += kSlot;
+          cur = kPop;
+        }
+      }
+      if ((uint32_t)cur < (uint32_t)kPop) {
+        uint32_t key[4];
+        int32_t base;
+        visit_q(nodes + cur, o, inv, best, key, base);
+        sort_keys<4>(key);
+        const int32_t from = cur;
+        cur = (int32_t)key[0] >= 0 ? child_ref(key[0], from, base) : kPop;
+        if ((int32_t)key[1] >= 0) {
+          // the other children, the farthest first
+          if ((int32_t)key[2] >= 0) {
+            if ((int32_t)key[3] >= 0) {
+              stack_store(top, key[3], child_ref(key[3], from, base));
+              top += kSlot;
+            }
+            stack_store(top, key[2], child_ref(key[2], from, base));
+            top += kSlot;
+          }
+          stack_store(top, key[1], child_ref(key[1], from, base));
+          top += kSlot;
+          if (top >= s_base + (kStackSlots - 2) * kSlot) {
+            // Fewer than three slots are left: reclaim those given away, and if
+            // that was not enough move the lower entries to the local array.
+            uint32_t at, key_m;
+            int32_t ref_m;
+            if (low != bottom) {
+              const uint32_t shift = low - bottom;
+              for (at = low; at < top; at += kSlot) {
+                stack_load(at, key_m, ref_m);
+                stack_store(at - shift, key_m, ref_m);
+              }
+              top -= shift;
+              low = bottom;
+            }
+            if (top >= s_base + (kStackSlots - 2) * kSlot) {
+              if (moved + kStackMove > kStackLocal) {
+                int64_t *mark = &s_ray[(threadIdx.x & ~31u) + (lead & 0xFF)];
+                if (*mark >= 0) *mark += kOverflow;
+                cur = kDone;
+                leaf = leaf2 = 0;
+              } else {
+                at = bottom + kSlot;
+                for (int k = 0; k < kStackMove; ++k, at += kSlot) {
+                  stack_load(at, key_m, ref_m);
+                  stk[moved + k] = (uint64_t)key_m << 32 | (uint32_t)ref_m;
+                }
+                for (; at < top; at += kSlot) {
+                  stack_load(at, key_m, ref_m);
+                  stack_store(at - kStackMove * kSlot, key_m, ref_m);
+                }
+                top -= kStackMove * kSlot;
+                moved += kStackMove;
+              }
+            }
+          }
+        }
+      }
+      if (cur < 0 && leaf2 == 0) {
+        leaf2 = leaf;
+        leaf = cur;
+        cur = kPop;
+      }
+      ++turns;
+      seeking = __ballot_sync(kAll, leaf == 0 && cur < kDone);
+    } while (__popc(seeking) > kLeafWait
+                 ? !(phase >= 2 && idle != 0u && turns >= kHelpTurns)
+                 : seeking != 0u && phase >= 2 && turns < kHelpTurns && !__any_sync(kAll, leaf != 0));
+    if (phase >= 2 && phase <= kHelpAfter) phase += turns;
+
+    // Test the (up to two) parked leaves together.
+    if (leaf != 0) {
+      const uint32_t s1 = (uint32_t)leaf & 0x7FFFFFFFu, s2 = (uint32_t)leaf2 & 0x7FFFFFFFu;
+      const int32_t e1 = ~__ldg(nodes[s1 >> 2].leaf + (s1 & 3u));
+      const int32_t e2 = leaf2 == 0 ? -1 : ~__ldg(nodes[s2 >> 2].leaf + (s2 & 3u));
+      // an unused slot holds no range
+      const int n1 = e1 < 0 ? 0 : (e1 & 7) + 1;
+      const int total = e2 < 0 ? n1 : n1 + (e2 & 7) + 1;
+      const int32_t f1 = (int32_t)((uint32_t)e1 >> 3), f2 = (int32_t)((uint32_t)e2 >> 3) - n1;
+      for (int j = 0; j < total; ++j) {
+        const int32_t g = (j < n1 ? f1 : f2) + j;
+        const float4 *p = (const float4 *)(tris + g);
+        const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+        float t;
+        if (!pluecker_t2(make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z), make_float3(c.x, c.y, c.z), o, d,
+                         pack2(one, one), t))
+          continue;
+        if (ANY) {
+          if (t >= tmin && !(t > best)) {
+            // a one-triangle scene is tested without a box
+            const float3 ie = make_float3(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z));
+            if (hit_any_box(tris, g, j < n1 ? e1 : e2, o, ie, best) || __ldg(&nodes[s1 >> 2].step) == kLoneStep) {
+              prim = g;
+              cur = kDone;
+              break;
+            }
+          }
+        } else if (t >= tmin && t <= best * (1.0f + kNear)) {
+          if (t < best || (prim < 0 && t == best)) {
+            tie = best <= t * (1.0f + kNear) ? kSome : kNone;
+            best = t;
+            prim = g;
+          } else if (t == best) {
+            tie = tie == kNone || tie == kSome ? g : kMany;
+          } else if (tie == kNone) {
+            tie = kSome;
+          }
+        }
+      }
+      leaf = 0;
+      leaf2 = 0;
+    }
+  }
+}
+
 template <int W, bool ANY, bool MT = false>
 __global__ void __launch_bounds__(128)
-    k_trace_retry(const NodeW<(W == 2 ? 4 : W)> *__restrict__ nodes, const Node2 *__restrict__ nodes2,
-                  const TriRec *__restrict__ tris,
-                  const int32_t *__restrict__ roots, const int64_t *__restrict__ ray_off, int n_scenes, RaySoA R, Out O,
-                  Scratch S) {
+    k_trace_retry(const NodeW<8> *__restrict__ wide, const Node2 *__restrict__ nodes2,
+                  const TriRec *__restrict__ tris, const int32_t *__restrict__ roots,
+                  const int64_t *__restrict__ ray_off, int n_scenes, RaySoA R, Out O, Scratch S) {
   const uint32_t cnt = min((int64_t)*S.ovf_count, S.ovf_cap);
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
     const int64_t i = S.ovf[j];
@@ -503,24 +1342,25 @@ __global__ void __launch_bounds__(128)
     float tmin, tmax;
     load_ray(R, i, o, d, inv, tmin, tmax);
     const int32_t root = scene_root(roots, ray_off, n_scenes, i);
-    if (W == 2) {
-      bool have;
-      int32_t prim;
-      float best;
-      if (!trace_bvh2<ANY, kRetryStack, MT>(nodes2, tris, root, o, d, inv, tmin, tmax, have, prim, best)) {
-        atomicOr(S.err, kErrStack);
-        continue;
-      }
-      write_result(O, i, ANY, have, prim, best, tmax);
+    bool have;
+    int32_t prim;
+    float best;
+    bool done;
+    if constexpr (W == 2) {
+      done = trace_bvh2<ANY, kRetryStack, MT>(nodes2, tris, root, o, d, inv, tmin, tmax, have, prim, best);
     } else {
-      Tracer<(W == 2 ? 4 : W), ANY, kRetryStack> tr;
+      Tracer<W, ANY, kRetryStack> tr;
       tr.o = o; tr.d = d; tr.inv = inv; tr.tmin = tmin; tr.tmax = tmax;
       tr.start(root);
-      while (!tr.step(nodes, tris)) {
+      while (!tr.step(wide, tris)) {
       }
-      if (tr.overflow) atomicOr(S.err, kErrStack);
-      else write_result(O, i, ANY, tr.have, tr.prim, tr.best, tr.tmax);
+      done = !tr.overflow;
+      have = tr.have;
+      prim = tr.prim;
+      best = tr.best;
     }
+    if (!done) atomicOr(S.err, kErrStack);
+    else write_result(O, i, ANY, have, prim, best, tmax);
   }
 }
 
@@ -610,14 +1450,14 @@ static int ensure_trace_scratch(flg_ctx ctx) {
   ctx->ovf_cap = 1 << 20;
   // Two sets (index 0: default stream, 1: staging second stream).
   FLG_CUDA(ctx, cudaMalloc((void **)&ctx->d_ovf, sizeof(int64_t) * ctx->ovf_cap * 2));
-  FLG_CUDA(ctx, cudaMalloc((void **)&ctx->d_ovf_count, sizeof(uint32_t) * 2));
-  FLG_CUDA(ctx, cudaMalloc((void **)&ctx->d_work, sizeof(unsigned long long) * 2));
+  FLG_CUDA(ctx, cudaMalloc((void **)&ctx->d_trace_ctr, sizeof(unsigned long long) * 8));
+  FLG_CUDA(ctx, cudaMemsetAsync(ctx->d_trace_ctr, 0, sizeof(unsigned long long) * 8, ctx->stream));
   return FLG_OK;
 }
 
 static Scratch scratch_for(flg_ctx ctx, int set) {
-  return Scratch{ctx->d_ovf + set * ctx->ovf_cap, ctx->d_ovf_count + set, ctx->ovf_cap, ctx->d_work + set,
-                 ctx->d_err};
+  unsigned long long *c = ctx->d_trace_ctr + 2 * set;  // [0] rays taken, [1] entries of the list
+  return Scratch{ctx->d_ovf + (set & 1) * ctx->ovf_cap, (uint32_t *)(c + 1), ctx->ovf_cap, c, ctx->d_err};
 }
 
 static int check_rays(flg_ctx ctx, const flg_rays *r, int64_t n) {
@@ -641,7 +1481,7 @@ static int check_rays(flg_ctx ctx, const flg_rays *r, int64_t n) {
 // kLeafWait = 4 give 21 % more rays/s.  Finished lanes are refilled from the
 // global ray counter once `refill` of them are idle.
 // ----------------------------------------------------------------------------
-constexpr int kLeafWait = 4;
+constexpr int kLeafWaitWW = 4;
 // Shared-memory stack entries per lane (a power of two; 32 KB per 256-thread
 // CTA).  16 measured 3.7 % faster than a local-memory stack, 8 gave 2 %.
 constexpr int kStackTop = 16;
@@ -762,7 +1602,7 @@ __global__ void __launch_bounds__(256, 4)
       // their first leaf: waiting for the last few cost more idle node
       // iterations than the leaf tests they would have joined.
       const bool ready = !active || leaf != kNone || cur == kNone || (cur < 0 && leaf != kNone);
-      if (__popc(__ballot_sync(0xFFFFFFFFu, !ready)) <= kLeafWait) break;
+      if (__popc(__ballot_sync(0xFFFFFFFFu, !ready)) <= kLeafWaitWW) break;
     }
 
     // Test the (up to two) parked leaves together.
@@ -788,6 +1628,57 @@ __global__ void __launch_bounds__(256, 4)
     leaf = kNone;
     leaf2 = kNone;
   }
+}
+
+// One trace over the 4-wide layout: the traversal, then the hit values (any
+// hit: the overflow list).
+//
+// A warp runs through the paths of its rays in turn, so the fewer it has the
+// sooner they end; but past two warps per scheduler thinner warps only add
+// instructions.  A batch too small to give eight full warps to every SM is
+// spread over that many (4,096 rays on 20,001 triangles: 72 us, against 92 us
+// in full warps and 96 us in one-ray warps), and its blocks are made smaller
+// until they cover the SMs.  Refills at 8 idle lanes at most: with the
+// quantised nodes 8 beat 16 and 24 (24.0 against 25.6 and 29.6 ms on 31.6 M
+// scattered rays).
+template <bool ANY>
+static int launch4(flg_ctx ctx, cudaStream_t st, flg_bvh b, const RaySoA &R, int64_t n, const Out &O,
+                   const Scratch &S, const int64_t *ray_off, int n_scenes, const flg_trace_opts &op) {
+  const int lanes = (int)std::min<int64_t>(32, ceil_div(n, (int64_t)ctx->num_sms * 8));
+  int threads = op.block_threads, per_sm = 0;
+  while (threads > 32 && ceil_div(n, (int64_t)lanes * (threads / 32)) < ctx->num_sms) threads >>= 1;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace4<ANY>, threads, 0);
+  if (per_sm < 1) per_sm = 1;
+  const int64_t g = std::min<int64_t>((int64_t)per_sm * ctx->num_sms, ceil_div(n, (int64_t)lanes * (threads / 32)));
+  const int refill = std::max(1, std::min(8, op.refill_lanes));
+  const Exact4 X{b->d_nodes2, b->d_tris, Ranges{b->d_rfirst, b->d_rcount}, b->leaf_size, b->d_root, ray_off, n_scenes};
+  if (!ANY) ctx->trace4_open = true;  // until the kernel that clears the counters is launched
+  k_trace4<ANY><<<(unsigned)g, threads, 0, st>>>((const NodeQ *)b->d_wide, b->d_tris, b->d_wide_root, ray_off, n_scenes,
+                                                 R, n, O, S, refill, lanes, 1.0f);
+  FLG_LAUNCH_CHECK(ctx, "k_trace4");
+  stage_mark(ctx, st, "trace");
+  if (ANY) {
+    k_trace_retry4<<<(unsigned)ctx->num_sms, 128, 0, st>>>(R, O, X, S);
+    FLG_LAUNCH_CHECK(ctx, "k_trace_retry4");
+    stage_mark(ctx, st, "trace_retry");
+  } else {
+    k_settle4<<<grid_for(n, 128, ctx->num_sms), 128, 0, st>>>(R, n, O, X, S);
+    FLG_LAUNCH_CHECK(ctx, "k_settle4");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid_for(n, 256, (int64_t)ctx->num_sms * 16));
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    FLG_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_trace_finish4, R, n, O, (const TriRec *)b->d_tris, S));
+    FLG_LAUNCH_CHECK(ctx, "k_trace_finish4");
+    ctx->trace4_open = false;
+    stage_mark(ctx, st, "trace_finish");
+  }
+  return FLG_OK;
 }
 
 template <int W, bool ANY>
@@ -923,11 +1814,14 @@ int trace_enqueue(flg_ctx ctx, cudaStream_t st, int set, flg_bvh b, const flg_ra
   }
   Out O{hits ? hits->prim : nullptr, hits ? hits->t : nullptr, hits ? hits->u : nullptr,
         hits ? hits->v : nullptr, occ};
-  Scratch S = scratch_for(ctx, set);
-  stage_mark(ctx, st, "start");
-  FLG_CUDA(ctx, cudaMemsetAsync(S.ovf_count, 0, sizeof(uint32_t), st));
-  FLG_CUDA(ctx, cudaMemsetAsync(S.work, 0, sizeof(unsigned long long), st));
   const bool any = occ != nullptr;
+  // Closest hits over the 4-wide layout end with their counters cleared, so
+  // they keep a pair of their own (sets 2 and 3).
+  const bool clears = b->width == 4 && !any && op.tri_test == 0;
+  Scratch S = scratch_for(ctx, clears ? set + 2 : set);
+  stage_mark(ctx, st, "start");
+  if (!clears || ctx->trace4_open)
+    FLG_CUDA(ctx, cudaMemsetAsync(S.work, 0, 2 * sizeof(unsigned long long), st));  // both counters
   if (op.tri_test == 1) {
     // The live renderer's Moller-Trumbore test: one ray per thread over the
     // BVH2 layout (kept by every handle), overflow retried with a deep stack.
@@ -958,8 +1852,8 @@ int trace_enqueue(flg_ctx ctx, cudaStream_t st, int set, flg_bvh b, const flg_ra
     else
       k_trace_bvh2<false><<<g, 256, 0, st>>>(b->d_nodes2, b->d_tris, b->d_root, ray_off_dev, n_scenes, R, n, O, S);
   } else if (b->width == 4) {
-    if (any) launch_wide<4, true>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op);
-    else launch_wide<4, false>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op);
+    return any ? launch4<true>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op)
+               : launch4<false>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op);
   } else {
     if (any) launch_wide<8, true>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op);
     else launch_wide<8, false>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op);
@@ -967,23 +1861,16 @@ int trace_enqueue(flg_ctx ctx, cudaStream_t st, int set, flg_bvh b, const flg_ra
   FLG_LAUNCH_CHECK(ctx, "trace kernel");
   stage_mark(ctx, st, "trace");
   const unsigned rg = (unsigned)ctx->num_sms;
-  const void *wide = b->d_wide;
+  const NodeW<8> *wide = (const NodeW<8> *)b->d_wide;
   const int32_t *roots = b->width == 2 ? b->d_root : b->d_wide_root;
-#define FLG_RETRY(WW)                                                                                       \
-  if (any)                                                                                                  \
-    k_trace_retry<WW, true><<<rg, 128, 0, st>>>((const NodeW<(WW == 2 ? 4 : WW)> *)wide, b->d_nodes2,       \
-                                                b->d_tris, roots, ray_off_dev, n_scenes, R, O, S);          \
-  else                                                                                                      \
-    k_trace_retry<WW, false><<<rg, 128, 0, st>>>((const NodeW<(WW == 2 ? 4 : WW)> *)wide, b->d_nodes2,      \
-                                                 b->d_tris, roots, ray_off_dev, n_scenes, R, O, S);
-  if (b->width == 2) {
-    FLG_RETRY(2)
-  } else if (b->width == 4) {
-    FLG_RETRY(4)
-  } else {
-    FLG_RETRY(8)
-  }
-#undef FLG_RETRY
+  if (b->width == 2 && any)
+    k_trace_retry<2, true><<<rg, 128, 0, st>>>(wide, b->d_nodes2, b->d_tris, roots, ray_off_dev, n_scenes, R, O, S);
+  else if (b->width == 2)
+    k_trace_retry<2, false><<<rg, 128, 0, st>>>(wide, b->d_nodes2, b->d_tris, roots, ray_off_dev, n_scenes, R, O, S);
+  else if (any)
+    k_trace_retry<8, true><<<rg, 128, 0, st>>>(wide, b->d_nodes2, b->d_tris, roots, ray_off_dev, n_scenes, R, O, S);
+  else
+    k_trace_retry<8, false><<<rg, 128, 0, st>>>(wide, b->d_nodes2, b->d_tris, roots, ray_off_dev, n_scenes, R, O, S);
   FLG_LAUNCH_CHECK(ctx, "trace retry kernel");
   stage_mark(ctx, st, "trace_retry");
   return finish_enqueue(ctx, st, R, n, O, b, any);
@@ -1402,11 +2289,10 @@ FLG_API int flg_trace_closest_noalloc(flg_ctx ctx, flg_bvh bvh, const flg_rays *
     FLG_LAUNCH_CHECK(ctx, "k_trace_bvh2");
     k_trace_retry<2, false><<<rg, 128, 0, st>>>(nullptr, bvh->d_nodes2, bvh->d_tris, bvh->d_root, nullptr, 1, R, O, S);
   } else if (bvh->width == 4) {
-    k_trace_wide<4, false, 64><<<g, 256, 0, st>>>((const NodeW<4> *)bvh->d_wide, bvh->d_tris, bvh->d_wide_root,
-                                                  nullptr, 1, R, n, O, S);
-    FLG_LAUNCH_CHECK(ctx, "k_trace_wide");
-    k_trace_retry<4, false><<<rg, 128, 0, st>>>((const NodeW<4> *)bvh->d_wide, bvh->d_nodes2, bvh->d_tris,
-                                                bvh->d_wide_root, nullptr, 1, R, O, S);
+    flg_trace_opts op{};
+    op.block_threads = 256;
+    op.refill_lanes = 16;
+    return launch4<false>(ctx, st, bvh, R, n, O, S, nullptr, 1, op);
   } else {
     k_trace_wide<8, false, 64><<<g, 256, 0, st>>>((const NodeW<8> *)bvh->d_wide, bvh->d_tris, bvh->d_wide_root,
                                                   nullptr, 1, R, n, O, S);

@@ -110,12 +110,14 @@ typedef struct flg_build_opts {
 enum { FLG_BUILDER_LBVH = 0, FLG_BUILDER_PLOC = 1, FLG_BUILDER_SAH = 2, FLG_BUILDER_TREELET = 3 };
 
 typedef struct flg_trace_opts {
-  int32_t stack_depth;    /* 32 or 64 (0 = 64); overflowing rays are retried deeper */
+  int32_t stack_depth;    /* 8-wide layout: 32 or 64 (0 = 64); overflowing rays are retried deeper */
   int32_t block_threads;  /* threads per block (0 = 256) */
-  int32_t persistent;     /* 0: one ray per thread; 1: persistent work-stealing kernel;
-                             2: persistent while-while kernel with speculative leaf
-                             postponing (wide layouts) */
-  int32_t refill_lanes;   /* persistent: refill a warp once this many lanes idle (0 = 16) */
+  int32_t persistent;     /* 8-wide layout: 0: one ray per thread; 1: persistent work-stealing
+                             kernel; 2: persistent while-while kernel with speculative leaf
+                             postponing.  The 4-wide layout always takes the persistent
+                             while-while kernel, which is the fastest of the three on it */
+  int32_t refill_lanes;   /* persistent: refill a warp once this many lanes idle (0 = 16; the
+                             4-wide layout's kernel refills at 8 at the latest) */
   int32_t ray_sort;       /* 0: none; 1: sort rays by direction octant and origin cell */
   int32_t tri_test;       /* 0: watertight Pluecker (intersector.hpp:63-101, the experimental
                              path); 1: the live renderer's Moller-Trumbore Triangle::intersect

@@ -1,0 +1,143 @@
+"""The 4-wide quantised layout where its boxes, its stack or its tie rules
+could go wrong: the hits must still be those of the exact boxes (oracle DEV
+arithmetic: ids equal but for exact ties, t/u/v bit-equal where they agree;
+occlusion bits equal)."""
+import numpy as np
+import pytest
+
+import geometry as G
+import gpu_util as U
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(kind):
+    rng = np.random.default_rng(404)
+    pos = G.random_soup(3000, rng, half=0.05).reshape(-1, 3, 3)
+    rays = G.sphere_rays(20000, rng)
+    if kind == "duplicates":          # every hit is an exact tie, within and across leaf ranges
+        pos = np.concatenate([pos, pos, pos[::-1]])
+    elif kind == "planes":            # overlapping axis-aligned triangles: flat boxes, equal and nearly equal t
+        pos[:, :, 2] = np.float32(0.25) * np.round(4 * pos[:, :1, 2])
+    elif kind == "far":               # coordinates large against the boxes
+        pos += np.float32(4096.0)
+        rays[0:3] += np.float32(4096.0)
+    elif kind == "axis":              # zero direction components
+        a = rng.integers(0, 3, rays.shape[1])
+        rays[3:6] = 0.0
+        rays[3 + a, np.arange(rays.shape[1])] = np.where(rng.random(rays.shape[1]) < 0.5, 1.0, -1.0)
+        rays[0:3] = rng.random((3, rays.shape[1])) * 1.2 - 0.1
+    elif kind == "tiny":
+        pos *= np.float32(2.0 ** -24)
+        rays[0:3] *= np.float32(2.0 ** -24)
+        rays[6] = 0.0
+    elif kind == "huge":              # the distances' numerators still fit fp32
+        pos *= np.float32(2.0 ** 30)
+        rays[0:3] *= np.float32(2.0 ** 30)
+    elif kind == "nonfinite":         # a box without bounds above every other one
+        pos[7, 1] = (np.inf, 0.5, -np.inf)
+        pos[8] = np.nan
+    elif kind == "slivers":           # the stack leaves shared memory
+        pos, rays = G.sliver_comb(64, rng)
+    return np.ascontiguousarray(pos.reshape(-1, 3).astype(np.float32)), rays.astype(np.float32)
+
+
+KINDS = ["duplicates", "planes", "far", "axis", "tiny", "huge", "nonfinite", "slivers"]
+
+
+@pytest.mark.parametrize("leaf", [1, 3, 8])
+@pytest.mark.parametrize("kind", KINDS)
+def test_quantised_boxes_change_no_hit(ctx, oracle, kind, leaf):
+    pos, r8 = _scene(kind)
+    b, _ = U.gpu_build(ctx, pos, width=4, leaf=leaf)
+    exact, _ = U.gpu_build(ctx, pos, width=8, leaf=leaf)  # fp32 boxes
+    rd, _ = U.rays_dev(r8)
+    hg, he = U.host(b.intersect(rd)), U.host(exact.intersect(rd))
+    occ, occ_e = b.intersectP(rd).cpu().numpy(), exact.intersectP(rd).cpu().numpy()
+    ctx.sync()
+    if kind == "nonfinite":  # the oracle's Morton codes of such a scene are its own
+        tri = pos.reshape(-1, 3, 3)
+        diff = np.nonzero(hg["prim"] != he["prim"])[0]
+        for i in diff:
+            k = [oracle.pluecker(tri[p, 0], tri[p, 1], tri[p, 2], r8[0:3, i], r8[3:6, i], oracle.MODE_DEV)
+                 for p in (hg["prim"][i], he["prim"][i]) if p >= 0]
+            assert len(k) == 2 and k[0][0] and k[1][0] and k[0][1][0] == k[1][1][0], i
+        assert np.array_equal(occ, occ_e)
+        return
+    tree = oracle.build_bvh(pos)
+    bad, ties, ho = U.compare_closest(oracle, pos, None, tree, r8, hg, oracle.MODE_DEV)
+    extra = 0
+    if leaf > 1:  # hits that a leaf range's box lets in and the reference's tighter boxes keep out
+        extra = np.count_nonzero((hg["prim"] >= 0) & (ho["prim"] < 0))
+        assert extra == np.count_nonzero((he["prim"] >= 0) & (ho["prim"] < 0))
+    if kind != "planes":  # there the order of visits decides between nearly equal t
+        assert bad == extra, (bad, ties, extra)
+    same = hg["prim"] == ho["prim"]
+    for k in ("t", "u", "v"):
+        assert np.array_equal(hg[k][same], ho[k][same]), k
+    assert np.array_equal(hg["prim"] >= 0, he["prim"] >= 0) and np.array_equal(occ, occ_e)
+
+
+def test_more_ties_than_the_list_holds(ctx):
+    """Over 2^20 rays that all end in a tie: the list overflows and the rays
+    are found by their marks.  Equal to tracing them in parts."""
+    import fledge_gb300 as F
+    import torch
+    pos, _ = _scene("duplicates")
+    b, _ = U.gpu_build(ctx, pos, width=4, leaf=1)
+    soa = F.gen_rays(ctx, 3 << 19, 77)
+    soa[3:6] = 0.5 - soa[0:3] + 0.2 * (soa[3:6] - 0.5)  # toward the middle: nearly all hit
+    whole = b.intersect(F.Rays.from_soa(soa))
+    assert int((whole["prim"] >= 0).sum()) > 1 << 20
+    for a in range(0, soa.shape[1], 1 << 19):
+        part = b.intersect(F.Rays.from_soa(soa[:, a:a + (1 << 19)].contiguous()))
+        for k in part:
+            assert torch.equal(part[k], whole[k][a:a + (1 << 19)]), k
+    ctx.sync()
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 4863, 4865, 155649])
+def test_small_batches_spread_over_warps(ctx, oracle, n):
+    """Ray counts around the edges of the spread of a small batch over warps
+    and blocks: equal to the same rays inside a large batch."""
+    import fledge_gb300 as F
+    import torch
+    pos = F.gen_triangles(ctx, 5000, 12)
+    b = F.RadixBVHBuilder(F.InternalTriangleMesh(pos), ctx)
+    b.build()
+    soa = F.gen_rays(ctx, 300000, 13)
+    whole = b.intersect(F.Rays.from_soa(soa))
+    occ = b.intersectP(F.Rays.from_soa(soa))
+    part = F.Rays.from_soa(soa[:, :n].contiguous())
+    hp = b.intersect(part)
+    for k in hp:
+        assert torch.equal(hp[k], whole[k][:n]), k
+    assert torch.equal(b.intersectP(part), occ[:n])
+    ctx.sync()
+
+
+def test_one_triangle_scenes_of_a_batch(ctx, oracle):
+    """Scenes of no, one and two triangles in one 4-wide batch, also after a
+    change of width: each equal to its own handle."""
+    import fledge_gb300 as F
+    import torch
+    counts = [1, 0, 2, 1, 1, 600, 1]
+    offs = np.concatenate([[0], np.cumsum(counts)])
+    pos = F.gen_triangles(ctx, int(offs[-1]), 5, half_extent=0.3)
+    per = 2000
+    soa = F.gen_rays(ctx, per * len(counts), 6)
+    bb = F.BatchedRadixBVHBuilder(F.InternalTriangleMesh(pos), offs, ctx, node_width=8)
+    bb.build()
+    bb.set_width(4)
+    h = bb.intersect_batched(F.Rays.from_soa(soa), per * np.arange(len(counts) + 1))
+    for s, c in enumerate(counts):
+        one = F.RadixBVHBuilder(F.InternalTriangleMesh(pos[3 * offs[s]:3 * offs[s + 1]].contiguous()), ctx, node_width=2)
+        one.build()
+        r = F.Rays.from_soa(soa[:, per * s:per * (s + 1)].contiguous())
+        ho = one.intersect(r)
+        for k in ho:
+            assert torch.equal(ho[k], h[k][per * s:per * (s + 1)]), (s, k)
+        four = F.RadixBVHBuilder(one.mesh, ctx, node_width=4)
+        four.build()
+        assert torch.equal(four.intersectP(r), one.intersectP(r))
+    ctx.sync()
