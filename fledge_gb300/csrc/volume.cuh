@@ -52,6 +52,51 @@ __device__ __forceinline__ float gat(const GridDev &G, int x, int y, int z) {
 
 __device__ __forceinline__ float lerpf(float a, float b, float w) { return a + (b - a) * w; }
 
+// The eight lattice values around (x, y, z), x fastest.  Almost every lookup
+// lies inside the lattice: one bounds test then stands for those of the eight
+// points, whose addresses follow from one base (dense), or from one brick slot
+// when they share a brick (7^3 / 8^3 = 67 % of the lookups in a sparse grid;
+// otherwise the offsets of both planes per axis are formed once).
+template <bool SP>
+__device__ __forceinline__ void grid_cell(const GridDev &G, int x, int y, int z, float (&v)[8]) {
+  if ((unsigned)x < (unsigned)(G.nx - 1) && (unsigned)y < (unsigned)(G.ny - 1) && (unsigned)z < (unsigned)(G.nz - 1)) {
+    if (!SP) {
+      const float *p = G.rho + ((int64_t)z * G.ny + y) * G.nx + x;
+      const int64_t sz = (int64_t)G.ny * G.nx;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) v[c] = __ldg(p + (c >> 2) * sz + (c >> 1 & 1) * (int64_t)G.nx + (c & 1));
+    } else {
+      const int bx = (unsigned)x / kBrick, by = (unsigned)y / kBrick, bz = (unsigned)z / kBrick;
+      const int ox = (unsigned)x % kBrick, oy = (unsigned)y % kBrick, oz = (unsigned)z % kBrick;
+      const int32_t *bp = G.bidx + ((int64_t)bz * G.bny + by) * G.bnx + bx;
+      if (ox < kBrick - 1 && oy < kBrick - 1 && oz < kBrick - 1) {
+        const int32_t slot = __ldg(bp);
+        const float *p = G.rho + (int64_t)slot * (kBrick * kBrick * kBrick) + (oz * kBrick + oy) * kBrick + ox;
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          v[c] = slot < 0 ? 0.0f : __ldg(p + (c >> 2) * kBrick * kBrick + (c >> 1 & 1) * kBrick + (c & 1));
+      } else {
+        // brick step and offset in the brick of the upper plane of each axis
+        const int sx = ox == kBrick - 1, sy = oy == kBrick - 1 ? G.bnx : 0;
+        const int64_t sz = oz == kBrick - 1 ? (int64_t)G.bny * G.bnx : 0;
+        const int ux = sx ? 0 : ox + 1, uy = sy ? 0 : oy + 1, uz = oz == kBrick - 1 ? 0 : oz + 1;
+        int32_t slot[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          slot[c] = __ldg(bp + (c & 4 ? sz : 0) + (c & 2 ? sy : 0) + (c & 1 ? sx : 0));
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          v[c] = slot[c] < 0 ? 0.0f
+                             : __ldg(G.rho + (int64_t)slot[c] * (kBrick * kBrick * kBrick) +
+                                     ((c & 4 ? uz : oz) * kBrick + (c & 2 ? uy : oy)) * kBrick + (c & 1 ? ux : ox));
+      }
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) v[c] = gat<SP>(G, x + (c & 1), y + (c >> 1 & 1), z + (c >> 2));
+  }
+}
+
 template <bool SP>
 __device__ __forceinline__ float sample_grid(const GridDev &G, float px, float py, float pz, int &x, int &y, int &z,
                                              float &fx, float &fy, float &fz) {
@@ -65,10 +110,12 @@ __device__ __forceinline__ float sample_grid(const GridDev &G, float px, float p
   fx = gx - x0;
   fy = gy - y0;
   fz = gz - z0;
-  float c00 = lerpf(gat<SP>(G, x, y, z), gat<SP>(G, x + 1, y, z), fx);
-  float c10 = lerpf(gat<SP>(G, x, y + 1, z), gat<SP>(G, x + 1, y + 1, z), fx);
-  float c01 = lerpf(gat<SP>(G, x, y, z + 1), gat<SP>(G, x + 1, y, z + 1), fx);
-  float c11 = lerpf(gat<SP>(G, x, y + 1, z + 1), gat<SP>(G, x + 1, y + 1, z + 1), fx);
+  float v[8];
+  grid_cell<SP>(G, x, y, z, v);
+  float c00 = lerpf(v[0], v[1], fx);
+  float c10 = lerpf(v[2], v[3], fx);
+  float c01 = lerpf(v[4], v[5], fx);
+  float c11 = lerpf(v[6], v[7], fx);
   float c0 = lerpf(c00, c10, fy);
   float c1 = lerpf(c01, c11, fy);
   return lerpf(c0, c1, fz);
@@ -95,41 +142,72 @@ __device__ __forceinline__ bool box_pbrt(const GridDev &G, const float3 &o, cons
   return true;
 }
 
-// Ratio tracking of one ray; returns T and the state after the last
-// roulette survival.
+// Ratio tracking of one ray, a step at a time: T so far in tr, and the state
+// after the last roulette survival (the adjoint's checkpoint).
+struct RatioState {
+  float3 o, d;
+  float t, t_max, tr;
+  float ck_t, ck_c;
+  uint32_t ck_k;
+  RayStream rs;
+};
+
+// False if the ray misses the grid's box (T = 1).
+__device__ __forceinline__ bool ratio_start(const GridDev &G, RatioState &s, float tmax, uint64_t seed, int64_t ray) {
+  s.ck_t = 0.0f;
+  s.ck_k = 0u;
+  s.ck_c = 1.0f;
+  s.tr = 1.0f;
+  float t_min;
+  if (!box_pbrt(G, s.o, s.d, tmax, t_min, s.t_max)) return false;
+  s.t = fmaxf(t_min, 0.0f);
+  s.t_max = fminf(s.t_max, tmax);
+  s.rs.init(seed, (uint64_t)ray, 0u);
+  s.ck_t = s.t;
+  return true;
+}
+
+// One step; false once the ray has left the box or been absorbed.
+template <bool SP>
+__device__ __forceinline__ bool ratio_step(const GridDev &G, float max_mu, float inv_maj, RatioState &s) {
+  const float u = s.rs.next();
+  s.t += -flg_logf(1.0f - u) / max_mu;
+  if (s.t >= s.t_max) return false;
+  int x, y, z;
+  float fx, fy, fz;
+  const float dens =
+      sample_grid<SP>(G, s.o.x + s.d.x * s.t, s.o.y + s.d.y * s.t, s.o.z + s.d.z * s.t, x, y, z, fx, fy, fz);
+  s.tr *= 1.0f - fmaxf(0.0f, dens * inv_maj);
+  if (s.tr < G.rr) {
+    const float q = fmaxf(0.05f, 1.0f - s.tr);
+    if (s.rs.next() < q) {
+      s.tr = 0.0f;
+      return false;
+    }
+    s.tr /= 1.0f - q;
+    s.ck_t = s.t;
+    s.ck_k = s.rs.k;
+    s.ck_c = s.tr;
+  }
+  return true;
+}
+
 template <bool SP>
 __device__ __forceinline__ float ratio_track(const GridDev &G, float maj, float inv_maj, const float3 &o,
                                              const float3 &d, float tmax, uint64_t seed, int64_t ray, float &ck_t,
                                              uint32_t &ck_k, float &ck_c) {
-  ck_t = 0.0f;
-  ck_k = 0u;
-  ck_c = 1.0f;
-  float t_min, t_max;
-  if (!box_pbrt(G, o, d, tmax, t_min, t_max)) return 1.0f;
-  float tr = 1.0f, t = fmaxf(t_min, 0.0f);
-  t_max = fminf(t_max, tmax);
-  const float max_mu = G.sigma_t * maj;
-  RayStream rs;
-  rs.init(seed, (uint64_t)ray, 0u);
-  ck_t = t;
-  for (int step_ = 0; step_ < kMaxTrackSteps; ++step_) {
-    float u = rs.next();
-    t += -flg_logf(1.0f - u) / max_mu;
-    if (t >= t_max) break;
-    int x, y, z;
-    float fx, fy, fz;
-    float dens = sample_grid<SP>(G, o.x + d.x * t, o.y + d.y * t, o.z + d.z * t, x, y, z, fx, fy, fz);
-    tr *= 1.0f - fmaxf(0.0f, dens * inv_maj);
-    if (tr < G.rr) {
-      float q = fmaxf(0.05f, 1.0f - tr);
-      if (rs.next() < q) return 0.0f;
-      tr /= 1.0f - q;
-      ck_t = t;
-      ck_k = rs.k;
-      ck_c = tr;
-    }
+  RatioState s;
+  s.o = o;
+  s.d = d;
+  if (ratio_start(G, s, tmax, seed, ray)) {
+    const float max_mu = G.sigma_t * maj;
+    for (int step_ = 0; step_ < kMaxTrackSteps; ++step_)
+      if (!ratio_step<SP>(G, max_mu, inv_maj, s)) break;
   }
-  return tr;
+  ck_t = s.ck_t;
+  ck_k = s.ck_k;
+  ck_c = s.ck_c;
+  return s.tr;
 }
 
 // Kernel-side view of a grid handle.
@@ -155,34 +233,58 @@ inline GridDev grid_dev(flg_grid g) {
   return G;
 }
 
-// Delta tracking of one ray over [0, tmax] (volume.cpp:109-148): true on a
-// real collision, with its position in p.  Draws from rs: one uniform per
-// step plus one for the collision test.
+// Delta tracking of one ray over [0, tmax] (volume.cpp:109-148), a step at a
+// time.  Draws from rs: one uniform per step plus one for the collision test.
+struct DeltaState {
+  float3 o, d;
+  float t, t_max;
+  RayStream rs;
+};
+
+// False if the ray misses the grid's box.
+__device__ __forceinline__ bool delta_start(const GridDev &G, DeltaState &s, float tmax) {
+  float t_min;
+  if (!box_pbrt(G, s.o, s.d, tmax, t_min, s.t_max)) return false;
+  s.t = fmaxf(t_min, 0.0f);
+  s.t_max = fminf(s.t_max, tmax);
+  return true;
+}
+
+// One step: 1 a real collision (its position in p), -1 out of the box, 0 go on.
+template <bool SP>
+__device__ __forceinline__ int delta_step(const GridDev &G, float max_mu, DeltaState &s, float3 &p) {
+  const float u = s.rs.next();
+  s.t += -flg_logf(1.0f - u) / max_mu;
+  if (s.t >= s.t_max) return -1;
+  const float qx = s.o.x + s.d.x * s.t, qy = s.o.y + s.d.y * s.t, qz = s.o.z + s.d.z * s.t;
+  int x, y, z;
+  float fx, fy, fz;
+  const float dens = sample_grid<SP>(G, qx, qy, qz, x, y, z, fx, fy, fz);
+  const float p_s = G.sigma_s * dens / max_mu;
+  const float p_a = G.sigma_a * dens / max_mu;
+  const float p_n = 1.0f - p_s - p_a;
+  if (s.rs.next() > p_n) {
+    p = make_float3(qx, qy, qz);
+    return 1;
+  }
+  return 0;
+}
+
 template <bool SP>
 __device__ __forceinline__ bool delta_track(const GridDev &G, float maj, const float3 &o, const float3 &d,
                                             float tmax, RayStream &rs, float3 &p) {
-  float t_min, t_max;
-  if (!box_pbrt(G, o, d, tmax, t_min, t_max)) return false;
-  float t = fmaxf(t_min, 0.0f);
-  const float max_mu = G.sigma_t * maj;
-  t_max = fminf(t_max, tmax);
-  for (int step_ = 0; step_ < kMaxTrackSteps; ++step_) {
-    float u = rs.next();
-    t += -flg_logf(1.0f - u) / max_mu;
-    if (t >= t_max) break;
-    float qx = o.x + d.x * t, qy = o.y + d.y * t, qz = o.z + d.z * t;
-    int x, y, z;
-    float fx, fy, fz;
-    float dens = sample_grid<SP>(G, qx, qy, qz, x, y, z, fx, fy, fz);
-    float p_s = G.sigma_s * dens / max_mu;
-    float p_a = G.sigma_a * dens / max_mu;
-    float p_n = 1.0f - p_s - p_a;
-    if (rs.next() > p_n) {
-      p = make_float3(qx, qy, qz);
-      return true;
-    }
+  DeltaState s;
+  s.o = o;
+  s.d = d;
+  s.rs = rs;
+  int r = -1;
+  if (delta_start(G, s, tmax)) {
+    const float max_mu = G.sigma_t * maj;
+    r = 0;
+    for (int step_ = 0; step_ < kMaxTrackSteps && r == 0; ++step_) r = delta_step<SP>(G, max_mu, s, p);
   }
-  return false;
+  rs = s.rs;
+  return r == 1;
 }
 
 // Henyey-Greenstein phase function HGP(wi, wo, g) (math_utils.h:103-107).
