@@ -510,8 +510,9 @@ __global__ void __launch_bounds__(256)
 //     does not settle go on a list, and k_settle4 settles the equal pairs
 //     (first_of_two) and traces the others again over the exact boxes
 //     (retrace4): about one ray per million on random soups.
-//   * Any hit: an accepted triangle counts if its own box, or else the box of
-//     its leaf range, passes the exact slab test.
+//   * Any hit: an accepted triangle counts if its own box passes the exact slab
+//     test.  A ray that found only others is traced again over the exact boxes
+//     (k_trace_retry4).
 // ----------------------------------------------------------------------------
 constexpr float kNear = 4.76837158203125e-07f;  // 2^-21
 // prim between k_trace4 and the kernels after it: a sorted position (< 2^28) with
@@ -519,6 +520,7 @@ constexpr float kNear = 4.76837158203125e-07f;  // 2^-21
 // positions at the same t, or v = -1: trace it again.
 constexpr int32_t kPending = 1 << 30;
 constexpr int32_t kListed = INT32_MIN;
+constexpr uint8_t kOccListed = 2;  // in occ: an any-hit ray on the list
 
 __device__ __forceinline__ float max3f(float a, float b, float c) {
   float r;
@@ -850,29 +852,6 @@ __device__ __noinline__ int32_t first_of_two(const Exact4 &X, const RaySoA &RS, 
   return min(p, q);
 }
 
-// Whether an any-hit candidate counts: its box, or that of its leaf range
-// (enc), passes the exact slab test.  Both only fail where the quantised
-// boxes let a ray in that the exact ones keep out.
-__device__ __forceinline__ bool hit_any_box(const TriRec *__restrict__ tris, int64_t g, int32_t enc, const float3 &o,
-                                            const float3 &inv, float tmax) {
-  float lo[3], hi[3];
-  tri_rec_box(tris, g, lo, hi);
-  float t0 = slab_exact(lo, hi, o, inv, tmax);
-  if (t0 == t0) return true;
-  const int64_t first = (int64_t)((uint32_t)enc >> 3);
-  const int count = (enc & 7) + 1;
-  for (int j = 0; j < count; ++j) {
-    float l[3], h[3];
-    tri_rec_box(tris, first + j, l, h);
-    for (int a = 0; a < 3; ++a) {
-      lo[a] = fminf(lo[a], l[a]);
-      hi[a] = fmaxf(hi[a], h[a]);
-    }
-  }
-  t0 = slab_exact(lo, hi, o, inv, tmax);
-  return t0 == t0;
-}
-
 // Final values of a closest hit: sorted position g, fp32 t.
 __device__ __forceinline__ void finish_hit(const RaySoA &R, const Out &O, const TriRec *__restrict__ tris, int64_t i,
                                            int32_t g, float best) {
@@ -943,13 +922,15 @@ __global__ void __launch_bounds__(256, 4)
   }
 }
 
-// Any-hit rays whose stack overflowed.
+// Any-hit rays that k_trace4 left open.
 __global__ void __launch_bounds__(128)
-    k_trace_retry4(const __grid_constant__ RaySoA R, Out O, const __grid_constant__ Exact4 X, Scratch S) {
-  const uint32_t cnt = min((int64_t)*S.ovf_count, S.ovf_cap);
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
-    const int64_t i = S.ovf[j];
-    O.occ[i] = retrace4<true>(X, R, i, S.err).prim >= 0 ? 1 : 0;
+    k_trace_retry4(const __grid_constant__ RaySoA R, int64_t n, Out O, const __grid_constant__ Exact4 X, Scratch S) {
+  const uint32_t cnt = *S.ovf_count;
+  const bool listed = cnt <= S.ovf_cap;  // else look for the marks
+  const int64_t end = listed ? (int64_t)cnt : n;
+  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < end; j += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = listed ? S.ovf[j] : j;
+    if (O.occ[i] == kOccListed) O.occ[i] = retrace4<true>(X, R, i, S.err).prim >= 0 ? 1 : 0;
   }
 }
 
@@ -1004,7 +985,9 @@ __global__ void __launch_bounds__(256, 4)
   constexpr int32_t kPop = 0x7FFFFFFD, kDone = 0x7FFFFFFE, kIdle = 0x7FFFFFFF;
   constexpr uint32_t kSlot = 256 * sizeof(uint64_t);  // bytes between a thread's slots
   constexpr unsigned kAll = 0xFFFFFFFFu;
-  constexpr int64_t kOverflow = INT64_MIN;  // on a ray's index: its stack overflowed
+  // On a ray's index: trace it again over the exact boxes (its stack
+  // overflowed, or an any-hit candidate's own box kept it out).
+  constexpr int64_t kAgain = INT64_MIN;
   // A second candidate near the closest hit: none, one within kNear but not
   // equal, two or more equal, or (>= 0) the one that is equal.
   constexpr int32_t kNone = -1, kSome = -2, kMany = -3;
@@ -1074,11 +1057,14 @@ __global__ void __launch_bounds__(256, 4)
     // Retire finished rays.
     if (cur == kDone && leaf == 0 && lead == lane) {
       const int64_t ray = s_ray[threadIdx.x];
+      const int64_t at = ray < 0 ? ray - kAgain : ray;
       if (ANY) {
-        if (ray < 0 && prim < 0) record_overflow(S, ray - kOverflow);
-        else O.occ[ray < 0 ? ray - kOverflow : ray] = prim >= 0 ? 1 : 0;
+        O.occ[at] = prim >= 0 ? 1 : ray < 0 ? kOccListed : 0;
+        if (ray < 0 && prim < 0) {
+          const uint32_t k = atomicAdd(S.ovf_count, 1u);
+          if (k < S.ovf_cap) S.ovf[k] = at;  // past the end the mark is looked for
+        }
       } else {
-        const int64_t at = ray < 0 ? ray - kOverflow : ray;
         bool listed = ray < 0;
         int32_t other = -1;
         if (prim >= 0 && !listed) {
@@ -1253,7 +1239,7 @@ __global__ void __launch_bounds__(256, 4)
             if (top >= s_base + (kStackSlots - 2) * kSlot) {
               if (moved + kStackMove > kStackLocal) {
                 int64_t *mark = &s_ray[(threadIdx.x & ~31u) + (lead & 0xFF)];
-                if (*mark >= 0) *mark += kOverflow;
+                if (*mark >= 0) *mark += kAgain;
                 cur = kDone;
                 leaf = leaf2 = 0;
               } else {
@@ -1304,13 +1290,17 @@ __global__ void __launch_bounds__(256, 4)
           continue;
         if (ANY) {
           if (t >= tmin && !(t > best)) {
-            // a one-triangle scene is tested without a box
             const float3 ie = make_float3(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z));
-            if (hit_any_box(tris, g, j < n1 ? e1 : e2, o, ie, best) || __ldg(&nodes[s1 >> 2].step) == kLoneStep) {
+            float lo[3], hi[3];
+            tri_rec_box(tris, g, lo, hi);
+            const float t0 = slab_exact(lo, hi, o, ie, best);
+            if (t0 == t0) {
               prim = g;
               cur = kDone;
               break;
             }
+            int64_t *mark = &s_ray[(threadIdx.x & ~31u) + (lead & 0xFF)];
+            if (*mark >= 0) *mark += kAgain;
           }
         } else if (t >= tmin && t <= best * (1.0f + kNear)) {
           if (t < best || (prim < 0 && t == best)) {
@@ -1658,7 +1648,7 @@ static int launch4(flg_ctx ctx, cudaStream_t st, flg_bvh b, const RaySoA &R, int
   FLG_LAUNCH_CHECK(ctx, "k_trace4");
   stage_mark(ctx, st, "trace");
   if (ANY) {
-    k_trace_retry4<<<(unsigned)ctx->num_sms, 128, 0, st>>>(R, O, X, S);
+    k_trace_retry4<<<(unsigned)ctx->num_sms, 128, 0, st>>>(R, n, O, X, S);
     FLG_LAUNCH_CHECK(ctx, "k_trace_retry4");
     stage_mark(ctx, st, "trace_retry");
   } else {
