@@ -953,20 +953,26 @@ __global__ void __launch_bounds__(128)
 // nodes as the average, so without more the last of them set the time of a
 // launch (of half of it on camera rays of a surface), and the longest that of
 // a small batch.  Once the counter is exhausted, idle lanes of a warp
-// therefore help the others: each takes the lowest stack entry (the farthest,
-// and mostly the largest, subtree) of a lane that has one, with a copy of its
-// ray, and walks it as a ray of its own.  The lane that took the ray from the
-// counter leads: it collects its helpers' hits under the rules for a second
-// candidate of the same ray, and retires once they are done.  Lanes of one
-// ray share the closest t at every turn of the outer loop.
+// therefore help the others: each takes one of their stack entries, the lowest
+// (farthest, and mostly largest) subtrees first, with a copy of the ray, and
+// walks it as a ray of its own.  The lane that took the ray from the counter
+// leads: at every turn of the outer loop it collects the group's closest hit,
+// under the rules for a second candidate of the same ray, and all take its t
+// for their limit; it retires once its helpers are done.
 constexpr int kLeafWait = 8;
 // Slots, the sentinel's included.  With the ray indices 32 KB per 256-thread
 // block: four blocks leave 124 KB of an SM for L1, a byte more only 92.
 constexpr int kStackSlots = 15;
 constexpr int kStackMove = 8;    // entries moved at a time
 constexpr int kStackLocal = 64;
-constexpr int kHelpAfter = 32;  // turns after the counter's end before lanes help
-constexpr int kHelpTurns = 8;
+// Turns of the node loop after the counter's end before lanes help, and
+// between two rounds of helping: 4 / 4; us at 32 / 8, 16 / 4, 8 / 4, 4 / 4:
+// 1 M camera rays on 327,680 triangles 199, 186, 183, 182 (240 without help),
+// 2 M shadow rays 511, 490, 479, 475, a 640x360 x 4 image 1319, 1206, 1145,
+// 1115, 4,096 rays on 20,001 triangles 60, 45, 42, 36 (96 at the time that every
+// ray walked alone).
+constexpr int kHelpAfter = 4;
+constexpr int kHelpTurns = 4;
 
 __device__ __forceinline__ void stack_store(uint32_t at, uint32_t key, int32_t ref) {
   asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at), "r"(key), "r"(ref) : "memory");
@@ -985,16 +991,18 @@ __global__ void __launch_bounds__(256, 4)
   constexpr int32_t kPop = 0x7FFFFFFD, kDone = 0x7FFFFFFE, kIdle = 0x7FFFFFFF;
   constexpr uint32_t kSlot = 256 * sizeof(uint64_t);  // bytes between a thread's slots
   constexpr unsigned kAll = 0xFFFFFFFFu;
-  // On a ray's index: trace it again over the exact boxes (its stack
-  // overflowed, or an any-hit candidate's own box kept it out).
-  constexpr int64_t kAgain = INT64_MIN;
+  // The upper word: bits 32 .. 47 of the ray's index; trace it again over the
+  // exact boxes (its stack overflowed, or an any-hit candidate's own box kept
+  // it out); and, as multiples of kHelper, its helpers at work.
+  constexpr uint32_t kRayHigh = 0xFFFFu, kAgain = 1u << 16, kHelper = 1u << 17;
   // A second candidate near the closest hit: none, one within kNear but not
   // equal, two or more equal, or (>= 0) the one that is equal.
   constexpr int32_t kNone = -1, kSome = -2, kMany = -3;
   __shared__ uint64_t s_stk[kStackSlots][256];
-  __shared__ int64_t s_ray[256];
+  __shared__ uint32_t s_ray[2][256];  // the ray's index; in the upper word also its flags and helpers
   const uint32_t s_base = (uint32_t)__cvta_generic_to_shared(&s_stk[0][0]);
   const uint32_t bottom = s_base + threadIdx.x * (uint32_t)sizeof(uint64_t);
+  uint32_t *crew = s_ray[1] + (threadIdx.x & ~31u);  // the upper words of the warp's lanes
   stack_store(bottom, 0xFF800000u, kDone);  // the sentinel: -inf
   uint64_t stk[kStackLocal];
   float3 o = make_float3(0.f, 0.f, 0.f), d = o, inv = o;
@@ -1005,7 +1013,7 @@ __global__ void __launch_bounds__(256, 4)
   uint32_t top = bottom + kSlot;  // the next free slot
   int moved = 0;                  // entries in the local array
   int scene = -1;
-  int lead = 0;                   // the lane that leads this ray | its helpers at work << 8
+  int lead = 0;                   // the lane that leads this ray
   int phase = 0;                  // 0 at the start; 1 the counter has rays; then 2 + turns since it has none
   // The first `lanes` rays of every warp by its index, the others from the
   // counter, which starts behind them.
@@ -1013,59 +1021,63 @@ __global__ void __launch_bounds__(256, 4)
 
   while (true) {
     const int lane = threadIdx.x & 31;
-    // Lanes that help: shared limits, finished helpers.
-    if (phase > kHelpAfter && __any_sync(kAll, cur != kIdle && (lead & 0xFF) != lane)) {
-      const unsigned group = __match_any_sync(kAll, cur != kIdle ? lead & 0xFF : 32 + lane);
-      if (ANY) {
-        if (__reduce_or_sync(group, prim >= 0 ? 1u : 0u) && cur != kIdle) {
-          cur = kDone;
-          leaf = leaf2 = 0;
-        }
-      } else {
-        const float m = __uint_as_float(__reduce_min_sync(group, __float_as_uint(best)));
-        if (m < best) {
-          tie = prim >= 0 && best <= m * (1.0f + kNear) ? kSome : kNone;
-          prim = -1;
-          best = m;
-        }
-      }
-      for (unsigned done = __ballot_sync(kAll, cur == kDone && leaf == 0 && (lead & 0xFF) != lane); done != 0u;
-           done &= done - 1u) {
-        const int h = __ffs(done) - 1;
-        const int to = __shfl_sync(kAll, lead & 0xFF, h);
+    // Lanes that help hand their hits to the lane that leads, share its limit,
+    // and are idle again once they are done.
+    const bool helps = cur != kIdle && lead != lane;
+    if (phase > kHelpAfter && __any_sync(kAll, helps)) {
+      for (unsigned m = __ballot_sync(kAll, helps && (prim >= 0 || tie != kNone)); m != 0u; m &= m - 1u) {
+        const int h = __ffs(m) - 1;
+        const int to = __shfl_sync(kAll, lead, h);
         const float h_best = __shfl_sync(kAll, best, h);
         const int32_t h_prim = __shfl_sync(kAll, prim, h), h_tie = __shfl_sync(kAll, tie, h);
-        if (lane == h) cur = kIdle;
         if (lane == to) {
-          lead -= 1 << 8;
           if (ANY) {
-            prim = max(prim, h_prim);
+            prim = h_prim;
+            cur = kDone;
+            leaf = leaf2 = 0;
           } else if (h_prim < 0) {
-            if (h_tie != kNone && tie == kNone) tie = kSome;
+            if (tie == kNone) tie = kSome;
           } else if (h_best < best || (prim < 0 && h_best == best)) {
             tie = h_tie != kNone ? h_tie : best <= h_best * (1.0f + kNear) ? kSome : kNone;
             best = h_best;
             prim = h_prim;
           } else if (h_best == best) {
-            tie = tie < 0 && tie != kMany && h_tie < 0 && h_tie != kMany ? h_prim : kMany;
+            tie = (tie == kNone || tie == kSome) && (h_tie == kNone || h_tie == kSome) ? h_prim : kMany;
           } else if (h_best <= best * (1.0f + kNear) && tie == kNone) {
             tie = kSome;
           }
         }
       }
+      const float l_best = __shfl_sync(kAll, best, lead);
+      const int32_t l_prim = __shfl_sync(kAll, prim, lead);
+      if (helps) {
+        prim = -1;
+        tie = kNone;
+        if (!ANY) best = l_best;
+        if (ANY && l_prim >= 0) {
+          cur = kDone;
+          leaf = leaf2 = 0;
+        }
+        if (cur == kDone && leaf == 0) {
+          cur = kIdle;
+          atomicSub(crew + lead, kHelper);
+        }
+      }
+      __syncwarp();
     }
     // Retire finished rays.
-    if (cur == kDone && leaf == 0 && lead == lane) {
-      const int64_t ray = s_ray[threadIdx.x];
-      const int64_t at = ray < 0 ? ray - kAgain : ray;
+    if (cur == kDone && leaf == 0 && lead == lane && *(volatile uint32_t *)(crew + lane) < kHelper) {
+      const uint32_t flags = crew[lane];
+      const int64_t at = (int64_t)(flags & kRayHigh) << 32 | s_ray[0][threadIdx.x];
+      const bool redo = (flags & kAgain) != 0u;
       if (ANY) {
-        O.occ[at] = prim >= 0 ? 1 : ray < 0 ? kOccListed : 0;
-        if (ray < 0 && prim < 0) {
+        O.occ[at] = prim >= 0 ? 1 : redo ? kOccListed : 0;
+        if (redo && prim < 0) {
           const uint32_t k = atomicAdd(S.ovf_count, 1u);
           if (k < S.ovf_cap) S.ovf[k] = at;  // past the end the mark is looked for
         }
       } else {
-        bool listed = ray < 0;
+        bool listed = redo;
         int32_t other = -1;
         if (prim >= 0 && !listed) {
           // the winner's box, and that of a second triangle at the same t
@@ -1110,7 +1122,8 @@ __global__ void __launch_bounds__(256, 4)
         if ((int64_t)base + nidle >= n) phase = 2;
       }
       if (cur == kIdle && my < n) {
-        s_ray[threadIdx.x] = my;
+        s_ray[0][threadIdx.x] = (uint32_t)my;
+        crew[lane] = (uint32_t)(my >> 32);
         load_ray(R, my, o, d, inv, tmin, best);
         inv = make_float3(inv_q(inv.x), inv_q(inv.y), inv_q(inv.z));
         tie = kNone;
@@ -1124,28 +1137,25 @@ __global__ void __launch_bounds__(256, 4)
       }
     } else if (phase >= 2 && idle != 0u) {
       if (idle == kAll) break;
-      // Help: the r-th idle lane takes the lowest entry of the r-th lane that
-      // has one to give.
-      const unsigned donors =
-          phase > kHelpAfter ? __ballot_sync(kAll, cur < kDone && moved == 0 && top - low > kSlot) : 0u;
-      if (donors != 0u) {
-        const unsigned lt = (1u << lane) - 1u;
-        const int k = min(nidle, __popc(donors));
-        const bool give = (donors >> lane & 1u) && __popc(donors & lt) < k;
-        const bool take = cur == kIdle && __popc(idle & lt) < k;
-        int from = lane;
-        if (take) {  // the donors' r-th bit
-          int r = __popc(idle & lt);
-          from = 0;
+      // Help: of the entries in the lanes' stacks, in lane order and each lane's
+      // lowest first, the r-th idle lane takes the r-th.
+      int left = phase > kHelpAfter && cur < kDone && moved == 0 ? (int)((top - low) / kSlot) - 1 : 0;
+      int upto = left;  // entries in the lanes up to this one
 #pragma unroll
-          for (int w = 16; w >= 1; w >>= 1) {
-            const int c = __popc(donors >> from & ((1u << w) - 1u));
-            if (r >= c) {
-              r -= c;
-              from += w;
-            }
-          }
-        }
+      for (int w = 1; w < 32; w <<= 1) {
+        const int v = __shfl_up_sync(kAll, upto, w);
+        if (lane >= w) upto += v;
+      }
+      const int k = min(nidle, __shfl_sync(kAll, upto, 31));
+      if (k > 0) {
+        const int r = __popc(idle & ((1u << lane) - 1u));
+        const bool take = cur == kIdle && r < k;
+        int from = 0;  // the first lane whose entries reach past r
+#pragma unroll
+        for (int w = 16; w >= 1; w >>= 1)
+          if (__shfl_sync(kAll, upto, (from + w - 1) & 31) <= r) from += w;
+        if (!take) from = lane;
+        const int before = upto - left, give = max(0, min(left, k - before));
         o.x = __shfl_sync(kAll, o.x, from);
         o.y = __shfl_sync(kAll, o.y, from);
         o.z = __shfl_sync(kAll, o.z, from);
@@ -1157,8 +1167,8 @@ __global__ void __launch_bounds__(256, 4)
         inv.z = __shfl_sync(kAll, inv.z, from);
         tmin = __shfl_sync(kAll, tmin, from);
         best = __shfl_sync(kAll, best, from);
-        const int to = __shfl_sync(kAll, lead & 0xFF, from);
-        const uint32_t at = __shfl_sync(kAll, low, from) + kSlot;
+        lead = __shfl_sync(kAll, lead, from);
+        const uint32_t at = __shfl_sync(kAll, low, from) + (uint32_t)(1 + r - __shfl_sync(kAll, before, from)) * kSlot;
         if (take) {
           uint32_t key;
           stack_load(at, key, cur);
@@ -1167,13 +1177,11 @@ __global__ void __launch_bounds__(256, 4)
           low = bottom;
           top = bottom + kSlot;
           moved = 0;
-          lead = to;
+          atomicAdd(crew + lead, kHelper);
         }
-        __syncwarp();  // the entries are read before their slots become sentinels
-        for (unsigned m = __ballot_sync(kAll, take); m != 0u; m &= m - 1u)
-          if (__shfl_sync(kAll, to, __ffs(m) - 1) == lane) lead += 1 << 8;
-        if (give) {
-          low += kSlot;  // the slot given away becomes the sentinel
+        __syncwarp();  // the entries are read before a slot becomes a sentinel
+        if (give > 0) {
+          low += (uint32_t)give * kSlot;  // the last slot given away becomes the sentinel
           stack_store(low, 0xFF800000u, kDone);
         }
       }
@@ -1238,8 +1246,7 @@ __global__ void __launch_bounds__(256, 4)
             }
             if (top >= s_base + (kStackSlots - 2) * kSlot) {
               if (moved + kStackMove > kStackLocal) {
-                int64_t *mark = &s_ray[(threadIdx.x & ~31u) + (lead & 0xFF)];
-                if (*mark >= 0) *mark += kAgain;
+                atomicOr(crew + lead, kAgain);
                 cur = kDone;
                 leaf = leaf2 = 0;
               } else {
@@ -1299,8 +1306,7 @@ __global__ void __launch_bounds__(256, 4)
               cur = kDone;
               break;
             }
-            int64_t *mark = &s_ray[(threadIdx.x & ~31u) + (lead & 0xFF)];
-            if (*mark >= 0) *mark += kAgain;
+            atomicOr(crew + lead, kAgain);
           }
         } else if (t >= tmin && t <= best * (1.0f + kNear)) {
           if (t < best || (prim < 0 && t == best)) {
@@ -1624,17 +1630,17 @@ __global__ void __launch_bounds__(256, 4)
 // hit: the overflow list).
 //
 // A warp runs through the paths of its rays in turn, so the fewer it has the
-// sooner they end; but past two warps per scheduler thinner warps only add
-// instructions.  A batch too small to give eight full warps to every SM is
-// spread over that many (4,096 rays on 20,001 triangles: 72 us, against 92 us
-// in full warps and 96 us in one-ray warps), and its blocks are made smaller
+// sooner they end; but past a few warps per scheduler thinner warps only add
+// instructions.  A batch too small to give sixteen full warps to every SM is
+// spread over that many (before lanes helped: 4,096 rays on 20,001 triangles 72
+// us, 92 in full warps, 96 in one-ray warps), and its blocks are made smaller
 // until they cover the SMs.  Refills at 8 idle lanes at most: with the
 // quantised nodes 8 beat 16 and 24 (24.0 against 25.6 and 29.6 ms on 31.6 M
 // scattered rays).
 template <bool ANY>
 static int launch4(flg_ctx ctx, cudaStream_t st, flg_bvh b, const RaySoA &R, int64_t n, const Out &O,
                    const Scratch &S, const int64_t *ray_off, int n_scenes, const flg_trace_opts &op) {
-  const int lanes = (int)std::min<int64_t>(32, ceil_div(n, (int64_t)ctx->num_sms * 8));
+  const int lanes = (int)std::min<int64_t>(32, ceil_div(n, (int64_t)ctx->num_sms * 16));
   int threads = op.block_threads, per_sm = 0;
   while (threads > 32 && ceil_div(n, (int64_t)lanes * (threads / 32)) < ctx->num_sms) threads >>= 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace4<ANY>, threads, 0);
