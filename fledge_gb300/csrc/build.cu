@@ -3,6 +3,7 @@
 //
 // Pipeline (one CUDA stream, no host synchronisation, no allocation in
 // flg_bvh_rebuild so the whole build can be captured in a CUDA graph):
+//   0. k_build_setup   everything the build starts from
 //   1. k_scene_bounds  union of triangle AABBs per scene (prestage reduce,
 //                      radix_bvh.cpp:49-60), block reduce + ordered atomics
 //   2. k_morton_hist   30-bit Morton code per triangle (radix_bvh.cpp:63-73)
@@ -16,7 +17,7 @@
 //                      neighbouring code deltas; the second arrival at a split
 //                      polls for its sibling's hand-over record (no fence per
 //                      level) and writes the finished node
-//   6. (optional) collapse to 4- or 8-wide nodes (collapse.cu)
+//   5. (optional) collapse to 4- or 8-wide nodes (collapse.cu)
 #include <cuda/atomic>
 
 #include <algorithm>
@@ -27,8 +28,6 @@
 #include "internal.h"
 
 namespace flg {
-
-int64_t sort_tiles(int64_t n);
 
 // Scene of triangle t given the scene `prev` of an earlier triangle of the
 // same thread (-1: none yet): one binary search, then a forward walk.
@@ -48,25 +47,63 @@ __device__ __forceinline__ void atomic_max_f(float *a, float v) {
   else atomicMin((unsigned int *)a, __float_as_uint(v));
 }
 
-__global__ void k_init_boxes(float *box, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    for (int k = 0; k < 3; ++k) {
-      box[6 * i + k] = 3.402823466e+38f;
-      box[6 * i + 3 + k] = -3.402823466e+38f;
+// Everything a build starts from, in one launch (as fills and copies these
+// were eight, 2 us each of a 20,001-triangle build): empty scene boxes, zeroed
+// digit counts, look-back words and tile counters, the scene passes' counts,
+// the collapse's counters and first queue, and, after a climb that gave up,
+// the climb's slots and counters (its mark is cleared by the next kernel).
+struct BuildSetup {
+  float *box;
+  int32_t n_scenes;
+  uint32_t *hist, *tile_ctr;
+  int64_t n_hist;
+  int32_t n_ctr;
+  uint4 *lookback;
+  int64_t n_lookback;  // 16-byte words
+  uint32_t *scene_hist;
+  const uint32_t *scene_hist_init;
+  int32_t n_scene_hist;
+  int32_t *wide_ctr;
+  int32_t n_wide_ctr;  // their initial values follow them
+  int2 *queue;
+  const int2 *queue_init;
+  int32_t n_queue;
+  float4 *slots;
+  uint32_t *flags;
+  int64_t n_nodes;
+  const uint32_t *dirty;
+};
+
+__global__ void __launch_bounds__(256) k_build_setup(BuildSetup B) {
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = t0; i < 6 * (int64_t)B.n_scenes; i += step)
+    B.box[i] = i % 6 < 3 ? 3.402823466e+38f : -3.402823466e+38f;
+  for (int64_t i = t0; i < B.n_hist; i += step) B.hist[i] = 0u;
+  for (int64_t i = t0; i < B.n_ctr; i += step) B.tile_ctr[i] = 0u;
+  for (int64_t i = t0; i < B.n_lookback; i += step) B.lookback[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int64_t i = t0; i < B.n_scene_hist; i += step) B.scene_hist[i] = B.scene_hist_init[i];
+  for (int64_t i = t0; i < B.n_wide_ctr; i += step) B.wide_ctr[i] = B.wide_ctr[B.n_wide_ctr + i];
+  for (int64_t i = t0; i < B.n_queue; i += step) B.queue[i] = B.queue_init[i];
+  if (B.n_nodes > 0 && *B.dirty != 0u) {
+    const float u = __int_as_float(kBoxUnset);
+    for (int64_t i = t0; i < B.n_nodes; i += step) {
+      B.slots[2 * i] = B.slots[2 * i + 1] = make_float4(u, u, u, u);
+      B.flags[i] = 0u;
     }
   }
 }
 
 constexpr int kBoundsThreads = 256;
-constexpr int kBoundsChunk = 8192;
+// Triangles per block: one round of the threads for small builds, more (fewer
+// atomics per scene) once that gives every SM its eight blocks.
+constexpr int kBoundsChunkMax = 8192;
 
 __global__ void __launch_bounds__(kBoundsThreads)
     k_scene_bounds(const float *__restrict__ pos, const int32_t *__restrict__ idx, int64_t n_tri,
-                   const int64_t *__restrict__ tri_off, int n_scenes, float *scene_box) {
+                   const int64_t *__restrict__ tri_off, int n_scenes, int chunk, float *scene_box) {
   __shared__ float s_red[6][kBoundsThreads / 32];
-  const int64_t start = (int64_t)blockIdx.x * kBoundsChunk;
-  const int64_t end = min(start + (int64_t)kBoundsChunk, n_tri);
+  const int64_t start = (int64_t)blockIdx.x * chunk;
+  const int64_t end = min(start + (int64_t)chunk, n_tri);
   if (start >= end) return;
   const int s0 = find_segment(tri_off, n_scenes, start);
   const int s1 = find_segment(tri_off, n_scenes, end - 1);
@@ -133,8 +170,9 @@ __device__ __forceinline__ uint32_t morton_of(const float *__restrict__ pos, con
 __global__ void __launch_bounds__(256)
     k_morton_hist(const float *__restrict__ pos, const int32_t *__restrict__ idx, int64_t n_tri,
                   const int64_t *__restrict__ tri_off, int n_scenes, const float *__restrict__ scene_box,
-                  uint32_t *__restrict__ keys, uint32_t *__restrict__ hist, int n_hist_passes) {
+                  uint32_t *__restrict__ keys, uint32_t *__restrict__ hist, int n_hist_passes, uint32_t *dirty) {
   __shared__ uint32_t s_hist[4][256];
+  if (blockIdx.x == 0 && threadIdx.x == 0) *dirty = 0u;
   for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) (&s_hist[0][0])[i] = 0u;
   __syncthreads();
   int s = -1;  // scene of t: t only grows, so it is searched once and then advanced
@@ -159,9 +197,10 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     k_morton_seg(const float *__restrict__ pos, const int32_t *__restrict__ idx, const int64_t *__restrict__ tri_off,
                  int n_scenes, const int32_t *__restrict__ tile_start, int tile, const float *__restrict__ scene_box,
-                 uint32_t *__restrict__ keys, uint32_t *__restrict__ hist) {
+                 uint32_t *__restrict__ keys, uint32_t *__restrict__ hist, uint32_t *dirty) {
   __shared__ uint32_t s_hist[4][256];
   __shared__ int s_scene;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *dirty = 0u;
   for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) (&s_hist[0][0])[i] = 0u;
   if (threadIdx.x == 0) s_scene = find_segment32(tile_start, n_scenes, (int32_t)blockIdx.x);
   __syncthreads();
@@ -181,27 +220,6 @@ __global__ void __launch_bounds__(256)
     const uint32_t c = (&s_hist[0][0])[i];
     if (c) atomicAdd(&h[i], c);
   }
-}
-
-// Exclusive scan of each scene's digit counts per pass, offset by the
-// scene's first position: the global start of every (scene, pass, digit)
-// bucket.  One block of 256 threads per (scene, pass).
-__global__ void k_scan_seg(const uint32_t *__restrict__ hist, const int64_t *__restrict__ tri_off,
-                           uint32_t *__restrict__ off) {
-  __shared__ uint32_t s_w[8];
-  const int sp = blockIdx.x, d = threadIdx.x, lane = d & 31, warp = d >> 5;
-  const uint32_t c = hist[(size_t)sp * 256 + d];
-  uint32_t x = c;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) s_w[warp] = x;
-  __syncthreads();
-  uint32_t pre = 0;
-  for (int w = 0; w < warp; ++w) pre += s_w[w];
-  off[(size_t)sp * 256 + d] = (uint32_t)tri_off[sp / 4] + pre + x - c;
 }
 
 // delta of radix_bvh.hpp:68-74 between neighbouring sorted positions i and
@@ -271,17 +289,14 @@ __device__ __forceinline__ bool slot_take(float4 *slot, float *lo, float *hi, in
 }
 
 // Sets every climb slot to the unset pattern and every arrival counter to 0
-// (at allocation, and before a build that follows one whose climb gave up).
-__global__ void k_climb_reset(float4 *slots, uint32_t *flags, int64_t n, const uint32_t *dirty) {
-  if (dirty && *dirty == 0u) return;
+// (at allocation).
+__global__ void k_climb_reset(float4 *slots, uint32_t *flags, int64_t n) {
   const float u = __int_as_float(kBoxUnset);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     slots[2 * i] = slots[2 * i + 1] = make_float4(u, u, u, u);
     flags[i] = 0u;
   }
 }
-
-__global__ void k_climb_clean(uint32_t *dirty) { *dirty = 0u; }
 
 // Karras tree construction fused with the bottom-up refit (radix_bvh.cpp:
 // 118-199), built from the leaves up (Apetrei 2014): a node covering sorted
@@ -437,51 +452,58 @@ int build_enqueue(flg_ctx ctx, flg_bvh b) {
   const int64_t n = b->n_tri;
   if (n <= 0) return FLG_OK;
   stage_mark(ctx, st, "start");
-  const unsigned fill_grid = grid_for(b->n_scenes, 128);
-  k_init_boxes<<<fill_grid, 128, 0, st>>>(b->d_scene_box, b->n_scenes);
-  FLG_LAUNCH_CHECK(ctx, "k_init_boxes");
-  if (b->builder == FLG_BUILDER_SAH) {
-    // Top-down from the scene bounds; no Morton codes or sort.
-    k_scene_bounds<<<grid_for(n, kBoundsChunk), kBoundsThreads, 0, st>>>(b->pos, b->idx, n, b->d_tri_off,
-                                                                       b->n_scenes, b->d_scene_box);
-    FLG_LAUNCH_CHECK(ctx, "k_scene_bounds");
-    stage_mark(ctx, st, "bounds");
-    int rc = sah_build(ctx, b);
-    if (rc) return rc;
-    if (b->width > 2) return collapse_enqueue(ctx, b, b->width, b->leaf_size);
-    return FLG_OK;
+  const bool sah = b->builder == FLG_BUILDER_SAH;  // top-down from the scene bounds: no codes, sort or climb
+  BuildSetup B = {};
+  B.box = b->d_scene_box;
+  B.n_scenes = b->n_scenes;
+  if (!sah) {
+    B.hist = b->d_tile_start ? b->d_shist : b->d_hist;
+    B.n_hist = b->d_tile_start ? 4 * 256 * (int64_t)b->n_scenes : 256 * (int64_t)b->n_morton_passes;
+    B.tile_ctr = b->d_tile_ctr;
+    B.n_ctr = b->n_passes;
+    B.lookback = (uint4 *)b->d_lookback;
+    B.n_lookback = 64 * b->n_tiles * b->n_passes;
+    B.scene_hist = b->d_hist + 256 * b->n_morton_passes;
+    B.scene_hist_init = b->d_hist + 256 * b->n_passes;
+    B.n_scene_hist = 256 * (b->n_passes - b->n_morton_passes);
+    B.slots = b->d_slots;
+    B.flags = b->d_flags;
+    B.n_nodes = b->n_nodes;
+    B.dirty = b->d_dirty;
   }
-  if (b->d_tile_start) {
-    FLG_CUDA(ctx, cudaMemsetAsync(b->d_shist, 0, sizeof(uint32_t) * 4 * 256 * (size_t)b->n_scenes, st));
-  } else {
-    FLG_CUDA(ctx, cudaMemsetAsync(b->d_hist, 0, sizeof(uint32_t) * 256 * b->n_morton_passes, st));
+  if (b->width > 2 && b->d_wide_ctr) {
+    B.wide_ctr = b->d_wide_ctr;
+    B.n_wide_ctr = collapse_ctr_words();
+    B.queue = b->d_queue[0];
+    B.queue_init = b->d_queue_init;
+    B.n_queue = b->n_wide_roots;
   }
-  if (b->n_passes > b->n_morton_passes)
-    FLG_CUDA(ctx, cudaMemcpyAsync(b->d_hist + 256 * b->n_morton_passes,
-                                  b->d_hist + 512 * b->n_passes,
-                                  sizeof(uint32_t) * 256 * (b->n_passes - b->n_morton_passes),
-                                  cudaMemcpyDeviceToDevice, st));
-  FLG_CUDA(ctx, cudaMemsetAsync(b->d_lookback, 0,
-                                sizeof(uint32_t) * 256 * (size_t)b->n_tiles * b->n_passes, st));
-  FLG_CUDA(ctx, cudaMemsetAsync(b->d_tile_ctr, 0, sizeof(uint32_t) * b->n_passes, st));
+  k_build_setup<<<grid_for(std::max<int64_t>(B.n_lookback, 6 * (int64_t)b->n_scenes), 256, (int64_t)ctx->num_sms * 8),
+                  256, 0, st>>>(B);
+  FLG_LAUNCH_CHECK(ctx, "k_build_setup");
   stage_mark(ctx, st, "setup");
-
-  k_scene_bounds<<<grid_for(n, kBoundsChunk), kBoundsThreads, 0, st>>>(b->pos, b->idx, n, b->d_tri_off,
-                                                                     b->n_scenes, b->d_scene_box);
+  const int chunk = (int)std::min<int64_t>(
+      kBoundsChunkMax, ceil_div(ceil_div(n, (int64_t)ctx->num_sms * 8), kBoundsThreads) * kBoundsThreads);
+  k_scene_bounds<<<grid_for(n, chunk), kBoundsThreads, 0, st>>>(b->pos, b->idx, n, b->d_tri_off, b->n_scenes, chunk,
+                                                              b->d_scene_box);
   FLG_LAUNCH_CHECK(ctx, "k_scene_bounds");
   stage_mark(ctx, st, "bounds");
+  if (sah) {
+    int rc = sah_build(ctx, b);
+    if (rc) return rc;
+    if (b->width > 2) return collapse_enqueue(ctx, b, b->width);
+    return FLG_OK;
+  }
   uint32_t *morton_out = (b->n_passes % 2 == 0) ? b->d_keys : b->d_keys_alt;
   if (b->d_tile_start) {
     k_morton_seg<<<(unsigned)b->n_tiles, 256, 0, st>>>(b->pos, b->idx, b->d_tri_off, b->n_scenes, b->d_tile_start,
-                                                      (int)sort_tile(), b->d_scene_box, morton_out, b->d_shist);
+                                                      (int)sort_tile(b->sort_items), b->d_scene_box, morton_out,
+                                                      b->d_shist, b->d_dirty);
     FLG_LAUNCH_CHECK(ctx, "k_morton_seg");
-    k_scan_seg<<<(unsigned)(4 * b->n_scenes), 256, 0, st>>>(b->d_shist, b->d_tri_off,
-                                                             b->d_shist + 4 * 256 * (size_t)b->n_scenes);
-    FLG_LAUNCH_CHECK(ctx, "k_scan_seg");
   } else {
     const unsigned g_elem = grid_for(n, 256, (int64_t)ctx->num_sms * 8);
     k_morton_hist<<<g_elem, 256, 0, st>>>(b->pos, b->idx, n, b->d_tri_off, b->n_scenes, b->d_scene_box,
-                                          morton_out, b->d_hist, b->n_morton_passes);
+                                          morton_out, b->d_hist, b->n_morton_passes, b->d_dirty);
     FLG_LAUNCH_CHECK(ctx, "k_morton_hist");
   }
   stage_mark(ctx, st, "morton");
@@ -491,7 +513,7 @@ int build_enqueue(flg_ctx ctx, flg_bvh b) {
     rc = ploc_build(ctx, b);
     if (rc) return rc;
     stage_mark(ctx, st, "ploc");
-    if (b->width > 2) return collapse_enqueue(ctx, b, b->width, b->leaf_size);
+    if (b->width > 2) return collapse_enqueue(ctx, b, b->width);
     return FLG_OK;
   }
   // Lanes take their next leaf as soon as they stop climbing, so one wave
@@ -501,12 +523,6 @@ int build_enqueue(flg_ctx ctx, flg_bvh b) {
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_climb, 256, 0) != cudaSuccess || v < 1) v = 1;
     return v;
   }();
-  const unsigned g_nodes = grid_for(b->n_nodes, 256, (int64_t)ctx->num_sms * 8);
-  k_climb_reset<<<g_nodes, 256, 0, st>>>(b->d_slots, b->d_flags, b->n_nodes, b->d_dirty);
-  FLG_LAUNCH_CHECK(ctx, "k_climb_reset");
-  k_climb_clean<<<1, 1, 0, st>>>(b->d_dirty);
-  FLG_LAUNCH_CHECK(ctx, "k_climb_clean");
-  stage_mark(ctx, st, "climb_reset");
   k_climb<<<grid_for(n, 256, (int64_t)ctx->num_sms * climb_per_sm), 256, 0, st>>>(
       b->pos, b->idx, n, b->d_tri_off, b->n_scenes, b->d_keys, b->d_perm, b->d_nodes2, b->d_flags, b->d_slots,
       b->d_tris, ctx->spin_limit, ctx->d_err, b->d_dirty);
@@ -516,7 +532,7 @@ int build_enqueue(flg_ctx ctx, flg_bvh b) {
     rc = treelet_build(ctx, b);
     if (rc) return rc;
   }
-  if (b->width > 2) return collapse_enqueue(ctx, b, b->width, b->leaf_size);
+  if (b->width > 2) return collapse_enqueue(ctx, b, b->width);
   return FLG_OK;
 }
 
@@ -576,16 +592,17 @@ static int bvh_create(flg_ctx ctx, const float *pos, const int32_t *idx, const i
   b->n_morton_passes = 4;
   int scene_passes = 0;
   if (n_scenes > 1) scene_passes = n_scenes <= 256 ? 1 : n_scenes <= 65536 ? 2 : 3;
-  b->n_tiles = sort_tiles(n);
+  b->sort_items = sort_items(ctx, n);
+  b->n_tiles = sort_tiles(n, b->sort_items);
   // Batched builds whose scenes average at least 4 sort tiles sort each
   // scene in its own run of tiles (per-scene digit offsets, look-back chains
   // restarting at each scene) instead of appending scene passes.
   std::vector<int32_t> tile_start;
-  if (n_scenes > 1 && n >= 4 * (int64_t)sort_tile() * n_scenes) {
+  if (n_scenes > 1 && n >= 4 * sort_tile(b->sort_items) * n_scenes) {
     tile_start.resize(n_scenes + 1);
     tile_start[0] = 0;
     for (int s = 0; s < n_scenes; ++s)
-      tile_start[s + 1] = tile_start[s] + (int32_t)sort_tiles(tri_off_host[s + 1] - tri_off_host[s]);
+      tile_start[s + 1] = tile_start[s] + (int32_t)sort_tiles(tri_off_host[s + 1] - tri_off_host[s], b->sort_items);
     b->n_tiles = tile_start[n_scenes];
     scene_passes = 0;
   }
@@ -608,11 +625,11 @@ static int bvh_create(flg_ctx ctx, const float *pos, const int32_t *idx, const i
   A(&b->d_dirty, 1);
   A(&b->d_nodes2, b->n_nodes);
   A(&b->d_tris, n);
-  // hist: [passes][256] counts, [passes][256] offsets, [passes][256] static scene counts
-  A(&b->d_hist, 3 * 256 * (size_t)b->n_passes);
+  // hist: [passes][256] counts, then the scene passes' static counts
+  A(&b->d_hist, 2 * 256 * (size_t)b->n_passes);
   if (!tile_start.empty()) {
     A(&b->d_tile_start, n_scenes + 1);
-    A(&b->d_shist, 2 * 4 * 256 * (size_t)n_scenes);  // per-scene counts, then bucket starts
+    A(&b->d_shist, 4 * 256 * (size_t)n_scenes);  // per-scene counts
   }
   A(&b->d_lookback, 256 * (size_t)b->n_tiles * b->n_passes);
   A(&b->d_tile_ctr, b->n_passes);
@@ -641,16 +658,16 @@ static int bvh_create(flg_ctx ctx, const float *pos, const int32_t *idx, const i
   if (e == cudaSuccess && !tile_start.empty())
     e = cudaMemcpyAsync(b->d_tile_start, tile_start.data(), sizeof(int32_t) * (n_scenes + 1),
                         cudaMemcpyHostToDevice, st);
-  // Static scene counts live after counts and offsets; build_enqueue copies
-  // the scene passes' part into place each build.
+  // Static scene counts live after the counts; every build's setup copies them
+  // into place.
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(b->d_hist + 512 * (size_t)b->n_passes, sh.data() + 256 * b->n_morton_passes,
+    e = cudaMemcpyAsync(b->d_hist + 256 * (size_t)b->n_passes, sh.data() + 256 * b->n_morton_passes,
                         sizeof(uint32_t) * 256 * (b->n_passes - b->n_morton_passes), cudaMemcpyHostToDevice, st);
   // Node records zeroed (unused slots hold refs 0), climb scratch unset.
   if (e == cudaSuccess && b->n_nodes > 0) e = cudaMemsetAsync(b->d_nodes2, 0, sizeof(Node2) * (size_t)b->n_nodes, st);
   if (e == cudaSuccess) {
     k_climb_reset<<<grid_for(b->n_nodes, 256, (int64_t)ctx->num_sms * 8), 256, 0, st>>>(b->d_slots, b->d_flags,
-                                                                                      b->n_nodes, nullptr);
+                                                                                      b->n_nodes);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemsetAsync(b->d_dirty, 0, sizeof(uint32_t), st);

@@ -1,7 +1,6 @@
 // collapse.cu — re-lays out a built Karras BVH2 as 4- or 8-wide nodes for
 // traversal.  Top-down, level by level (one cooperative launch with a grid
-// barrier between levels; one launch per level under stream capture): each
-// queued BVH2 node becomes a wide node whose children are found by
+// barrier between levels): each queued BVH2 node becomes a wide node whose children are found by
 // repeatedly opening the child with the largest surface area (Wald, Benthin,
 // Boulos 2008 style collapsing).
 // A BVH2 subtree covers a contiguous run of sorted triangles, so any subtree
@@ -18,6 +17,8 @@
 namespace flg {
 
 constexpr int kMaxLevels = 64;
+constexpr int kCollapseThreads = 128;
+constexpr int kCollapseNodes = 4;
 // 4-wide layouts hold leaf ranges of at most this many triangles, whatever
 // the handle's leaf_size: with quantised nodes a visit costs about as much as
 // a triangle test, and ranges of 1 / 2 / 3 / 4 traced 24 batched scenes in
@@ -26,26 +27,26 @@ constexpr int kMaxLevels = 64;
 // k_trace4's superset argument does not depend on the ranges, and retrace4 and
 // first_of_two form the exact tree with leaf_size.
 constexpr int kLeaf4 = 2;
-// Collapse counters: [0] wide nodes allocated, [1 + L] queue size of level L,
-// [kMaxLevels + 2 .. + 3] the one-launch collapse's barrier; the initial
-// values of these kCtrLive words follow as a static copy.
-constexpr int kCtrLive = kMaxLevels + 4;
+// Collapse counters: [0] wide nodes allocated, [1] its initial value, [2 .. 4]
+// the barrier; the initial values of these kCtrLive words follow as a static
+// copy.
+constexpr int kCtrLive = 5;
 
-// One wide node per queued BVH2 node of a level (cnt items in q_in).  The
-// new wide slots and queue entries of a warp are claimed with one atomic per
-// counter (warp prefix sum of the lanes' internal children): per-child
-// atomics on the two shared counters serialised in L2.  Queue entries are
-// read through L2 (__ldcg): in the one-launch collapse this SM may still
-// hold lines of the same buffer from two levels before.
+// One wide node per queued BVH2 node of a level (cnt items in q_in).  A warp
+// claims the slots of its new wide nodes with one atomic on node_ctr (prefix
+// sum of the lanes' internal children); the queue of the next level holds the
+// new nodes in slot order, so a node's place in it is its slot less the level's
+// first (q_base).  Claims by block cost more in barriers than they save (4 M
+// triangles: 230 against 220 us).  Queue entries are read through L2 (__ldcg):
+// this SM may still hold lines of the same buffer from two levels before.
 template <int W>
 __device__ __forceinline__ void collapse_level(const Node2 *__restrict__ nodes2, const Ranges &R, int leaf_size,
                                                const int2 *__restrict__ q_in, int cnt, int2 *__restrict__ q_out,
-                                               int32_t *q_out_count, int32_t *node_ctr, int64_t cap,
+                                               int q_base, int32_t *node_ctr, int64_t cap,
                                                typename WideRec<W>::T *__restrict__ wide, uint32_t *err) {
   const int lane = threadIdx.x & 31;
   // Warp-uniform loop: all lanes of a warp share it0.
-  for (int it0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) & ~31u); it0 < cnt;
-       it0 += gridDim.x * blockDim.x) {
+  for (int it0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) & ~31u); it0 < cnt; it0 += gridDim.x * blockDim.x) {
     const int it = it0 + lane;
     const bool valid = it < cnt;
     int2 item = make_int2(0, 0);
@@ -70,14 +71,9 @@ __device__ __forceinline__ void collapse_level(const Node2 *__restrict__ nodes2,
       const int v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
       if (lane >= o) incl += v;
     }
-    const int total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    int slot0 = 0, q0 = 0;
-    if (lane == 31 && total > 0) {
-      slot0 = atomicAdd(node_ctr, total);
-      q0 = atomicAdd(q_out_count, total);
-    }
+    int slot0 = 0;
+    if (lane == 31 && incl > 0) slot0 = atomicAdd(node_ctr, incl);
     slot0 = __shfl_sync(0xFFFFFFFFu, slot0, 31) + incl - need;
-    q0 = __shfl_sync(0xFFFFFFFFu, q0, 31) + incl - need;
     if (!valid || nc == 0) continue;
     int32_t child[W];
 #pragma unroll
@@ -87,13 +83,12 @@ __device__ __forceinline__ void collapse_level(const Node2 *__restrict__ nodes2,
         if (c[k].ref < 0 || c[k].count <= leaf_size) {
           child[k] = ~((c[k].first << 3) | (c[k].count - 1));
         } else {
-          const int slot = slot0++;
+          const int slot = slot0++, q = slot - q_base;
           if (slot >= cap) {
             atomicOr(err, kErrQueue);
-            if (q0 < cap) q_out[q0] = make_int2(-1, -1);  // the next level skips it
-            ++q0;
+            if (q < cap) q_out[q] = make_int2(-1, -1);  // the next level skips it
           } else {
-            q_out[q0++] = make_int2(c[k].ref, slot);
+            q_out[q] = make_int2(c[k].ref, slot);
             child[k] = slot;
           }
         }
@@ -133,28 +128,22 @@ __device__ __forceinline__ void collapse_level(const Node2 *__restrict__ nodes2,
   }
 }
 
-template <int W>
-__global__ void __launch_bounds__(128)
-    k_collapse_level(const Node2 *__restrict__ nodes2, Ranges R, int leaf_size,
-                     const int2 *__restrict__ q_in, const int32_t *__restrict__ q_in_count, int2 *__restrict__ q_out,
-                     int32_t *q_out_count, int32_t *node_ctr, int64_t cap, typename WideRec<W>::T *__restrict__ wide,
-                     uint32_t *err) {
-  // Counts beyond the queue capacity only arise from a corrupted tree.
-  const int cnt = (int)min((int64_t)*q_in_count, cap);
-  collapse_level<W>(nodes2, R, leaf_size, q_in, cnt, q_out, q_out_count, node_ctr, cap, wide, err);
-}
-
 // Barrier over all CTAs of a cooperative launch (all resident): bar[0]
 // counts arrivals, bar[1] is the generation.  Fences make each CTA's writes
 // of the level visible before it arrives and the others' after it leaves.
+// The last CTA to arrive notes *ctr in bar[2]; every thread returns that
+// value (the next barrier, which all have to reach first, replaces it).
 // The wait is bounded: on a timeout the error word is set and the CTA goes
 // on (the tree is then wrong, the device keeps answering).
-__device__ __forceinline__ void grid_barrier(uint32_t *bar, uint32_t limit, uint32_t *err) {
+__device__ __forceinline__ int grid_barrier(uint32_t *bar, const int32_t *ctr, uint32_t limit, uint32_t *err) {
+  __shared__ int s_now;
   __syncthreads();
   if (threadIdx.x == 0) {
     const uint32_t gen = ld_volatile(bar + 1);
     __threadfence();
     if (atomicAdd(bar, 1u) == gridDim.x - 1) {
+      __threadfence();
+      *(volatile uint32_t *)(bar + 2) = ld_volatile((const uint32_t *)ctr);
       *(volatile uint32_t *)bar = 0u;
       __threadfence();
       atomicAdd(bar + 1, 1u);
@@ -168,29 +157,29 @@ __device__ __forceinline__ void grid_barrier(uint32_t *bar, uint32_t limit, uint
       }
     }
     __threadfence();
+    s_now = (int)ld_volatile(bar + 2);
   }
   __syncthreads();
+  return s_now;
 }
 
 // The whole collapse in one cooperative launch: level after level with a
 // grid barrier between them, until a level is empty.  Replaces up to 64
 // launches (most of them empty) by one.
 template <int W>
-__global__ void __launch_bounds__(128)
-    k_collapse_all(const Node2 *__restrict__ nodes2, Ranges R, int leaf_size, int2 *q0, int2 *q1, int32_t *ctr,
-                   uint32_t *bar, int64_t cap, typename WideRec<W>::T *__restrict__ wide, uint32_t spin_limit, uint32_t *err) {
-  for (int L = 0; L < kMaxLevels; ++L) {
+__global__ void __launch_bounds__(kCollapseThreads)
+    k_collapse_all(const Node2 *__restrict__ nodes2, Ranges R, int leaf_size, int n_roots, int2 *q0, int2 *q1,
+                   int32_t *ctr, uint32_t *bar, int64_t cap, typename WideRec<W>::T *__restrict__ wide,
+                   uint32_t spin_limit, uint32_t *err) {
+  int cnt = n_roots, end = ctr[1];  // the level's queue; where its new nodes begin (ctr[0] moves on)
+  for (int L = 0; L < kMaxLevels && cnt > 0; ++L) {
+    collapse_level<W>(nodes2, R, leaf_size, (L & 1) ? q1 : q0, cnt, (L & 1) ? q0 : q1, end, ctr, cap, wide, err);
+    const int now = grid_barrier(bar, ctr, spin_limit, err);
     // Counts beyond the queue capacity only arise from a corrupted tree.
-    const int cnt = (int)min((int64_t)(int32_t)ld_volatile((const uint32_t *)(ctr + 1 + L)), cap);
-    if (cnt == 0) break;  // the same value in every CTA: read after the last barrier
-    collapse_level<W>(nodes2, R, leaf_size, (L & 1) ? q1 : q0, cnt, (L & 1) ? q0 : q1, ctr + 2 + L, ctr, cap, wide,
-                      err);
-    grid_barrier(bar, spin_limit, err);
+    cnt = (int)min((int64_t)(now - end), cap);
+    end = now;
   }
-}
-
-__global__ void k_collapse_check(const int32_t *last_count, uint32_t *err) {
-  if (*last_count > 0) atomicOr(err, kErrQueue);
+  if (blockIdx.x == 0 && threadIdx.x == 0 && cnt > 0) atomicOr(err, kErrQueue);  // deeper than kMaxLevels
 }
 
 int collapse_reserve(flg_ctx ctx, flg_bvh b) {
@@ -246,8 +235,7 @@ int collapse_reserve(flg_ctx ctx, flg_bvh b) {
   }
   b->n_wide_roots = (int32_t)q.size();
   std::vector<int32_t> ctr(2 * kCtrLive, 0);
-  ctr[0] = ctr[kCtrLive] = slots;
-  ctr[1] = ctr[kCtrLive + 1] = b->n_wide_roots;
+  ctr[0] = ctr[1] = ctr[kCtrLive] = ctr[kCtrLive + 1] = slots;
   cudaStream_t st = ctx->stream;
   cudaError_t e = cudaMemcpyAsync(b->d_wide_root, roots.data(), sizeof(int32_t) * b->n_scenes,
                                   cudaMemcpyHostToDevice, st);
@@ -269,62 +257,41 @@ static int collapse_levels(flg_ctx ctx, flg_bvh b) {
   Rec *wide = (Rec *)b->d_wide;
   const Ranges R{b->d_rfirst, b->d_rcount};
   const int leaf = W == 4 ? std::min<int>(b->leaf_size, kLeaf4) : b->leaf_size;
-  // Level sizes are only known on the device.  Default: one cooperative
-  // launch of one resident wave that walks the levels with a grid barrier in
-  // between and stops at the first empty one.  Under stream capture: one
-  // launch of one resident wave per level (the empty ones after the deepest
-  // exit at once).
-  static const int all_per_sm = [] {
+  // Level sizes are only known on the device: one cooperative launch walks the
+  // levels with a grid barrier in between.  A barrier costs by its CTAs, so a
+  // small tree takes fewer than a resident wave: one thread per kCollapseNodes
+  // nodes covers its widest levels.
+  static const int per_sm = [] {
     int v = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_collapse_all<W>, 128, 0) != cudaSuccess || v < 1)
-      v = 1;
-    return v;
-  }();
-  static const int level_per_sm = [] {
-    int v = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_collapse_level<W>, 128, 0) != cudaSuccess || v < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_collapse_all<W>, kCollapseThreads, 0) != cudaSuccess ||
+        v < 1)
       v = 1;
     return v;
   }();
   int32_t *ctr = b->d_wide_ctr;
-  if (!ctx->capturing) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ctx->num_sms * (unsigned)all_per_sm);
-    cfg.blockDim = dim3(128);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    uint32_t *bar = (uint32_t *)(ctr + kMaxLevels + 2);
-    FLG_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_collapse_all<W>, (const Node2 *)b->d_nodes2, R, leaf, b->d_queue[0],
-                                     b->d_queue[1], ctr, bar, (int64_t)b->wide_cap, wide, ctx->spin_limit,
-                                     ctx->d_err));
-    FLG_LAUNCH_CHECK(ctx, "k_collapse_all");
-  } else {
-    const unsigned grid = (unsigned)ctx->num_sms * (unsigned)level_per_sm;
-    for (int L = 0; L < kMaxLevels; ++L) {
-      k_collapse_level<W><<<grid, 128, 0, st>>>(b->d_nodes2, R, leaf, b->d_queue[L & 1], ctr + 1 + L,
-                                                b->d_queue[(L + 1) & 1], ctr + 2 + L, ctr, b->wide_cap, wide,
-                                                ctx->d_err);
-      FLG_LAUNCH_CHECK(ctx, "k_collapse_level");
-    }
-  }
-  k_collapse_check<<<1, 1, 0, st>>>(ctr + 1 + kMaxLevels, ctx->d_err);
-  FLG_LAUNCH_CHECK(ctx, "k_collapse_check");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid_for(ceil_div(b->n_nodes, kCollapseNodes), kCollapseThreads, (int64_t)ctx->num_sms * per_sm));
+  cfg.blockDim = dim3(kCollapseThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  FLG_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_collapse_all<W>, (const Node2 *)b->d_nodes2, R, leaf, (int)b->n_wide_roots,
+                                   b->d_queue[0], b->d_queue[1], ctr, (uint32_t *)(ctr + 2), (int64_t)b->wide_cap, wide,
+                                   ctx->spin_limit, ctx->d_err));
+  FLG_LAUNCH_CHECK(ctx, "k_collapse_all");
   return FLG_OK;
 }
 
-int collapse_enqueue(flg_ctx ctx, flg_bvh b, int width, int leaf_size) {
-  (void)leaf_size;
+int collapse_ctr_words() { return kCtrLive; }
+
+// Expects the counters and the first level's queue at their initial values
+// (k_build_setup, or flg_bvh_set_width's copies).
+int collapse_enqueue(flg_ctx ctx, flg_bvh b, int width) {
   if (b->n_wide_roots == 0) return FLG_OK;
   cudaStream_t st = ctx->stream;
-  FLG_CUDA(ctx, cudaMemcpyAsync(b->d_wide_ctr, b->d_wide_ctr + kCtrLive, sizeof(int32_t) * kCtrLive,
-                                cudaMemcpyDeviceToDevice, st));
-  FLG_CUDA(ctx, cudaMemcpyAsync(b->d_queue[0], b->d_queue_init, sizeof(int2) * b->n_wide_roots,
-                                cudaMemcpyDeviceToDevice, st));
   const int rc = width == 4 ? collapse_levels<4>(ctx, b) : collapse_levels<8>(ctx, b);
   if (rc == FLG_OK) stage_mark(ctx, st, "collapse");
   return rc;
@@ -350,5 +317,11 @@ FLG_API int flg_bvh_set_width(flg_ctx ctx, flg_bvh bvh, int32_t node_width, int3
     int rc = collapse_reserve(ctx, bvh);
     if (rc) return rc;
   }
-  return collapse_enqueue(ctx, bvh, node_width, leaf_size);
+  if (bvh->n_wide_roots > 0) {
+    FLG_CUDA(ctx, cudaMemcpyAsync(bvh->d_wide_ctr, bvh->d_wide_ctr + kCtrLive, sizeof(int32_t) * kCtrLive,
+                                  cudaMemcpyDeviceToDevice, ctx->stream));
+    FLG_CUDA(ctx, cudaMemcpyAsync(bvh->d_queue[0], bvh->d_queue_init, sizeof(int2) * bvh->n_wide_roots,
+                                  cudaMemcpyDeviceToDevice, ctx->stream));
+  }
+  return collapse_enqueue(ctx, bvh, node_width);
 }

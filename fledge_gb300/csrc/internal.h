@@ -140,13 +140,13 @@ struct flg_bvh_t {
   flg::Node2 *d_nodes2 = nullptr;
   flg::TriRec *d_tris = nullptr;
   // Sort scratch.
-  uint32_t *d_hist = nullptr;      // [passes][256] counts, then exclusive offsets
+  uint32_t *d_hist = nullptr;      // [passes][256] counts, then the scene passes' static counts
   uint32_t *d_lookback = nullptr;  // [passes][tiles][256]
   uint32_t *d_tile_ctr = nullptr;  // [passes]
-  int32_t n_passes = 0, n_morton_passes = 0;
+  int32_t n_passes = 0, n_morton_passes = 0, sort_items = 0;
   int64_t n_tiles = 0;
   // Segmented sorts: first sort tile of every scene (n_scenes + 1), per-scene
-  // digit counts [scene][pass][256] followed by the buckets' global starts.
+  // digit counts [scene][pass][256].
   int32_t *d_tile_start = nullptr;
   uint32_t *d_shist = nullptr;
   std::vector<uint32_t> scene_hist_h;  // scene-digit histograms (host)
@@ -288,10 +288,13 @@ inline unsigned grid_for(int64_t n, int threads, int64_t cap_blocks = 1 << 30) {
 // Defined in the build / trace translation units.
 int build_enqueue(flg_ctx ctx, flg_bvh b);
 int collapse_reserve(flg_ctx ctx, flg_bvh b);
-int collapse_enqueue(flg_ctx ctx, flg_bvh b, int width, int leaf_size);
+int collapse_enqueue(flg_ctx ctx, flg_bvh b, int width);
+int collapse_ctr_words();  // counters that a collapse starts from (d_wide_ctr, their values behind them)
 int sort_enqueue(flg_ctx ctx, flg_bvh b);
-int64_t sort_tiles(int64_t n);
-int64_t sort_tile();  // pairs per sort tile
+int sort_items(flg_ctx ctx, int64_t n);        // pairs per thread of a sort of n pairs
+int64_t sort_tile(int items);                  // pairs per sort tile
+int64_t sort_tiles(int64_t n, int items);
+constexpr int kSortItemsLarge = 12;            // the ray sort's
 int sort_pairs_enqueue(flg_ctx ctx, cudaStream_t st, int64_t n, int passes, uint32_t *const keys[2],
                        uint32_t *const vals[2], uint32_t *hist, uint32_t *lookback, uint32_t *tile_ctr);
 int ploc_reserve(flg_bvh b);

@@ -5,7 +5,8 @@
 // the sort is stable, so equal codes keep ascending original index.
 //
 // One launch per 8-bit digit.  Each CTA claims a tile of 3072 pairs (256
-// threads x 12) in launch order, ranks its keys with warp ballots and
+// threads x 12; 1024 pairs, 256 x 4, for arrays that would not give every SM a
+// tile) in launch order, ranks its keys with warp ballots and
 // shared-memory atomics, publishes its per-digit counts,
 // resolves its global offsets by looking back over earlier tiles, reorders
 // the tile in shared memory and writes runs of equal digits contiguously.
@@ -22,8 +23,8 @@ namespace flg {
 constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSortItems = 12;  // 12 x 4 CTAs per SM beat 8 / 16 items and 2 / 3 CTAs
+constexpr int kSortItemsSmall = 4;
 constexpr int kSortMinBlocks = 4;  // CTAs per SM the register budget allows
-constexpr int kSortTile = kSortThreads * kSortItems;
 constexpr int kRadix = 256;
 constexpr int kLookback = 4;  // predecessor tiles read per look-back step
 constexpr int kSceneStage = 2048;  // scene passes stage up to this many offsets in shared memory
@@ -57,18 +58,23 @@ __device__ __forceinline__ uint32_t sort_digit(uint32_t key, uint32_t val, int s
 // per (warp, digit); (4) publish the tile's counts and look back for the
 // global offsets; (5) scatter the pairs into shared memory in digit order
 // (one 8-byte store each) and write them out in runs of equal digits.
-template <bool kFirst, bool kScene>
+//
+// hist holds the digit counts of this pass (of every scene, scene_stride
+// apart, in a segmented sort); each CTA scans the 256 it needs beside its own
+// counts, which costs less than a launch to scan them once.
+template <bool kFirst, bool kScene, int kItems>
 __global__ void __launch_bounds__(kSortThreads, kSortMinBlocks)
     k_onesweep(const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
                uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, int64_t n, int shift,
-               const int64_t *__restrict__ tri_off, int n_scenes, const uint32_t *__restrict__ pass_off,
+               const int64_t *__restrict__ tri_off, int n_scenes, const uint32_t *__restrict__ hist,
                const int32_t *__restrict__ tile_start, int64_t scene_stride, uint32_t *lookback, uint32_t *tile_ctr,
                uint32_t *err, uint32_t spin_limit) {
-  __shared__ uint2 s_kv[kSortTile];
-  __shared__ uint8_t s_dig[kScene ? kSortTile : 1];
+  constexpr int kTile = kSortThreads * kItems;
+  __shared__ uint2 s_kv[kTile];
+  __shared__ uint8_t s_dig[kScene ? kTile : 1];
   __shared__ uint32_t s_whist[kSortWarps][kRadix];
   __shared__ int32_t s_glob[kRadix];
-  __shared__ uint32_t s_wsum[kSortWarps];
+  __shared__ uint32_t s_wsum[2][kSortWarps];
   __shared__ uint32_t s_tile;
   __shared__ int32_t s_off[kScene ? kSceneStage : 1];  // scene passes: the scene offsets
   __shared__ int32_t s_seg;                             // segmented sorts: the tile's scene
@@ -87,26 +93,39 @@ __global__ void __launch_bounds__(kSortThreads, kSortMinBlocks)
   // A segmented sort keeps every scene in its own run of tiles: the tile
   // covers part of [tri_off[s], tri_off[s+1]), the look-back stops at the
   // scene's first tile and the digit offsets are the scene's.
-  int64_t first_tile = 0, base = tile * kSortTile, seg_end = n;
+  int64_t first_tile = 0, base = tile * kTile, seg_end = n;
   if (tile_start) {
     const int sc = s_seg;
     first_tile = tile_start[sc];
-    base = tri_off[sc] + (tile - first_tile) * kSortTile;
+    base = tri_off[sc] + (tile - first_tile) * kTile;
     seg_end = tri_off[sc + 1];
-    pass_off += (size_t)sc * scene_stride;
+    hist += (size_t)sc * scene_stride;
   }
-  const bool full = base + kSortTile <= seg_end;
-  const int64_t wbase = base + (int64_t)warp * (kSortItems * 32) + lane;
+  // The pass's counts, scanned within each warp of digits; the warps' sums are
+  // added below.
+  {
+    const uint32_t c = hist[tid];
+    uint32_t x = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+      if (lane >= o) x += y;
+    }
+    s_glob[tid] = (int32_t)(x - c);
+    if (lane == 31) s_wsum[1][warp] = x;
+  }
+  const bool full = base + kTile <= seg_end;
+  const int64_t wbase = base + (int64_t)warp * (kItems * 32) + lane;
   // Pairs of this lane left in the input, as a 32-bit bound for the checks.
   const int64_t wrem64 = seg_end - wbase;
-  const int wrem = wrem64 > kSortTile ? kSortTile : (wrem64 < 0 ? 0 : (int)wrem64);
+  const int wrem = wrem64 > kTile ? kTile : (wrem64 < 0 ? 0 : (int)wrem64);
   const uint32_t *kin = keys_in + wbase;
   const uint32_t *vin = kFirst ? nullptr : vals_in + wbase;
 
-  uint32_t k[kSortItems], v[kSortItems], rank[kSortItems];
-  uint32_t dg[kScene ? kSortItems : 1];
+  uint32_t k[kItems], v[kItems], rank[kItems];
+  uint32_t dg[kScene ? kItems : 1];
 #pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
+  for (int j = 0; j < kItems; ++j) {
     const bool valid = full || j * 32 < wrem;
     k[j] = valid ? kin[j * 32] : 0xFFFFFFFFu;
     v[j] = valid ? (kFirst ? (uint32_t)wbase + (uint32_t)(j * 32) : vin[j * 32]) : 0u;
@@ -116,26 +135,26 @@ __global__ void __launch_bounds__(kSortThreads, kSortMinBlocks)
     // of fixed depth whose steps are interleaved over the thread's pairs
     // (largest s with off[s] <= value, as find_segment).
     if (staged) {
-      int sc[kScene ? kSortItems : 1];
+      int sc[kScene ? kItems : 1];
 #pragma unroll
-      for (int j = 0; j < kSortItems; ++j) sc[kScene ? j : 0] = 0;
+      for (int j = 0; j < kItems; ++j) sc[kScene ? j : 0] = 0;
       for (int step = n_scenes > 1 ? 1 << (31 - __clz(n_scenes - 1)) : 0; step >= 1; step >>= 1) {
 #pragma unroll
-        for (int j = 0; j < kSortItems; ++j) {
+        for (int j = 0; j < kItems; ++j) {
           const int c = sc[kScene ? j : 0] + step;
           if (c < n_scenes && s_off[kScene ? c : 0] <= (int32_t)v[j]) sc[kScene ? j : 0] = c;
         }
       }
 #pragma unroll
-      for (int j = 0; j < kSortItems; ++j) dg[kScene ? j : 0] = ((uint32_t)sc[kScene ? j : 0] >> shift) & 0xFFu;
+      for (int j = 0; j < kItems; ++j) dg[kScene ? j : 0] = ((uint32_t)sc[kScene ? j : 0] >> shift) & 0xFFu;
     } else {
 #pragma unroll
-      for (int j = 0; j < kSortItems; ++j) dg[kScene ? j : 0] = sort_digit<true>(k[j], v[j], shift, tri_off, n_scenes);
+      for (int j = 0; j < kItems; ++j) dg[kScene ? j : 0] = sort_digit<true>(k[j], v[j], shift, tri_off, n_scenes);
     }
   }
   const uint32_t lt = (1u << lane) - 1u;
 #pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
+  for (int j = 0; j < kItems; ++j) {
     const bool valid = full || j * 32 < wrem;
     const uint32_t d = !valid ? 256u : kScene ? dg[kScene ? j : 0] : ((k[j] >> shift) & 0xFFu);
     // Lanes holding the same digit: one ballot per digit bit (and one for
@@ -178,12 +197,12 @@ __global__ void __launch_bounds__(kSortThreads, kSortMinBlocks)
     uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
     if (lane >= o) x += y;
   }
-  if (lane == 31) s_wsum[warp] = x;
+  if (lane == 31) s_wsum[0][warp] = x;
   __syncthreads();
   uint32_t wpre = 0;
 #pragma unroll
   for (int w = 0; w < kSortWarps; ++w)
-    if (w < warp) wpre += s_wsum[w];
+    if (w < warp) wpre += s_wsum[0][w];
   const uint32_t tstart = wpre + x - tile_count;
 #pragma unroll
   for (int w = 0; w < kSortWarps; ++w) s_whist[w][d] += tstart;
@@ -221,11 +240,15 @@ __global__ void __launch_bounds__(kSortThreads, kSortMinBlocks)
     }
     st_volatile(lb + d, ((excl + tile_count) & kValMask) | kFlagPrefix);
   }
-  s_glob[d] = (int32_t)(pass_off[d] + excl) - (int32_t)tstart;
+  uint32_t bucket = (uint32_t)s_glob[d] + (tile_start ? (uint32_t)tri_off[s_seg] : 0u);
+#pragma unroll
+  for (int w = 0; w < kSortWarps; ++w)
+    if (w < warp) bucket += s_wsum[1][w];
+  s_glob[d] = (int32_t)(bucket + excl) - (int32_t)tstart;
   __syncthreads();
 
 #pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
+  for (int j = 0; j < kItems; ++j) {
     const uint32_t dj = kScene ? dg[kScene ? j : 0] : ((k[j] >> shift) & 0xFFu);
     if (full || j * 32 < wrem) {
       const uint32_t pos = s_whist[warp][dj] + rank[j];
@@ -235,7 +258,7 @@ __global__ void __launch_bounds__(kSortThreads, kSortMinBlocks)
   }
   __syncthreads();
   const int64_t rem = seg_end - base;
-  const int tile_valid = rem < kSortTile ? (int)rem : kSortTile;
+  const int tile_valid = rem < kTile ? (int)rem : kTile;
   for (int i = tid; i < tile_valid; i += kSortThreads) {
     const uint2 kv = s_kv[i];
     const uint32_t di = kScene ? (uint32_t)s_dig[kScene ? i : 0] : ((kv.x >> shift) & 0xFFu);
@@ -247,49 +270,28 @@ __global__ void __launch_bounds__(kSortThreads, kSortMinBlocks)
   }
 }
 
-// Launches one pass (the template pair for first / scene passes).
+// Launches one pass.
+template <int kItems>
 static void launch_pass(cudaStream_t st, unsigned grid, bool first, bool scene, const uint32_t *in_k,
                         const uint32_t *in_v, uint32_t *out_k, uint32_t *out_v, int64_t n, int shift,
-                        const int64_t *tri_off, int n_scenes, const uint32_t *pass_off, const int32_t *tile_start,
+                        const int64_t *tri_off, int n_scenes, const uint32_t *hist, const int32_t *tile_start,
                         int64_t scene_stride, uint32_t *lb, uint32_t *tile_ctr, uint32_t *err, uint32_t spin_limit) {
-  if (first && scene)
-    k_onesweep<true, true><<<grid, kSortThreads, 0, st>>>(in_k, in_v, out_k, out_v, n, shift, tri_off, n_scenes,
-                                                          pass_off, tile_start, scene_stride, lb, tile_ctr, err,
-                                                          spin_limit);
-  else if (first)
-    k_onesweep<true, false><<<grid, kSortThreads, 0, st>>>(in_k, in_v, out_k, out_v, n, shift, tri_off, n_scenes,
-                                                           pass_off, tile_start, scene_stride, lb, tile_ctr, err,
-                                                           spin_limit);
-  else if (scene)
-    k_onesweep<false, true><<<grid, kSortThreads, 0, st>>>(in_k, in_v, out_k, out_v, n, shift, tri_off, n_scenes,
-                                                           pass_off, tile_start, scene_stride, lb, tile_ctr, err,
-                                                           spin_limit);
-  else
-    k_onesweep<false, false><<<grid, kSortThreads, 0, st>>>(in_k, in_v, out_k, out_v, n, shift, tri_off, n_scenes,
-                                                            pass_off, tile_start, scene_stride, lb, tile_ctr, err,
-                                                            spin_limit);
+  auto *kern = first ? (scene ? k_onesweep<true, true, kItems> : k_onesweep<true, false, kItems>)
+                     : (scene ? k_onesweep<false, true, kItems> : k_onesweep<false, false, kItems>);
+  kern<<<grid, kSortThreads, 0, st>>>(in_k, in_v, out_k, out_v, n, shift, tri_off, n_scenes, hist, tile_start,
+                                      scene_stride, lb, tile_ctr, err, spin_limit);
 }
 
-// Exclusive scan of each pass's 256 digit counts (one block per pass).
-__global__ void k_scan_hist(const uint32_t *__restrict__ hist, uint32_t *__restrict__ off) {
-  __shared__ uint32_t s_w[8];
-  const int p = blockIdx.x, d = threadIdx.x, lane = d & 31, warp = d >> 5;
-  uint32_t c = hist[p * kRadix + d];
-  uint32_t x = c;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) s_w[warp] = x;
-  __syncthreads();
-  uint32_t pre = 0;
-  for (int w = 0; w < warp; ++w) pre += s_w[w];
-  off[p * kRadix + d] = pre + x - c;
+// Pairs per thread of a sort of n pairs: the large tile once it gives every SM
+// one.  Below that its CTAs are few and their phases long: the four passes
+// over 5,000 pairs take 58 us with the large tile and 33 with the small one,
+// over 20,001 59 and 41, over 400,000 73 and 66; over 600,000 76 and 77, over
+// 4,000,003 192 and 290 (three times the look-back words to write and read).
+int sort_items(flg_ctx ctx, int64_t n) {
+  return n >= (int64_t)ctx->num_sms * kSortThreads * kSortItems ? kSortItems : kSortItemsSmall;
 }
-
-int64_t sort_tiles(int64_t n) { return ceil_div(n, kSortTile); }
-int64_t sort_tile() { return kSortTile; }
+int64_t sort_tile(int items) { return (int64_t)kSortThreads * items; }
+int64_t sort_tiles(int64_t n, int items) { return ceil_div(n, sort_tile(items)); }
 
 // Enqueues the passes.  Expects: b->d_kbuf[0] holds the unsorted codes and
 // b->d_hist[0 .. n_morton_passes) the code histograms; the scene-pass
@@ -298,18 +300,9 @@ int64_t sort_tile() { return kSortTile; }
 int sort_enqueue(flg_ctx ctx, flg_bvh b) {
   const int64_t n = b->n_tri;
   if (n <= 0) return FLG_OK;
-  uint32_t *hist = b->d_hist;
-  uint32_t *off = b->d_hist + (size_t)b->n_passes * kRadix;
-  int64_t scene_stride = 0;
-  if (b->d_tile_start) {
-    // Segmented: the bucket starts are per scene ([scene][pass][digit], from
-    // k_scan_seg).
-    off = b->d_shist + 4 * kRadix * (size_t)b->n_scenes;
-    scene_stride = 4 * kRadix;
-  } else {
-    k_scan_hist<<<b->n_passes, kRadix, 0, ctx->stream>>>(hist, off);
-    FLG_LAUNCH_CHECK(ctx, "k_scan_hist");
-  }
+  // Segmented: the counts are per scene ([scene][pass][digit]).
+  const uint32_t *hist = b->d_tile_start ? b->d_shist : b->d_hist;
+  const int64_t scene_stride = b->d_tile_start ? 4 * kRadix : 0;
   const unsigned grid = (unsigned)b->n_tiles;
   // Ping-pong: pass p reads buffer (p & 1) and writes buffer ((p + 1) & 1).
   uint32_t *kb[2] = {b->n_passes % 2 == 0 ? b->d_keys : b->d_keys_alt,
@@ -322,9 +315,10 @@ int sort_enqueue(flg_ctx ctx, flg_bvh b) {
     uint32_t *lb = b->d_lookback + (size_t)p * b->n_tiles * kRadix;
     uint32_t *in_k = kb[p & 1], *out_k = kb[(p + 1) & 1];
     uint32_t *in_v = vb[p & 1], *out_v = vb[(p + 1) & 1];
-    launch_pass(ctx->stream, grid, p == 0, scene_pass, in_k, in_v, out_k, out_v, n, shift, b->d_tri_off, b->n_scenes,
-                off + (size_t)p * kRadix, b->d_tile_start, scene_stride, lb, b->d_tile_ctr + p, ctx->d_err,
-                ctx->spin_limit);
+    auto *launch = b->sort_items == kSortItems ? launch_pass<kSortItems> : launch_pass<kSortItemsSmall>;
+    launch(ctx->stream, grid, p == 0, scene_pass, in_k, in_v, out_k, out_v, n, shift, b->d_tri_off, b->n_scenes,
+           hist + (size_t)p * kRadix, b->d_tile_start, scene_stride, lb, b->d_tile_ctr + p, ctx->d_err,
+           ctx->spin_limit);
     FLG_LAUNCH_CHECK(ctx, "k_onesweep");
     stage_mark(ctx, ctx->stream, scene_pass ? "sort_scene_pass" : "sort_pass");
   }
@@ -334,21 +328,19 @@ int sort_enqueue(flg_ctx ctx, flg_bvh b) {
 // Generic (key, index) sort used by the ray sort: keys[0] holds n keys and
 // hist[0 .. passes) their per-pass digit counts; the sorted keys and the
 // original indices end in keys[passes & 1] / vals[passes & 1].  hist needs
-// 2 * passes * 256 words, lookback passes * tiles * 256, tile_ctr passes.
+// passes * 256 words, lookback passes * tiles * 256 (sort_tiles of the large
+// tile), tile_ctr passes.
 int sort_pairs_enqueue(flg_ctx ctx, cudaStream_t st, int64_t n, int passes, uint32_t *const keys[2],
                        uint32_t *const vals[2], uint32_t *hist, uint32_t *lookback, uint32_t *tile_ctr) {
   if (n <= 0) return FLG_OK;
-  const int64_t tiles = sort_tiles(n);
-  uint32_t *off = hist + (size_t)passes * kRadix;
+  const int64_t tiles = sort_tiles(n, kSortItems);
   FLG_CUDA(ctx, cudaMemsetAsync(lookback, 0, sizeof(uint32_t) * kRadix * (size_t)tiles * passes, st));
   FLG_CUDA(ctx, cudaMemsetAsync(tile_ctr, 0, sizeof(uint32_t) * passes, st));
-  k_scan_hist<<<passes, kRadix, 0, st>>>(hist, off);
-  FLG_LAUNCH_CHECK(ctx, "k_scan_hist");
   for (int p = 0; p < passes; ++p) {
     uint32_t *lb = lookback + (size_t)p * tiles * kRadix;
-    launch_pass(st, (unsigned)tiles, p == 0, false, keys[p & 1], vals[p & 1], keys[(p + 1) & 1], vals[(p + 1) & 1], n,
-                8 * p, nullptr, 1, off + (size_t)p * kRadix, nullptr, 0, lb, tile_ctr + p, ctx->d_err,
-                ctx->spin_limit);
+    launch_pass<kSortItems>(st, (unsigned)tiles, p == 0, false, keys[p & 1], vals[p & 1], keys[(p + 1) & 1],
+                            vals[(p + 1) & 1], n, 8 * p, nullptr, 1, hist + (size_t)p * kRadix, nullptr, 0, lb,
+                            tile_ctr + p, ctx->d_err, ctx->spin_limit);
     FLG_LAUNCH_CHECK(ctx, "k_onesweep");
     stage_mark(ctx, st, "ray_sort_pass");
   }

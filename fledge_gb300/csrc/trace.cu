@@ -768,57 +768,15 @@ __device__ __forceinline__ void tri_rec_box(const TriRec *__restrict__ tris, int
   tri_box(make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z), make_float3(c.x, c.y, c.z), lo, hi);
 }
 
-// A child of a wide node on the walk of first_of_two: as Cand, but with the
-// record that holds its box (4-wide: BVH2 node x 2 + side) for the box.
-struct WalkCand {
-  int32_t ref, first, count, box;
-  float area;
-};
-__device__ __forceinline__ void walk_cands(const Exact4 &X, int32_t node, WalkCand &a, WalkCand &b) {
-  const float4 *np = (const float4 *)(X.nodes2 + node);
-  Node2 nd;
-  nd.a = __ldg(np);
-  nd.b = __ldg(np + 1);
-  nd.c = __ldg(np + 2);
-  nd.d = __ldg((const int4 *)(np + 3));
-  Cand c, e;
-  child_cands(nd, X.R, c, e);
-  a = WalkCand{c.ref, c.first, c.count, 2 * node, half_area(c)};
-  b = WalkCand{e.ref, e.first, e.count, 2 * node + 1, half_area(e)};
-}
-
 // Which of two sorted positions of a scene the exact traversal of a ray tests
 // first: at the wide node where their paths part, the child that is entered
-// first; within a leaf range, the lower one.  Walks down from the root,
-// forming each wide node's children as open_wide does.
+// first; within a leaf range, the lower one.
 __device__ __noinline__ int32_t first_of_two(const Exact4 &X, const RaySoA &RS, int64_t ray, int32_t p, int32_t q) {
   int32_t cur = scene_root(X.roots, X.ray_off, X.n_scenes, ray);
   for (int level = 0; cur >= 0 && level < 4096; ++level) {
     WalkCand c[4];
-    int nc = 2;
-    walk_cands(X, cur, c[0], c[1]);
-    while (nc < 4) {
-      int best = -1;
-      float ba = -1.0f;
-      int32_t r = 0;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (k < nc && c[k].ref >= 0 && c[k].count > X.leaf_size && c[k].area > ba) {
-          ba = c[k].area;
-          best = k;
-          r = c[k].ref;
-        }
-      }
-      if (best < 0) break;
-      WalkCand a, b;
-      walk_cands(X, r, a, b);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (k == best) c[k] = a;
-        if (k == nc) c[k] = b;
-      }
-      ++nc;
-    }
+    int nc;
+    walk_open(X.nodes2, X.R, X.leaf_size, cur, c, nc);
     int32_t next = INT32_MIN, bp = -1, bq = -1, sp = 0, sq = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -840,9 +798,8 @@ __device__ __noinline__ int32_t first_of_two(const Exact4 &X, const RaySoA &RS, 
       float tmin, tmax;
       load_ray(RS, ray, o, d, inv, tmin, tmax);
       auto key = [&](int32_t box, int slot) {
-        const Node2 &nd = X.nodes2[box >> 1];
-        const float4 ab = (box & 1) ? nd.b : nd.a;
-        const float lo[3] = {ab.x, ab.z, (box & 1) ? nd.c.z : nd.c.x}, hi[3] = {ab.y, ab.w, (box & 1) ? nd.c.w : nd.c.y};
+        float lo[3], hi[3];
+        walk_box(X.nodes2, box, lo, hi);
         return (__float_as_uint(slab_exact(lo, hi, o, inv, 3.402823466e+38f)) & 0x7FFFFFFCu) | (uint32_t)slot;
       };
       return key(bp, sp) < key(bq, sq) ? p : q;
@@ -1761,7 +1718,7 @@ int trace_enqueue(flg_ctx ctx, cudaStream_t st, int set, flg_bvh b, const flg_ra
   if (op.ray_sort) {
     // Scratch: keys and indices (2 x 2), digit counts and offsets, look-back,
     // tile counters, the sorted rays (8 arrays) and their hits (4 arrays).
-    const int64_t tiles = sort_tiles(n);
+    const int64_t tiles = sort_tiles(n, kSortItemsLarge);
     const size_t w = (size_t)n * 4;
     const size_t need = 4 * w + 2 * 4 * 256 * 4 + (size_t)4 * tiles * 256 * 4 + 64 + 8 * w + 4 * w + 16 * 256;
     if (ctx->rs_bytes < need) {

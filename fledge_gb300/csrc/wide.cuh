@@ -103,6 +103,85 @@ __device__ __forceinline__ void open_wide(const Node2 *__restrict__ nodes2, cons
   }
 }
 
+// A child of a 4-wide node by what chooses it: as Cand, with its area and the
+// place of its box (BVH2 node x 2 + side) instead of the box, which keeps the
+// choice of four children in half the registers.
+struct WalkCand {
+  int32_t ref, first, count, box;
+  float area;
+};
+
+__device__ __forceinline__ void walk_cands(const Node2 *__restrict__ nodes2, const Ranges &R, int32_t node,
+                                           WalkCand &a, WalkCand &b) {
+  const float4 *np = (const float4 *)(nodes2 + node);
+  Node2 nd;
+  nd.a = __ldg(np);
+  nd.b = __ldg(np + 1);
+  nd.c = __ldg(np + 2);
+  nd.d = __ldg((const int4 *)(np + 3));
+  Cand c, e;
+  child_cands(nd, R, c, e);
+  a = WalkCand{c.ref, c.first, c.count, 2 * node, half_area(c)};
+  b = WalkCand{e.ref, e.first, e.count, 2 * node + 1, half_area(e)};
+}
+
+// Box of a WalkCand.
+__device__ __forceinline__ void walk_box(const Node2 *__restrict__ nodes2, int32_t box, float *lo, float *hi) {
+  const float4 *np = (const float4 *)(nodes2 + (box >> 1));
+  const float4 ab = __ldg(np + (box & 1));
+  const float2 z = __ldg((const float2 *)(np + 2) + (box & 1));
+  lo[0] = ab.x;
+  hi[0] = ab.y;
+  lo[1] = ab.z;
+  hi[1] = ab.w;
+  lo[2] = z.x;
+  hi[2] = z.y;
+}
+
+// The children of a 4-wide node, as open_wide<4> picks them.  The records of
+// both children of `node` that may be opened are read at once: the first
+// opening takes one of them and the second usually the other.
+__device__ __forceinline__ void walk_open(const Node2 *__restrict__ nodes2, const Ranges &R, int leaf_size,
+                                          int32_t node, WalkCand (&c)[4], int &nc) {
+  nc = 2;
+  walk_cands(nodes2, R, node, c[0], c[1]);
+  const int32_t r0 = c[0].ref >= 0 && c[0].count > leaf_size ? c[0].ref : -1;
+  const int32_t r1 = c[1].ref >= 0 && c[1].count > leaf_size ? c[1].ref : -1;
+  WalkCand g0[2], g1[2];
+  if (r0 >= 0) walk_cands(nodes2, R, r0, g0[0], g0[1]);
+  if (r1 >= 0) walk_cands(nodes2, R, r1, g1[0], g1[1]);
+  while (nc < 4) {
+    int best = -1;
+    float ba = -1.0f;
+    int32_t r = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k < nc && c[k].ref >= 0 && c[k].count > leaf_size && c[k].area > ba) {
+        ba = c[k].area;
+        best = k;
+        r = c[k].ref;
+      }
+    }
+    if (best < 0) break;
+    WalkCand a, b;
+    if (r == r0) {
+      a = g0[0];
+      b = g0[1];
+    } else if (r == r1) {
+      a = g1[0];
+      b = g1[1];
+    } else {
+      walk_cands(nodes2, R, r, a, b);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k == best) c[k] = a;
+      if (k == nc) c[k] = b;
+    }
+    ++nc;
+  }
+}
+
 // Quantises the children's boxes of a 4-wide node (NodeQ): per axis an origin
 // and a power-of-two step; every child's lower plane rounds down and its
 // upper plane up, both with at least 1/64 step to spare.  The slack covers
