@@ -23,6 +23,7 @@ __global__ void __launch_bounds__(256)
                   int64_t n, const int32_t *__restrict__ prim, const float *__restrict__ hu,
                   const float *__restrict__ hv, const float *__restrict__ gt, const float *__restrict__ gu,
                   const float *__restrict__ gv, float *__restrict__ grad) {
+  after_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int32_t p = prim[i];
@@ -78,9 +79,8 @@ FLG_API int flg_hit_adjoint(flg_ctx ctx, const float *pos, const int32_t *idx, i
   if (!pos || !dL_dpos || !rays->dx || !rays->dy || !rays->dz || !hits->prim || !hits->u || !hits->v)
     return set_error(ctx, FLG_ERR_ARG, "NULL pointer");
   if (!idx && n_vert != 3 * n_tri) return set_error(ctx, FLG_ERR_ARG, "soup needs n_vert == 3*n_tri");
-  k_hit_adjoint<<<(unsigned)ceil_div(n, 256), 256, 0, ctx->stream>>>(pos, idx, n_tri, rays->dx, rays->dy, rays->dz,
-                                                                      n, hits->prim, hits->u, hits->v, dL_dt, dL_du,
-                                                                      dL_dv, dL_dpos);
+  FLG_CUDA(ctx, launch_after(k_hit_adjoint, (unsigned)ceil_div(n, 256), 256, ctx->stream, pos, idx, n_tri, rays->dx,
+                             rays->dy, rays->dz, n, hits->prim, hits->u, hits->v, dL_dt, dL_du, dL_dv, dL_dpos));
   FLG_LAUNCH_CHECK(ctx, "k_hit_adjoint");
   return FLG_OK;
 }

@@ -75,6 +75,7 @@ struct BuildSetup {
 };
 
 __global__ void __launch_bounds__(256) k_build_setup(BuildSetup B) {
+  after_wait();
   const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = t0; i < 6 * (int64_t)B.n_scenes; i += step)
     B.box[i] = i % 6 < 3 ? 3.402823466e+38f : -3.402823466e+38f;
@@ -102,6 +103,7 @@ __global__ void __launch_bounds__(kBoundsThreads)
     k_scene_bounds(const float *__restrict__ pos, const int32_t *__restrict__ idx, int64_t n_tri,
                    const int64_t *__restrict__ tri_off, int n_scenes, int chunk, float *scene_box) {
   __shared__ float s_red[6][kBoundsThreads / 32];
+  after_wait();
   const int64_t start = (int64_t)blockIdx.x * chunk;
   const int64_t end = min(start + (int64_t)chunk, n_tri);
   if (start >= end) return;
@@ -172,6 +174,7 @@ __global__ void __launch_bounds__(256)
                   const int64_t *__restrict__ tri_off, int n_scenes, const float *__restrict__ scene_box,
                   uint32_t *__restrict__ keys, uint32_t *__restrict__ hist, int n_hist_passes, uint32_t *dirty) {
   __shared__ uint32_t s_hist[4][256];
+  after_wait();
   if (blockIdx.x == 0 && threadIdx.x == 0) *dirty = 0u;
   for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) (&s_hist[0][0])[i] = 0u;
   __syncthreads();
@@ -200,6 +203,7 @@ __global__ void __launch_bounds__(256)
                  uint32_t *__restrict__ keys, uint32_t *__restrict__ hist, uint32_t *dirty) {
   __shared__ uint32_t s_hist[4][256];
   __shared__ int s_scene;
+  after_wait();
   if (blockIdx.x == 0 && threadIdx.x == 0) *dirty = 0u;
   for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) (&s_hist[0][0])[i] = 0u;
   if (threadIdx.x == 0) s_scene = find_segment32(tile_start, n_scenes, (int32_t)blockIdx.x);
@@ -325,6 +329,7 @@ __global__ void __launch_bounds__(256)
             const int64_t *__restrict__ tri_off, int n_scenes, const uint32_t *__restrict__ keys,
             const uint32_t *__restrict__ perm, Node2 *__restrict__ nodes, uint32_t *flags, float4 *slots,
             TriRec *__restrict__ tris, uint32_t spin_limit, uint32_t *err, uint32_t *dirty) {
+  after_wait();
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt = (1u << lane) - 1u;
   const int64_t n_warps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -478,14 +483,16 @@ int build_enqueue(flg_ctx ctx, flg_bvh b) {
     B.queue_init = b->d_queue_init;
     B.n_queue = b->n_wide_roots;
   }
-  k_build_setup<<<grid_for(std::max<int64_t>(B.n_lookback, 6 * (int64_t)b->n_scenes), 256, (int64_t)ctx->num_sms * 8),
-                  256, 0, st>>>(B);
+  FLG_CUDA(ctx, launch_after(k_build_setup,
+                             grid_for(std::max<int64_t>(B.n_lookback, 6 * (int64_t)b->n_scenes), 256,
+                                      (int64_t)ctx->num_sms * 8),
+                             256, st, B));
   FLG_LAUNCH_CHECK(ctx, "k_build_setup");
   stage_mark(ctx, st, "setup");
   const int chunk = (int)std::min<int64_t>(
       kBoundsChunkMax, ceil_div(ceil_div(n, (int64_t)ctx->num_sms * 8), kBoundsThreads) * kBoundsThreads);
-  k_scene_bounds<<<grid_for(n, chunk), kBoundsThreads, 0, st>>>(b->pos, b->idx, n, b->d_tri_off, b->n_scenes, chunk,
-                                                              b->d_scene_box);
+  FLG_CUDA(ctx, launch_after(k_scene_bounds, grid_for(n, chunk), kBoundsThreads, st, b->pos, b->idx, n, b->d_tri_off,
+                             b->n_scenes, chunk, b->d_scene_box));
   FLG_LAUNCH_CHECK(ctx, "k_scene_bounds");
   stage_mark(ctx, st, "bounds");
   if (sah) {
@@ -496,14 +503,14 @@ int build_enqueue(flg_ctx ctx, flg_bvh b) {
   }
   uint32_t *morton_out = (b->n_passes % 2 == 0) ? b->d_keys : b->d_keys_alt;
   if (b->d_tile_start) {
-    k_morton_seg<<<(unsigned)b->n_tiles, 256, 0, st>>>(b->pos, b->idx, b->d_tri_off, b->n_scenes, b->d_tile_start,
-                                                      (int)sort_tile(b->sort_items), b->d_scene_box, morton_out,
-                                                      b->d_shist, b->d_dirty);
+    FLG_CUDA(ctx, launch_after(k_morton_seg, (unsigned)b->n_tiles, 256, st, b->pos, b->idx, b->d_tri_off, b->n_scenes,
+                               b->d_tile_start, (int)sort_tile(b->sort_items), b->d_scene_box, morton_out, b->d_shist,
+                               b->d_dirty));
     FLG_LAUNCH_CHECK(ctx, "k_morton_seg");
   } else {
     const unsigned g_elem = grid_for(n, 256, (int64_t)ctx->num_sms * 8);
-    k_morton_hist<<<g_elem, 256, 0, st>>>(b->pos, b->idx, n, b->d_tri_off, b->n_scenes, b->d_scene_box,
-                                          morton_out, b->d_hist, b->n_morton_passes, b->d_dirty);
+    FLG_CUDA(ctx, launch_after(k_morton_hist, g_elem, 256, st, b->pos, b->idx, n, b->d_tri_off, b->n_scenes,
+                               b->d_scene_box, morton_out, b->d_hist, b->n_morton_passes, b->d_dirty));
     FLG_LAUNCH_CHECK(ctx, "k_morton_hist");
   }
   stage_mark(ctx, st, "morton");
@@ -523,9 +530,9 @@ int build_enqueue(flg_ctx ctx, flg_bvh b) {
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_climb, 256, 0) != cudaSuccess || v < 1) v = 1;
     return v;
   }();
-  k_climb<<<grid_for(n, 256, (int64_t)ctx->num_sms * climb_per_sm), 256, 0, st>>>(
-      b->pos, b->idx, n, b->d_tri_off, b->n_scenes, b->d_keys, b->d_perm, b->d_nodes2, b->d_flags, b->d_slots,
-      b->d_tris, ctx->spin_limit, ctx->d_err, b->d_dirty);
+  FLG_CUDA(ctx, launch_after(k_climb, grid_for(n, 256, (int64_t)ctx->num_sms * climb_per_sm), 256, st, b->pos, b->idx, n,
+                             b->d_tri_off, b->n_scenes, b->d_keys, b->d_perm, b->d_nodes2, b->d_flags, b->d_slots,
+                             b->d_tris, ctx->spin_limit, ctx->d_err, b->d_dirty));
   FLG_LAUNCH_CHECK(ctx, "k_climb");
   stage_mark(ctx, st, "climb");
   if (b->builder == FLG_BUILDER_TREELET) {

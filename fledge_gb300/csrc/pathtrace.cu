@@ -182,6 +182,7 @@ struct PtQueues {
 };
 
 __global__ void k_pt_camera(PtScene S, Halton H, int s0, int n_path, PtQueues Q, int qa) {
+  after_wait();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n_path) return;
   const int i = p % Q.n_pix, s = s0 + p / Q.n_pix;
@@ -244,6 +245,7 @@ __device__ __forceinline__ int queue_slot(bool want, int32_t *counter) {
 __global__ void __launch_bounds__(256, 4)
     k_pt_shade(PtScene S, Halton H, int s0, int depth, int64_t n_in, PtQueues Q, int qa, const int32_t *__restrict__ prim,
                const float *__restrict__ th, const float *__restrict__ uh, const float *__restrict__ vh) {
+  after_wait();
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = q < n_in;
   const int qb = qa ^ 1;
@@ -459,6 +461,7 @@ __global__ void __launch_bounds__(256, 4)
 // from an offset origin.  Contributions carry the transmittance so far.
 __global__ void k_pt_shadow_step(PtScene S, int64_t n, const int32_t *__restrict__ prim, const float *__restrict__ th,
                                  PtQueues Q, int in) {
+  after_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = i < n;
   float *const *sx = in == 0 ? Q.sx : Q.sx2;
@@ -522,6 +525,7 @@ __global__ void k_pt_shadow_step(PtScene S, int64_t n, const int32_t *__restrict
 // ratio-tracking transmittance of the shadow segment (VolEstimateTr,
 // integrator.cpp:40-66).
 __global__ void k_pt_shadow(PtScene S, int s0, int depth, int64_t n, const uint8_t *__restrict__ occ, PtQueues Q) {
+  after_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n || occ[i]) return;
   const int pid = Q.spath[i];
@@ -548,6 +552,7 @@ __global__ void k_pt_shadow(PtScene S, int s0, int depth, int64_t n, const uint8
 // Adds the wavefront's K samples of every pixel to the image, in sample
 // order (a fixed summation order: the image does not depend on scheduling).
 __global__ void k_pt_reduce(const float *__restrict__ rad, int n_pix, int k_samples, float *radiance) {
+  after_wait();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;  // pixel * 3 + channel
   if (e >= 3 * (int64_t)n_pix) return;
   float acc = radiance[e];
@@ -753,7 +758,7 @@ static int pathtrace_run(flg_ctx ctx, flg_bvh bvh, flg_grid grid, const flg_mesh
     const int k = s0 == 0 ? 1 : (int)std::min<int64_t>(kmax, spp - s0);
     const int64_t n_path = (int64_t)k * n;
     int qa = 0;
-    k_pt_camera<<<(unsigned)ceil_div(n_path, 256), 256, 0, st>>>(S, H, s0, (int)n_path, Q, qa);
+    FLG_CUDA(ctx, launch_after(k_pt_camera, (unsigned)ceil_div(n_path, 256), 256, st, S, H, s0, (int)n_path, Q, qa));
     FLG_LAUNCH_CHECK(ctx, "k_pt_camera");
     int64_t n_a = n_path;
     // Without interfaces an iteration is a bounce; with them a path may pass
@@ -769,8 +774,8 @@ static int pathtrace_run(flg_ctx ctx, flg_bvh bvh, flg_grid grid, const flg_mesh
       if (rc) return rc;
       n_closest += n_a;
       FLG_CUDA(ctx, cudaMemsetAsync(Q.counts, 0, 2 * sizeof(int32_t), st));
-      k_pt_shade<<<(unsigned)ceil_div(n_a, 256), 256, 0, st>>>(S, H, s0, depth, n_a, Q, qa, hh.prim, hh.t, hh.u,
-                                                                hh.v);
+      FLG_CUDA(ctx, launch_after(k_pt_shade, (unsigned)ceil_div(n_a, 256), 256, st, S, H, s0, depth, n_a, Q, qa, hh.prim,
+                                 hh.t, hh.u, hh.v));
       FLG_LAUNCH_CHECK(ctx, "k_pt_shade");
       FLG_CUDA(ctx, cudaMemcpyAsync(counts, Q.counts, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
       FLG_CUDA(ctx, cudaStreamSynchronize(st));
@@ -787,7 +792,7 @@ static int pathtrace_run(flg_ctx ctx, flg_bvh bvh, flg_grid grid, const flg_mesh
           if (rc) return rc;
           n_shadow += n_s;
           FLG_CUDA(ctx, cudaMemsetAsync(Q.counts + 2, 0, sizeof(int32_t), st));
-          k_pt_shadow_step<<<(unsigned)ceil_div(n_s, 256), 256, 0, st>>>(S, n_s, sh.prim, sh.t, Q, in);
+          FLG_CUDA(ctx, launch_after(k_pt_shadow_step, (unsigned)ceil_div(n_s, 256), 256, st, S, n_s, sh.prim, sh.t, Q, in));
           FLG_LAUNCH_CHECK(ctx, "k_pt_shadow_step");
           int32_t nn = 0;
           FLG_CUDA(ctx, cudaMemcpyAsync(&nn, Q.counts + 2, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
@@ -799,13 +804,14 @@ static int pathtrace_run(flg_ctx ctx, flg_bvh bvh, flg_grid grid, const flg_mesh
         rc = trace_enqueue(ctx, st, 0, bvh, &sr, counts[1], opts, nullptr, 1, nullptr, occ);
         if (rc) return rc;
         n_shadow += counts[1];
-        k_pt_shadow<<<(unsigned)ceil_div(counts[1], 256), 256, 0, st>>>(S, s0, depth, counts[1], occ, Q);
+        FLG_CUDA(ctx, launch_after(k_pt_shadow, (unsigned)ceil_div(counts[1], 256), 256, st, S, s0, depth,
+                                   (int64_t)counts[1], occ, Q));
         FLG_LAUNCH_CHECK(ctx, "k_pt_shadow");
       }
       n_a = counts[0];
       qa ^= 1;
     }
-    k_pt_reduce<<<(unsigned)ceil_div(3 * n, 256), 256, 0, st>>>(Q.rad, (int)n, k, radiance);
+    FLG_CUDA(ctx, launch_after(k_pt_reduce, (unsigned)ceil_div(3 * n, 256), 256, st, Q.rad, (int)n, k, radiance));
     FLG_LAUNCH_CHECK(ctx, "k_pt_reduce");
     s0 += k;
   }

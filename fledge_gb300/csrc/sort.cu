@@ -80,11 +80,12 @@ __global__ void __launch_bounds__(kSortThreads, kSortMinBlocks)
   __shared__ int32_t s_seg;                             // segmented sorts: the tile's scene
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int i = tid; i < kSortWarps * kRadix; i += kSortThreads) (&s_whist[0][0])[i] = 0u;
+  after_wait();
   if (tid == 0) {
     s_tile = atomicAdd(tile_ctr, 1u);
     if (tile_start) s_seg = find_segment32(tile_start, n_scenes, (int32_t)s_tile);
   }
-  for (int i = tid; i < kSortWarps * kRadix; i += kSortThreads) (&s_whist[0][0])[i] = 0u;
   const bool staged = kScene && n_scenes <= kSceneStage;
   if (staged)
     for (int i = tid; i < n_scenes; i += kSortThreads) s_off[kScene ? i : 0] = (int32_t)tri_off[i];
@@ -272,14 +273,14 @@ __global__ void __launch_bounds__(kSortThreads, kSortMinBlocks)
 
 // Launches one pass.
 template <int kItems>
-static void launch_pass(cudaStream_t st, unsigned grid, bool first, bool scene, const uint32_t *in_k,
+static cudaError_t launch_pass(cudaStream_t st, unsigned grid, bool first, bool scene, const uint32_t *in_k,
                         const uint32_t *in_v, uint32_t *out_k, uint32_t *out_v, int64_t n, int shift,
                         const int64_t *tri_off, int n_scenes, const uint32_t *hist, const int32_t *tile_start,
                         int64_t scene_stride, uint32_t *lb, uint32_t *tile_ctr, uint32_t *err, uint32_t spin_limit) {
   auto *kern = first ? (scene ? k_onesweep<true, true, kItems> : k_onesweep<true, false, kItems>)
                      : (scene ? k_onesweep<false, true, kItems> : k_onesweep<false, false, kItems>);
-  kern<<<grid, kSortThreads, 0, st>>>(in_k, in_v, out_k, out_v, n, shift, tri_off, n_scenes, hist, tile_start,
-                                      scene_stride, lb, tile_ctr, err, spin_limit);
+  return launch_after(kern, grid, kSortThreads, st, in_k, in_v, out_k, out_v, n, shift, tri_off, n_scenes, hist,
+                      tile_start, scene_stride, lb, tile_ctr, err, spin_limit);
 }
 
 // Pairs per thread of a sort of n pairs: the large tile once it gives every SM
@@ -316,9 +317,9 @@ int sort_enqueue(flg_ctx ctx, flg_bvh b) {
     uint32_t *in_k = kb[p & 1], *out_k = kb[(p + 1) & 1];
     uint32_t *in_v = vb[p & 1], *out_v = vb[(p + 1) & 1];
     auto *launch = b->sort_items == kSortItems ? launch_pass<kSortItems> : launch_pass<kSortItemsSmall>;
-    launch(ctx->stream, grid, p == 0, scene_pass, in_k, in_v, out_k, out_v, n, shift, b->d_tri_off, b->n_scenes,
-           hist + (size_t)p * kRadix, b->d_tile_start, scene_stride, lb, b->d_tile_ctr + p, ctx->d_err,
-           ctx->spin_limit);
+    FLG_CUDA(ctx, launch(ctx->stream, grid, p == 0, scene_pass, in_k, in_v, out_k, out_v, n, shift, b->d_tri_off,
+                         b->n_scenes, hist + (size_t)p * kRadix, b->d_tile_start, scene_stride, lb, b->d_tile_ctr + p,
+                         ctx->d_err, ctx->spin_limit));
     FLG_LAUNCH_CHECK(ctx, "k_onesweep");
     stage_mark(ctx, ctx->stream, scene_pass ? "sort_scene_pass" : "sort_pass");
   }
@@ -338,9 +339,10 @@ int sort_pairs_enqueue(flg_ctx ctx, cudaStream_t st, int64_t n, int passes, uint
   FLG_CUDA(ctx, cudaMemsetAsync(tile_ctr, 0, sizeof(uint32_t) * passes, st));
   for (int p = 0; p < passes; ++p) {
     uint32_t *lb = lookback + (size_t)p * tiles * kRadix;
-    launch_pass<kSortItems>(st, (unsigned)tiles, p == 0, false, keys[p & 1], vals[p & 1], keys[(p + 1) & 1],
-                            vals[(p + 1) & 1], n, 8 * p, nullptr, 1, hist + (size_t)p * kRadix, nullptr, 0, lb,
-                            tile_ctr + p, ctx->d_err, ctx->spin_limit);
+    FLG_CUDA(ctx, launch_pass<kSortItems>(st, (unsigned)tiles, p == 0, false, keys[p & 1], vals[p & 1],
+                                          keys[(p + 1) & 1], vals[(p + 1) & 1], n, 8 * p, nullptr, 1,
+                                          hist + (size_t)p * kRadix, nullptr, 0, lb, tile_ctr + p, ctx->d_err,
+                                          ctx->spin_limit));
     FLG_LAUNCH_CHECK(ctx, "k_onesweep");
     stage_mark(ctx, st, "ray_sort_pass");
   }

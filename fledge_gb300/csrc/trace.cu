@@ -837,6 +837,7 @@ __device__ __noinline__ ExactHit retrace_closest(const Exact4 &X, const RaySoA &
 // k_trace_finish4 may start at once: the two work on different rays.
 __global__ void __launch_bounds__(128)
     k_settle4(const __grid_constant__ RaySoA R, int64_t n, Out O, const __grid_constant__ Exact4 X, Scratch S) {
+  after_wait();
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t cnt = *S.ovf_count;
   const bool listed = cnt <= S.ovf_cap;  // else look for the marks
@@ -872,7 +873,7 @@ __global__ void __launch_bounds__(256, 4)
   }
   // k_settle4 has ended and its writes are visible: so they are to what
   // follows this kernel
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  after_wait();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *S.work = 0ull;
     *S.ovf_count = 0u;
@@ -882,6 +883,7 @@ __global__ void __launch_bounds__(256, 4)
 // Any-hit rays that k_trace4 left open.
 __global__ void __launch_bounds__(128)
     k_trace_retry4(const __grid_constant__ RaySoA R, int64_t n, Out O, const __grid_constant__ Exact4 X, Scratch S) {
+  after_wait();
   const uint32_t cnt = *S.ovf_count;
   const bool listed = cnt <= S.ovf_cap;  // else look for the marks
   const int64_t end = listed ? (int64_t)cnt : n;
@@ -961,6 +963,7 @@ __global__ void __launch_bounds__(256, 4)
   const uint32_t bottom = s_base + threadIdx.x * (uint32_t)sizeof(uint64_t);
   uint32_t *crew = s_ray[1] + (threadIdx.x & ~31u);  // the upper words of the warp's lanes
   stack_store(bottom, 0xFF800000u, kDone);  // the sentinel: -inf
+  after_wait();
   uint64_t stk[kStackLocal];
   float3 o = make_float3(0.f, 0.f, 0.f), d = o, inv = o;
   float tmin = 0.f;
@@ -1606,27 +1609,19 @@ static int launch4(flg_ctx ctx, cudaStream_t st, flg_bvh b, const RaySoA &R, int
   const int refill = std::max(1, std::min(8, op.refill_lanes));
   const Exact4 X{b->d_nodes2, b->d_tris, Ranges{b->d_rfirst, b->d_rcount}, b->leaf_size, b->d_root, ray_off, n_scenes};
   if (!ANY) ctx->trace4_open = true;  // until the kernel that clears the counters is launched
-  k_trace4<ANY><<<(unsigned)g, threads, 0, st>>>((const NodeQ *)b->d_wide, b->d_tris, b->d_wide_root, ray_off, n_scenes,
-                                                 R, n, O, S, refill, lanes, 1.0f);
+  FLG_CUDA(ctx, launch_after(k_trace4<ANY>, (unsigned)g, threads, st, (const NodeQ *)b->d_wide, b->d_tris,
+                             b->d_wide_root, ray_off, n_scenes, R, n, O, S, refill, lanes, 1.0f));
   FLG_LAUNCH_CHECK(ctx, "k_trace4");
   stage_mark(ctx, st, "trace");
   if (ANY) {
-    k_trace_retry4<<<(unsigned)ctx->num_sms, 128, 0, st>>>(R, n, O, X, S);
+    FLG_CUDA(ctx, launch_after(k_trace_retry4, (unsigned)ctx->num_sms, 128, st, R, n, O, X, S));
     FLG_LAUNCH_CHECK(ctx, "k_trace_retry4");
     stage_mark(ctx, st, "trace_retry");
   } else {
-    k_settle4<<<grid_for(n, 128, ctx->num_sms), 128, 0, st>>>(R, n, O, X, S);
+    FLG_CUDA(ctx, launch_after(k_settle4, grid_for(n, 128, ctx->num_sms), 128, st, R, n, O, X, S));
     FLG_LAUNCH_CHECK(ctx, "k_settle4");
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid_for(n, 256, (int64_t)ctx->num_sms * 16));
-    cfg.blockDim = dim3(256);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    FLG_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_trace_finish4, R, n, O, (const TriRec *)b->d_tris, S));
+    FLG_CUDA(ctx, launch_after(k_trace_finish4, grid_for(n, 256, (int64_t)ctx->num_sms * 16), 256, st, R, n, O, b->d_tris,
+                               S));
     FLG_LAUNCH_CHECK(ctx, "k_trace_finish4");
     ctx->trace4_open = false;
     stage_mark(ctx, st, "trace_finish");

@@ -69,6 +69,7 @@ template <bool SP>
 __global__ void __launch_bounds__(256, 4)
     k_volume_tr(GridDev G, VRays R, int64_t n, uint64_t seed, float *__restrict__ T, float *__restrict__ ck_t,
                 uint32_t *__restrict__ ck_k, float *__restrict__ ck_c) {
+  after_wait();
   const float maj = __ldg(G.params), inv_maj = __ldg(G.params + 1);
   const float max_mu = G.sigma_t * maj;
   WarpChunk chunk(n);
@@ -122,6 +123,7 @@ __global__ void __launch_bounds__(256, 4)
     k_volume_tr_adj(GridDev G, VRays R, int64_t n, uint64_t seed, const float *__restrict__ dLdT,
                     const float *__restrict__ T, const float *__restrict__ ck_t, const uint32_t *__restrict__ ck_k,
                     float *__restrict__ grad, int64_t nv) {
+  after_wait();
   const float maj = __ldg(G.params), inv_maj = __ldg(G.params + 1);
   const float max_mu = G.sigma_t * maj;
   const bool aligned = (reinterpret_cast<uintptr_t>(grad) & 15u) == 0u;
@@ -207,6 +209,7 @@ template <bool SP>
 __global__ void __launch_bounds__(256, 4)
     k_volume_sample(GridDev G, VRays R, int64_t n, uint64_t seed, uint8_t *__restrict__ success,
                     float *__restrict__ p, float *__restrict__ weight) {
+  after_wait();
   const float maj = __ldg(G.params);
   const float max_mu = G.sigma_t * maj;
   WarpChunk chunk(n);
@@ -470,8 +473,8 @@ FLG_API int flg_volume_tr(flg_ctx ctx, flg_grid grid, const flg_rays *rays, int6
   if (ckpt && (!ckpt->t || !ckpt->k || !ckpt->c)) return set_error(ctx, FLG_ERR_ARG, "checkpoint array is NULL");
   if (n == 0) return FLG_OK;
   auto *kern = grid->bidx ? k_volume_tr<true> : k_volume_tr<false>;
-  kern<<<track_blocks(ctx, n), 256, 0, ctx->stream>>>(
-      grid_dev(grid), V, n, seed, T, ckpt ? ckpt->t : nullptr, ckpt ? ckpt->k : nullptr, ckpt ? ckpt->c : nullptr);
+  FLG_CUDA(ctx, launch_after(kern, track_blocks(ctx, n), 256, ctx->stream, grid_dev(grid), V, n, seed, T,
+                             ckpt ? ckpt->t : nullptr, ckpt ? ckpt->k : nullptr, ckpt ? ckpt->c : nullptr));
   FLG_LAUNCH_CHECK(ctx, "k_volume_tr");
   return FLG_OK;
 }
@@ -487,8 +490,8 @@ FLG_API int flg_volume_tr_adjoint(flg_ctx ctx, flg_grid grid, const flg_rays *ra
   if (n == 0) return FLG_OK;
   auto *kern = grid->bidx ? k_volume_tr_adj<true> : k_volume_tr_adj<false>;
   const int64_t nv = grid->bidx ? grid->n_bricks * kBrick * kBrick * kBrick : (int64_t)grid->nx * grid->ny * grid->nz;
-  kern<<<track_blocks(ctx, n), 256, 0, ctx->stream>>>(grid_dev(grid), V, n, seed, dLdT, T, ckpt ? ckpt->t : nullptr,
-                                                      ckpt ? ckpt->k : nullptr, grad, nv);
+  FLG_CUDA(ctx, launch_after(kern, track_blocks(ctx, n), 256, ctx->stream, grid_dev(grid), V, n, seed, dLdT, T,
+                             ckpt ? ckpt->t : nullptr, ckpt ? ckpt->k : nullptr, grad, nv));
   FLG_LAUNCH_CHECK(ctx, "k_volume_tr_adj");
   return FLG_OK;
 }
@@ -502,7 +505,7 @@ FLG_API int flg_volume_sample(flg_ctx ctx, flg_grid grid, const flg_rays *rays, 
   if (n > 0 && (!success || !p || !weight)) return set_error(ctx, FLG_ERR_ARG, "NULL output");
   if (n == 0) return FLG_OK;
   auto *kern = grid->bidx ? k_volume_sample<true> : k_volume_sample<false>;
-  kern<<<track_blocks(ctx, n), 256, 0, ctx->stream>>>(grid_dev(grid), V, n, seed, success, p, weight);
+  FLG_CUDA(ctx, launch_after(kern, track_blocks(ctx, n), 256, ctx->stream, grid_dev(grid), V, n, seed, success, p, weight));
   FLG_LAUNCH_CHECK(ctx, "k_volume_sample");
   return FLG_OK;
 }
