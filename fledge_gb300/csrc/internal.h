@@ -98,7 +98,7 @@ struct flg_ctx_t {
   int64_t *d_ovf = nullptr;
   int64_t ovf_cap = 0;
   unsigned long long *d_trace_ctr = nullptr;
-  bool trace4_open = false;              // a 4-wide trace's launches were cut short: clear its counters
+  bool trace4_open[2] = {false, false};  // by scratch set: a 4-wide trace's launches were cut short: clear its counters
   int64_t *d_ray_off = nullptr;          // device copy of batched ray offsets
   int64_t ray_off_cap = 0;
   std::vector<int64_t> ray_off_h;        // host copy of what d_ray_off holds

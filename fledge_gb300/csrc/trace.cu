@@ -43,7 +43,7 @@ struct Out {
 
 struct Scratch {
   int64_t *ovf;
-  uint32_t *ovf_count;
+  uint32_t *ovf_count;  // and above it the blocks that are done (clear_counters)
   int64_t ovf_cap;
   unsigned long long *work;
   uint32_t *err;
@@ -829,17 +829,41 @@ __device__ __forceinline__ void finish_hit(const RaySoA &R, const Out &O, const 
   O.v[i] = v;
 }
 
+// Those of the closest hits that k_trace4 is sure of; the rays that k_settle4
+// works on are left alone: neither kListed nor a finished id has kPending.
+__device__ __forceinline__ void finish_pending(const RaySoA &R, int64_t n, const Out &O,
+                                               const TriRec *__restrict__ tris) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t g = O.prim[i];
+    if (g < 0 || !(g & kPending)) continue;
+    finish_hit(R, O, tris, i, g & ~kPending, O.t[i]);
+  }
+}
+
 __device__ __noinline__ ExactHit retrace_closest(const Exact4 &X, const RaySoA &R, int64_t i, uint32_t *err) {
   return retrace4<false>(X, R, i, err);
 }
 
+// Clears the trace's counters for the next one, in the last block to get here
+// (the word above the list's length counts them, and wraps to 0).
+__device__ __forceinline__ void clear_counters(const Scratch &S) {
+  __syncthreads();  // every thread has read the list's length
+  if (threadIdx.x == 0 && atomicInc(S.ovf_count + 1, gridDim.x - 1) == gridDim.x - 1) {
+    *S.work = 0ull;
+    *S.ovf_count = 0u;
+  }
+}
+
 // Settles the rays that k_trace4 left open and writes their final values.
-// k_trace_finish4 may start at once: the two work on different rays.
+// ALL: also those of the others, in place of k_trace_finish4, which else may
+// start at once, as the two work on different rays.
+template <bool ALL>
 __global__ void __launch_bounds__(128)
     k_settle4(const __grid_constant__ RaySoA R, int64_t n, Out O, const __grid_constant__ Exact4 X, Scratch S) {
   after_wait();
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (!ALL) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t cnt = *S.ovf_count;
+  if (ALL) finish_pending(R, n, O, X.tris);
   const bool listed = cnt <= S.ovf_cap;  // else look for the marks
   const int64_t end = listed ? (int64_t)cnt : n;
   for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < end; j += (int64_t)gridDim.x * blockDim.x) {
@@ -858,19 +882,15 @@ __global__ void __launch_bounds__(128)
       O.v[i] = 0.0f;
     }
   }
+  if (ALL) clear_counters(S);
 }
 
 // Hit values of every closest hit of k_trace4, one ray per thread (as
-// k_trace_finish), beside k_settle4, whose latency it hides; the rays of that
-// are left alone: neither kListed nor a finished id has kPending.  Then clears
-// the trace's counters for the next one.
+// k_trace_finish), beside k_settle4, whose latency it hides.  Then clears the
+// trace's counters for the next one.
 __global__ void __launch_bounds__(256, 4)
     k_trace_finish4(RaySoA R, int64_t n, Out O, const TriRec *__restrict__ tris, Scratch S) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t g = O.prim[i];
-    if (g < 0 || !(g & kPending)) continue;
-    finish_hit(R, O, tris, i, g & ~kPending, O.t[i]);
-  }
+  finish_pending(R, n, O, tris);
   // k_settle4 has ended and its writes are visible: so they are to what
   // follows this kernel
   after_wait();
@@ -891,6 +911,7 @@ __global__ void __launch_bounds__(128)
     const int64_t i = listed ? S.ovf[j] : j;
     if (O.occ[i] == kOccListed) O.occ[i] = retrace4<true>(X, R, i, S.err).prim >= 0 ? 1 : 0;
   }
+  clear_counters(S);
 }
 
 // The traversal: while-while with speculative leaf postponing (Aila & Laine,
@@ -1597,35 +1618,46 @@ __global__ void __launch_bounds__(256, 4)
 // until they cover the SMs.  Refills at 8 idle lanes at most: with the
 // quantised nodes 8 beat 16 and 24 (24.0 against 25.6 and 29.6 ms on 31.6 M
 // scattered rays).
+//
+// As long as k_settle4's blocks cover the rays in one wave (3 of 128 threads
+// per SM) they also compute the hit values: a launch less (1 to 20,000 rays on
+// 20,480 triangles 2 us less of host time, which is what bounds up to 5,000;
+// 57,000 rays 48.9 against 48.4 us).  Above, k_trace_finish4 has more than
+// twice the warps.
 template <bool ANY>
 static int launch4(flg_ctx ctx, cudaStream_t st, flg_bvh b, const RaySoA &R, int64_t n, const Out &O,
-                   const Scratch &S, const int64_t *ray_off, int n_scenes, const flg_trace_opts &op) {
+                   const Scratch &S, const int64_t *ray_off, int n_scenes, const flg_trace_opts &op, bool &open) {
   const int lanes = (int)std::min<int64_t>(32, ceil_div(n, (int64_t)ctx->num_sms * 16));
-  int threads = op.block_threads, per_sm = 0;
+  int threads = op.block_threads;
   while (threads > 32 && ceil_div(n, (int64_t)lanes * (threads / 32)) < ctx->num_sms) threads >>= 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace4<ANY>, threads, 0);
-  if (per_sm < 1) per_sm = 1;
-  const int64_t g = std::min<int64_t>((int64_t)per_sm * ctx->num_sms, ceil_div(n, (int64_t)lanes * (threads / 32)));
+  int64_t g = ceil_div(n, (int64_t)lanes * (threads / 32));
+  if (g > ctx->num_sms) {  // no more than can be resident
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace4<ANY>, threads, 0);
+    g = std::min<int64_t>(g, (int64_t)std::max(per_sm, 1) * ctx->num_sms);
+  }
   const int refill = std::max(1, std::min(8, op.refill_lanes));
   const Exact4 X{b->d_nodes2, b->d_tris, Ranges{b->d_rfirst, b->d_rcount}, b->leaf_size, b->d_root, ray_off, n_scenes};
-  if (!ANY) ctx->trace4_open = true;  // until the kernel that clears the counters is launched
+  open = true;  // until the kernel that clears the counters is launched
   FLG_CUDA(ctx, launch_after(k_trace4<ANY>, (unsigned)g, threads, st, (const NodeQ *)b->d_wide, b->d_tris,
                              b->d_wide_root, ray_off, n_scenes, R, n, O, S, refill, lanes, 1.0f));
   FLG_LAUNCH_CHECK(ctx, "k_trace4");
   stage_mark(ctx, st, "trace");
   if (ANY) {
-    FLG_CUDA(ctx, launch_after(k_trace_retry4, (unsigned)ctx->num_sms, 128, st, R, n, O, X, S));
+    FLG_CUDA(ctx, launch_after(k_trace_retry4, grid_for(n, 128, ctx->num_sms), 128, st, R, n, O, X, S));
     FLG_LAUNCH_CHECK(ctx, "k_trace_retry4");
-    stage_mark(ctx, st, "trace_retry");
+  } else if (n <= (int64_t)ctx->num_sms * 3 * 128) {
+    FLG_CUDA(ctx, launch_after(k_settle4<true>, grid_for(n, 128, (int64_t)ctx->num_sms * 3), 128, st, R, n, O, X, S));
+    FLG_LAUNCH_CHECK(ctx, "k_settle4");
   } else {
-    FLG_CUDA(ctx, launch_after(k_settle4, grid_for(n, 128, ctx->num_sms), 128, st, R, n, O, X, S));
+    FLG_CUDA(ctx, launch_after(k_settle4<false>, grid_for(n, 128, ctx->num_sms), 128, st, R, n, O, X, S));
     FLG_LAUNCH_CHECK(ctx, "k_settle4");
     FLG_CUDA(ctx, launch_after(k_trace_finish4, grid_for(n, 256, (int64_t)ctx->num_sms * 16), 256, st, R, n, O, b->d_tris,
                                S));
     FLG_LAUNCH_CHECK(ctx, "k_trace_finish4");
-    ctx->trace4_open = false;
-    stage_mark(ctx, st, "trace_finish");
   }
+  open = false;
+  stage_mark(ctx, st, ANY ? "trace_retry" : "trace_finish");
   return FLG_OK;
 }
 
@@ -1763,12 +1795,12 @@ int trace_enqueue(flg_ctx ctx, cudaStream_t st, int set, flg_bvh b, const flg_ra
   Out O{hits ? hits->prim : nullptr, hits ? hits->t : nullptr, hits ? hits->u : nullptr,
         hits ? hits->v : nullptr, occ};
   const bool any = occ != nullptr;
-  // Closest hits over the 4-wide layout end with their counters cleared, so
-  // they keep a pair of their own (sets 2 and 3).
-  const bool clears = b->width == 4 && !any && op.tri_test == 0;
+  // Traces over the 4-wide layout end with their counters cleared, so they
+  // keep a pair of their own (sets 2 and 3).
+  const bool clears = b->width == 4 && op.tri_test == 0;
   Scratch S = scratch_for(ctx, clears ? set + 2 : set);
   stage_mark(ctx, st, "start");
-  if (!clears || ctx->trace4_open)
+  if (!clears || ctx->trace4_open[set])
     FLG_CUDA(ctx, cudaMemsetAsync(S.work, 0, 2 * sizeof(unsigned long long), st));  // both counters
   if (op.tri_test == 1) {
     // The live renderer's Moller-Trumbore test: one ray per thread over the
@@ -1800,8 +1832,8 @@ int trace_enqueue(flg_ctx ctx, cudaStream_t st, int set, flg_bvh b, const flg_ra
     else
       k_trace_bvh2<false><<<g, 256, 0, st>>>(b->d_nodes2, b->d_tris, b->d_root, ray_off_dev, n_scenes, R, n, O, S);
   } else if (b->width == 4) {
-    return any ? launch4<true>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op)
-               : launch4<false>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op);
+    return any ? launch4<true>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op, ctx->trace4_open[set])
+               : launch4<false>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op, ctx->trace4_open[set]);
   } else {
     if (any) launch_wide<8, true>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op);
     else launch_wide<8, false>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op);
@@ -2240,7 +2272,8 @@ FLG_API int flg_trace_closest_noalloc(flg_ctx ctx, flg_bvh bvh, const flg_rays *
     flg_trace_opts op{};
     op.block_threads = 256;
     op.refill_lanes = 16;
-    return launch4<false>(ctx, st, bvh, R, n, O, S, nullptr, 1, op);
+    bool open;  // the counters are cleared above, on every call
+    return launch4<false>(ctx, st, bvh, R, n, O, S, nullptr, 1, op, open);
   } else {
     k_trace_wide<8, false, 64><<<g, 256, 0, st>>>((const NodeW<8> *)bvh->d_wide, bvh->d_tris, bvh->d_wide_root,
                                                   nullptr, 1, R, n, O, S);

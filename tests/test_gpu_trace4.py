@@ -141,3 +141,26 @@ def test_one_triangle_scenes_of_a_batch(ctx, oracle):
         four.build()
         assert torch.equal(four.intersectP(r), one.intersectP(r))
     ctx.sync()
+
+
+@pytest.mark.parametrize("over", [0, 1])
+def test_where_settling_also_finishes(ctx, oracle, over):
+    """On either side of the rule that lets one kernel settle and finish:
+    every hit a tie, closest and any hit in turn on the counters that the trace
+    before them has cleared."""
+    import torch
+    pos, _ = _scene("duplicates")
+    n = torch.cuda.get_device_properties(0).multi_processor_count * 384 + over
+    r8 = G.sphere_rays(n, np.random.default_rng(12))
+    b, _ = U.gpu_build(ctx, pos, width=4)
+    rd, _ = U.rays_dev(r8)
+    tree = oracle.build_bvh(pos)
+    for _ in range(3):
+        h = U.host(b.intersect(rd))
+        occ = b.intersectP(rd).cpu().numpy()
+        bad, _, ho = U.compare_closest(oracle, pos, None, tree, r8, h, oracle.MODE_DEV)
+        assert bad == 0
+        same = h["prim"] == ho["prim"]
+        assert np.array_equal(h["t"][same], ho["t"][same])
+        assert np.array_equal(occ != 0, ho["prim"] >= 0)
+    ctx.sync()
