@@ -294,10 +294,9 @@ __global__ void __launch_bounds__(256, 4)
         bool scatter = false;
         float3 ps = p;
         if (S.medium == 1) {
-          RayStream rs;
-          rs.init(S.seed, path_stream_id(pix, s, depth, 0), 0u);
-          scatter = S.G.bidx ? delta_track<true>(S.G, __ldg(S.G.params), o, d, th[q], rs, ps)
-                             : delta_track<false>(S.G, __ldg(S.G.params), o, d, th[q], rs, ps);
+          const int64_t id = (int64_t)path_stream_id(pix, s, depth, 0);
+          scatter = S.G.bidx ? delta_track<true>(S.G, __ldg(S.G.params), o, d, th[q], S.seed, id, ps)
+                             : delta_track<false>(S.G, __ldg(S.G.params), o, d, th[q], S.seed, id, ps);
           if (scatter) {
             const float wgt = S.G.sigma_s / S.G.sigma_t;
             beta = make_float3(beta.x * wgt, beta.y * wgt, beta.z * wgt);

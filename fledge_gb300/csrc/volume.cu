@@ -37,11 +37,16 @@ __device__ __forceinline__ void load_vray(const VRays &R, int64_t i, float3 &o, 
 // Rays take very different numbers of steps (geometric: the longest of 32 takes
 // about four times the mean), so a warp does not run 32 rays to their end: it
 // owns a contiguous chunk of the rays, and lanes whose ray has ended take the
-// next ones together once kVolRefill of them are idle.  A lane's step is one
-// turn of the warp's loop.  Together with one bounds test and one address per
-// lattice cell (grid_cell), us before -> after: delta tracking of 2 M rays
-// through a 192^3 sparse grid 927 -> 547, of 1 M rays through a 256^3 dense one
-// 83 -> 52; ratio tracking of the latter 85 -> 78, its adjoint 85 -> 82.
+// next ones together once kVolRefill of them are idle.  A lane's step (of delta
+// tracking: two, a Philox block's draws) is one turn of the warp's loop.
+// Together with one bounds test and one address per lattice cell (grid_cell), us
+// before -> after: delta tracking of 2 M rays through a 192^3 sparse grid 927 ->
+// 547 and, two steps to a turn, 460; of 1 M rays through a 256^3 dense one 83 ->
+// 52 -> 47; ratio tracking of the latter 85 -> 75, its adjoint 85 -> 79.  Ratio
+// tracking, which waits for scattered sectors of the grid (29 % of L2's and 30 %
+// of DRAM's rate, L1 at 41 %), gains nothing from turns of four draws (76 us,
+// the adjoint 85), nor from lookups of steps ahead.  Refills at 4 idle lanes: 454
+// and 81 us; at 16 520 and 77.
 constexpr int kVolRefill = 8;
 
 struct WarpChunk {
@@ -213,9 +218,8 @@ __global__ void __launch_bounds__(256, 4)
   const float maj = __ldg(G.params);
   const float max_mu = G.sigma_t * maj;
   WarpChunk chunk(n);
-  DeltaState s;
+  TrackState s;
   int64_t ray = -1;
-  int steps = 0;
   while (true) {
     bool left;
     const int64_t my = chunk.take(ray >= 0, left);
@@ -225,15 +229,11 @@ __global__ void __launch_bounds__(256, 4)
       ray = my;
       float tmax;
       load_vray(R, ray, s.o, s.d, tmax);
-      s.rs.init(seed, (uint64_t)ray, 0u);
-      r = delta_start(G, s, tmax) ? 0 : -1;
-      steps = 0;
+      s.ray = ray;
+      r = s.start(G, tmax) ? 0 : -1;
     }
     float3 q = make_float3(0.0f, 0.0f, 0.0f);
-    if (r == 0) {
-      r = delta_step<SP>(G, max_mu, s, q);
-      if (r == 0 && ++steps >= kMaxTrackSteps) r = -1;
-    }
+    if (r == 0) r = delta_turn<SP>(G, max_mu, seed, s, q);
     if (r != 0 && ray >= 0) {
       const bool ok = r == 1;
       success[ray] = ok ? 1 : 0;

@@ -54,9 +54,11 @@ __device__ __forceinline__ float lerpf(float a, float b, float w) { return a + (
 
 // The eight lattice values around (x, y, z), x fastest.  Almost every lookup
 // lies inside the lattice: one bounds test then stands for those of the eight
-// points, whose addresses follow from one base (dense), or from one brick slot
-// when they share a brick (7^3 / 8^3 = 67 % of the lookups in a sparse grid;
-// otherwise the offsets of both planes per axis are formed once).
+// points, whose addresses follow from one base (dense), or from the brick slots
+// and the offsets of both planes per axis (sparse; seven of the slots are loaded
+// only where the cell straddles bricks, which a third of the lookups do: nearly
+// every warp has both kinds, and one path for them takes fewer instructions than
+// two).
 template <bool SP>
 __device__ __forceinline__ void grid_cell(const GridDev &G, int x, int y, int z, float (&v)[8]) {
   if ((unsigned)x < (unsigned)(G.nx - 1) && (unsigned)y < (unsigned)(G.ny - 1) && (unsigned)z < (unsigned)(G.nz - 1)) {
@@ -66,30 +68,26 @@ __device__ __forceinline__ void grid_cell(const GridDev &G, int x, int y, int z,
 #pragma unroll
       for (int c = 0; c < 8; ++c) v[c] = __ldg(p + (c >> 2) * sz + (c >> 1 & 1) * (int64_t)G.nx + (c & 1));
     } else {
-      const int bx = (unsigned)x / kBrick, by = (unsigned)y / kBrick, bz = (unsigned)z / kBrick;
-      const int ox = (unsigned)x % kBrick, oy = (unsigned)y % kBrick, oz = (unsigned)z % kBrick;
-      const int32_t *bp = G.bidx + ((int64_t)bz * G.bny + by) * G.bnx + bx;
-      if (ox < kBrick - 1 && oy < kBrick - 1 && oz < kBrick - 1) {
-        const int32_t slot = __ldg(bp);
-        const float *p = G.rho + (int64_t)slot * (kBrick * kBrick * kBrick) + (oz * kBrick + oy) * kBrick + ox;
+      const unsigned ox = (unsigned)x % kBrick, oy = (unsigned)y % kBrick, oz = (unsigned)z % kBrick;
+      const int32_t *bp = G.bidx + ((int64_t)((unsigned)z / kBrick) * G.bny + (unsigned)y / kBrick) * G.bnx +
+                          (unsigned)x / kBrick;
+      // brick step and offset in the brick of the upper plane of each axis
+      const bool nx = ox == kBrick - 1, ny = oy == kBrick - 1, nz = oz == kBrick - 1;
+      const int64_t sx = nx, sy = ny ? G.bnx : 0, sz = nz ? (int64_t)G.bny * G.bnx : 0;
+      const unsigned ux = nx ? 0 : ox + 1, uy = (ny ? 0 : oy + 1) * kBrick, uz = (nz ? 0 : oz + 1) * kBrick * kBrick;
+      const unsigned ly = oy * kBrick, lz = oz * kBrick * kBrick;
+      int32_t slot[8];
+      slot[0] = __ldg(bp);
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
-          v[c] = slot < 0 ? 0.0f : __ldg(p + (c >> 2) * kBrick * kBrick + (c >> 1 & 1) * kBrick + (c & 1));
-      } else {
-        // brick step and offset in the brick of the upper plane of each axis
-        const int sx = ox == kBrick - 1, sy = oy == kBrick - 1 ? G.bnx : 0;
-        const int64_t sz = oz == kBrick - 1 ? (int64_t)G.bny * G.bnx : 0;
-        const int ux = sx ? 0 : ox + 1, uy = sy ? 0 : oy + 1, uz = oz == kBrick - 1 ? 0 : oz + 1;
-        int32_t slot[8];
+      for (int c = 1; c < 8; ++c)
+        slot[c] = ((c & 1) && nx) || ((c & 2) && ny) || ((c & 4) && nz)
+                      ? __ldg(bp + (c & 4 ? sz : 0) + (c & 2 ? sy : 0) + (c & 1 ? sx : 0))
+                      : slot[0];
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
-          slot[c] = __ldg(bp + (c & 4 ? sz : 0) + (c & 2 ? sy : 0) + (c & 1 ? sx : 0));
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          v[c] = slot[c] < 0 ? 0.0f
-                             : __ldg(G.rho + (int64_t)slot[c] * (kBrick * kBrick * kBrick) +
-                                     ((c & 4 ? uz : oz) * kBrick + (c & 2 ? uy : oy)) * kBrick + (c & 1 ? ux : ox));
-      }
+      for (int c = 0; c < 8; ++c)
+        v[c] = slot[c] < 0 ? 0.0f
+                           : __ldg(G.rho + (int64_t)slot[c] * (kBrick * kBrick * kBrick) +
+                                   ((c & 4 ? uz : lz) + (c & 2 ? uy : ly) + (c & 1 ? ux : ox)));
     }
   } else {
 #pragma unroll
@@ -141,6 +139,35 @@ __device__ __forceinline__ bool box_pbrt(const GridDev &G, const float3 &o, cons
   t1o = t1;
   return true;
 }
+
+// What the trackers keep of a ray.  They work in turns of a Philox block's four
+// draws, so that the lanes of a warp compute their blocks together: drawn one
+// by one, some lane of every warp needs a new block at every step.
+struct TrackState {
+  float3 o, d;
+  float t, t_max;
+  uint32_t k;  // draws taken
+  int steps;
+  int64_t ray;
+
+  // The block of draw k.
+  __device__ __forceinline__ uint4 block(uint64_t seed) const {
+    return philox4x32_10(make_uint4(k >> 2, (uint32_t)ray, (uint32_t)((uint64_t)ray >> 32), 0x7e5u), (uint32_t)seed,
+                         (uint32_t)(seed >> 32));
+  }
+  // False if the ray misses the grid's box.
+  __device__ __forceinline__ bool start(const GridDev &G, float tmax) {
+    float t_min;
+    k = 0u;
+    steps = 0;
+    if (!box_pbrt(G, o, d, tmax, t_min, t_max)) return false;
+    t = fmaxf(t_min, 0.0f);
+    t_max = fminf(t_max, tmax);
+    return true;
+  }
+};
+
+__device__ __forceinline__ float free_path(uint32_t x, float max_mu) { return -flg_logf(1.0f - u01(x)) / max_mu; }
 
 // Ratio tracking of one ray, a step at a time: T so far in tr, and the state
 // after the last roulette survival (the adjoint's checkpoint).
@@ -233,57 +260,46 @@ inline GridDev grid_dev(flg_grid g) {
   return G;
 }
 
-// Delta tracking of one ray over [0, tmax] (volume.cpp:109-148), a step at a
-// time.  Draws from rs: one uniform per step plus one for the collision test.
-struct DeltaState {
-  float3 o, d;
-  float t, t_max;
-  RayStream rs;
-};
-
-// False if the ray misses the grid's box.
-__device__ __forceinline__ bool delta_start(const GridDev &G, DeltaState &s, float tmax) {
-  float t_min;
-  if (!box_pbrt(G, s.o, s.d, tmax, t_min, s.t_max)) return false;
-  s.t = fmaxf(t_min, 0.0f);
-  s.t_max = fminf(s.t_max, tmax);
-  return true;
-}
-
-// One step: 1 a real collision (its position in p), -1 out of the box, 0 go on.
+// One turn of delta tracking (volume.cpp:109-148): two steps, each with one
+// uniform for its free path and one for its collision test.  1: a real
+// collision (its position in p), -1: out of the box, 0: go on.
 template <bool SP>
-__device__ __forceinline__ int delta_step(const GridDev &G, float max_mu, DeltaState &s, float3 &p) {
-  const float u = s.rs.next();
-  s.t += -flg_logf(1.0f - u) / max_mu;
-  if (s.t >= s.t_max) return -1;
-  const float qx = s.o.x + s.d.x * s.t, qy = s.o.y + s.d.y * s.t, qz = s.o.z + s.d.z * s.t;
-  int x, y, z;
-  float fx, fy, fz;
-  const float dens = sample_grid<SP>(G, qx, qy, qz, x, y, z, fx, fy, fz);
-  const float p_s = G.sigma_s * dens / max_mu;
-  const float p_a = G.sigma_a * dens / max_mu;
-  const float p_n = 1.0f - p_s - p_a;
-  if (s.rs.next() > p_n) {
-    p = make_float3(qx, qy, qz);
-    return 1;
+__device__ __forceinline__ int delta_turn(const GridDev &G, float max_mu, uint64_t seed, TrackState &s, float3 &p) {
+  const uint4 b = s.block(seed);  // k is a multiple of 4
+  s.k += 4u;
+#pragma unroll
+  for (int w = 0; w < 4; w += 2) {
+    s.t += free_path(w ? b.z : b.x, max_mu);
+    if (s.t >= s.t_max) return -1;
+    const float qx = s.o.x + s.d.x * s.t, qy = s.o.y + s.d.y * s.t, qz = s.o.z + s.d.z * s.t;
+    int x, y, z;
+    float fx, fy, fz;
+    const float dens = sample_grid<SP>(G, qx, qy, qz, x, y, z, fx, fy, fz);
+    const float p_s = G.sigma_s * dens / max_mu;
+    const float p_a = G.sigma_a * dens / max_mu;
+    const float p_n = 1.0f - p_s - p_a;
+    if (u01(w ? b.w : b.y) > p_n) {
+      p = make_float3(qx, qy, qz);
+      return 1;
+    }
+    if (++s.steps >= kMaxTrackSteps) return -1;
   }
   return 0;
 }
 
 template <bool SP>
 __device__ __forceinline__ bool delta_track(const GridDev &G, float maj, const float3 &o, const float3 &d,
-                                            float tmax, RayStream &rs, float3 &p) {
-  DeltaState s;
+                                            float tmax, uint64_t seed, int64_t ray, float3 &p) {
+  TrackState s;
   s.o = o;
   s.d = d;
-  s.rs = rs;
+  s.ray = ray;
   int r = -1;
-  if (delta_start(G, s, tmax)) {
+  if (s.start(G, tmax)) {
     const float max_mu = G.sigma_t * maj;
-    r = 0;
-    for (int step_ = 0; step_ < kMaxTrackSteps && r == 0; ++step_) r = delta_step<SP>(G, max_mu, s, p);
+    do r = delta_turn<SP>(G, max_mu, seed, s, p);
+    while (r == 0);
   }
-  rs = s.rs;
   return r == 1;
 }
 
