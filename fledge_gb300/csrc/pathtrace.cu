@@ -31,6 +31,7 @@
 // triangle is chosen uniformly and a point on it by UniformSampleTriangle
 // (math_utils.h:90-93), with the area pdf converted to solid angle.
 #include <algorithm>
+#include <array>
 #include <cstring>
 #include <cmath>
 #include <vector>
@@ -42,58 +43,102 @@
 namespace flg {
 
 constexpr int kPtPrimes = 64;
-__constant__ int c_primes[kPtPrimes] = {
+constexpr int kPrimes[kPtPrimes] = {
     2,   3,   5,   7,   11,  13,  17,  19,  23,  29,  31,  37,  41,  43,  47,  53,  59,  61,  67,  71,  73,  79,
     83,  89,  97,  101, 103, 107, 109, 113, 127, 131, 137, 139, 149, 151, 157, 163, 167, 173, 179, 181, 191, 193,
     197, 199, 211, 223, 227, 229, 233, 239, 241, 251, 257, 263, 269, 271, 277, 281, 283, 293, 307, 311};
 
+// A dimension's base, 1 / base in fp32, and ceil(2^64 / base): the upper 64 bits
+// of its product with a are a / base for every a < 2^32 (Granlund and
+// Montgomery, Division by Invariant Integers using Multiplication, 1994: the
+// error a (base magic - 2^64) / 2^64 stays below 1 / base).
+struct HaltonDim {
+  uint64_t magic;
+  uint32_t base;
+  float inv;
+};
+struct HaltonDims {
+  HaltonDim d[kPtPrimes];
+};
+constexpr HaltonDims make_dims() {
+  HaltonDims t{};
+  for (int i = 0; i < kPtPrimes; ++i) {
+    t.d[i].magic = ~(uint64_t)0 / (uint64_t)kPrimes[i] + 1u;
+    t.d[i].base = (uint32_t)kPrimes[i];
+    t.d[i].inv = 1.0f / (float)kPrimes[i];
+  }
+  return t;
+}
+// The largest multiple of each base below 2^32, its neighbours and the last
+// number: where the error is largest.
+constexpr bool dims_divide() {
+  const HaltonDims t = make_dims();
+  for (int i = 0; i < kPtPrimes; ++i) {
+    const uint64_t base = t.d[i].base, top = ~(uint32_t)0 / base * base;
+    for (uint64_t a : {top - 1, top, top + 1, (uint64_t)~(uint32_t)0})
+      if (a <= ~(uint32_t)0 &&
+          (a * (t.d[i].magic >> 32) + (a * (t.d[i].magic & ~(uint32_t)0) >> 32)) >> 32 != a / base)
+        return false;
+  }
+  return true;
+}
+static_assert(dims_divide());
+__constant__ HaltonDims c_dims = make_dims();
+
+// The scales are at most 128 and 243 and an image takes at most 65535 samples,
+// so indices and offsets fit 32 bits.
 struct Halton {
-  uint64_t scale0, scale1, stride, inv0, inv1;
+  uint32_t scale0, scale1, stride, inv0, inv1;
   int exp0, exp1;
 };
 
-// RadicalInverse_ (sampler.h), in fp32 as the reference evaluates it.
-__device__ __forceinline__ float radical_inverse(int base, uint64_t a) {
-  const float inv_base = 1.0f / (float)base;
+// RadicalInverse_ (sampler.h), in fp32 as the reference evaluates it.  Its
+// quotients are products with a magic number: as 64-bit divisions they were most
+// of k_pt_shade's instructions.
+__device__ __forceinline__ float radical_inverse(const HaltonDim &D, uint32_t a) {
+  const uint32_t base = D.base, m_hi = (uint32_t)(D.magic >> 32), m_lo = (uint32_t)D.magic;
+  const float inv_base = D.inv;
   uint64_t rev = 0;
   float inv_n = 1.0f;
   while (a) {
-    const uint64_t next = a / (uint64_t)base;
-    const uint64_t digit = a - next * (uint64_t)base;
-    rev = rev * (uint64_t)base + digit;
+    const uint32_t next = (uint32_t)(((uint64_t)a * m_hi + __umulhi(a, m_lo)) >> 32);
+    rev = rev * base + (a - next * base);
     inv_n *= inv_base;
     a = next;
   }
   return (float)rev * inv_n;
 }
 
-__device__ __forceinline__ uint64_t inverse_radical_inverse(int base, uint64_t inverse, int n_digits) {
-  uint64_t index = 0;
+template <uint32_t BASE>
+__device__ __forceinline__ uint32_t inverse_radical_inverse(uint32_t inverse, int n_digits) {
+  uint32_t index = 0;
   for (int i = 0; i < n_digits; ++i) {
-    const uint64_t digit = inverse % (uint64_t)base;
-    inverse /= (uint64_t)base;
-    index = index * (uint64_t)base + digit;
+    const uint32_t digit = inverse % BASE;
+    inverse /= BASE;
+    index = index * BASE + digit;
   }
   return index;
 }
 
 // HaltonSampler::getIndexForSample offset of pixel (x, y) (sampler.h:200-221).
-__device__ __forceinline__ uint64_t halton_pixel_offset(const Halton &H, int x, int y) {
+__device__ __forceinline__ uint32_t halton_pixel_offset(const Halton &H, int x, int y) {
   if (H.stride <= 1) return 0;
-  const uint64_t pm0 = (uint64_t)(x % 128), pm1 = (uint64_t)(y % 128);
-  uint64_t off = inverse_radical_inverse(2, pm0, H.exp0) * (H.stride / H.scale0) * H.inv0;
-  off += inverse_radical_inverse(3, pm1, H.exp1) * (H.stride / H.scale1) * H.inv1;
+  const uint32_t pm0 = (uint32_t)(x % 128), pm1 = (uint32_t)(y % 128);
+  uint32_t off = inverse_radical_inverse<2>(pm0, H.exp0) * (H.stride / H.scale0) * H.inv0;
+  off += inverse_radical_inverse<3>(pm1, H.exp1) * (H.stride / H.scale1) * H.inv1;
   return off % H.stride;
 }
 
 // HaltonSampler::get1D for dimension `dim` of sample `index` (sampler.h:233-244).
-__device__ __forceinline__ float halton(const Halton &H, uint64_t index, int dim) {
-  float v;
-  if (dim == 0) v = radical_inverse(2, index / H.scale0);
-  else if (dim == 1) v = radical_inverse(3, index / H.scale1);
-  else v = radical_inverse(c_primes[dim < kPtPrimes ? dim : kPtPrimes - 1], index);
-  return fminf(v, 0.99999994f);
+__device__ __forceinline__ float halton(const Halton &H, uint32_t index, int dim) {
+  const uint32_t a = dim == 0 ? index / H.scale0 : dim == 1 ? index / H.scale1 : index;
+  return fminf(radical_inverse(c_dims.d[dim < kPtPrimes ? dim : kPtPrimes - 1], a), 0.99999994f);
 }
+
+// Participating medium: none, a grid's medium filling its box, or a homogeneous
+// medium bounded by the interface triangles [iface_first, iface_first +
+// iface_count).
+enum { kMedNone, kMedDense, kMedSparse, kMedMesh };
 
 struct PtScene {
   const float *pos;
@@ -103,9 +148,6 @@ struct PtScene {
   float eye[3], fwd[3], right[3], up[3];
   float fov_ratio, aspect;
   int width, height, spp, max_depth;
-  // Participating medium: 0 none, 1 the grid's medium filling its box,
-  // 2 a homogeneous medium bounded by the interface triangles
-  // [iface_first, iface_first + iface_count).
   int medium;
   GridDev G;
   float g;
@@ -187,7 +229,7 @@ __global__ void k_pt_camera(PtScene S, Halton H, int s0, int n_path, PtQueues Q,
   if (p >= n_path) return;
   const int i = p % Q.n_pix, s = s0 + p / Q.n_pix;
   const int x = i % S.width, y = i / S.width;
-  const uint64_t off = halton_pixel_offset(H, x, y);
+  const uint32_t off = halton_pixel_offset(H, x, y);
   float px, py;
   int cnt;
   if (s == 0) {  // eval_pixel's first ray goes through the pixel centre
@@ -197,7 +239,7 @@ __global__ void k_pt_camera(PtScene S, Halton H, int s0, int n_path, PtQueues Q,
   } else {
     // sample 1 continues the dimensions left by sample 0; later samples
     // follow HaltonSampler::reset (integrator.cpp:148-156)
-    const uint64_t index = off + (uint64_t)(s - 1) * H.stride;
+    const uint32_t index = off + (uint32_t)(s - 1) * H.stride;
     cnt = s == 1 ? Q.cnt_end[i] : 0;
     px = (float)x + halton(H, index, cnt);
     py = (float)y + halton(H, index, cnt + 1);
@@ -214,7 +256,7 @@ __global__ void k_pt_camera(PtScene S, Halton H, int s0, int n_path, PtQueues Q,
   Q.beta[3 * p] = Q.beta[3 * p + 1] = Q.beta[3 * p + 2] = 1.0f;
   Q.rad[3 * p] = Q.rad[3 * p + 1] = Q.rad[3 * p + 2] = 0.0f;
   Q.cnt[p] = cnt;
-  if (S.medium == 2) {  // camera rays start outside any medium
+  if (S.medium == kMedMesh) {  // camera rays start outside any medium
     Q.bnc[p] = 0;
     Q.seg[p] = 0;
     Q.inmed[p] = 0;
@@ -240,8 +282,11 @@ __device__ __forceinline__ int queue_slot(bool want, int32_t *counter) {
 // estimation toward one light triangle (Lambertian or Henyey-Greenstein
 // factor; the shadow ray's transmittance is applied in k_pt_shadow); the
 // continuation ray (cosine-weighted bounce or HGSampleP).
-// 4 CTAs per SM (64 registers, no spills; 74 without the bound): +1.3 % on a
-// 1080p / 16-spp render of a 1.3 M-triangle mesh.
+// 4 CTAs per SM (64 registers; 74 without the bound): +1.3 % on a 1080p / 16-spp
+// render of a 1.3 M-triangle mesh.  With a kernel per kind of medium and 32-bit
+// Halton digits, images of 640 x 360 at 4 samples 1060 -> 1015 us, of 1280 x 720
+// at 8 3330 -> 3055 us, the latter in a grid medium 4070 -> 3790 us.
+template <int MED>
 __global__ void __launch_bounds__(256, 4)
     k_pt_shade(PtScene S, Halton H, int s0, int depth, int64_t n_in, PtQueues Q, int qa, const int32_t *__restrict__ prim,
                const float *__restrict__ th, const float *__restrict__ uh, const float *__restrict__ vh) {
@@ -255,7 +300,7 @@ __global__ void __launch_bounds__(256, 4)
   float3 so = o, sd = o, contrib = o, nd = o, no = o;
   float smax = 0.0f;
   const float inv_spp = 1.0f / (float)S.spp;
-  const bool meshmed = S.medium == 2;
+  constexpr bool meshmed = MED == kMedMesh;
   int bnc = depth, sg = depth;     // bounces and segments so far (equal without interfaces)
   bool inmed = false, nmed = false, smed = false;  // inside now / after this vertex / shadow ray start
   if (valid) {
@@ -273,8 +318,8 @@ __global__ void __launch_bounds__(256, 4)
     }
     const int32_t h = prim[q];
     const int x = pix % S.width, y = pix / S.width;
-    const uint64_t off = halton_pixel_offset(H, x, y);
-    const uint64_t index = off + (uint64_t)(s > 0 ? s - 1 : 0) * H.stride;
+    const uint32_t off = halton_pixel_offset(H, x, y);
+    const uint32_t index = off + (uint32_t)(s > 0 ? s - 1 : 0) * H.stride;
     if (h >= 0) {
       const float3 a = pt_vertex(S, h, 0), b = pt_vertex(S, h, 1), c = pt_vertex(S, h, 2);
       const float u = uh[q], v = vh[q], w = 1.0f - u - v;
@@ -293,10 +338,9 @@ __global__ void __launch_bounds__(256, 4)
         // Volume::sample over the segment up to the surface (volume.cpp:109-148)
         bool scatter = false;
         float3 ps = p;
-        if (S.medium == 1) {
+        if (MED == kMedDense || MED == kMedSparse) {
           const int64_t id = (int64_t)path_stream_id(pix, s, depth, 0);
-          scatter = S.G.bidx ? delta_track<true>(S.G, __ldg(S.G.params), o, d, th[q], S.seed, id, ps)
-                             : delta_track<false>(S.G, __ldg(S.G.params), o, d, th[q], S.seed, id, ps);
+          scatter = delta_track<MED == kMedSparse>(S.G, __ldg(S.G.params), o, d, th[q], S.seed, id, ps);
           if (scatter) {
             const float wgt = S.G.sigma_s / S.G.sigma_t;
             beta = make_float3(beta.x * wgt, beta.y * wgt, beta.z * wgt);
@@ -523,6 +567,7 @@ __global__ void k_pt_shadow_step(PtScene S, int64_t n, const int32_t *__restrict
 // Unoccluded shadow rays add their contribution; with a medium, times the
 // ratio-tracking transmittance of the shadow segment (VolEstimateTr,
 // integrator.cpp:40-66).
+template <int MED>
 __global__ void k_pt_shadow(PtScene S, int s0, int depth, int64_t n, const uint8_t *__restrict__ occ, PtQueues Q) {
   after_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -530,16 +575,14 @@ __global__ void k_pt_shadow(PtScene S, int s0, int depth, int64_t n, const uint8
   const int pid = Q.spath[i];
   const int p = pid % Q.n_pix, s = s0 + pid / Q.n_pix;
   float tr = 1.0f;
-  if (S.medium) {
+  if (MED != kMedNone) {
     const float3 o = make_float3(Q.sx[0][i], Q.sx[1][i], Q.sx[2][i]);
     const float3 d = make_float3(Q.sx[3][i], Q.sx[4][i], Q.sx[5][i]);
     float ct, cc;
     uint32_t ck;
     const int64_t id = (int64_t)path_stream_id(p, s, depth, 1);
-    tr = S.G.bidx ? ratio_track<true>(S.G, __ldg(S.G.params), __ldg(S.G.params + 1), o, d, Q.sx[6][i], S.seed, id,
-                                      ct, ck, cc)
-                  : ratio_track<false>(S.G, __ldg(S.G.params), __ldg(S.G.params + 1), o, d, Q.sx[6][i], S.seed, id,
-                                       ct, ck, cc);
+    tr = ratio_track<MED == kMedSparse>(S.G, __ldg(S.G.params), __ldg(S.G.params + 1), o, d, Q.sx[6][i], S.seed, id,
+                                        ct, ck, cc);
     if (tr == 0.0f) return;
   }
   // A path has at most one shadow ray per bounce: no other thread adds to it.
@@ -591,13 +634,13 @@ static void host_halton(int width, int height, Halton &H) {
     if (x < 0) x += b;
     return (uint64_t)x;
   };
-  H.scale0 = scale[0];
-  H.scale1 = scale[1];
+  H.scale0 = (uint32_t)scale[0];
+  H.scale1 = (uint32_t)scale[1];
   H.exp0 = ex[0];
   H.exp1 = ex[1];
-  H.stride = scale[0] * scale[1];
-  H.inv0 = mul_inverse((int64_t)scale[1], (int64_t)scale[0]);
-  H.inv1 = mul_inverse((int64_t)scale[0], (int64_t)scale[1]);
+  H.stride = (uint32_t)(scale[0] * scale[1]);
+  H.inv0 = (uint32_t)mul_inverse((int64_t)scale[1], (int64_t)scale[0]);
+  H.inv1 = (uint32_t)mul_inverse((int64_t)scale[0], (int64_t)scale[1]);
 }
 
 }  // namespace flg
@@ -630,7 +673,7 @@ static int pathtrace_run(flg_ctx ctx, flg_bvh bvh, flg_grid grid, const flg_mesh
   }
   PtScene S;
   std::memset(&S, 0, sizeof(S));
-  S.medium = grid ? 1 : mm ? 2 : 0;
+  S.medium = mm ? kMedMesh : !grid ? kMedNone : grid->bidx ? kMedSparse : kMedDense;
   if (mm) {
     S.iface_first = mm->first;
     S.iface_count = mm->count;
@@ -749,6 +792,11 @@ static int pathtrace_run(flg_ctx ctx, flg_bvh bvh, flg_grid grid, const flg_mesh
   }
   if (bp > (char *)ctx->pt_buf + need) return set_error(ctx, FLG_ERR_STATE, "internal buffer layout");
 
+  // A kernel per kind of medium: together they took more registers than four
+  // blocks leave, and spilled in every render.
+  static constexpr auto shade =
+      std::array{k_pt_shade<kMedNone>, k_pt_shade<kMedDense>, k_pt_shade<kMedSparse>, k_pt_shade<kMedMesh>};
+  static constexpr auto shadow = std::array{k_pt_shadow<kMedNone>, k_pt_shadow<kMedDense>, k_pt_shadow<kMedSparse>};
   cudaStream_t st = ctx->stream;
   FLG_CUDA(ctx, cudaMemsetAsync(radiance, 0, 3 * sizeof(float) * n, st));
   int64_t n_closest = 0, n_shadow = 0;
@@ -773,7 +821,7 @@ static int pathtrace_run(flg_ctx ctx, flg_bvh bvh, flg_grid grid, const flg_mesh
       if (rc) return rc;
       n_closest += n_a;
       FLG_CUDA(ctx, cudaMemsetAsync(Q.counts, 0, 2 * sizeof(int32_t), st));
-      FLG_CUDA(ctx, launch_after(k_pt_shade, (unsigned)ceil_div(n_a, 256), 256, st, S, H, s0, depth, n_a, Q, qa, hh.prim,
+      FLG_CUDA(ctx, launch_after(shade[S.medium], (unsigned)ceil_div(n_a, 256), 256, st, S, H, s0, depth, n_a, Q, qa, hh.prim,
                                  hh.t, hh.u, hh.v));
       FLG_LAUNCH_CHECK(ctx, "k_pt_shade");
       FLG_CUDA(ctx, cudaMemcpyAsync(counts, Q.counts, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
@@ -803,7 +851,7 @@ static int pathtrace_run(flg_ctx ctx, flg_bvh bvh, flg_grid grid, const flg_mesh
         rc = trace_enqueue(ctx, st, 0, bvh, &sr, counts[1], opts, nullptr, 1, nullptr, occ);
         if (rc) return rc;
         n_shadow += counts[1];
-        FLG_CUDA(ctx, launch_after(k_pt_shadow, (unsigned)ceil_div(counts[1], 256), 256, st, S, s0, depth,
+        FLG_CUDA(ctx, launch_after(shadow[S.medium], (unsigned)ceil_div(counts[1], 256), 256, st, S, s0, depth,
                                    (int64_t)counts[1], occ, Q));
         FLG_LAUNCH_CHECK(ctx, "k_pt_shadow");
       }
