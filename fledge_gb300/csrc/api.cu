@@ -108,6 +108,9 @@ FLG_API int flg_ctx_destroy(flg_ctx c) {
   cudaFree(c->d_ray_off);
   cudaFree(c->stage);
   cudaFree(c->pt_buf);
+  cudaFreeHost(c->pt_counts);
+  for (cudaEvent_t e : c->pt_event)
+    if (e) cudaEventDestroy(e);
   cudaFree(c->rs_buf);
   for (cudaEvent_t e : c->stage_pool) cudaEventDestroy(e);
   delete c;

@@ -108,6 +108,10 @@ struct flg_ctx_t {
   // Wavefront queues of flg_pathtrace (grown on demand).
   void *pt_buf = nullptr;
   size_t pt_bytes = 0;
+  // Path tracer: the queue lengths of its last iterations, in pinned host memory
+  // that the device writes, and an event behind each.
+  int32_t *pt_counts = nullptr;
+  cudaEvent_t pt_event[4] = {};
   // Ray-sort scratch of trace_enqueue (grown on demand).
   void *rs_buf = nullptr;
   size_t rs_bytes = 0;
@@ -339,8 +343,11 @@ constexpr int kFlagScanTile = 4096;
 __global__ void k_scan_tiles(const int32_t *in, int n, int32_t *out, int32_t *tsum);
 __global__ void k_scan_sums(int32_t *tsum, int nt, int32_t *total_out);
 #endif
+// n_dev: the number of rays in device memory, of which n is the most it can be;
+// for the traces that trace_takes_device_count() names.
 int trace_enqueue(flg_ctx ctx, cudaStream_t st, int set, flg_bvh b, const flg_rays *rays, int64_t n,
                   const flg_trace_opts *opts, const int64_t *ray_off_dev, int n_scenes, flg_hits *hits,
-                  uint8_t *occ);
+                  uint8_t *occ, const int32_t *n_dev = nullptr);
+bool trace_takes_device_count(flg_bvh b, const flg_trace_opts *opts);
 
 }  // namespace flg

@@ -49,6 +49,14 @@ struct Scratch {
   uint32_t *err;
 };
 
+// Rays of a launch: their number, or the most there can be where it stands in
+// device memory.
+struct RayCount {
+  int64_t most;
+  const int32_t *at;
+  __device__ __forceinline__ int64_t get() const { return at ? (int64_t)*at : most; }
+};
+
 constexpr int kRetryStack = 256;
 
 __device__ __forceinline__ void load_ray(const RaySoA &R, int64_t i, float3 &o, float3 &d, float3 &inv,
@@ -859,10 +867,11 @@ __device__ __forceinline__ void clear_counters(const Scratch &S) {
 // start at once, as the two work on different rays.
 template <bool ALL>
 __global__ void __launch_bounds__(128)
-    k_settle4(const __grid_constant__ RaySoA R, int64_t n, Out O, const __grid_constant__ Exact4 X, Scratch S) {
+    k_settle4(const __grid_constant__ RaySoA R, RayCount N, Out O, const __grid_constant__ Exact4 X, Scratch S) {
   after_wait();
   if (!ALL) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t cnt = *S.ovf_count;
+  const int64_t n = N.get();
   if (ALL) finish_pending(R, n, O, X.tris);
   const bool listed = cnt <= S.ovf_cap;  // else look for the marks
   const int64_t end = listed ? (int64_t)cnt : n;
@@ -889,8 +898,8 @@ __global__ void __launch_bounds__(128)
 // k_trace_finish), beside k_settle4, whose latency it hides.  Then clears the
 // trace's counters for the next one.
 __global__ void __launch_bounds__(256, 4)
-    k_trace_finish4(RaySoA R, int64_t n, Out O, const TriRec *__restrict__ tris, Scratch S) {
-  finish_pending(R, n, O, tris);
+    k_trace_finish4(RaySoA R, RayCount N, Out O, const TriRec *__restrict__ tris, Scratch S) {
+  finish_pending(R, N.get(), O, tris);
   // k_settle4 has ended and its writes are visible: so they are to what
   // follows this kernel
   after_wait();
@@ -902,11 +911,11 @@ __global__ void __launch_bounds__(256, 4)
 
 // Any-hit rays that k_trace4 left open.
 __global__ void __launch_bounds__(128)
-    k_trace_retry4(const __grid_constant__ RaySoA R, int64_t n, Out O, const __grid_constant__ Exact4 X, Scratch S) {
+    k_trace_retry4(const __grid_constant__ RaySoA R, RayCount N, Out O, const __grid_constant__ Exact4 X, Scratch S) {
   after_wait();
   const uint32_t cnt = *S.ovf_count;
   const bool listed = cnt <= S.ovf_cap;  // else look for the marks
-  const int64_t end = listed ? (int64_t)cnt : n;
+  const int64_t end = listed ? (int64_t)cnt : N.get();
   for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < end; j += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = listed ? S.ovf[j] : j;
     if (O.occ[i] == kOccListed) O.occ[i] = retrace4<true>(X, R, i, S.err).prim >= 0 ? 1 : 0;
@@ -961,10 +970,12 @@ __device__ __forceinline__ void stack_load(uint32_t at, uint32_t &key, int32_t &
   asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(key), "=r"(ref) : "r"(at) : "memory");
 }
 
-template <bool ANY>
+// COUNTED: the number of rays stands in device memory (as a runtime choice it
+// made long launches 0.5 % slower).
+template <bool ANY, bool COUNTED>
 __global__ void __launch_bounds__(256, 4)
     k_trace4(const NodeQ *__restrict__ nodes, const TriRec *__restrict__ tris, const int32_t *__restrict__ roots,
-             const int64_t *__restrict__ ray_off, int n_scenes, RaySoA R, int64_t n, Out O, Scratch S, int refill,
+             const int64_t *__restrict__ ray_off, int n_scenes, RaySoA R, RayCount N, Out O, Scratch S, int refill,
              int lanes, float one) {
   // What a lane does next: a node (0 .. kPop - 1), a leaf (< 0), a pop, nothing
   // more for its ray, or nothing.  No parked leaf: 0.
@@ -1091,6 +1102,7 @@ __global__ void __launch_bounds__(256, 4)
     const unsigned idle = __ballot_sync(kAll, cur == kIdle);
     const int nidle = __popc(idle);
     if (phase < 2 && nidle >= refill) {
+      const int64_t n = COUNTED ? (int64_t)*N.at : N.most;
       int64_t my;
       if (phase == 0) {
         my = lane < lanes ? ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * lanes + lane : n;
@@ -1625,34 +1637,36 @@ __global__ void __launch_bounds__(256, 4)
 // 57,000 rays 48.9 against 48.4 us).  Above, k_trace_finish4 has more than
 // twice the warps.
 template <bool ANY>
-static int launch4(flg_ctx ctx, cudaStream_t st, flg_bvh b, const RaySoA &R, int64_t n, const Out &O,
-                   const Scratch &S, const int64_t *ray_off, int n_scenes, const flg_trace_opts &op, bool &open) {
+static int launch4(flg_ctx ctx, cudaStream_t st, flg_bvh b, const RaySoA &R, int64_t n, const int32_t *n_dev,
+                   const Out &O, const Scratch &S, const int64_t *ray_off, int n_scenes, const flg_trace_opts &op, bool &open) {
   const int lanes = (int)std::min<int64_t>(32, ceil_div(n, (int64_t)ctx->num_sms * 16));
   int threads = op.block_threads;
   while (threads > 32 && ceil_div(n, (int64_t)lanes * (threads / 32)) < ctx->num_sms) threads >>= 1;
   int64_t g = ceil_div(n, (int64_t)lanes * (threads / 32));
   if (g > ctx->num_sms) {  // no more than can be resident
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace4<ANY>, threads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace4<ANY, false>, threads, 0);
     g = std::min<int64_t>(g, (int64_t)std::max(per_sm, 1) * ctx->num_sms);
   }
   const int refill = std::max(1, std::min(8, op.refill_lanes));
+  const RayCount N{n, n_dev};
   const Exact4 X{b->d_nodes2, b->d_tris, Ranges{b->d_rfirst, b->d_rcount}, b->leaf_size, b->d_root, ray_off, n_scenes};
   open = true;  // until the kernel that clears the counters is launched
-  FLG_CUDA(ctx, launch_after(k_trace4<ANY>, (unsigned)g, threads, st, (const NodeQ *)b->d_wide, b->d_tris,
-                             b->d_wide_root, ray_off, n_scenes, R, n, O, S, refill, lanes, 1.0f));
+  FLG_CUDA(ctx, launch_after(n_dev ? k_trace4<ANY, true> : k_trace4<ANY, false>, (unsigned)g, threads, st,
+                             (const NodeQ *)b->d_wide, b->d_tris, b->d_wide_root, ray_off, n_scenes, R, N, O, S, refill,
+                             lanes, 1.0f));
   FLG_LAUNCH_CHECK(ctx, "k_trace4");
   stage_mark(ctx, st, "trace");
   if (ANY) {
-    FLG_CUDA(ctx, launch_after(k_trace_retry4, grid_for(n, 128, ctx->num_sms), 128, st, R, n, O, X, S));
+    FLG_CUDA(ctx, launch_after(k_trace_retry4, grid_for(n, 128, ctx->num_sms), 128, st, R, N, O, X, S));
     FLG_LAUNCH_CHECK(ctx, "k_trace_retry4");
   } else if (n <= (int64_t)ctx->num_sms * 3 * 128) {
-    FLG_CUDA(ctx, launch_after(k_settle4<true>, grid_for(n, 128, (int64_t)ctx->num_sms * 3), 128, st, R, n, O, X, S));
+    FLG_CUDA(ctx, launch_after(k_settle4<true>, grid_for(n, 128, (int64_t)ctx->num_sms * 3), 128, st, R, N, O, X, S));
     FLG_LAUNCH_CHECK(ctx, "k_settle4");
   } else {
-    FLG_CUDA(ctx, launch_after(k_settle4<false>, grid_for(n, 128, ctx->num_sms), 128, st, R, n, O, X, S));
+    FLG_CUDA(ctx, launch_after(k_settle4<false>, grid_for(n, 128, ctx->num_sms), 128, st, R, N, O, X, S));
     FLG_LAUNCH_CHECK(ctx, "k_settle4");
-    FLG_CUDA(ctx, launch_after(k_trace_finish4, grid_for(n, 256, (int64_t)ctx->num_sms * 16), 256, st, R, n, O, b->d_tris,
+    FLG_CUDA(ctx, launch_after(k_trace_finish4, grid_for(n, 256, (int64_t)ctx->num_sms * 16), 256, st, R, N, O, b->d_tris,
                                S));
     FLG_LAUNCH_CHECK(ctx, "k_trace_finish4");
   }
@@ -1721,9 +1735,13 @@ static int finish_enqueue(flg_ctx ctx, cudaStream_t st, const RaySoA &R, int64_t
   return FLG_OK;
 }
 
+bool trace_takes_device_count(flg_bvh b, const flg_trace_opts *opts) {
+  return b->width == 4 && (!opts || (opts->tri_test == 0 && opts->ray_sort == 0));
+}
+
 int trace_enqueue(flg_ctx ctx, cudaStream_t st, int set, flg_bvh b, const flg_rays *rays, int64_t n,
                   const flg_trace_opts *opts, const int64_t *ray_off_dev, int n_scenes, flg_hits *hits,
-                  uint8_t *occ) {
+                  uint8_t *occ, const int32_t *n_dev) {
   flg_trace_opts op{};
   if (opts) op = *opts;
   if (op.stack_depth == 0) op.stack_depth = 64;
@@ -1742,6 +1760,8 @@ int trace_enqueue(flg_ctx ctx, cudaStream_t st, int set, flg_bvh b, const flg_ra
   if (n == 0) return FLG_OK;
   RaySoA R{rays->ox, rays->oy, rays->oz, rays->dx, rays->dy, rays->dz, rays->tmin, rays->tmax,
            rays->tmin_const, rays->tmax_const};
+  if (n_dev && !trace_takes_device_count(b, &op))
+    return set_error(ctx, FLG_ERR_STATE, "this trace needs its number of rays on the host");
   if (op.ray_sort) {
     // Scratch: keys and indices (2 x 2), digit counts and offsets, look-back,
     // tile counters, the sorted rays (8 arrays) and their hits (4 arrays).
@@ -1832,8 +1852,8 @@ int trace_enqueue(flg_ctx ctx, cudaStream_t st, int set, flg_bvh b, const flg_ra
     else
       k_trace_bvh2<false><<<g, 256, 0, st>>>(b->d_nodes2, b->d_tris, b->d_root, ray_off_dev, n_scenes, R, n, O, S);
   } else if (b->width == 4) {
-    return any ? launch4<true>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op, ctx->trace4_open[set])
-               : launch4<false>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op, ctx->trace4_open[set]);
+    return any ? launch4<true>(ctx, st, b, R, n, n_dev, O, S, ray_off_dev, n_scenes, op, ctx->trace4_open[set])
+               : launch4<false>(ctx, st, b, R, n, n_dev, O, S, ray_off_dev, n_scenes, op, ctx->trace4_open[set]);
   } else {
     if (any) launch_wide<8, true>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op);
     else launch_wide<8, false>(ctx, st, b, R, n, O, S, ray_off_dev, n_scenes, op);
@@ -2273,7 +2293,7 @@ FLG_API int flg_trace_closest_noalloc(flg_ctx ctx, flg_bvh bvh, const flg_rays *
     op.block_threads = 256;
     op.refill_lanes = 16;
     bool open;  // the counters are cleared above, on every call
-    return launch4<false>(ctx, st, bvh, R, n, O, S, nullptr, 1, op, open);
+    return launch4<false>(ctx, st, bvh, R, n, nullptr, O, S, nullptr, 1, op, open);
   } else {
     k_trace_wide<8, false, 64><<<g, 256, 0, st>>>((const NodeW<8> *)bvh->d_wide, bvh->d_tris, bvh->d_wide_root,
                                                   nullptr, 1, R, n, O, S);
