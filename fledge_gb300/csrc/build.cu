@@ -50,7 +50,7 @@ __device__ __forceinline__ void atomic_max_f(float *a, float v) {
 // Everything a build starts from, in one launch (as fills and copies these
 // were eight, 2 us each of a 20,001-triangle build): empty scene boxes, zeroed
 // digit counts, look-back words and tile counters, the scene passes' counts,
-// the collapse's counters and first queue, and, after a climb that gave up,
+// the collapse's counters, and, after a climb that gave up,
 // the climb's slots and counters (its mark is cleared by the next kernel).
 struct BuildSetup {
   float *box;
@@ -65,9 +65,6 @@ struct BuildSetup {
   int32_t n_scene_hist;
   int32_t *wide_ctr;
   int32_t n_wide_ctr;  // their initial values follow them
-  int2 *queue;
-  const int2 *queue_init;
-  int32_t n_queue;
   float4 *slots;
   uint32_t *flags;
   int64_t n_nodes;
@@ -84,7 +81,6 @@ __global__ void __launch_bounds__(256) k_build_setup(BuildSetup B) {
   for (int64_t i = t0; i < B.n_lookback; i += step) B.lookback[i] = make_uint4(0u, 0u, 0u, 0u);
   for (int64_t i = t0; i < B.n_scene_hist; i += step) B.scene_hist[i] = B.scene_hist_init[i];
   for (int64_t i = t0; i < B.n_wide_ctr; i += step) B.wide_ctr[i] = B.wide_ctr[B.n_wide_ctr + i];
-  for (int64_t i = t0; i < B.n_queue; i += step) B.queue[i] = B.queue_init[i];
   if (B.n_nodes > 0 && *B.dirty != 0u) {
     const float u = __int_as_float(kBoxUnset);
     for (int64_t i = t0; i < B.n_nodes; i += step) {
@@ -479,9 +475,6 @@ int build_enqueue(flg_ctx ctx, flg_bvh b) {
   if (b->width > 2 && b->d_wide_ctr) {
     B.wide_ctr = b->d_wide_ctr;
     B.n_wide_ctr = collapse_ctr_words();
-    B.queue = b->d_queue[0];
-    B.queue_init = b->d_queue_init;
-    B.n_queue = b->n_wide_roots;
   }
   FLG_CUDA(ctx, launch_after(k_build_setup,
                              grid_for(std::max<int64_t>(B.n_lookback, 6 * (int64_t)b->n_scenes), 256,

@@ -1,8 +1,9 @@
 // collapse.cu — re-lays out a built Karras BVH2 as 4- or 8-wide nodes for
-// traversal.  Top-down, level by level (one cooperative launch with a grid
-// barrier between levels): each queued BVH2 node becomes a wide node whose children are found by
-// repeatedly opening the child with the largest surface area (Wald, Benthin,
-// Boulos 2008 style collapsing).
+// traversal, top-down: a BVH2 node becomes a wide node whose children are found
+// by repeatedly opening the child with the largest surface area (Wald, Benthin,
+// Boulos 2008 style collapsing).  Large scenes go level by level in one
+// cooperative launch with a grid barrier between levels (k_collapse_all),
+// smaller ones in subtrees (k_collapse_top, k_collapse_rest).
 // A BVH2 subtree covers a contiguous run of sorted triangles, so any subtree
 // with at most leaf_size triangles becomes a leaf range [first, first+count).
 // The Karras topology itself (the parity object) is unchanged.
@@ -27,104 +28,150 @@ constexpr int kCollapseNodes = 4;
 // k_trace4's superset argument does not depend on the ranges, and retrace4 and
 // first_of_two form the exact tree with leaf_size.
 constexpr int kLeaf4 = 2;
-// Collapse counters: [0] wide nodes allocated, [1] its initial value, [2 .. 4]
-// the barrier; the initial values of these kCtrLive words follow as a static
-// copy.
-constexpr int kCtrLive = 5;
+// Counters of a collapse; the initial values of these kCtrLive words follow as a
+// static copy.
+enum {
+  kCtrNodes = 0,  // slots taken
+  kCtrFirst = 1,  // slots that the roots have
+  kCtrBar = 2,    // k_collapse_all's barrier: arrivals, generation, kCtrNodes when all had arrived
+  kCtrReady = 5,  // k_collapse_top: subtrees listed
+  kCtrClaim = 6,  // subtrees taken
+  kCtrLive = 7
+};
 
-// One wide node per queued BVH2 node of a level (cnt items in q_in).  A warp
-// claims the slots of its new wide nodes with one atomic on node_ctr (prefix
-// sum of the lanes' internal children); the queue of the next level holds the
-// new nodes in slot order, so a node's place in it is its slot less the level's
-// first (q_base).  Claims by block cost more in barriers than they save (4 M
-// triangles: 230 against 220 us).  Queue entries are read through L2 (__ldcg):
-// this SM may still hold lines of the same buffer from two levels before.
+// Child k of an opened node becomes a wide node of its own.
 template <int W>
-__device__ __forceinline__ void collapse_level(const Node2 *__restrict__ nodes2, const Ranges &R, int leaf_size,
-                                               const int2 *__restrict__ q_in, int cnt, int2 *__restrict__ q_out,
-                                               int q_base, int32_t *node_ctr, int64_t cap,
-                                               typename WideRec<W>::T *__restrict__ wide, uint32_t *err) {
+__device__ __forceinline__ bool is_inner(const Cand (&c)[W], int nc, int k, int leaf_size) {
+  return k < nc && c[k].ref >= 0 && c[k].count > leaf_size;
+}
+
+// Record of an opened node whose inner children take the slots from slot0 on
+// (those from cap on: unused, the caller has set the error word).
+template <int W>
+__device__ __forceinline__ typename WideRec<W>::T wide_record(const Cand (&c)[W], int nc, int leaf_size, int slot0,
+                                                              int64_t cap) {
+  int32_t child[W];
+  int slot = slot0;
+#pragma unroll
+  for (int k = 0; k < W; ++k) {
+    child[k] = kEmptyChild;
+    if (is_inner<W>(c, nc, k, leaf_size)) {
+      if (slot < cap) child[k] = slot;
+      ++slot;
+    } else if (k < nc) {
+      child[k] = ~((c[k].first << 3) | (c[k].count - 1));
+    }
+  }
+  typename WideRec<W>::T out;
+  if constexpr (W == 4) {
+    quantise(c, nc, out);
+    out.base = 0;
+    out.kind = 0u;
+    uint32_t rank = 0u;
+#pragma unroll
+    for (int k = 3; k >= 0; --k)
+      if (child[k] >= 0 && child[k] != kEmptyChild) out.base = child[k];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const bool inner = child[k] >= 0 && child[k] != kEmptyChild;
+      out.kind |= (inner ? rank : 0x80u | (uint32_t)k) << (8 * k);
+      rank += inner ? 1u : 0u;
+      out.leaf[k] = inner ? kEmptyChild : child[k];
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      const float inf = __int_as_float(0x7f800000);  // unused slots: +inf boxes, which no ray enters
+      out.lox[k] = k < nc ? c[k].lo[0] : inf;
+      out.loy[k] = k < nc ? c[k].lo[1] : inf;
+      out.loz[k] = k < nc ? c[k].lo[2] : inf;
+      out.hix[k] = k < nc ? c[k].hi[0] : inf;
+      out.hiy[k] = k < nc ? c[k].hi[1] : inf;
+      out.hiz[k] = k < nc ? c[k].hi[2] : inf;
+      out.child[k] = child[k];
+    }
+  }
+  return out;
+}
+
+// Opens item (BVH2 node, wide slot); nc stays 0 if it names neither: a hole left
+// by an overflow, or a broken tree.
+template <int W>
+__device__ __forceinline__ void open_item(const Node2 *__restrict__ nodes2, const Ranges &R, int leaf_size,
+                                          const int2 &item, int64_t cap, Cand (&c)[W], int &nc, uint32_t *err) {
+  // cap = BVH2 node count + 1: item.x names a BVH2 node, item.y a wide slot.
+  if (item.x < 0 || item.y < 0 || item.x >= cap - 1 || item.y >= cap) atomicOr(err, kErrQueue);
+  else open_wide<W>(nodes2, R, leaf_size, item.x, c, nc);
+}
+
+// What a collapse works on.
+struct Collapse {
+  const Node2 *nodes2;
+  Ranges R;
+  int leaf_size;
+  int64_t cap;        // slots
+  const int2 *roots;  // (BVH2 node, slot)
+  int n_roots;
+  int2 *queue[2];     // k_collapse_all: the nodes of a level, (BVH2 node, slot)
+  int small;          // k_collapse_top: most triangles of a subtree that it lists
+  int32_t *ref;       // BVH2 node by slot
+  int32_t *ready;     // slots of the listed subtrees
+  int32_t *large[2];  // slots of the large nodes of a level
+  int32_t *ctr;
+  uint32_t spin_limit, *err;
+};
+
+__device__ __forceinline__ int warp_inclusive(int v, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xFFFFFFFFu, v, o);
+    if (lane >= o) v += x;
+  }
+  return v;
+}
+
+// k_collapse_all: one wide node per queued BVH2 node of a level (cnt items in
+// q_in).  A warp claims the slots of its new wide nodes with one atomic (prefix
+// sum of the lanes' inner children); the queue of the next level holds the new
+// nodes in slot order, so a node's place in it is its slot less the level's
+// first (q_base).  Claims by block cost more in barriers than they save (4 M
+// triangles: 230 against 220 us), as do separate lists of slots (246).  Queue
+// entries are read through L2 (__ldcg): this SM may still hold lines of the same
+// buffer from two levels before.
+template <int W>
+__device__ __forceinline__ void collapse_level(const Collapse &X, const int2 *__restrict__ q_in, int cnt,
+                                               int2 *__restrict__ q_out, int q_base,
+                                               typename WideRec<W>::T *__restrict__ wide) {
   const int lane = threadIdx.x & 31;
   // Warp-uniform loop: all lanes of a warp share it0.
   for (int it0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) & ~31u); it0 < cnt; it0 += gridDim.x * blockDim.x) {
     const int it = it0 + lane;
-    const bool valid = it < cnt;
     int2 item = make_int2(0, 0);
     Cand c[W];
     int nc = 0;
-    if (valid) {
+    if (it < cnt) {
       item = __ldcg(q_in + it);
-      // cap = BVH2 node count + 1: item.x names a BVH2 node, item.y a wide slot.
-      if (item.x < 0 || item.y < 0 || item.x >= cap - 1 || item.y >= cap)
-        atomicOr(err, kErrQueue);  // a hole left by an overflowing level
-      else
-        open_wide<W>(nodes2, R, leaf_size, item.x, c, nc);
+      open_item<W>(X.nodes2, X.R, X.leaf_size, item, X.cap, c, nc, X.err);
     }
-    // Children that become wide nodes of the next level.
     int need = 0;
 #pragma unroll
-    for (int k = 0; k < W; ++k)
-      if (k < nc && c[k].ref >= 0 && c[k].count > leaf_size) ++need;
-    int incl = need;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    int slot0 = 0;
-    if (lane == 31 && incl > 0) slot0 = atomicAdd(node_ctr, incl);
-    slot0 = __shfl_sync(0xFFFFFFFFu, slot0, 31) + incl - need;
-    if (!valid || nc == 0) continue;
-    int32_t child[W];
+    for (int k = 0; k < W; ++k) need += is_inner<W>(c, nc, k, X.leaf_size) ? 1 : 0;
+    const int incl = warp_inclusive(need, lane);
+    int base = 0;
+    if (lane == 31 && incl > 0) base = atomicAdd(X.ctr + kCtrNodes, incl);
+    base = __shfl_sync(0xFFFFFFFFu, base, 31);
+    if (nc == 0) continue;
+    const int slot0 = base + incl - need;
+    int slot = slot0;
 #pragma unroll
     for (int k = 0; k < W; ++k) {
-      child[k] = kEmptyChild;
-      if (k < nc) {
-        if (c[k].ref < 0 || c[k].count <= leaf_size) {
-          child[k] = ~((c[k].first << 3) | (c[k].count - 1));
-        } else {
-          const int slot = slot0++, q = slot - q_base;
-          if (slot >= cap) {
-            atomicOr(err, kErrQueue);
-            if (q < cap) q_out[q] = make_int2(-1, -1);  // the next level skips it
-          } else {
-            q_out[q] = make_int2(c[k].ref, slot);
-            child[k] = slot;
-          }
-        }
-      }
+      if (!is_inner<W>(c, nc, k, X.leaf_size)) continue;
+      const int q = slot - q_base;
+      if (slot >= X.cap) atomicOr(X.err, kErrQueue);
+      if (q < X.cap) q_out[q] = slot < X.cap ? make_int2(c[k].ref, slot) : make_int2(-1, -1);  // the next level skips it
+      ++slot;
     }
-    typename WideRec<W>::T out;
-    if constexpr (W == 4) {
-      quantise(c, nc, out);
-      // This lane's inner children took consecutive slots.
-      out.base = 0;
-      out.kind = 0u;
-      uint32_t rank = 0u;
-#pragma unroll
-      for (int k = 3; k >= 0; --k)
-        if (child[k] >= 0 && child[k] != kEmptyChild) out.base = child[k];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const bool inner = child[k] >= 0 && child[k] != kEmptyChild;
-        out.kind |= (inner ? rank : 0x80u | (uint32_t)k) << (8 * k);
-        rank += inner ? 1u : 0u;
-        out.leaf[k] = inner ? kEmptyChild : child[k];
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < W; ++k) {
-        const float inf = __int_as_float(0x7f800000);  // unused slots: +inf boxes, which no ray enters
-        out.lox[k] = k < nc ? c[k].lo[0] : inf;
-        out.loy[k] = k < nc ? c[k].lo[1] : inf;
-        out.loz[k] = k < nc ? c[k].lo[2] : inf;
-        out.hix[k] = k < nc ? c[k].hi[0] : inf;
-        out.hiy[k] = k < nc ? c[k].hi[1] : inf;
-        out.hiz[k] = k < nc ? c[k].hi[2] : inf;
-        out.child[k] = child[k];
-      }
-    }
-    wide[item.y] = out;
+    wide[item.y] = wide_record<W>(c, nc, X.leaf_size, slot0, X.cap);
   }
 }
 
@@ -164,22 +211,194 @@ __device__ __forceinline__ int grid_barrier(uint32_t *bar, const int32_t *ctr, u
 }
 
 // The whole collapse in one cooperative launch: level after level with a
-// grid barrier between them, until a level is empty.  Replaces up to 64
-// launches (most of them empty) by one.
+// grid barrier between them, until a level is empty.
 template <int W>
 __global__ void __launch_bounds__(kCollapseThreads)
-    k_collapse_all(const Node2 *__restrict__ nodes2, Ranges R, int leaf_size, int n_roots, int2 *q0, int2 *q1,
-                   int32_t *ctr, uint32_t *bar, int64_t cap, typename WideRec<W>::T *__restrict__ wide,
-                   uint32_t spin_limit, uint32_t *err) {
-  int cnt = n_roots, end = ctr[1];  // the level's queue; where its new nodes begin (ctr[0] moves on)
+    k_collapse_all(const __grid_constant__ Collapse X, typename WideRec<W>::T *__restrict__ wide) {
+  int cnt = X.n_roots, end = X.ctr[kCtrFirst];  // the level's queue; where its new nodes begin
   for (int L = 0; L < kMaxLevels && cnt > 0; ++L) {
-    collapse_level<W>(nodes2, R, leaf_size, (L & 1) ? q1 : q0, cnt, (L & 1) ? q0 : q1, end, ctr, cap, wide, err);
-    const int now = grid_barrier(bar, ctr, spin_limit, err);
+    collapse_level<W>(X, L == 0 ? X.roots : X.queue[L & 1], cnt, X.queue[(L + 1) & 1], end, wide);
+    const int now = grid_barrier((uint32_t *)X.ctr + kCtrBar, X.ctr + kCtrNodes, X.spin_limit, X.err);
     // Counts beyond the queue capacity only arise from a corrupted tree.
-    cnt = (int)min((int64_t)(now - end), cap);
+    cnt = (int)min((int64_t)(now - end), X.cap);
     end = now;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0 && cnt > 0) atomicOr(err, kErrQueue);  // deeper than kMaxLevels
+  if (blockIdx.x == 0 && threadIdx.x == 0 && cnt > 0) atomicOr(X.err, kErrQueue);  // deeper than kMaxLevels
+}
+
+// Up to kTopMax triangles a collapse is two launches without a wait for another
+// SM.  k_collapse_top, one CTA, opens level after level the nodes of more than
+// `small` triangles and lists their other inner children; k_collapse_rest gives
+// these subtrees to warps.  A level of k_collapse_all takes 4 us, half of it in
+// the barrier, whatever its size, and the last ones, of a few nodes each, are
+// half of them.  us per collapse, k_collapse_all -> this: 5,000 triangles 48 ->
+// 29, 20,001 54 -> 31, 65,536 62 -> 37, 200,000 73 -> 46, 600,000 97 -> 80,
+// 1,000,000 108 -> 105, 2,000,000 152 -> 196.  `small`: n / 700, at least 128.
+// The top CTA is bound by instructions, so smaller subtrees cost (20,001
+// triangles in subtrees of 64: 51 us); and a warp takes long over larger ones
+// (200,000 in n / 256: 79).  Large scenes keep the levels: a warp's steps run
+// with half of the lanes.
+constexpr int64_t kTopMax = 1 << 20;
+constexpr int kTopThreads = 256;
+constexpr int kTopRoots = 1024;
+constexpr int kTopSplit = 700;
+constexpr int kSmallTree = 128;
+
+// Entries that this kernel writes and reads go through L2.
+__device__ __forceinline__ int2 item_at(const Collapse &X, int slot) {
+  return make_int2(slot >= 0 && slot < X.cap ? __ldcg(X.ref + slot) : -1, slot);
+}
+
+// Lists the inner children of an opened node, which take the slots from slot0 on:
+// the large ones from list[large] on, the others from X.ready[other] on.
+template <int W>
+__device__ __forceinline__ void list_children(const Collapse &X, const Cand (&c)[W], int nc, int slot0, int32_t *list,
+                                              int large, int64_t most, int other) {
+  int slot = slot0;
+#pragma unroll
+  for (int k = 0; k < W; ++k) {
+    if (!is_inner<W>(c, nc, k, X.leaf_size)) continue;
+    const bool big = c[k].count > X.small;
+    int &at = big ? large : other;
+    if (slot < X.cap && at < (big ? most : X.cap)) {
+      X.ref[slot] = c[k].ref;
+      (big ? list : X.ready)[at] = slot;
+    } else {
+      atomicOr(X.err, kErrQueue);  // counts that do not add up: a broken tree
+    }
+    ++at;
+    ++slot;
+  }
+}
+
+// Inner children of an opened node, and in the upper half the large ones.
+template <int W>
+__device__ __forceinline__ int count_children(const Collapse &X, const Cand (&c)[W], int nc) {
+  int need = 0;
+#pragma unroll
+  for (int k = 0; k < W; ++k)
+    if (is_inner<W>(c, nc, k, X.leaf_size)) need += c[k].count > X.small ? 0x10001 : 1;
+  return need;
+}
+
+// The listed subtrees.  A warp takes one, opens up to 32 of its nodes at a time,
+// claims the slots of their inner children with one atomic and stacks them as
+// one run of slots.  Last in, first out: a run on the stack lies deeper in the
+// tree than the one below it, so kMaxLevels runs suffice.
+template <int W>
+__device__ __forceinline__ void collapse_rest(const Collapse &X, int n_ready,
+                                              typename WideRec<W>::T *__restrict__ wide) {
+  __shared__ int2 s_run[kCollapseThreads / 32][kMaxLevels];
+  const int lane = threadIdx.x & 31;
+  int2 *run = s_run[threadIdx.x >> 5];
+  const int warps = gridDim.x * (kCollapseThreads / 32);
+  const int take = min(max(n_ready / (2 * warps), 1), 32);  // at a time
+  int mine = (blockIdx.x * (kCollapseThreads / 32) + (threadIdx.x >> 5)) * take;
+  int depth = 0;
+  while (true) {
+    int slot = -1;
+    if (depth == 0) {
+      if (mine >= n_ready) break;
+      if (lane < take && mine + lane < n_ready) slot = __ldcg(X.ready + mine + lane);
+      if (lane == 0) mine = warps * take + atomicAdd(X.ctr + kCtrClaim, take);
+      mine = __shfl_sync(0xFFFFFFFFu, mine, 0);
+    } else {
+      const int2 r = run[depth - 1];
+      const int m = min(r.y, 32);
+      if (lane < m) slot = r.x + r.y - m + lane;
+      __syncwarp();
+      if (r.y == m) --depth;
+      else if (lane == 0) run[depth - 1].y = r.y - m;
+    }
+    Cand c[W];
+    int nc = 0;
+    if (slot >= 0) open_item<W>(X.nodes2, X.R, X.leaf_size, item_at(X, slot), X.cap, c, nc, X.err);
+    int need = 0;
+#pragma unroll
+    for (int k = 0; k < W; ++k) need += is_inner<W>(c, nc, k, X.leaf_size) ? 1 : 0;
+    const int incl = warp_inclusive(need, lane);
+    const int all = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    int base = 0;
+    if (lane == 0 && all > 0) base = atomicAdd(X.ctr + kCtrNodes, all);
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    if (nc > 0) {
+      const int slot0 = base + incl - need;
+      int to = slot0;
+#pragma unroll
+      for (int k = 0; k < W; ++k) {
+        if (!is_inner<W>(c, nc, k, X.leaf_size)) continue;
+        if (to < X.cap) X.ref[to] = c[k].ref;
+        ++to;
+      }
+      wide[slot] = wide_record<W>(c, nc, X.leaf_size, slot0, X.cap);
+    }
+    if (all > 0) {
+      // only a broken tree needs more slots, or more levels, than there are
+      const int left = base < X.cap ? (int)min((int64_t)all, X.cap - base) : 0;
+      if ((left < all || depth == kMaxLevels) && lane == 0) atomicOr(X.err, kErrQueue);
+      if (left > 0 && depth < kMaxLevels) {
+        if (lane == 0) run[depth] = make_int2(base, left);
+        ++depth;
+      }
+    }
+    __syncwarp();
+  }
+}
+
+template <int W>
+__global__ void __launch_bounds__(kTopThreads)
+    k_collapse_top(const __grid_constant__ Collapse X, typename WideRec<W>::T *__restrict__ wide) {
+  __shared__ int s_wsum[kTopThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  after_wait();
+  int slots = X.ctr[kCtrFirst], n_ready = 0;
+  int cnt = X.n_roots;
+  for (int L = 0; L < kMaxLevels && cnt > 0; ++L) {
+    const int32_t *in = X.large[L & 1];
+    int next = 0;
+    for (int it0 = 0; it0 < cnt; it0 += kTopThreads) {
+      int2 item = make_int2(0, 0);
+      Cand c[W];
+      int nc = 0;
+      if (it0 + tid < cnt) {
+        item = L == 0 ? X.roots[it0 + tid] : item_at(X, __ldcg(in + it0 + tid));
+        open_item<W>(X.nodes2, X.R, X.leaf_size, item, X.cap, c, nc, X.err);
+      }
+      const int need = count_children<W>(X, c, nc), incl = warp_inclusive(need, lane);
+      if (lane == 31) s_wsum[warp] = incl;
+      __syncthreads();
+      int before = incl - need, all = 0;
+#pragma unroll
+      for (int w = 0; w < kTopThreads / 32; ++w) {
+        const int x = s_wsum[w];
+        if (w < warp) before += x;
+        all += x;
+      }
+      if (nc > 0) {
+        const int slot0 = slots + (before & 0xFFFF);
+        list_children<W>(X, c, nc, slot0, X.large[(L + 1) & 1], next + (before >> 16), X.cap,
+                         n_ready + (before & 0xFFFF) - (before >> 16));
+        wide[item.y] = wide_record<W>(c, nc, X.leaf_size, slot0, X.cap);
+      }
+      slots += all & 0xFFFF;
+      next += all >> 16;
+      n_ready += (all & 0xFFFF) - (all >> 16);
+      __syncthreads();
+    }
+    cnt = (int)min((int64_t)next, X.cap);
+  }
+  if (tid == 0) {
+    X.ctr[kCtrNodes] = slots;
+    X.ctr[kCtrReady] = (int32_t)min((int64_t)n_ready, X.cap);
+    if (cnt > 0) atomicOr(X.err, kErrQueue);  // deeper than kMaxLevels
+  }
+}
+
+template <int W>
+__global__ void __launch_bounds__(kCollapseThreads)
+    k_collapse_rest(const __grid_constant__ Collapse X, typename WideRec<W>::T *__restrict__ wide) {
+  after_wait();
+  collapse_rest<W>(X, X.ctr[kCtrReady], wide);
 }
 
 int collapse_reserve(flg_ctx ctx, flg_bvh b) {
@@ -235,7 +454,7 @@ int collapse_reserve(flg_ctx ctx, flg_bvh b) {
   }
   b->n_wide_roots = (int32_t)q.size();
   std::vector<int32_t> ctr(2 * kCtrLive, 0);
-  ctr[0] = ctr[1] = ctr[kCtrLive] = ctr[kCtrLive + 1] = slots;
+  for (int i : {(int)kCtrNodes, (int)kCtrFirst}) ctr[i] = ctr[kCtrLive + i] = slots;
   cudaStream_t st = ctx->stream;
   cudaError_t e = cudaMemcpyAsync(b->d_wide_root, roots.data(), sizeof(int32_t) * b->n_scenes,
                                   cudaMemcpyHostToDevice, st);
@@ -255,12 +474,40 @@ static int collapse_levels(flg_ctx ctx, flg_bvh b) {
   cudaStream_t st = ctx->stream;
   using Rec = typename WideRec<W>::T;
   Rec *wide = (Rec *)b->d_wide;
-  const Ranges R{b->d_rfirst, b->d_rcount};
-  const int leaf = W == 4 ? std::min<int>(b->leaf_size, kLeaf4) : b->leaf_size;
-  // Level sizes are only known on the device: one cooperative launch walks the
-  // levels with a grid barrier in between.  A barrier costs by its CTAs, so a
-  // small tree takes fewer than a resident wave: one thread per kCollapseNodes
-  // nodes covers its widest levels.
+  Collapse X;
+  X.nodes2 = b->d_nodes2;
+  X.R = Ranges{b->d_rfirst, b->d_rcount};
+  X.leaf_size = W == 4 ? std::min<int>(b->leaf_size, kLeaf4) : b->leaf_size;
+  X.roots = b->d_queue_init;
+  X.n_roots = b->n_wide_roots;
+  X.cap = b->wide_cap;
+  X.queue[0] = b->d_queue[0];
+  X.queue[1] = b->d_queue[1];
+  X.small = 0;
+  X.ref = (int32_t *)b->d_queue[0];
+  X.ready = X.ref + X.cap;
+  X.large[0] = (int32_t *)b->d_queue[1];
+  X.large[1] = X.large[0] + X.cap;
+  X.ctr = b->d_wide_ctr;
+  X.spin_limit = ctx->spin_limit;
+  X.err = ctx->d_err;
+  static const int rest_per_sm = [] {
+    int v = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_collapse_rest<W>, kCollapseThreads, 0) != cudaSuccess ||
+        v < 1)
+      v = 1;
+    return v;
+  }();
+  if (b->n_tri <= kTopMax && b->n_wide_roots <= kTopRoots) {
+    X.small = (int)std::max<int64_t>(kSmallTree, ceil_div(b->n_tri, kTopSplit));
+    FLG_CUDA(ctx, launch_after(k_collapse_top<W>, 1, kTopThreads, st, X, wide));
+    FLG_LAUNCH_CHECK(ctx, "k_collapse_top");
+    FLG_CUDA(ctx, launch_after(k_collapse_rest<W>,
+                               grid_for(b->n_nodes, 2 * kCollapseThreads, (int64_t)ctx->num_sms * rest_per_sm),
+                               kCollapseThreads, st, X, wide));
+    FLG_LAUNCH_CHECK(ctx, "k_collapse_rest");
+    return FLG_OK;
+  }
   static const int per_sm = [] {
     int v = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_collapse_all<W>, kCollapseThreads, 0) != cudaSuccess ||
@@ -268,7 +515,6 @@ static int collapse_levels(flg_ctx ctx, flg_bvh b) {
       v = 1;
     return v;
   }();
-  int32_t *ctr = b->d_wide_ctr;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid_for(ceil_div(b->n_nodes, kCollapseNodes), kCollapseThreads, (int64_t)ctx->num_sms * per_sm));
   cfg.blockDim = dim3(kCollapseThreads);
@@ -278,17 +524,15 @@ static int collapse_levels(flg_ctx ctx, flg_bvh b) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  FLG_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_collapse_all<W>, (const Node2 *)b->d_nodes2, R, leaf, (int)b->n_wide_roots,
-                                   b->d_queue[0], b->d_queue[1], ctr, (uint32_t *)(ctr + 2), (int64_t)b->wide_cap, wide,
-                                   ctx->spin_limit, ctx->d_err));
+  FLG_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_collapse_all<W>, X, wide));
   FLG_LAUNCH_CHECK(ctx, "k_collapse_all");
   return FLG_OK;
 }
 
 int collapse_ctr_words() { return kCtrLive; }
 
-// Expects the counters and the first level's queue at their initial values
-// (k_build_setup, or flg_bvh_set_width's copies).
+// Expects the counters at their initial values (k_build_setup, or
+// flg_bvh_set_width's copy).
 int collapse_enqueue(flg_ctx ctx, flg_bvh b, int width) {
   if (b->n_wide_roots == 0) return FLG_OK;
   cudaStream_t st = ctx->stream;
@@ -317,11 +561,8 @@ FLG_API int flg_bvh_set_width(flg_ctx ctx, flg_bvh bvh, int32_t node_width, int3
     int rc = collapse_reserve(ctx, bvh);
     if (rc) return rc;
   }
-  if (bvh->n_wide_roots > 0) {
+  if (bvh->n_wide_roots > 0)
     FLG_CUDA(ctx, cudaMemcpyAsync(bvh->d_wide_ctr, bvh->d_wide_ctr + kCtrLive, sizeof(int32_t) * kCtrLive,
                                   cudaMemcpyDeviceToDevice, ctx->stream));
-    FLG_CUDA(ctx, cudaMemcpyAsync(bvh->d_queue[0], bvh->d_queue_init, sizeof(int2) * bvh->n_wide_roots,
-                                  cudaMemcpyDeviceToDevice, ctx->stream));
-  }
   return collapse_enqueue(ctx, bvh, node_width);
 }

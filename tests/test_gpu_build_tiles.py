@@ -89,3 +89,44 @@ def test_captured_build_traces_like_the_oracle(oracle, width, counts):
             assert bad == 0, (trial, k)
     ctx2.lib.flg_graph_destroy(g)
     ctx2.close()
+
+
+@pytest.mark.parametrize("width", [4, 8])
+@pytest.mark.parametrize("n", [(1 << 20), (1 << 20) + 1])
+def test_either_collapse_of_a_scene(ctx, width, n):
+    """On either side of the rule for collapsing in subtrees: the hits of the
+    binary tree, which has none to collapse."""
+    import fledge_gb300 as F
+    pos = F.gen_triangles(ctx, n, 21)
+    rays = F.Rays.from_soa(F.gen_rays(ctx, 20000, 22), tmin=1e-4)
+    out = []
+    for w in (2, width):
+        b = F.RadixBVHBuilder(F.InternalTriangleMesh(pos), ctx, node_width=w)
+        b.build()
+        b.build()
+        out.append(U.host(b.intersect(rays)))
+    ctx.sync()
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k]), k
+
+
+@pytest.mark.parametrize("scenes", [1024, 1025])
+def test_either_collapse_of_a_batch(ctx, scenes):
+    import fledge_gb300 as F
+    rng = np.random.default_rng(5)
+    counts = rng.integers(0, 40, scenes)
+    counts[7] = 3000
+    counts[counts < 2] = 2  # as many roots as scenes
+    offs = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+    roff = np.arange(scenes + 1, dtype=np.int64) * 20
+    pos = U.dev(G.random_soup(int(offs[-1]), rng, half=0.1))
+    rays, _ = U.rays_dev(G.sphere_rays(int(roff[-1]), rng))
+    out = []
+    for w in (2, 4):
+        b = F.BatchedRadixBVHBuilder(F.InternalTriangleMesh(pos), offs, ctx, node_width=w)
+        b.build()
+        b.build()
+        out.append(U.host(b.intersect_batched(rays, roff)))
+    ctx.sync()
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k]), k
