@@ -9,6 +9,8 @@
 //   2. k_morton_hist   30-bit Morton code per triangle (radix_bvh.cpp:63-73)
 //                      plus the digit histograms of every sort pass
 //   3. sort            onesweep radix sort (sort.cu)
+//   (a single scene of up to 32,768 triangles: 0 to 3 in one cluster,
+//   k_small_sort)
 //   4. k_climb         the Karras tree (radix_bvh.cpp:118-161) and its refit
 //                      (radix_bvh.cpp:163-199) in one bottom-up pass: lanes
 //                      over sorted leaves gather the triangle into the sorted
@@ -69,10 +71,10 @@ struct BuildSetup {
   uint32_t *flags;
   int64_t n_nodes;
   const uint32_t *dirty;
+  uint32_t *dirty_out;  // the same, for k_small_sort
 };
 
-__global__ void __launch_bounds__(256) k_build_setup(BuildSetup B) {
-  after_wait();
+__device__ __forceinline__ void build_setup(const BuildSetup &B) {
   const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = t0; i < 6 * (int64_t)B.n_scenes; i += step)
     B.box[i] = i % 6 < 3 ? 3.402823466e+38f : -3.402823466e+38f;
@@ -88,6 +90,11 @@ __global__ void __launch_bounds__(256) k_build_setup(BuildSetup B) {
       B.flags[i] = 0u;
     }
   }
+}
+
+__global__ void __launch_bounds__(256) k_build_setup(BuildSetup B) {
+  after_wait();
+  build_setup(B);
 }
 
 constexpr int kBoundsThreads = 256;
@@ -144,6 +151,22 @@ __global__ void __launch_bounds__(kBoundsThreads)
   }
 }
 
+// The correctly rounded (lo + hi) / 2: 0.5 is exact.
+__device__ __forceinline__ float box_center(float lo, float hi) { return (lo + hi) * 0.5f; }
+
+// Morton code of a box center against the scene box sb.
+__device__ __forceinline__ uint32_t morton_at(const float (&c)[3], const float *sb) {
+  uint32_t q[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    float slo = sb[k], shi = sb[3 + k];
+    float e = shi - slo;
+    float nrm = e == 0.0f ? 0.0f : __fdiv_rn(c[k] - slo, e);
+    q[k] = to_u32(nrm * 1024.0f);
+  }
+  return (left_shift3(q[2]) << 2) | (left_shift3(q[1]) << 1) | left_shift3(q[0]);
+}
+
 // Morton code of triangle t against its scene box sb (radix_bvh.cpp:63-73,
 // experimental_utils.hpp:33-45).
 __device__ __forceinline__ uint32_t morton_of(const float *__restrict__ pos, const int32_t *__restrict__ idx,
@@ -152,16 +175,10 @@ __device__ __forceinline__ uint32_t morton_of(const float *__restrict__ pos, con
   tri_verts(pos, idx, t, p0, p1, p2);
   float lo[3], hi[3];
   tri_box(p0, p1, p2, lo, hi);
-  uint32_t q[3];
+  float c[3];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    float slo = sb[k], shi = sb[3 + k];
-    float e = shi - slo;
-    float c = (lo[k] + hi[k]) * 0.5f;  // = the correctly rounded (lo + hi) / 2: 0.5 is exact
-    float nrm = e == 0.0f ? 0.0f : __fdiv_rn(c - slo, e);
-    q[k] = to_u32(nrm * 1024.0f);
-  }
-  return (left_shift3(q[2]) << 2) | (left_shift3(q[1]) << 1) | left_shift3(q[0]);
+  for (int k = 0; k < 3; ++k) c[k] = box_center(lo[k], hi[k]);
+  return morton_at(c, sb);
 }
 
 // Morton code of every triangle and the per-pass digit histograms.
@@ -220,6 +237,244 @@ __global__ void __launch_bounds__(256)
     const uint32_t c = (&s_hist[0][0])[i];
     if (c) atomicAdd(&h[i], c);
   }
+}
+
+// Scene bounds, codes and their sort of one scene of at most kSmallMax triangles,
+// in one thread block cluster: setup, bounds, codes and four onesweep passes are
+// seven launches whose kernels each wait for L2 a few times and do next to
+// nothing.  Here a CTA keeps a run of `tile` = 1024 x ITEMS positions in its
+// registers and shared memory, and what a launch boundary did is a cluster
+// barrier.  A pass: each warp ranks its keys as k_onesweep does, each CTA sends
+// its digit counts to all others, and then the pairs to the CTAs that own their
+// new positions.  Padding has keys above every code and stays at the end.
+// Builds, us, seven launches -> this: 700 triangles 65 -> 58, 5,000 69 -> 61, 16,384
+// 79 -> 72, 20,001 82 -> 78, 32,768 96 -> 93; with three and four positions per
+// thread (40,000 and 60,000 triangles) 98 -> 98 and 101 -> 104: each adds 5 us for
+// the scattered 8-byte stores into other SMs.  Clusters of 8 CTAs, the most that
+// need no opt-in: 16,384 74, 20,001 81.
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr int kSmallCtas = 16;
+constexpr int kSmallItems = 2;
+constexpr int64_t kSmallMax = (int64_t)kSmallThreads * kSmallCtas * kSmallItems;
+
+// The address of a shared variable in CTA r of the cluster.
+__device__ __forceinline__ uint32_t in_cta(const void *p, uint32_t r) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(r));
+  return a;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ void cluster_barrier() {
+  cluster_arrive();
+  cluster_wait();
+}
+
+template <int ITEMS>
+__global__ void __launch_bounds__(kSmallThreads, 1)
+    k_small_sort(const float *__restrict__ pos, const int32_t *__restrict__ idx, int n, float *__restrict__ scene_box,
+                 uint32_t *__restrict__ keys, uint32_t *__restrict__ perm, BuildSetup B) {
+  constexpr int kTile = kSmallThreads * ITEMS;
+  extern __shared__ uint2 s_kv[];  // [kTile]
+  __shared__ uint32_t s_whist[kSmallWarps][256];
+  __shared__ uint32_t s_tot[kSmallCtas][256];
+  __shared__ uint32_t s_base[256];
+  __shared__ uint32_t s_wsum[8];
+  __shared__ float s_red[6][kSmallWarps];
+  __shared__ float s_box[kSmallCtas][6];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ctas = gridDim.x, me = blockIdx.x;  // one cluster
+  const int first = warp * 32 * ITEMS + lane;   // of this lane's items in the tile, 32 apart
+  cluster_arrive();
+  after_wait();
+  build_setup(B);
+
+  // Bounds.
+  float v[6] = {3.402823466e+38f, 3.402823466e+38f, 3.402823466e+38f,
+                -3.402823466e+38f, -3.402823466e+38f, -3.402823466e+38f};
+  float c[ITEMS][3];
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const int t = me * kTile + first + j * 32;
+    if (t < n) {
+      float3 p0, p1, p2;
+      tri_verts(pos, idx, t, p0, p1, p2);
+      float lo[3], hi[3];
+      tri_box(p0, p1, p2, lo, hi);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        v[k] = fminf(v[k], lo[k]);
+        v[3 + k] = fmaxf(v[3 + k], hi[k]);
+        c[j][k] = box_center(lo[k], hi[k]);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) c[j][k] = 0.0f;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      v[k] = fminf(v[k], __shfl_xor_sync(0xFFFFFFFFu, v[k], o));
+      v[3 + k] = fmaxf(v[3 + k], __shfl_xor_sync(0xFFFFFFFFu, v[3 + k], o));
+    }
+  }
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < 6; ++k) s_red[k][warp] = v[k];
+  __syncthreads();
+  cluster_wait();  // every CTA runs: its shared memory can be written
+  if (warp < 6) {
+    float r = s_red[warp][lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float x = __shfl_xor_sync(0xFFFFFFFFu, r, o);
+      r = warp < 3 ? fminf(r, x) : fmaxf(r, x);
+    }
+    if (lane < ctas)
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(in_cta(&s_box[me][warp], lane)), "f"(r) : "memory");
+  }
+  cluster_barrier();
+  float sb[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    sb[k] = s_box[0][k];
+    for (int r = 1; r < ctas; ++r) sb[k] = k < 3 ? fminf(sb[k], s_box[r][k]) : fmaxf(sb[k], s_box[r][k]);
+  }
+  if (me == 0 && tid == 0) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) scene_box[k] = sb[k];
+    *B.dirty_out = 0u;  // every CTA has seen it
+  }
+
+  // Codes.
+  uint32_t key[ITEMS], val[ITEMS], rank[ITEMS];
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    val[j] = (uint32_t)(me * kTile + first + j * 32);
+    key[j] = (int)val[j] < n ? morton_at(c[j], sb) : 0xFFFFFFFFu;
+  }
+
+  // Sort.
+  const uint32_t lt = (1u << lane) - 1u;
+  for (int shift = 0; shift < 32; shift += 8) {
+#pragma unroll
+    for (int i = 0; i < 256; i += 32) s_whist[warp][i + lane] = 0u;
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const uint32_t d = (key[j] >> shift) & 0xFFu;
+      uint32_t peers = 0xFFFFFFFFu;
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, (d >> b) & 1u);
+        peers &= ((d >> b) & 1u) ? m : ~m;
+      }
+      // one lane per digit: no atomic needed
+      const uint32_t before = s_whist[warp][d];
+      __syncwarp();
+      if ((peers & lt) == 0u) s_whist[warp][d] = before + __popc(peers);
+      __syncwarp();
+      rank[j] = before + __popc(peers & lt);
+    }
+    __syncthreads();
+    if (tid < 256) {
+      uint32_t total = 0u;
+#pragma unroll
+      for (int w = 0; w < kSmallWarps; ++w) {
+        const uint32_t x = s_whist[w][tid];
+        s_whist[w][tid] = total;
+        total += x;
+      }
+      for (int r = 0; r < ctas; ++r)
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(in_cta(&s_tot[me][tid], r)), "r"(total) : "memory");
+    }
+    cluster_barrier();  // and the pairs of the pass before are all in registers
+    if (tid < 256) {
+      uint32_t all = 0u, before = 0u;
+      for (int r = 0; r < ctas; ++r) {
+        if (r == me) before = all;
+        all += s_tot[r][tid];
+      }
+      uint32_t x = all;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane == 31) s_wsum[warp] = x;
+      s_base[tid] = x - all + before;
+    }
+    __syncthreads();
+    if (tid < 256) {
+      uint32_t sum = 0u;
+#pragma unroll
+      for (int w = 0; w < 7; ++w)
+        if (w < warp) sum += s_wsum[w];
+      s_base[tid] += sum;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const uint32_t d = (key[j] >> shift) & 0xFFu;
+      const uint32_t to = s_base[d] + s_whist[warp][d] + rank[j];
+      const uint32_t owner = to / (uint32_t)kTile;
+      asm volatile("st.shared::cluster.v2.u32 [%0], {%1, %2};" ::"r"(in_cta(s_kv + (to - owner * kTile), owner)),
+                   "r"(key[j]), "r"(val[j])
+                   : "memory");
+    }
+    cluster_barrier();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const uint2 kv = s_kv[first + j * 32];
+      key[j] = kv.x;
+      val[j] = kv.y;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const int at = me * kTile + first + j * 32;
+    if (at < n) {
+      keys[at] = key[j];
+      perm[at] = val[j];
+    }
+  }
+}
+
+// k_small_sort with as few positions per thread, and then as few CTAs, as hold
+// the scene.
+template <int ITEMS>
+static cudaError_t launch_small(flg_ctx ctx, flg_bvh b, const BuildSetup &B) {
+  if constexpr (ITEMS < kSmallItems) {
+    if (b->n_tri > (int64_t)kSmallThreads * kSmallCtas * ITEMS) return launch_small<ITEMS + 1>(ctx, b, B);
+  }
+  constexpr int kBytes = kSmallThreads * ITEMS * (int)sizeof(uint2);
+  if (!(ctx->small_sort_ready >> ITEMS & 1u)) {
+    cudaError_t e = cudaFuncSetAttribute(k_small_sort<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_small_sort<ITEMS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    ctx->small_sort_ready |= 1u << ITEMS;
+  }
+  unsigned ctas = 1;
+  while ((int64_t)ctas * kSmallThreads * ITEMS < b->n_tri) ctas *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(kSmallThreads);
+  cfg.dynamicSmemBytes = kBytes;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ctas;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, k_small_sort<ITEMS>, b->pos, b->idx, (int)b->n_tri, b->d_scene_box, b->d_keys,
+                            b->d_perm, B);
 }
 
 // delta of radix_bvh.hpp:68-74 between neighbouring sorted positions i and
@@ -457,7 +712,14 @@ int build_enqueue(flg_ctx ctx, flg_bvh b) {
   BuildSetup B = {};
   B.box = b->d_scene_box;
   B.n_scenes = b->n_scenes;
+  const bool small = !sah && b->n_scenes == 1 && n <= kSmallMax;
   if (!sah) {
+    B.slots = b->d_slots;
+    B.flags = b->d_flags;
+    B.n_nodes = b->n_nodes;
+    B.dirty = B.dirty_out = b->d_dirty;
+  }
+  if (!sah && !small) {
     B.hist = b->d_tile_start ? b->d_shist : b->d_hist;
     B.n_hist = b->d_tile_start ? 4 * 256 * (int64_t)b->n_scenes : 256 * (int64_t)b->n_morton_passes;
     B.tile_ctr = b->d_tile_ctr;
@@ -467,48 +729,51 @@ int build_enqueue(flg_ctx ctx, flg_bvh b) {
     B.scene_hist = b->d_hist + 256 * b->n_morton_passes;
     B.scene_hist_init = b->d_hist + 256 * b->n_passes;
     B.n_scene_hist = 256 * (b->n_passes - b->n_morton_passes);
-    B.slots = b->d_slots;
-    B.flags = b->d_flags;
-    B.n_nodes = b->n_nodes;
-    B.dirty = b->d_dirty;
   }
   if (b->width > 2 && b->d_wide_ctr) {
     B.wide_ctr = b->d_wide_ctr;
     B.n_wide_ctr = collapse_ctr_words();
   }
-  FLG_CUDA(ctx, launch_after(k_build_setup,
-                             grid_for(std::max<int64_t>(B.n_lookback, 6 * (int64_t)b->n_scenes), 256,
-                                      (int64_t)ctx->num_sms * 8),
-                             256, st, B));
-  FLG_LAUNCH_CHECK(ctx, "k_build_setup");
-  stage_mark(ctx, st, "setup");
-  const int chunk = (int)std::min<int64_t>(
-      kBoundsChunkMax, ceil_div(ceil_div(n, (int64_t)ctx->num_sms * 8), kBoundsThreads) * kBoundsThreads);
-  FLG_CUDA(ctx, launch_after(k_scene_bounds, grid_for(n, chunk), kBoundsThreads, st, b->pos, b->idx, n, b->d_tri_off,
-                             b->n_scenes, chunk, b->d_scene_box));
-  FLG_LAUNCH_CHECK(ctx, "k_scene_bounds");
-  stage_mark(ctx, st, "bounds");
-  if (sah) {
-    int rc = sah_build(ctx, b);
-    if (rc) return rc;
-    if (b->width > 2) return collapse_enqueue(ctx, b, b->width);
-    return FLG_OK;
-  }
-  uint32_t *morton_out = (b->n_passes % 2 == 0) ? b->d_keys : b->d_keys_alt;
-  if (b->d_tile_start) {
-    FLG_CUDA(ctx, launch_after(k_morton_seg, (unsigned)b->n_tiles, 256, st, b->pos, b->idx, b->d_tri_off, b->n_scenes,
-                               b->d_tile_start, (int)sort_tile(b->sort_items), b->d_scene_box, morton_out, b->d_shist,
-                               b->d_dirty));
-    FLG_LAUNCH_CHECK(ctx, "k_morton_seg");
+  if (small) {
+    B.n_scenes = 0;  // the box is written whole
+    FLG_CUDA(ctx, launch_small<1>(ctx, b, B));
+    FLG_LAUNCH_CHECK(ctx, "k_small_sort");
+    stage_mark(ctx, st, "small_sort");
   } else {
-    const unsigned g_elem = grid_for(n, 256, (int64_t)ctx->num_sms * 8);
-    FLG_CUDA(ctx, launch_after(k_morton_hist, g_elem, 256, st, b->pos, b->idx, n, b->d_tri_off, b->n_scenes,
-                               b->d_scene_box, morton_out, b->d_hist, b->n_morton_passes, b->d_dirty));
-    FLG_LAUNCH_CHECK(ctx, "k_morton_hist");
+    FLG_CUDA(ctx, launch_after(k_build_setup,
+                               grid_for(std::max<int64_t>(B.n_lookback, 6 * (int64_t)b->n_scenes), 256,
+                                        (int64_t)ctx->num_sms * 8),
+                               256, st, B));
+    FLG_LAUNCH_CHECK(ctx, "k_build_setup");
+    stage_mark(ctx, st, "setup");
+    const int chunk = (int)std::min<int64_t>(
+        kBoundsChunkMax, ceil_div(ceil_div(n, (int64_t)ctx->num_sms * 8), kBoundsThreads) * kBoundsThreads);
+    FLG_CUDA(ctx, launch_after(k_scene_bounds, grid_for(n, chunk), kBoundsThreads, st, b->pos, b->idx, n, b->d_tri_off,
+                               b->n_scenes, chunk, b->d_scene_box));
+    FLG_LAUNCH_CHECK(ctx, "k_scene_bounds");
+    stage_mark(ctx, st, "bounds");
+    if (sah) {
+      int rc = sah_build(ctx, b);
+      if (rc) return rc;
+      if (b->width > 2) return collapse_enqueue(ctx, b, b->width);
+      return FLG_OK;
+    }
+    uint32_t *morton_out = (b->n_passes % 2 == 0) ? b->d_keys : b->d_keys_alt;
+    if (b->d_tile_start) {
+      FLG_CUDA(ctx, launch_after(k_morton_seg, (unsigned)b->n_tiles, 256, st, b->pos, b->idx, b->d_tri_off, b->n_scenes,
+                                 b->d_tile_start, (int)sort_tile(b->sort_items), b->d_scene_box, morton_out, b->d_shist,
+                                 b->d_dirty));
+      FLG_LAUNCH_CHECK(ctx, "k_morton_seg");
+    } else {
+      const unsigned g_elem = grid_for(n, 256, (int64_t)ctx->num_sms * 8);
+      FLG_CUDA(ctx, launch_after(k_morton_hist, g_elem, 256, st, b->pos, b->idx, n, b->d_tri_off, b->n_scenes,
+                                 b->d_scene_box, morton_out, b->d_hist, b->n_morton_passes, b->d_dirty));
+      FLG_LAUNCH_CHECK(ctx, "k_morton_hist");
+    }
+    stage_mark(ctx, st, "morton");
+    if (int rc = sort_enqueue(ctx, b)) return rc;
   }
-  stage_mark(ctx, st, "morton");
-  int rc = sort_enqueue(ctx, b);
-  if (rc) return rc;
+  int rc;
   if (b->builder == FLG_BUILDER_PLOC) {
     rc = ploc_build(ctx, b);
     if (rc) return rc;

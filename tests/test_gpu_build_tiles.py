@@ -130,3 +130,16 @@ def test_either_collapse_of_a_batch(ctx, scenes):
     ctx.sync()
     for k in out[0]:
         assert np.array_equal(out[0][k], out[1][k]), k
+
+
+@pytest.mark.parametrize("n", [1, 2, 2048, 2049, 8193, 16384, 16385, 20001, 32767, 32768, 32769])
+def test_cluster_sort_edges(ctx, oracle, n):
+    """Cluster sizes, positions per thread and the last size of the sort in one
+    cluster; the second scene has only three different codes."""
+    for pos in (G.random_soup(n, np.random.default_rng(n)),
+                np.tile(G.random_soup(3, np.random.default_rng(1)), ((n + 2) // 3, 1))[:3 * n]):
+        b, _ = U.gpu_build(ctx, pos)
+        b.build()
+        if n > 1:
+            U.assert_same_topology(b.topology(), oracle.build_bvh(pos))
+    ctx.sync()
