@@ -41,13 +41,14 @@ __device__ __forceinline__ void load_vray(const VRays &R, int64_t i, float3 &o, 
 // tracking: two, a Philox block's draws) is one turn of the warp's loop.
 // Together with one bounds test and one address per lattice cell (grid_cell), us
 // before -> after: delta tracking of 2 M rays through a 192^3 sparse grid 927 ->
-// 547 and, two steps to a turn, 460; of 1 M rays through a 256^3 dense one 83 ->
+// 547, with two steps to a turn 460, and with 32-bit addresses and refills at 4
+// idle lanes 434 (8: 446); of 1 M rays through a 256^3 dense one 83 ->
 // 52 -> 47; ratio tracking of the latter 85 -> 75, its adjoint 85 -> 79.  Ratio
 // tracking, which waits for scattered sectors of the grid (29 % of L2's and 30 %
 // of DRAM's rate, L1 at 41 %), gains nothing from turns of four draws (76 us,
-// the adjoint 85), nor from lookups of steps ahead.  Refills at 4 idle lanes: 454
-// and 81 us; at 16 520 and 77.
-constexpr int kVolRefill = 8;
+// the adjoint 85), nor from lookups of steps ahead; with refills at 4 idle lanes it
+// takes 81 us, at 16 77.
+constexpr int kVolRefill = 8, kSampleRefill = 4;
 
 struct WarpChunk {
   int64_t next, end;
@@ -59,11 +60,12 @@ struct WarpChunk {
   }
   // The ray that this lane takes now, or -1; all lanes call it.  `left`: false
   // once every lane is idle and the chunk is empty.
+  template <int REFILL = kVolRefill>
   __device__ __forceinline__ int64_t take(bool busy, bool &left) {
     const unsigned idle = __ballot_sync(0xFFFFFFFFu, !busy);
     const int nidle = __popc(idle);
     left = next < end || nidle < 32;
-    if (next >= end || nidle < kVolRefill) return -1;
+    if (next >= end || nidle < REFILL) return -1;
     const int64_t my = next + __popc(idle & ((1u << (threadIdx.x & 31u)) - 1u));
     next += nidle;
     return !busy && my < end ? my : -1;
@@ -222,7 +224,7 @@ __global__ void __launch_bounds__(256, 4)
   int64_t ray = -1;
   while (true) {
     bool left;
-    const int64_t my = chunk.take(ray >= 0, left);
+    const int64_t my = chunk.take<kSampleRefill>(ray >= 0, left);
     if (!left) break;
     int r = ray >= 0 ? 0 : -1;
     if (my >= 0) {

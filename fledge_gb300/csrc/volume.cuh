@@ -68,26 +68,27 @@ __device__ __forceinline__ void grid_cell(const GridDev &G, int x, int y, int z,
 #pragma unroll
       for (int c = 0; c < 8; ++c) v[c] = __ldg(p + (c >> 2) * sz + (c >> 1 & 1) * (int64_t)G.nx + (c & 1));
     } else {
+      // 32 bits hold a brick's index: a lattice that fits in memory has fewer
       const unsigned ox = (unsigned)x % kBrick, oy = (unsigned)y % kBrick, oz = (unsigned)z % kBrick;
-      const int32_t *bp = G.bidx + ((int64_t)((unsigned)z / kBrick) * G.bny + (unsigned)y / kBrick) * G.bnx +
-                          (unsigned)x / kBrick;
+      const uint32_t brick = ((unsigned)z / kBrick * (uint32_t)G.bny + (unsigned)y / kBrick) * (uint32_t)G.bnx +
+                             (unsigned)x / kBrick;
       // brick step and offset in the brick of the upper plane of each axis
       const bool nx = ox == kBrick - 1, ny = oy == kBrick - 1, nz = oz == kBrick - 1;
-      const int64_t sx = nx, sy = ny ? G.bnx : 0, sz = nz ? (int64_t)G.bny * G.bnx : 0;
-      const unsigned ux = nx ? 0 : ox + 1, uy = (ny ? 0 : oy + 1) * kBrick, uz = (nz ? 0 : oz + 1) * kBrick * kBrick;
-      const unsigned ly = oy * kBrick, lz = oz * kBrick * kBrick;
+      const uint32_t sx = nx, sy = ny ? G.bnx : 0, sz = nz ? (uint32_t)G.bny * (uint32_t)G.bnx : 0;
+      const uint32_t ux = nx ? 0 : ox + 1, uy = (ny ? 0 : oy + 1) * kBrick, uz = (nz ? 0 : oz + 1) * kBrick * kBrick;
+      const uint32_t ly = oy * kBrick, lz = oz * kBrick * kBrick;
       int32_t slot[8];
-      slot[0] = __ldg(bp);
+      slot[0] = __ldg(G.bidx + brick);
 #pragma unroll
       for (int c = 1; c < 8; ++c)
         slot[c] = ((c & 1) && nx) || ((c & 2) && ny) || ((c & 4) && nz)
-                      ? __ldg(bp + (c & 4 ? sz : 0) + (c & 2 ? sy : 0) + (c & 1 ? sx : 0))
+                      ? __ldg(G.bidx + (brick + (c & 4 ? sz : 0) + (c & 2 ? sy : 0) + (c & 1 ? sx : 0)))
                       : slot[0];
 #pragma unroll
-      for (int c = 0; c < 8; ++c)
-        v[c] = slot[c] < 0 ? 0.0f
-                           : __ldg(G.rho + (int64_t)slot[c] * (kBrick * kBrick * kBrick) +
-                                   ((c & 4 ? uz : lz) + (c & 2 ? uy : ly) + (c & 1 ? ux : ox)));
+      for (int c = 0; c < 8; ++c) {
+        const float *p = G.rho + ((c & 4 ? uz : lz) + (c & 2 ? uy : ly) + (c & 1 ? ux : ox));
+        v[c] = slot[c] < 0 ? 0.0f : __ldg(p + (int64_t)slot[c] * (kBrick * kBrick * kBrick));
+      }
     }
   } else {
 #pragma unroll
