@@ -98,6 +98,11 @@ FLG_API int flg_ctx_destroy(flg_ctx c) {
     cudaStreamSynchronize(c->copy_stream);
     cudaStreamDestroy(c->copy_stream);
   }
+  if (c->pt_side) {
+    cudaStreamSynchronize(c->pt_side);
+    cudaStreamDestroy(c->pt_side);
+  }
+  if (c->pt_fork) cudaEventDestroy(c->pt_fork);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   for (int k = 0; k < 4; ++k)
     if (c->ev[k]) cudaEventDestroy(c->ev[k]);

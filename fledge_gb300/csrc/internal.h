@@ -113,6 +113,9 @@ struct flg_ctx_t {
   // that the device writes, and an event behind each.
   int32_t *pt_counts = nullptr;
   cudaEvent_t pt_event[4] = {};
+  // Its stream for shadow rays, and the event between the two.
+  cudaStream_t pt_side = nullptr;
+  cudaEvent_t pt_fork = nullptr;
   // Ray-sort scratch of trace_enqueue (grown on demand).
   void *rs_buf = nullptr;
   size_t rs_bytes = 0;
