@@ -68,3 +68,30 @@ def test_adjoint_into_unaligned_buffers(ctx, oracle, shape, offset):
     assert np.all(np.abs(g - np.asarray(ref).reshape(-1)) <= 1e-4 * scale)
     rest = torch.cat([buf[:offset], buf[offset + rho.size:]])
     assert bool((rest == 7.0).all())
+
+
+@pytest.mark.parametrize("side_by_side", [True, False])
+@pytest.mark.parametrize("over", [0, 1])
+def test_many_rays(ctx, oracle, over, side_by_side):
+    """On either side of the rule for warps of 256 rays: every ray's result is
+    that of the same ray (the same stream) in the oracle, checked at the ends
+    and in a seeded sample, and no ray is left out."""
+    import fledge_gb300 as F
+    n = torch.cuda.get_device_properties(0).multi_processor_count * 4 * 8 * 512 + over
+    rho = _grid((9, 8, 17))
+    rng = np.random.default_rng(4)
+    r8 = G.sphere_rays(n, rng)
+    if side_by_side:
+        r8[0:3] = np.array([[0.5], [0.5], [-2.0]], np.float32)
+        d = np.stack([np.linspace(-0.3, 0.3, n), np.full(n, 0.05), np.ones(n)])
+        r8[3:6] = d / np.linalg.norm(d, axis=0)
+    r8 = r8.astype(np.float32)
+    rd, _ = U.rays_dev(r8)
+    vol = F.DenseGridVolume(U.dev(rho), medium=F.Medium(3.2, 0.8, 0.3), ctx=ctx)
+    T, ck = vol.tr(rd, 5, checkpoint=True)
+    T, k = T.cpu().numpy(), ck["k"].cpu().numpy().view(np.uint32)
+    ok = vol.sample(rd, 6)[0].cpu().numpy()
+    To, cko = oracle.volume_tr(rho, (0.0,) * 3, (1.0,) * 3, Medium, r8, 5, want_ckpt=True)
+    so = np.asarray(oracle.volume_sample(rho, (0.0,) * 3, (1.0,) * 3, Medium, r8, 6)[0])
+    assert np.array_equal(T, To) and np.array_equal(k, cko["k"]) and np.array_equal(ok.reshape(-1), so.reshape(-1))
+    ctx.sync()
