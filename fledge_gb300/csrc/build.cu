@@ -443,29 +443,12 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
   }
 }
 
-// k_small_sort with as few positions per thread, and then as few CTAs, as hold
-// the scene.
-template <int ITEMS>
-static cudaError_t launch_small(flg_ctx ctx, flg_bvh b, const BuildSetup &B) {
-  if constexpr (ITEMS < kSmallItems) {
-    if (b->n_tri > (int64_t)kSmallThreads * kSmallCtas * ITEMS) return launch_small<ITEMS + 1>(ctx, b, B);
-  }
-  constexpr int kBytes = kSmallThreads * ITEMS * (int)sizeof(uint2);
-  if (!(ctx->small_sort_ready >> ITEMS & 1u)) {
-    cudaError_t e = cudaFuncSetAttribute(k_small_sort<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_small_sort<ITEMS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-    ctx->small_sort_ready |= 1u << ITEMS;
-  }
-  unsigned ctas = 1;
-  while ((int64_t)ctas * kSmallThreads * ITEMS < b->n_tri) ctas *= 2;
-  cudaLaunchConfig_t cfg = {};
+static void small_config(flg_ctx ctx, int items, unsigned ctas, cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&attr)[2]) {
+  cfg = {};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(kSmallThreads);
-  cfg.dynamicSmemBytes = kBytes;
+  cfg.dynamicSmemBytes = kSmallThreads * items * sizeof(uint2);
   cfg.stream = ctx->stream;
-  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = ctas;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
@@ -473,8 +456,38 @@ static cudaError_t launch_small(flg_ctx ctx, flg_bvh b, const BuildSetup &B) {
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, k_small_sort<ITEMS>, b->pos, b->idx, (int)b->n_tri, b->d_scene_box, b->d_keys,
-                            b->d_perm, B);
+}
+
+// Allows k_small_sort its shared memory and its cluster size; false if the device
+// (a slice of one, say) has no room for such a cluster.
+template <int ITEMS>
+static bool allow_small(flg_ctx ctx) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[2];
+  small_config(ctx, ITEMS, kSmallCtas, cfg, attr);
+  cfg.numAttrs = 1;
+  int n = 0;
+  const bool ok = cudaFuncSetAttribute(k_small_sort<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)cfg.dynamicSmemBytes) == cudaSuccess &&
+                  cudaFuncSetAttribute(k_small_sort<ITEMS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                      cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&n, k_small_sort<ITEMS>, &cfg) == cudaSuccess && n > 0;
+  if (!ok) cudaGetLastError();
+  return ok;
+}
+
+// k_small_sort with as few positions per thread, and then as few CTAs, as hold
+// the scene.
+static_assert(kSmallItems == 2);
+static cudaError_t launch_small(flg_ctx ctx, flg_bvh b, const BuildSetup &B) {
+  const int items = b->n_tri <= (int64_t)kSmallThreads * kSmallCtas ? 1 : 2;
+  unsigned ctas = 1;
+  while ((int64_t)ctas * kSmallThreads * items < b->n_tri) ctas *= 2;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[2];
+  small_config(ctx, items, ctas, cfg, attr);
+  return cudaLaunchKernelEx(&cfg, items == 1 ? k_small_sort<1> : k_small_sort<2>, b->pos, b->idx, (int)b->n_tri,
+                            b->d_scene_box, b->d_keys, b->d_perm, B);
 }
 
 // delta of radix_bvh.hpp:68-74 between neighbouring sorted positions i and
@@ -712,7 +725,9 @@ int build_enqueue(flg_ctx ctx, flg_bvh b) {
   BuildSetup B = {};
   B.box = b->d_scene_box;
   B.n_scenes = b->n_scenes;
-  const bool small = !sah && b->n_scenes == 1 && n <= kSmallMax;
+  bool small = !sah && b->n_scenes == 1 && n <= kSmallMax;
+  if (small && ctx->small_sort == 0) ctx->small_sort = allow_small<1>(ctx) && allow_small<2>(ctx) ? 1 : -1;
+  small = small && ctx->small_sort > 0;
   if (!sah) {
     B.slots = b->d_slots;
     B.flags = b->d_flags;
@@ -736,7 +751,7 @@ int build_enqueue(flg_ctx ctx, flg_bvh b) {
   }
   if (small) {
     B.n_scenes = 0;  // the box is written whole
-    FLG_CUDA(ctx, launch_small<1>(ctx, b, B));
+    FLG_CUDA(ctx, launch_small(ctx, b, B));
     FLG_LAUNCH_CHECK(ctx, "k_small_sort");
     stage_mark(ctx, st, "small_sort");
   } else {

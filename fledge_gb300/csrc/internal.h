@@ -108,7 +108,7 @@ struct flg_ctx_t {
   // Wavefront queues of flg_pathtrace (grown on demand).
   void *pt_buf = nullptr;
   size_t pt_bytes = 0;
-  uint32_t small_sort_ready = 0;  // bit i: k_small_sort<i> is set up on this device
+  int small_sort = 0;  // k_small_sort on this device: 0 not asked yet, 1 set up, -1 no room for its cluster
   // Path tracer: the queue lengths of its last iterations, in pinned host memory
   // that the device writes, and an event behind each.
   int32_t *pt_counts = nullptr;

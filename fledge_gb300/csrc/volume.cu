@@ -75,7 +75,7 @@ struct WarpChunk {
   }
   // After 32 rays have been taken together (`mine`: one of them is this lane's):
   // a warp whose rays lie side by side takes all of the next ones together, too.
-  __device__ __forceinline__ void judge(const GridDev &G, bool mine, const float3 &o, const float3 &d) {
+  __device__ __forceinline__ void adapt(const GridDev &G, bool mine, const float3 &o, const float3 &d) {
     const int src = __ffs(__ballot_sync(0xFFFFFFFFu, mine)) - 1;
     const float ox = (o.x - __shfl_sync(0xFFFFFFFFu, o.x, src)) * G.scale[0];
     const float oy = (o.y - __shfl_sync(0xFFFFFFFFu, o.y, src)) * G.scale[1];
@@ -92,7 +92,7 @@ struct WarpChunk {
 template <bool SP>
 __global__ void __launch_bounds__(256, 4)
     k_volume_tr(GridDev G, VRays R, int64_t n, uint64_t seed, float *__restrict__ T, float *__restrict__ ck_t,
-                uint32_t *__restrict__ ck_k, float *__restrict__ ck_c, bool judge) {
+                uint32_t *__restrict__ ck_k, float *__restrict__ ck_c, bool adapt) {
   after_wait();
   const float maj = __ldg(G.params), inv_maj = __ldg(G.params + 1);
   const float max_mu = G.sigma_t * maj;
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(256, 4)
       go = ratio_start(G, s, tmax, seed, ray);
       steps = 0;
     }
-    if (judge && chunk.fresh) chunk.judge(G, my >= 0, s.o, s.d);
+    if (adapt && chunk.fresh) chunk.adapt(G, my >= 0, s.o, s.d);
     if (go) go = ratio_step<SP>(G, max_mu, inv_maj, s) && ++steps < kMaxTrackSteps;
     if (!go && ray >= 0) {
       T[ray] = s.tr;
@@ -289,7 +289,7 @@ __global__ void k_grid_inv(float *params) {
 // come in order as others end: neighbouring chunks are under way at the same time,
 // so that rays that lie side by side find the grid in L2, and rays that miss the box
 // leave no SM idle.  Ratio tracking then also looks whether a warp's rays lie side by
-// side (WarpChunk::judge).  us, one wave -> this (one ray per thread before): 8.3 M
+// side (WarpChunk::adapt).  us, one wave -> this (one ray per thread before): 8.3 M
 // camera rays through 512^3 ratio tracking 1370 -> 790 (745), adjoint 1222 -> 755
 // (955), delta tracking 628 -> 458 (533), through a sparse grid 1721 -> 1574 (2622).
 // Scattered rays: 4.2 M through 256^3 271 -> 275 (301), 8.4 M through 100^3 485 -> 470
