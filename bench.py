@@ -52,7 +52,7 @@ SEED_C0, SEED_C2, SEED_C3 = S.SEED_SOUP, S.SEED_VOLUME, S.SEED_BATCH
 BYTES_PER_RAY = 24 + 16
 STAGE_BYTES_PER_TRI = {"bounds": 36, "morton": 48, "sort_pass": 16, "climb": 120}
 BYTES_PER_TRI = 268
-TRACE_PROFILE = os.path.join(ROOT, "profiles", "k_trace_ww_config3.json")
+TRACE_PROFILE = os.path.join(ROOT, "profiles", "k_trace4_config3.json")
 TRACE_SOURCES = ["fledge_gb300/csrc/trace.cu", "fledge_gb300/csrc/common.cuh", "fledge_gb300/csrc/internal.h"]
 TUNED = os.path.join(ROOT, "fledge_gb300", "tuned", "batched_config3.json")
 
@@ -833,7 +833,7 @@ def _graph_step(torch, F, ctx, b, pos, rays, hits, topts, dev):
     ctx2.sync()
     ctx2.lib.flg_graph_destroy(g)
     ctx2.close()
-    res["launches_per_step"] = "build (about 14 kernels) + trace (3), one graph launch when replayed"
+    res["launches_per_step"] = "build (10 kernels) + trace (3), one graph launch when replayed"
     return res
 
 
@@ -1003,8 +1003,7 @@ def run_c4(ctx, torch, F, dev, pk):
     sh = torch.cat([hp[:, hit], sd[:, hit], torch.full((1, n_sh), 1e-4, device=dev),
                     (dist[hit] * (1 - 1e-4))[None, :]], 0).contiguous()
     srays = F.Rays(*[sh[k] for k in range(8)])
-    # Coherent camera rays keep one thread per ray (4271 against 3627 Mrays/s persistent); the
-    # scattered shadow rays take the persistent while-while kernel (2765 against 2354 Mrays/s).
+    # (Options of the fp32 layouts; the 4-wide one has a single kernel.)
     sopts = dict(persistent=2, refill_lanes=16)
     occ = b.intersectP(srays, **sopts)
     sms = _time(torch, lambda: b.intersectP(srays, out=occ, **sopts), 3, s)
