@@ -233,7 +233,8 @@ __global__ void __launch_bounds__(kCollapseThreads)
 // the barrier, whatever its size, and the last ones, of a few nodes each, are
 // half of them.  us per collapse, k_collapse_all -> this: 5,000 triangles 48 ->
 // 29, 20,001 54 -> 31, 65,536 62 -> 37, 200,000 73 -> 46, 600,000 97 -> 80,
-// 1,000,000 108 -> 105, 2,000,000 152 -> 196.  `small`: n / 700, at least 128.
+// 1,000,000 108 -> 105, 2,000,000 152 -> 196.  `small`: 1.4 n / 2^k for the k at which
+// n / 2^k falls to 181, at most 10.
 // The top CTA is bound by instructions, so smaller subtrees cost (20,001
 // triangles in subtrees of 64: 51 us); and a warp takes long over larger ones
 // (200,000 in n / 256: 79).  Large scenes keep the levels: a warp's steps run
@@ -241,8 +242,8 @@ __global__ void __launch_bounds__(kCollapseThreads)
 constexpr int64_t kTopMax = 1 << 20;
 constexpr int kTopThreads = 256;
 constexpr int kTopRoots = 1024;
-constexpr int kTopSplit = 700;
-constexpr int kSmallTree = 128;
+constexpr int kTopSplit = 1024;
+constexpr int kSmallTree = 181;
 
 // Entries that this kernel writes and reads go through L2.
 __device__ __forceinline__ int2 item_at(const Collapse &X, int slot) {
@@ -499,7 +500,12 @@ static int collapse_levels(flg_ctx ctx, flg_bvh b) {
     return v;
   }();
   if (b->n_tri <= kTopMax && b->n_wide_roots <= kTopRoots) {
-    X.small = (int)std::max<int64_t>(kSmallTree, ceil_div(b->n_tri, kTopSplit));
+    // n / 2^k triangles are what a node of depth k has on average: cut between two
+    // depths, not through the middle of one (builds with small = max(128, n / 700)
+    // against this, us: 8,192 triangles 77 -> 67, 32,768 93 -> 84, 45,000 100 -> 95).
+    int64_t nodes = 1;
+    while (nodes < kTopSplit && b->n_tri > kSmallTree * nodes) nodes *= 2;
+    X.small = (int)(b->n_tri * 181 / (128 * nodes));
     FLG_CUDA(ctx, launch_after(k_collapse_top<W>, 1, kTopThreads, st, X, wide));
     FLG_LAUNCH_CHECK(ctx, "k_collapse_top");
     FLG_CUDA(ctx, launch_after(k_collapse_rest<W>,
