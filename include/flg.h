@@ -398,7 +398,10 @@ typedef struct flg_pt_stats {
 /* Renders the image into radiance (device, 3 floats per pixel, row-major,
  * mean over spp) as a wavefront: camera rays, closest hit, shading with
  * queue compaction, shadow rays with any hit, per bounce.  bvh must be built
- * over the same mesh.  Synchronises once per bounce. */
+ * over the same mesh.  Waits once per bounce for the lengths of its queues:
+ * over a 4-wide handle (default tri_test and ray_sort) those of two bounces
+ * before, while shadow rays are traced on a stream of the context's own;
+ * the context's stream is behind that one when the call returns. */
 FLG_API int flg_pathtrace(flg_ctx ctx, flg_bvh bvh, const flg_pt_scene *scene, const flg_pt_camera *cam,
                           int32_t spp, int32_t max_depth, const flg_trace_opts *opts, float *radiance,
                           flg_pt_stats *stats);
