@@ -34,7 +34,7 @@ constexpr int32_t kBoxUnset = (int32_t)0xFFC0DEADu;
 constexpr int32_t kEmptyChild = 0x7FFFFFFF;
 
 // 4-wide node: the children's boxes in 8 bits per plane, as (origin + byte x
-// 2^(e - 127)) per axis, conservative (quantise, wide.cuh).  The traversal is
+// step) per axis with a power-of-two step, conservative (quantise, wide.cuh).  The traversal is
 // bound by its divergent 16-byte loads, one L1 wavefront per lane and load:
 // this record takes 3 per visit against 6 and the refs for the same boxes in
 // fp32.  Inner children sit in consecutive slots; a leaf child's range is read
@@ -42,7 +42,7 @@ constexpr int32_t kEmptyChild = 0x7FFFFFFF;
 // re-decided per hit (k_trace4, k_trace_finish4).
 struct alignas(16) NodeQ {
   float org[3];
-  uint32_t step;    // exponents: y << 23 | z << 15 | x << 7
+  uint32_t step;    // biased exponents of 2^16 steps: y << 23 | z << 15 | x << 7
   uint32_t qlo[3];  // per axis, byte k: child k's lower plane
   uint32_t qhi[3];
   int32_t base;     // slot of the first inner child
@@ -50,9 +50,9 @@ struct alignas(16) NodeQ {
   int32_t leaf[4];  // leaf children: ~range
 };
 static_assert(sizeof(NodeQ) == 64, "NodeQ layout");
-// Step word of the node of a one-triangle scene: infinite on every axis (a
-// word that quantise gives to no node with a finite box).
-constexpr uint32_t kLoneStep = 255u << 23 | 255u << 15 | 255u << 7;
+// Step word of the node of a one-triangle scene: infinite on every axis, and a
+// mark in a bit that no exponent uses.
+constexpr uint32_t kLoneStep = 255u << 23 | 255u << 15 | 255u << 7 | 1u;
 
 // 8-wide node, structure of arrays inside the record (14 16-byte loads per
 // visit).

@@ -508,7 +508,8 @@ __global__ void __launch_bounds__(256)
 // reference's slab test, children nearest first, first found kept among equal
 // t), although the boxes the traversal reads are a little larger:
 //   * A quantised box contains the exact one with room for every rounding of
-//     visit_q, so the leaves visited are a superset of the exact ones.
+//     visit_q, so the leaves visited are a superset of the exact ones.  (A ray
+//     whose direction leaves no such room is traced over the exact boxes: inv_q.)
 //   * Closest hit: a finished ray's winner stands if its own box, which its
 //     leaf range's and every ancestor's box contain, passes the exact slab
 //     test with tnear <= t: then the exact traversal reaches it, whatever it
@@ -541,11 +542,51 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
   return r;
 }
 
-// Inverse direction for the quantised slab test: the infinite inverse of a
-// zero component becomes +-2^90, so that plane distances stay finite (an
-// infinite one would be NaN after the multiply-add and drop the axis).
-__device__ __forceinline__ float inv_q(float inv) {
-  return fabsf(inv) <= 3.402823466e+38f ? inv : copysignf(1.2379400392853803e27f, inv);
+// Inverse directions with a component below kInvMin or from kInvMax on, for the
+// quantised slab test.  False if the ray has to be traced over the exact boxes.
+//
+// An infinite component (of a direction's zero, or below 2^-128) would make every
+// plane distance of its axis NaN and drop the axis, so +-B takes its place, the
+// largest power of two for which 2^16 steps of the scene's root, and so of every
+// node, times B stay finite (2^90 if the root's step is infinite).  An exact plane
+// distance is +-inf there; the quantised one has its sign, except that an origin
+// between an exact plane and the quantised one is inside: no box is lost by that.
+// But the far distance of a box that the origin is inside of is finite now.  It is
+// at least 1/128 step x B, what quantise adds less the rounding of the distance,
+// and the step at least 2^-40 and at least 2^-30 of the origin's coordinate,
+// which lies between the planes.  Boxes nearer than that (`sure`), and than the
+// 2^126 of visit_q, are tested as the exact test tests them; and no box that the
+// exact test accepts is farther (`far`) than tmax, or than the root's far plane on
+// an axis of a finite component.
+constexpr uint32_t kInvMin = (127u - 100u) << 23, kInvMax = (127u + 64u) << 23;  // 2^-100 (the step is at least 2^-40), 2^64
+__device__ __forceinline__ uint32_t above_min(float inv) { return (__float_as_uint(inv) & 0x7FFFFFFFu) - kInvMin; }
+__device__ __forceinline__ bool odd_inv(const float3 &inv) {
+  return max(max(above_min(inv.x), above_min(inv.y)), above_min(inv.z)) >= kInvMax - kInvMin;
+}
+__device__ __forceinline__ bool is_finite(float x) { return fabsf(x) <= 3.402823466e+38f; }
+__device__ __forceinline__ bool inv_q(const NodeQ *__restrict__ root, const float3 &o, const float3 &d, float tmax,
+                                      float3 &inv) {
+  const uint4 A = __ldg((const uint4 *)root);
+  const float oo[3] = {o.x, o.y, o.z}, dd[3] = {d.x, d.y, d.z};
+  const uint32_t org[3] = {A.x, A.y, A.z}, e[3] = {A.w >> 7 & 255u, A.w >> 23, A.w >> 15 & 255u};
+  float *const ii[3] = {&inv.x, &inv.y, &inv.z};
+  float far = tmax, sure = 8.507059173023462e+37f;  // 2^126
+  bool hits = A.w != kLoneStep;  // one triangle, in a box that constrains nothing
+  bool small = false;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    if (is_finite(*ii[a])) {
+      // 256 steps cover the box
+      far = fminf(far, (fabsf(__uint_as_float(org[a]) - oo[a]) + __uint_as_float(e[a] << 23) * 0.00390625f) * fabsf(*ii[a]));
+      small |= (__float_as_uint(*ii[a]) & 0x7FFFFFFFu) < kInvMin;
+    } else {
+      *ii[a] = copysignf(__uint_as_float((e[a] == 255u ? 217u : min(254u, 379u - e[a])) << 23), *ii[a]);
+      // half of it, for the roundings here
+      sure = fminf(sure, fmaxf(3.5527136788005009e-15f, fabsf(oo[a]) * 3.637978807091713e-12f) * fabsf(*ii[a]));
+    }
+    hits &= is_finite(oo[a]) && dd[a] == dd[a];  // else the ray hits nothing
+  }
+  return !hits || (!small && far < sure);
 }
 
 // Two fp32 values in one 64-bit register: sm_103a's packed add, multiply and
@@ -581,20 +622,26 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   return r;
 }
 
-// Byte k of w as the float 2^15 + byte: one byte permute puts it above the
-// last mantissa byte of 2^15.
+// Byte k of w as the float 1/2 + byte / 2^16: one byte permute puts it above the
+// last mantissa byte of 1/2.  (As 2^15 + byte, with s smaller by 2^16, the offset
+// 2^15 s would overflow before s itself, and planes at -inf reject the box
+// that planes at NaN leave alone.)
 template <int K>
 __device__ __forceinline__ float byte_f(uint32_t w) {
-  return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7404 | (K << 4)));
+  return __uint_as_float(__byte_perm(w, 0x3F000000u, 0x7604 | (K << 4)));
 }
 
 // Tests the children of a quantised node.  key[k]: tnear with child k's kind
 // byte in place of its low byte (masked off again, i.e. rounded down, when a
 // stack entry is culled); a miss is ~0.  Per axis the plane distance
-// of byte q is fma(2^15 + q, step inv, (origin - o) inv - 2^15 step inv).  Its
-// error is below 1/64 step (the boxes' slack) plus 2^-22 of itself, and the
+// of byte q is fma(1/2 + q / 2^16, s, (origin - o) inv - s / 2) with s = 2^16 step inv.
+// Its error is below 1/64 step (the boxes' slack) plus 2^-22 of itself, and the
 // exact test's own below 2^-23: with tnear scaled by 1 - 2^-20 the test passes
-// whenever the exact one does.
+// whenever the exact one does.  For that s must not be subnormal (rays with
+// an inverse below kInvMin are traced over the exact boxes).  Where s is infinite
+// the distances are NaN and the axis constrains nothing.  Where s is finite and
+// (origin - o) inv - s / 2 is not, the origin lies 2^15 steps or more outside and
+// the distances have the exact ones' sign; those are beyond 2^126.
 __device__ __forceinline__ void visit_q(const NodeQ *__restrict__ node, const float3 &o, const float3 &inv, float lim,
                                         uint32_t (&key)[4], int32_t &base) {
   const uint4 *np = (const uint4 *)node;
@@ -604,9 +651,9 @@ __device__ __forceinline__ void visit_q(const NodeQ *__restrict__ node, const fl
   const float ey = __uint_as_float(A.w & 0x7F800000u);
   const float ez = __uint_as_float((A.w << 8) & 0x7F800000u);
   const float sx = ex * inv.x, sy = ey * inv.y, sz = ez * inv.z;
-  const float bx = fmaf(-32768.0f, sx, (__uint_as_float(A.x) - o.x) * inv.x);
-  const float by = fmaf(-32768.0f, sy, (__uint_as_float(A.y) - o.y) * inv.y);
-  const float bz = fmaf(-32768.0f, sz, (__uint_as_float(A.z) - o.z) * inv.z);
+  const float bx = fmaf(-0.5f, sx, (__uint_as_float(A.x) - o.x) * inv.x);
+  const float by = fmaf(-0.5f, sy, (__uint_as_float(A.y) - o.y) * inv.y);
+  const float bz = fmaf(-0.5f, sz, (__uint_as_float(A.z) - o.z) * inv.z);
   // (near, far) pairs, the near one scaled
   constexpr float k = 0.99999905f;  // 1 - 2^-20
   const f32x2 sx2 = pack2(sx * k, sx), sy2 = pack2(sy * k, sy), sz2 = pack2(sz * k, sz);
@@ -989,8 +1036,9 @@ __global__ void __launch_bounds__(256, 4)
   constexpr uint32_t kSlot = 256 * sizeof(uint64_t);  // bytes between a thread's slots
   constexpr unsigned kAll = 0xFFFFFFFFu;
   // The upper word: bits 32 .. 47 of the ray's index; trace it again over the
-  // exact boxes (its stack overflowed, or an any-hit candidate's own box kept
-  // it out); and, as multiples of kHelper, its helpers at work.
+  // exact boxes (its stack overflowed, an any-hit candidate's own box kept
+  // it out, or its inverse direction is too small or too large); and, as
+  // multiples of kHelper, its helpers at work.
   constexpr uint32_t kRayHigh = 0xFFFFu, kAgain = 1u << 16, kHelper = 1u << 17;
   // A second candidate near the closest hit: none, one within kNear but not
   // equal, two or more equal, or (>= 0) the one that is equal.
@@ -1124,11 +1172,14 @@ __global__ void __launch_bounds__(256, 4)
         s_ray[0][threadIdx.x] = (uint32_t)my;
         crew[lane] = (uint32_t)(my >> 32);
         load_ray(R, my, o, d, inv, tmin, best);
-        inv = make_float3(inv_q(inv.x), inv_q(inv.y), inv_q(inv.z));
         tie = kNone;
         prim = -1;
         cur = scene_root_walk(roots, ray_off, n_scenes, my, scene);
         if (cur == kEmptyChild) cur = kDone;
+        if (odd_inv(inv) && cur != kDone && !inv_q(nodes + cur, o, d, best, inv)) {
+          crew[lane] |= kAgain;
+          cur = kDone;
+        }
         low = bottom;
         top = bottom + kSlot;
         moved = 0;

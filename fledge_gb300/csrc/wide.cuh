@@ -186,8 +186,9 @@ __device__ __forceinline__ void walk_open(const Node2 *__restrict__ nodes2, cons
 // and a power-of-two step; every child's lower plane rounds down and its
 // upper plane up, both with at least 1/64 step to spare.  The slack covers
 // the rounding of the traversal's plane distances, so that a box test on the
-// record never rejects a box that the exact test accepts (visit_q).  An axis
-// whose planes are not finite, or too far apart for fp32, gets an infinite
+// record never rejects a box that the exact test accepts (visit_q).  The
+// record holds the exponent of 2^16 steps, as visit_q takes it.  An axis
+// whose planes are not finite, or more than 2^118 apart, gets an infinite
 // step and zero bytes, which constrain nothing.
 __device__ __forceinline__ void quantise(const Cand (&c)[4], int nc, NodeQ &out) {
   out.step = 0u;
@@ -210,8 +211,8 @@ __device__ __forceinline__ void quantise(const Cand (&c)[4], int nc, NodeQ &out)
     e = max(e, 87u);
     uint32_t qlo = 0u, qhi = 0u;
     float org = 0.0f;
-    // ext < inf and not NaN (lo <= hi, so ext >= 0); the step stays normal
-    if (ext < __int_as_float(0x7f800000) && e <= 250u) {
+    // ext < inf and not NaN (lo <= hi, so ext >= 0); 2^16 steps stay finite
+    if (ext < __int_as_float(0x7f800000) && e <= 238u) {
       const float s = __uint_as_float(e << 23), rs = __uint_as_float((254u - e) << 23);
       org = __fsub_rd(lo, s * 0.03125f);
 #pragma unroll
@@ -222,6 +223,7 @@ __device__ __forceinline__ void quantise(const Cand (&c)[4], int nc, NodeQ &out)
         qlo |= (uint32_t)fminf(fmaxf(l, 0.0f), 255.0f) << (8 * k);
         qhi |= (uint32_t)fminf(fmaxf(h, 0.0f), 255.0f) << (8 * k);
       }
+      e += 16u;
     } else {
       e = 255u;
     }

@@ -78,6 +78,61 @@ def test_quantised_boxes_change_no_hit(ctx, oracle, kind, leaf):
     assert np.array_equal(hg["prim"] >= 0, he["prim"] >= 0) and np.array_equal(occ, occ_e)
 
 
+def _directions(kind, v, n, rng):
+    """Unit rays through the unit cube whose direction has a zero or a very
+    small component, or a very small or large length."""
+    r = np.zeros((8, n), np.float32)
+    if kind == "sphere":
+        r[:] = G.sphere_rays(n, rng)
+    else:  # down the z axis from above, or from inside
+        r[0:3] = rng.random((3, n))
+        r[2, ::2] = 2.0
+        r[5] = -1.0
+    if kind == "tilt":
+        r[3] = v
+    else:
+        r[3:6] *= np.float32(v)
+    r[6], r[7] = 0.0, np.inf
+    return r
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e3, 1e6, 1.1e9, 4e9, 1e12, 1e18])
+@pytest.mark.parametrize("kind,v", [("axis", 1.0), ("axis", 1e-14), ("axis", 1e-28), ("axis", 1e31), ("sphere", 1e-36),
+                                    ("sphere", 1e31), ("tilt", 1e-10), ("tilt", 6e-17), ("tilt", 1e-33),
+                                    ("tilt", 5e-37), ("tilt", 1e-38), ("tilt", 1e-40)])
+def test_inverse_directions_at_the_ends_of_fp32(ctx, oracle, scale, kind, v):
+    """Distances to quantised planes that would overflow or lose their bits:
+    the hits stay those of fp32 boxes, for closest and any hit.  One scene is as
+    thick as it is wide, the other a millionth of that along x."""
+    rng = np.random.default_rng(91)
+    for thin in (False, True):
+        pos = G.random_soup(3000, rng, half=0.05).reshape(-1, 3)
+        r8 = _directions(kind, v, 20000, rng)
+        if thin:
+            pos[:, 0] = (pos[:, 0] - np.float32(0.5)) * np.float32(1e-6)
+            r8[0] = (r8[0] - np.float32(0.5)) * np.float32(1e-6)
+        pos *= np.float32(scale)
+        r8[0:3] *= np.float32(scale)
+        b, _ = U.gpu_build(ctx, pos, width=4)
+        exact, _ = U.gpu_build(ctx, pos, width=8)
+        rd, _ = U.rays_dev(r8)
+        hg, he = U.host(b.intersect(rd)), U.host(exact.intersect(rd))
+        occ, occ_e = b.intersectP(rd).cpu().numpy(), exact.intersectP(rd).cpu().numpy()
+        ctx.sync()
+        assert np.array_equal(hg["prim"] >= 0, he["prim"] >= 0), (thin, np.count_nonzero(hg["prim"] >= 0))
+        assert np.array_equal(occ, occ_e), thin
+        tri = pos.reshape(-1, 3, 3)
+        for i in np.nonzero(hg["prim"] != he["prim"])[0]:  # at the same distance, else not another triangle
+            t = [oracle.pluecker(*tri[p], r8[0:3, i], r8[3:6, i], oracle.MODE_DEV)[1][0]
+                 for p in (hg["prim"][i], he["prim"][i])]
+            assert t[0] == t[1], (thin, i)
+        same = hg["prim"] == he["prim"]
+        for k in ("t", "u", "v"):
+            assert np.array_equal(hg[k][same], he[k][same], equal_nan=True), (thin, k)
+    if kind != "sphere" and abs(np.log10(v)) < 15 and scale < 1e12:
+        assert (hg["prim"] >= 0).mean() > 0.1
+
+
 def test_more_ties_than_the_list_holds(ctx):
     """Over 2^20 rays that all end in a tie: the list overflows and the rays
     are found by their marks.  Equal to tracing them in parts."""
