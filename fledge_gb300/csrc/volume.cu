@@ -41,8 +41,8 @@ __device__ __forceinline__ void load_vray(const VRays &R, int64_t i, float3 &o, 
 // tracking: two, a Philox block's draws) is one turn of the warp's loop.
 // Together with one bounds test and one address per lattice cell (grid_cell), us
 // before -> after: delta tracking of 2 M rays through a 192^3 sparse grid 927 ->
-// 547, with two steps to a turn 460, and with 32-bit addresses and refills at 4
-// idle lanes 434 (8: 446); of 1 M rays through a 256^3 dense one 83 ->
+// 547, with two steps to a turn 460, with refills at 4 idle lanes 434 (8: 446), and
+// with a pointer to each of the two layers of bricks 1.5 % less; of 1 M rays through a 256^3 dense one 83 ->
 // 52 -> 47; ratio tracking of the latter 85 -> 75, its adjoint 85 -> 79.  Ratio
 // tracking, which waits for scattered sectors of the grid (29 % of L2's and 30 %
 // of DRAM's rate, L1 at 41 %), gains nothing from turns of four draws (76 us,

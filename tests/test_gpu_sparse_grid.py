@@ -136,3 +136,44 @@ def test_sparse_matches_oracle(ctx, oracle):
     # voxels of dropped bricks are not parameters: the oracle's gradient there
     # is what the dense grid would have received; the sparse grid has none
     assert np.all(gs[~stored] == 0)
+
+
+def test_table_of_more_than_2_to_32_bricks(ctx):
+    """A lattice whose brick table needs 64-bit indices (17 GB, all but one
+    layer of it empty), against the same bricks in a table of one layer: rays
+    along x and y inside the layer enter and leave both boxes at the same
+    distances, and all lattice coordinates are exact, so transmittance,
+    checkpoints, collisions and gradients are the same bits."""
+    import fledge_gb300 as F
+    if torch.cuda.mem_get_info()[0] < 24 << 30:
+        pytest.skip("needs 24 GB of device memory")
+    nb, layers, h = 2048, 1025, 2.0 ** -10  # 2048 x 2048 x 1024 = 2^32 bricks lie before the last layer
+    g = torch.Generator(device="cuda").manual_seed(3)
+    bricks = 2.0 * torch.rand(2 * 64 * 3, 8, 8, 8, device="cuda", generator=g)
+    layer = torch.full((1, nb, nb), -1, dtype=torch.int32, device="cuda")
+    layer[0, 5:8, 100:164] = torch.arange(64 * 3, dtype=torch.int32, device="cuda").view(3, 64)
+    layer[0, 300:364, 70:73] = torch.arange(64 * 3, 2 * 64 * 3, dtype=torch.int32, device="cuda").view(64, 3)
+    table = torch.full((layers, nb, nb), -1, dtype=torch.int32, device="cuda")
+    table[-1] = layer[0]
+    med = F.Medium(0.8, 0.2, 0.3, majorant=2.0)
+    n, z0 = 8 * nb, 8 * (layers - 1) * h
+    grids = [F.SparseGridVolume(t, bricks, (nz, n, n), (0.0, 0.0, lo), ((n - 1) * h, (n - 1) * h, z0 + 7 * h), med, ctx)
+             for t, nz, lo in ((table, 8 * layers, 0.0), (layer, 8, z0))]
+    m = 20000
+    rays = torch.zeros(6, m, device="cuda")
+    u = torch.rand(2, m, device="cuda", generator=g)
+    rays[2] = z0 + h * 7 * u[0]
+    rays[0, ::2], rays[1, ::2], rays[3, ::2] = -1.0, h * (8 * 5 + 24 * u[1, ::2]), 1.0
+    rays[0, 1::2], rays[1, 1::2], rays[4, 1::2] = h * (8 * 70 + 24 * u[1, 1::2]), -1.0, 1.0
+    rd = F.Rays.from_soa(rays)
+    out = []
+    for v in grids:
+        T, ck = v.tr(rd, 5, checkpoint=True)
+        out.append([T, *ck.values(), *v.sample(rd, 6), v.tr_adjoint(rd, 5, torch.ones_like(T), T, ck)])
+    ctx.sync()
+    for a, b in zip(*[o[:-1] for o in out]):
+        assert torch.equal(a, b)
+    T, grad = out[1][0], out[1][-1]
+    # 512 cells at the majorant 2 are one expected step: a share of exp(-1) takes none there
+    assert (T < 1).float().mean() > 0.6 and float(grad.abs().max()) > 0
+    assert torch.allclose(out[0][-1], grad, rtol=1e-4, atol=1e-4 * float(grad.abs().max()))
