@@ -133,6 +133,58 @@ def test_inverse_directions_at_the_ends_of_fp32(ctx, oracle, scale, kind, v):
         assert (hg["prim"] >= 0).mean() > 0.1
 
 
+def test_hits_in_front_of_their_own_box(ctx, oracle):
+    """Two triangles per scene: a sliver of 1e-7 to 1e-6 along the ray, whose
+    fp32 t may lie well in front of its box, and a triangle across the ray about
+    where that box begins.  Which box the ray enters first, and whether the
+    other one begins beyond that hit, decides, as with fp32 boxes (8-wide;
+    distances that agree but for the bits which the child's number replaces may
+    be in either order)."""
+    import fledge_gb300 as F
+    n = 1 << 17
+    rng = np.random.default_rng(5)
+    d = np.zeros((n, 3))
+    d[np.arange(n), rng.integers(0, 3, n)] = 1.0
+    d += 0.3 * (rng.random((n, 3)) - 0.5)
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    o = rng.random((n, 3))
+    u = np.cross(d, [0.37, 0.61, 0.7])
+    u /= np.linalg.norm(u, axis=1, keepdims=True)
+    v = np.cross(d, u)
+    s = 1e-7 * 10.0 ** rng.random((n, 1))
+    ang = 2 * np.pi * rng.random((n, 1))
+
+    def corner(k, t, r):
+        x = ang + 2 * np.pi / 3 * k
+        return o + t * d + r * (np.cos(x) * u + np.sin(x) * v)
+
+    along = 0.2 * (rng.random((n, 3)) - 0.5)
+    across = 1 + along.min(1, keepdims=True) + (rng.random((n, 1)) - 0.8) * np.exp(9 * rng.random((n, 1)) - 13)
+    tri = np.stack([np.stack([corner(k, 1 + along[:, k:k + 1], s) for k in range(3)], 1),
+                    np.stack([corner(k, across, 0.01) for k in range(3)], 1)], 1).astype(np.float32)
+    r8 = np.zeros((8, n), np.float32)
+    r8[0:3], r8[3:6], r8[7] = o.T, d.T, np.inf
+    rd, _ = U.rays_dev(r8)
+    hits = []
+    for w in (4, 8):
+        b = F.BatchedRadixBVHBuilder(F.InternalTriangleMesh(U.dev(tri.reshape(-1, 3))), 2 * np.arange(n + 1), ctx, node_width=w)
+        b.build()
+        hits.append(U.host(b.intersect_batched(rd, np.arange(n + 1))))
+    ctx.sync()
+    assert (hits[1]["prim"] == 0).sum() > 100
+    inv = np.float32(1) / r8[3:6].T
+    planes = (np.where(inv[:, None] < 0, tri.max(2), tri.min(2)) - r8[0:3].T[:, None]) * inv[:, None]
+    near = np.maximum(planes.max(2), np.float32(0)).view(np.int32)
+    same = hits[0]["prim"] == hits[1]["prim"]
+    assert np.count_nonzero(~same) < 100
+    for i in np.nonzero(~same)[0]:
+        t = [np.float32(oracle.pluecker(*tri[i, k], r8[0:3, i], r8[3:6, i], oracle.MODE_DEV)[1][0]).view(np.int32)
+             for k in (0, 1)]
+        assert min(abs(near[i, 0] - near[i, 1]), abs(near[i, 0] - t[1]), abs(near[i, 1] - t[0])) < 8, i
+    for k in ("t", "u", "v"):
+        assert np.array_equal(hits[0][k][same], hits[1][k][same]), k
+
+
 def test_more_ties_than_the_list_holds(ctx):
     """Over 2^20 rays that all end in a tie: the list overflows and the rays
     are found by their marks.  Equal to tracing them in parts."""
