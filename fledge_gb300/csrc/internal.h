@@ -39,7 +39,7 @@ constexpr int32_t kEmptyChild = 0x7FFFFFFF;
 // this record takes 3 per visit against 6 and the refs for the same boxes in
 // fp32.  Inner children sit in consecutive slots; a leaf child's range is read
 // when the leaf is tested.  What the exact boxes decide beyond that is
-// re-decided per hit (k_trace4, k_trace_finish4).
+// re-decided per hit (k_trace4, k_settle4).
 struct alignas(16) NodeQ {
   float org[3];
   uint32_t step;    // biased exponents of 2^16 steps: y << 23 | z << 15 | x << 7
@@ -299,9 +299,9 @@ inline unsigned grid_for(int64_t n, int threads, int64_t cap_blocks = 1 << 30) {
 // touches global memory.  Takes the 2 us between dependent kernels out of the
 // chains of short ones that builds, traces and bounces are: a rebuild of 20,001
 // triangles 125 -> 103 us, of 4,000,003 824 -> 782; one image of 640 x 360
-// 1120 -> 1055.  No kernel lets its successor start before it ends itself
-// (except k_settle4): that made builds 1 to 4 % slower, the early blocks being
-// in the way of the ones at work.
+// 1120 -> 1055.  No kernel lets its successor start before it ends itself: that
+// made builds 1 to 4 % slower, the early blocks being in the way of the ones at
+// work, and what a kernel two before has written is only visible after the wait.
 template <class... P, class... A>
 cudaError_t launch_after(void (*kern)(P...), unsigned grid, unsigned threads, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg = {};

@@ -11,7 +11,7 @@
 //   k_trace4            4-wide: while-while traversal with parked leaves, one
 //                       ray per thread or persistent warps that refill idle
 //                       lanes from a global ray counter (work stealing across
-//                       scenes of a batch); k_trace_finish4 after it
+//                       scenes of a batch); k_settle4 or k_trace_retry4 after it
 //   k_trace_bvh2        one ray per thread over BVH2, leaf triangles tested
 //                       directly as the reference does (no leaf box test)
 //   k_trace_wide, k_trace_persistent, k_trace_ww   the same three schedules
@@ -890,8 +890,9 @@ __device__ __forceinline__ void finish_hit(const RaySoA &R, const Out &O, const 
   O.v[i] = v;
 }
 
-// Those of the closest hits that k_trace4 is sure of; the rays that k_settle4
-// works on are left alone: neither kListed nor a finished id has kPending.
+// Those of the closest hits that k_trace4 is sure of, one ray per thread; the rays
+// that other threads settle are left alone: neither kListed nor a finished id
+// has kPending.
 __device__ __forceinline__ void finish_pending(const RaySoA &R, int64_t n, const Out &O,
                                                const TriRec *__restrict__ tris) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -901,8 +902,20 @@ __device__ __forceinline__ void finish_pending(const RaySoA &R, int64_t n, const
   }
 }
 
-__device__ __noinline__ ExactHit retrace_closest(const Exact4 &X, const RaySoA &R, int64_t i, uint32_t *err) {
-  return retrace4<false>(X, R, i, err);
+// Final values of a listed ray.
+__device__ __noinline__ void settle(const RaySoA &R, const Out &O, const Exact4 &X, int64_t i, uint32_t *err) {
+  const int32_t q = __float_as_int(O.v[i]);
+  ExactHit h{__float_as_int(O.u[i]), O.t[i]};
+  if (q >= 0) h.prim = first_of_two(X, R, i, h.prim, q);
+  else h = retrace4<false>(X, R, i, err);
+  if (h.prim >= 0) {
+    finish_hit(R, O, X.tris, i, h.prim, h.t);
+  } else {
+    O.prim[i] = -1;
+    O.t[i] = h.t;
+    O.u[i] = 0.0f;
+    O.v[i] = 0.0f;
+  }
 }
 
 // Clears the trace's counters for the next one, in the last block to get here
@@ -915,51 +928,30 @@ __device__ __forceinline__ void clear_counters(const Scratch &S) {
   }
 }
 
-// Settles the rays that k_trace4 left open and writes their final values.
-// ALL: also those of the others, in place of k_trace_finish4, which else may
-// start at once, as the two work on different rays.
-template <bool ALL>
-__global__ void __launch_bounds__(128)
+// Settles the rays that k_trace4 left open and writes the final values of all.
+// The list comes first: the walks of its rays take longer than the others'
+// values, which hide them.  Up to kSettleWide rays with registers for the walks
+// (five blocks of 128 threads per SM), above with as few as the values need: 921,600
+// camera rays 222 -> 218 us against 64 registers, 1 M rays on layers of quads 258 ->
+// 248; 31.6 M rays 20.15 -> 20.05 ms against five blocks of 128.
+constexpr int64_t kSettleWide = 1 << 21;
+template <int THREADS, int BLOCKS>
+__global__ void __launch_bounds__(THREADS, BLOCKS)
     k_settle4(const __grid_constant__ RaySoA R, RayCount N, Out O, const __grid_constant__ Exact4 X, Scratch S) {
   after_wait();
-  if (!ALL) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t cnt = *S.ovf_count;
   const int64_t n = N.get();
-  if (ALL) finish_pending(R, n, O, X.tris);
+  const int64_t t = (int64_t)blockIdx.x * THREADS + threadIdx.x, threads = (int64_t)gridDim.x * THREADS;
   const bool listed = cnt <= S.ovf_cap;  // else look for the marks
   const int64_t end = listed ? (int64_t)cnt : n;
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < end; j += (int64_t)gridDim.x * blockDim.x) {
+  // a short list: a ray to a warp
+  const int64_t first = end <= threads / 32 ? (t & 31) * (threads / 32) + (t >> 5) : t;
+  for (int64_t j = first; j < end; j += threads) {
     const int64_t i = listed ? S.ovf[j] : j;
-    if (O.prim[i] != kListed) continue;
-    const int32_t q = __float_as_int(O.v[i]);
-    ExactHit h{__float_as_int(O.u[i]), O.t[i]};
-    if (q >= 0) h.prim = first_of_two(X, R, i, h.prim, q);
-    else h = retrace_closest(X, R, i, S.err);
-    if (h.prim >= 0) {
-      finish_hit(R, O, X.tris, i, h.prim, h.t);
-    } else {
-      O.prim[i] = -1;
-      O.t[i] = h.t;
-      O.u[i] = 0.0f;
-      O.v[i] = 0.0f;
-    }
+    if (O.prim[i] == kListed) settle(R, O, X, i, S.err);
   }
-  if (ALL) clear_counters(S);
-}
-
-// Hit values of every closest hit of k_trace4, one ray per thread (as
-// k_trace_finish), beside k_settle4, whose latency it hides.  Then clears the
-// trace's counters for the next one.
-__global__ void __launch_bounds__(256, 4)
-    k_trace_finish4(RaySoA R, RayCount N, Out O, const TriRec *__restrict__ tris, Scratch S) {
-  finish_pending(R, N.get(), O, tris);
-  // k_settle4 has ended and its writes are visible: so they are to what
-  // follows this kernel
-  after_wait();
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    *S.work = 0ull;
-    *S.ovf_count = 0u;
-  }
+  finish_pending(R, n, O, X.tris);
+  clear_counters(S);
 }
 
 // Any-hit rays that k_trace4 left open.
@@ -1693,12 +1685,6 @@ __global__ void __launch_bounds__(256, 4)
 // until they cover the SMs.  Refills at 8 idle lanes at most: with the
 // quantised nodes 8 beat 16 and 24 (24.0 against 25.6 and 29.6 ms on 31.6 M
 // scattered rays).
-//
-// As long as k_settle4's blocks cover the rays in one wave (3 of 128 threads
-// per SM) they also compute the hit values: a launch less (1 to 20,000 rays on
-// 20,480 triangles 2 us less of host time, which is what bounds up to 5,000;
-// 57,000 rays 48.9 against 48.4 us).  Above, k_trace_finish4 has more than
-// twice the warps.
 template <bool ANY>
 static int launch4(flg_ctx ctx, cudaStream_t st, flg_bvh b, const RaySoA &R, int64_t n, const int32_t *n_dev,
                    const Out &O, const Scratch &S, const int64_t *ray_off, int n_scenes, const flg_trace_opts &op, bool &open) {
@@ -1723,15 +1709,11 @@ static int launch4(flg_ctx ctx, cudaStream_t st, flg_bvh b, const RaySoA &R, int
   if (ANY) {
     FLG_CUDA(ctx, launch_after(k_trace_retry4, grid_for(n, 128, ctx->num_sms), 128, st, R, N, O, X, S));
     FLG_LAUNCH_CHECK(ctx, "k_trace_retry4");
-  } else if (n <= (int64_t)ctx->num_sms * 3 * 128) {
-    FLG_CUDA(ctx, launch_after(k_settle4<true>, grid_for(n, 128, (int64_t)ctx->num_sms * 3), 128, st, R, N, O, X, S));
-    FLG_LAUNCH_CHECK(ctx, "k_settle4");
   } else {
-    FLG_CUDA(ctx, launch_after(k_settle4<false>, grid_for(n, 128, ctx->num_sms), 128, st, R, N, O, X, S));
+    FLG_CUDA(ctx, n > kSettleWide
+                      ? launch_after(k_settle4<256, 4>, grid_for(n, 256, (int64_t)ctx->num_sms * 16), 256, st, R, N, O, X, S)
+                      : launch_after(k_settle4<128, 5>, grid_for(n, 128, (int64_t)ctx->num_sms * 32), 128, st, R, N, O, X, S));
     FLG_LAUNCH_CHECK(ctx, "k_settle4");
-    FLG_CUDA(ctx, launch_after(k_trace_finish4, grid_for(n, 256, (int64_t)ctx->num_sms * 16), 256, st, R, N, O, b->d_tris,
-                               S));
-    FLG_LAUNCH_CHECK(ctx, "k_trace_finish4");
   }
   open = false;
   stage_mark(ctx, st, ANY ? "trace_retry" : "trace_finish");

@@ -271,3 +271,26 @@ def test_where_settling_also_finishes(ctx, oracle, over):
         assert np.array_equal(h["t"][same], ho["t"][same])
         assert np.array_equal(occ != 0, ho["prim"] >= 0)
     ctx.sync()
+
+
+@pytest.mark.parametrize("over", [0, 1])
+def test_where_settling_changes_its_blocks(ctx, over):
+    """On either side of the 2^21 rays above which the settling kernel runs in
+    other blocks, among them more ties than its list holds and few: equal to
+    tracing the rays in parts."""
+    import fledge_gb300 as F
+    import torch
+    n = (1 << 21) + over
+    soa = F.gen_rays(ctx, n, 78)
+    soa[3:6] = 0.5 - soa[0:3] + 0.2 * (soa[3:6] - 0.5)
+    for kind in ("duplicates", "planes"):
+        b, _ = U.gpu_build(ctx, _scene(kind)[0], width=4, leaf=1)
+        whole = b.intersect(F.Rays.from_soa(soa))
+        occ = b.intersectP(F.Rays.from_soa(soa))
+        for a in range(0, n, 700001):
+            r = F.Rays.from_soa(soa[:, a:a + 700001].contiguous())
+            part = b.intersect(r)
+            for k in part:
+                assert torch.equal(part[k], whole[k][a:a + 700001]), (kind, k)
+            assert torch.equal(b.intersectP(r), occ[a:a + 700001]), kind
+        ctx.sync()
