@@ -748,6 +748,7 @@ struct Exact4 {
   const int32_t *roots;  // BVH2 roots per scene
   const int64_t *ray_off;
   int32_t n_scenes;
+  int64_t most;          // stack entries of a walk: each node and leaf range once, at most
 };
 
 // Ray `ray` over the exact boxes, in the exact order: the children of a wide
@@ -773,8 +774,11 @@ __device__ __forceinline__ ExactHit retrace4(const Exact4 &X, const RaySoA &RS, 
   bool have = false;
   int sp = 0;
   stk[sp++] = (uint32_t)(root < 0 ? ~((~root) << 3) : root);
-  // (a ray visits far fewer nodes; the bound ends a walk over a broken tree)
-  for (int visits = 0; sp > 0 && visits < (1 << 22); ++visits) {
+  for (int64_t left = X.most; sp > 0; --left) {
+    if (left == 0) {  // a broken tree
+      atomicOr(err, kErrQueue);
+      break;
+    }
     const uint64_t e = stk[--sp];
     if (__uint_as_float((uint32_t)(e >> 32)) > best) continue;
     const int32_t cur = (int32_t)(uint32_t)e;
@@ -1699,7 +1703,8 @@ static int launch4(flg_ctx ctx, cudaStream_t st, flg_bvh b, const RaySoA &R, int
   }
   const int refill = std::max(1, std::min(8, op.refill_lanes));
   const RayCount N{n, n_dev};
-  const Exact4 X{b->d_nodes2, b->d_tris, Ranges{b->d_rfirst, b->d_rcount}, b->leaf_size, b->d_root, ray_off, n_scenes};
+  const Exact4 X{b->d_nodes2, b->d_tris, Ranges{b->d_rfirst, b->d_rcount}, b->leaf_size, b->d_root, ray_off, n_scenes,
+                 2 * b->n_tri};
   open = true;  // until the kernel that clears the counters is launched
   FLG_CUDA(ctx, launch_after(n_dev ? k_trace4<ANY, true> : k_trace4<ANY, false>, (unsigned)g, threads, st,
                              (const NodeQ *)b->d_wide, b->d_tris, b->d_wide_root, ray_off, n_scenes, R, N, O, S, refill,

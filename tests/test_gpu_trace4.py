@@ -294,3 +294,20 @@ def test_where_settling_changes_its_blocks(ctx, over):
                 assert torch.equal(part[k], whole[k][a:a + 700001]), (kind, k)
             assert torch.equal(b.intersectP(r), occ[a:a + 700001]), kind
         ctx.sync()
+
+
+def test_a_walk_of_more_than_2_to_22_entries(ctx):
+    """A ray over the exact boxes (its direction is too long for the quantised
+    ones) that enters the boxes of 3.4 million equal triangles before the one
+    that it hits: the walk, about 4 s long, is not cut short."""
+    import fledge_gb300 as F
+    import torch
+    n = 3400000
+    pos = torch.tensor([[0.0, 0, 0.1], [1, 0, 3], [0, 1, 3]], device="cuda").repeat(n + 1, 1)
+    pos[3 * n:] = torch.tensor([[0.2, 0.2, 1.0], [0.6, 0.2, 1], [0.2, 0.6, 1]], device="cuda")
+    b = F.RadixBVHBuilder(F.InternalTriangleMesh(pos), ctx)
+    b.build()
+    r = torch.tensor([[0.3], [0.3], [-1.0], [0.0], [0.0], [2.0 ** 103]], device="cuda")
+    h = b.intersect(F.Rays.from_soa(r, tmin=0.0))
+    ctx.sync()
+    assert int(h["prim"][0]) == n and float(h["t"][0]) == 2.0 ** -102
