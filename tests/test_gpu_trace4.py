@@ -185,6 +185,47 @@ def test_hits_in_front_of_their_own_box(ctx, oracle):
         assert np.array_equal(hits[0][k][same], hits[1][k][same]), k
 
 
+@pytest.mark.parametrize("leaf", [1, 3, 8])
+@pytest.mark.parametrize("kind", ["soup", "copies3", "copies7", "copies9", "duplicates", "planes", "quads", "slivers"])
+def test_ids_are_those_of_the_walk_over_exact_boxes(ctx, kind, leaf):
+    """Directions 2^104 times as long take every ray over the exact boxes, with
+    all its arithmetic scaled by a power of two: the same ids (and distances, but
+    for the last bit: the low parts of their refinement become subnormal), also
+    where several triangles share the closest distance and the order of visits
+    decides (`copies<k>`: k equal triangles each, next to each other or not)."""
+    import fledge_gb300 as F
+    import torch
+    rng = np.random.default_rng(58)
+    rays = G.sphere_rays(200000, rng)
+    if kind.startswith("copies"):
+        tri = G.random_soup(1500, rng, half=0.05).reshape(-1, 9)
+        k = int(kind[6:])
+        pos = np.concatenate([np.repeat(tri[:750], k, 0), np.tile(tri[750:], (k, 1))])
+    elif kind == "quads":  # layers of squares, their diagonals and edges shared
+        x, y, z = np.meshgrid(np.arange(24) / 24, np.arange(24) / 24, (0.1, 0.3, 0.5, 0.7), indexing="ij")
+        c = [np.stack([x.ravel() + i / 24, y.ravel() + j / 24, z.ravel()], 1) for i, j in ((0, 0), (1, 0), (1, 1), (0, 1))]
+        pos = np.concatenate([np.concatenate([c[0], c[1], c[2]], 1), np.concatenate([c[0], c[2], c[3]], 1)])
+        rays[0:2, ::2] = rng.integers(0, 49, (2, 100000)) / 48  # every other one straight down through corners and edges
+        rays[2, ::2], rays[3:5, ::2], rays[5, ::2] = 2.0, 0.0, -1.0
+    elif kind == "slivers":
+        pos, rays = G.sliver_comb(64, rng)
+    else:
+        pos = G.random_soup(3000, rng, half=0.05) if kind == "soup" else _scene(kind)[0]
+    b, _ = U.gpu_build(ctx, np.ascontiguousarray(pos.reshape(-1, 3), np.float32), width=4, leaf=leaf)
+    rays = rays.astype(np.float32)
+    rays[6] = 0.0
+    long = rays.copy()
+    long[3:6] *= np.float32(2.0 ** 104)
+    (rd, _), (rl, _) = U.rays_dev(rays), U.rays_dev(long)
+    h, e = b.intersect(rd), b.intersect(rl)
+    ctx.sync()
+    assert (h["prim"] >= 0).float().mean() > 0.1
+    assert torch.equal(h["prim"], e["prim"]), int((h["prim"] != e["prim"]).sum())
+    hit = h["prim"] >= 0
+    assert ((h["t"] - e["t"] * 2.0 ** 104).abs() <= 2.0 ** -23 * h["t"])[hit].all()
+    assert torch.equal(b.intersectP(rd), b.intersectP(rl))
+
+
 def test_more_ties_than_the_list_holds(ctx):
     """Over 2^20 rays that all end in a tie: the list overflows and the rays
     are found by their marks.  Equal to tracing them in parts."""
