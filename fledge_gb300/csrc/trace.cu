@@ -554,19 +554,21 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
 // Inverse directions with a component below kInvMin or from kInvMax on, for the
 // quantised slab test.  False if the ray has to be traced over the exact boxes.
 //
-// An infinite component (of a direction's zero, or below 2^-128) would make every
-// plane distance of its axis NaN and drop the axis, so +-B takes its place, the
-// largest power of two for which 2^16 steps of the scene's root, and so of every
-// node, times B stay finite (2^90 if the root's step is infinite).  An exact plane
-// distance is +-inf there; the quantised one has its sign, except that an origin
-// between an exact plane and the quantised one is inside: no box is lost by that.
-// But the far distance of a box that the origin is inside of is finite now.  It is
-// at least 1/128 step x B, what quantise adds less the rounding of the distance,
-// and the step at least 2^-40 and at least 2^-30 of the origin's coordinate,
-// which lies between the planes.  Boxes nearer than that (`sure`), and than the
-// 2^126 of visit_q, are tested as the exact test tests them; and no box that the
+// An infinite component (of a direction's zero, or below 2^-128), or one so large
+// that 2^16 steps times it overflow, would make plane distances of its axis NaN
+// and drop the axis.  +-B takes its place, the largest power of two for which
+// 2^16 steps of the scene's root, and so of every node, times B stay finite (2^90
+// if the root's step is infinite).  The exact plane distances have the same signs
+// and are larger or infinite; an origin between an exact plane and the quantised
+// one is inside.  So no box is lost by its near planes.  But the far distance of
+// a box is smaller now.  It is at least 1/128 step x B, what quantise adds less
+// the rounding of the distance, and the step at least 2^-40 and at least 2^-30
+// of the box's coordinates, which are at least half the origin's if the far plane
+// is not half of that away.  Boxes nearer than that (`sure`), and than the 2^126
+// of visit_q, are tested as the exact test tests them; and no box that the
 // exact test accepts is farther (`far`) than tmax, or than the root's far plane on
-// an axis of a finite component.
+// another axis.  (1 M rays along z with 1e-38 along x: 10.2 ms with that axis
+// dropped, 0.67 with B.)
 constexpr uint32_t kInvMin = (127u - 100u) << 23, kInvMax = (127u + 64u) << 23;  // 2^-100 (the step is at least 2^-40), 2^64
 __device__ __forceinline__ uint32_t above_min(float inv) { return (__float_as_uint(inv) & 0x7FFFFFFFu) - kInvMin; }
 __device__ __forceinline__ bool odd_inv(const float3 &inv) {
@@ -584,14 +586,15 @@ __device__ __forceinline__ bool inv_q(const NodeQ *__restrict__ root, const floa
   bool small = false;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    if (is_finite(*ii[a])) {
+    const float b = __uint_as_float((e[a] == 255u ? 217u : min(254u, 379u - e[a])) << 23);
+    if (fabsf(*ii[a]) <= b) {
       // 256 steps cover the box
       far = fminf(far, (fabsf(__uint_as_float(org[a]) - oo[a]) + __uint_as_float(e[a] << 23) * 0.00390625f) * fabsf(*ii[a]));
       small |= (__float_as_uint(*ii[a]) & 0x7FFFFFFFu) < kInvMin;
     } else {
-      *ii[a] = copysignf(__uint_as_float((e[a] == 255u ? 217u : min(254u, 379u - e[a])) << 23), *ii[a]);
+      *ii[a] = copysignf(b, *ii[a]);
       // half of it, for the roundings here
-      sure = fminf(sure, fmaxf(3.5527136788005009e-15f, fabsf(oo[a]) * 3.637978807091713e-12f) * fabsf(*ii[a]));
+      sure = fminf(sure, fmaxf(3.5527136788005009e-15f, fabsf(oo[a]) * 3.637978807091713e-12f) * b);
     }
     hits &= is_finite(oo[a]) && dd[a] == dd[a];  // else the ray hits nothing
   }
