@@ -20,14 +20,6 @@ namespace flg {
 constexpr int kMaxLevels = 64;
 constexpr int kCollapseThreads = 128;
 constexpr int kCollapseNodes = 4;
-// 4-wide layouts hold leaf ranges of at most this many triangles, whatever
-// the handle's leaf_size: with quantised nodes a visit costs about as much as
-// a triangle test, and ranges of 1 / 2 / 3 / 4 traced 24 batched scenes in
-// 20.7 / 20.5 / 22.0 / 23.8 ms (64 k soup 890 / 913 / 985 / 1061 us, camera
-// rays 243 / 228 / 228 / 236).  The hits stay those of ranges of leaf_size:
-// k_trace4's superset argument does not depend on the ranges, and retrace4 and
-// first_of_two form the exact tree with leaf_size.
-constexpr int kLeaf4 = 2;
 // Counters of a collapse; the initial values of these kCtrLive words follow as a
 // static copy.
 enum {

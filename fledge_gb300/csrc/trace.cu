@@ -1707,6 +1707,8 @@ __global__ void __launch_bounds__(256, 4)
   }
 }
 
+constexpr int kRefill4 = 8;
+
 // One trace over the 4-wide layout: the traversal, then the hit values (any
 // hit: the overflow list).
 //
@@ -1715,7 +1717,7 @@ __global__ void __launch_bounds__(256, 4)
 // instructions.  A batch too small to give sixteen full warps to every SM is
 // spread over that many (before lanes helped: 4,096 rays on 20,001 triangles 72
 // us, 92 in full warps, 96 in one-ray warps), and its blocks are made smaller
-// until they cover the SMs.  Refills at 8 idle lanes at most: with the
+// until they cover the SMs.  Refills at kRefill4 idle lanes at most: with the
 // quantised nodes 8 beat 16 and 24 (24.0 against 25.6 and 29.6 ms on 31.6 M
 // scattered rays).
 template <bool ANY>
@@ -1730,7 +1732,7 @@ static int launch4(flg_ctx ctx, cudaStream_t st, flg_bvh b, const RaySoA &R, int
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace4<ANY, false>, threads, 0);
     g = std::min<int64_t>(g, (int64_t)std::max(per_sm, 1) * ctx->num_sms);
   }
-  const int refill = std::max(1, std::min(8, op.refill_lanes));
+  const int refill = std::max(1, std::min(kRefill4, op.refill_lanes));
   const RayCount N{n, n_dev};
   const Exact4 X{b->d_nodes2, b->d_tris, Ranges{b->d_rfirst, b->d_rcount}, b->leaf_size, b->d_root, ray_off, n_scenes,
                  2 * b->n_tri};
@@ -2099,9 +2101,11 @@ namespace flg {
 
 // Staged search of the traversal configuration on a given workload (node
 // width and leaf size, then the kernel, then the block size; single-scene
-// handles also try the ray-sort key).  Every trial is one untimed launch and
-// `reps` launches timed one by one with events; the trial's time is their
-// median.  Leaves the handle at the fastest layout.
+// handles also try the ray-sort key).  Options that a layout's kernel does not
+// read are not varied: the 4-wide one has leaf ranges of at most kLeaf4
+// triangles and one kernel, which refills at kRefill4 idle lanes at most.  Every
+// trial is one untimed launch and `reps` launches timed one by one with events;
+// the trial's time is their median.  Leaves the handle at the fastest layout.
 struct Tuner {
   flg_ctx ctx;
   flg_bvh bvh;
@@ -2163,7 +2167,7 @@ struct Tuner {
     // 1. layout, with the default kernel of each width
     for (int w : {2, 4, 8}) {
       for (int leaf : {1, 2, 3, 4}) {
-        if (w == 2 && leaf > 1) continue;
+        if ((w == 2 && leaf > 1) || (w == 4 && leaf > kLeaf4)) continue;
         rc = flg_bvh_set_width(ctx, bvh, w, leaf);
         if (rc) return rc;
         rc = trial(w, leaf, kernel_opts(w, 2, 8, 64, 256), "layout");
@@ -2174,7 +2178,12 @@ struct Tuner {
     rc = flg_bvh_set_width(ctx, bvh, w, leaf);
     if (rc) return rc;
     // 2. kernel on that layout
-    if (w > 2) {
+    if (w == 4) {
+      for (int refill : {2, 4, 6}) {
+        rc = trial(w, leaf, kernel_opts(w, 2, refill, 64, 256), "kernel");
+        if (rc) return rc;
+      }
+    } else if (w > 2) {
       for (int pers : {0, 1, 2})
         for (int refill : {4, 8, 16})
           for (int stack : {32, 64}) {
@@ -2188,9 +2197,11 @@ struct Tuner {
       if (rc) return rc;
     }
     // 3. block size
-    {
-      flg_trace_opts op = best;
-      op.block_threads = 128;
+    const flg_trace_opts kernel = best;
+    for (int threads : {64, 128}) {
+      if (threads == 64 && w != 4) continue;
+      flg_trace_opts op = kernel;
+      op.block_threads = threads;
       rc = trial(w, leaf, op, "block");
       if (rc) return rc;
     }

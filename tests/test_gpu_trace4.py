@@ -352,3 +352,32 @@ def test_a_walk_of_more_than_2_to_22_entries(ctx):
     h = b.intersect(F.Rays.from_soa(r, tmin=0.0))
     ctx.sync()
     assert int(h["prim"][0]) == n and float(h["t"][0]) == 2.0 ** -102
+
+
+@pytest.mark.parametrize("scenes", [1, 5])
+def test_the_tuner_tries_nothing_twice(ctx, scenes):
+    """Every trial on the 4-wide layout differs from the others in something
+    that its kernel reads: leaf ranges up to 2, refills up to 8 lanes, the block
+    size, the ray sort."""
+    import ctypes as C
+    import json
+
+    import fledge_gb300 as F
+    offs = np.arange(scenes + 1, dtype=np.int64) * 4000
+    mesh = F.InternalTriangleMesh(F.gen_triangles(ctx, int(offs[-1]), 21))
+    rays = F.Rays.from_soa(F.gen_rays(ctx, 10 * int(offs[-1]), 22), tmin=1e-4)
+    best, w, leaf, buf, r = F.FlgTraceOpts(), C.c_int32(), C.c_int32(), C.create_string_buffer(1 << 16), rays.struct()
+    if scenes == 1:
+        b = F.RadixBVHBuilder(mesh, ctx)
+        b.build()
+        ctx.check(ctx.lib.flg_autotune_trace(ctx.h, b.h, C.byref(r), rays.n, C.byref(best), C.byref(w), buf, len(buf)))
+    else:
+        b = F.BatchedRadixBVHBuilder(mesh, offs, ctx)
+        b.build()
+        ro = np.ascontiguousarray(10 * offs)
+        ctx.check(ctx.lib.flg_autotune_trace_batched(ctx.h, b.h, C.byref(r), ro.ctypes.data_as(C.POINTER(C.c_int64)), 3,
+                                                     C.byref(best), C.byref(w), C.byref(leaf), buf, len(buf)))
+    four = [(min(t["leaf_size"], 2), min(t["refill_lanes"], 8), t["block_threads"], t["ray_sort"])
+            for t in json.loads(buf.value.decode())["trials"] if t["node_width"] == 4]
+    assert w.value == 4 and len(four) > 6
+    assert len(set(four)) == len(four), four
