@@ -1026,10 +1026,13 @@ __global__ void __launch_bounds__(128)
 // under the rules for a second candidate of the same ray, and all take its t
 // for their limit; it retires once its helpers are done.
 //
-// leaf_wait (any hit): kLeafWait, but kLeafWaitAny in a tree of more than kLargeTree
-// triangles, where lanes find their first leaf at more different times
-// (2 M shadow rays on 330,000 triangles 468 -> 461 us, 12 M on 8 M triangles 2630 ->
-// 2785 Mrays/s; on 20,480 triangles 76 against 81 us).
+// leaf_wait: kLeafWait; for any hit (one scene) kLeafWaitAny in a tree of more than
+// kLargeTree triangles.  The deeper the tree, the more the turns differ at which
+// the lanes of a warp find their first leaf.  2 M shadow rays, 12 lanes against 8:
+// displaced spheres of 1,280 triangles 281 / 271 us, 5,120 325 / 317, 20,480 374 /
+// 370, 81,920 428 / 425, 327,680 490 / 492, 1.3 M 561 / 573 (200,000 rays: 5,120
+// 87 / 82, 20,480 108 / 104, 81,920 136 / 136, 1.3 M 220 / 225); soups of 65,536 to 8 M
+// triangles within 1 % of each other, 12 lanes ahead by 0.2 to 0.9 % at 2 M rays.
 constexpr int kLeafWait = 8, kLeafWaitAny = 12;
 constexpr int64_t kLargeTree = 1 << 18;
 // Slots, the sentinel's included.  With the ray indices 32 KB per 256-thread
