@@ -34,7 +34,9 @@ constexpr int32_t kBoxUnset = (int32_t)0xFFC0DEADu;
 constexpr int32_t kEmptyChild = 0x7FFFFFFF;
 
 // 4-wide node: the children's boxes in 8 bits per plane, as (origin + byte x
-// step) per axis with a power-of-two step, conservative (quantise, wide.cuh).  The traversal is
+// step) per axis with a power-of-two step, conservative (quantise, wide.cuh); the
+// idea is that of compressed wide nodes (Ylitie, Karras, Laine, "Efficient Incoherent
+// Ray Traversal on GPUs Through Compressed Wide BVHs", HPG 2017).  The traversal is
 // bound by its divergent 16-byte loads, one L1 wavefront per lane and load:
 // this record takes 3 per visit against 6 and the refs for the same boxes in
 // fp32.  Inner children sit in consecutive slots; a leaf child's range is read

@@ -8,14 +8,14 @@
 // gathered in sorted (leaf) order, 48 bytes each.
 //
 // Kernels:
-//   k_trace4            4-wide: while-while traversal with parked leaves, one
-//                       ray per thread or persistent warps that refill idle
-//                       lanes from a global ray counter (work stealing across
-//                       scenes of a batch); k_settle4 or k_trace_retry4 after it
+//   k_trace4            4-wide: while-while traversal with parked leaves;
+//                       persistent warps refill idle lanes from a global ray
+//                       counter (work stealing across scenes of a batch);
+//                       k_settle4 or k_trace_retry4 after it
 //   k_trace_bvh2        one ray per thread over BVH2, leaf triangles tested
 //                       directly as the reference does (no leaf box test)
-//   k_trace_wide, k_trace_persistent, k_trace_ww   the same three schedules
-//                       over 8-wide nodes
+//   k_trace_wide, k_trace_persistent, k_trace_ww   8-wide: one ray per thread,
+//                       persistent warps, and these with parked leaves
 //   k_trace_retry       rays whose short stack overflowed, with a deep stack
 #include <algorithm>
 #include <chrono>

@@ -42,12 +42,13 @@ __device__ __forceinline__ void load_vray(const VRays &R, int64_t i, float3 &o, 
 // Together with one bounds test and one address per lattice cell (grid_cell), us
 // before -> after: delta tracking of 2 M rays through a 192^3 sparse grid 927 ->
 // 547, with two steps to a turn 460, with refills at 4 idle lanes 434 (8: 446), and
-// with a pointer to each of the two layers of bricks 1.5 % less; of 1 M rays through a 256^3 dense one 83 ->
-// 52 -> 47; ratio tracking of the latter 85 -> 75, its adjoint 85 -> 79.  Ratio
-// tracking, which waits for scattered sectors of the grid (29 % of L2's and 30 %
-// of DRAM's rate, L1 at 41 %), gains nothing from turns of four draws (76 us,
-// the adjoint 85), nor from lookups of steps ahead; with refills at 4 idle lanes it
-// takes 81 us, at 16 77.
+// with a pointer to each of the two layers of bricks 1.5 % less; of 1 M rays
+// through a 256^3 dense one 83 -> 52 -> 47.  Ratio tracking of the latter became 5 %
+// faster, its adjoint 3 %: it waits for one dependent lookup after the other
+// (stalls on loads: 5.4 and 10.2 per issued instruction; L1 at 61 and 36 % of
+// its rate, L2 at 50 and 41, DRAM at 28 and 56, 17.7 and 12.1 of 32 lanes active).
+// It gains nothing from turns of four draws (75 -> 76 us, the adjoint 79 -> 85), nor
+// from lookups of steps ahead; with refills at 4 idle lanes it takes 81 us, at 16 77.
 constexpr int kVolRefill = 8, kSampleRefill = 4;
 
 struct WarpChunk {

@@ -183,7 +183,7 @@ __device__ __forceinline__ void walk_open(const Node2 *__restrict__ nodes2, cons
 }
 
 // Quantises the children's boxes of a 4-wide node (NodeQ): per axis an origin
-// and a power-of-two step; every child's lower plane rounds down and its
+// and a power-of-two step, as in Ylitie, Karras and Laine's nodes; every child's lower plane rounds down and its
 // upper plane up, both with at least 1/64 step to spare.  The slack covers
 // the rounding of the traversal's plane distances, so that a box test on the
 // record never rejects a box that the exact test accepts (visit_q).  The
