@@ -53,7 +53,8 @@ BYTES_PER_RAY = 24 + 16
 STAGE_BYTES_PER_TRI = {"bounds": 36, "morton": 48, "sort_pass": 16, "climb": 120}
 BYTES_PER_TRI = 268
 TRACE_PROFILE = os.path.join(ROOT, "profiles", "k_trace4_config3.json")
-TRACE_SOURCES = ["fledge_gb300/csrc/trace.cu", "fledge_gb300/csrc/common.cuh", "fledge_gb300/csrc/internal.h"]
+TRACE_SOURCES = ["fledge_gb300/csrc/trace.cu", "fledge_gb300/csrc/wide.cuh", "fledge_gb300/csrc/collapse.cu",
+                 "fledge_gb300/csrc/common.cuh", "fledge_gb300/csrc/internal.h"]
 TUNED = os.path.join(ROOT, "fledge_gb300", "tuned", "batched_config3.json")
 
 _T0 = time.perf_counter()
