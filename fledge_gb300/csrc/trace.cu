@@ -520,17 +520,22 @@ __global__ void __launch_bounds__(256)
 //     settles the equal pairs (first_of_two) and traces the others again over
 //     the exact boxes (retrace4), of which those around the hit decide where only
 //     rounding is in question: about one ray per million on random soups.
-//     Left open are triangles that were not tested, their boxes being beyond
-//     the hit, while their t is not: a grazing triangle's t loses its digits
-//     as N.D goes to 0.  The exact order may come to such a triangle before
-//     the hit, and this one, almost the same, after it: 34 of 131,072 rays, each
-//     through 16 slivers of 1e-7 to 1e-6 of the distance, none with slivers ten times
-//     as wide.
+//   * A triangle's fp32 t may also lie in front of its own box: by rounding at
+//     vertices and edges, the more the smaller the triangle is for its
+//     distance, and without bound for a grazing one, as N.D goes to 0.  The exact
+//     order may come to such a triangle before another hit whose t lies
+//     between, so boxes up to kBeyond of t beyond the hit are entered too.
+//     Left open are triangles that lie further than that in front of their box:
+//     none in 150 M rays at the vertices of spheres and soups from 3, 30 and 300
+//     sizes away; 34 of 131,072 rays, each through 16 slivers of 1e-7 to 1e-6 of the
+//     distance.
 //   * Any hit: an accepted triangle counts if its own box passes the exact slab
 //     test.  A ray that found only others is traced again over the exact boxes
 //     (k_trace_retry4).
 // ----------------------------------------------------------------------------
 constexpr float kNear = 4.76837158203125e-07f;  // 2^-21
+constexpr float kBeyond = 1.220703125e-04f;     // 2^-13: 2^-20 left 28 of 4.2 M such rays wrong, 2^-14 one
+constexpr float kAround = 9.765625e-04f;        // 2^-10: what retrace4 takes for the surroundings of a hit
 // prim between k_trace4 and the kernels after it: a sorted position (< 2^28) with
 // kPending, -1, or kListed for a listed ray.  A listed ray's u and v hold two
 // positions at the same t; or v = kByWalk: candidates within kNear; or v = -1:
@@ -648,8 +653,8 @@ __device__ __forceinline__ float byte_f(uint32_t w) {
 // stack entry is culled); a miss is ~0.  Per axis the plane distance
 // of byte q is fma(1/2 + q / 2^16, s, (origin - o) inv - s / 2) with s = 2^16 step inv.
 // Its error is below 1/64 step (the boxes' slack) plus 2^-22 of itself, and the
-// exact test's own below 2^-23: with tnear scaled by 1 - 2^-20 the test passes
-// whenever the exact one does.  For that s must not be subnormal (rays with
+// exact test's own below 2^-23: with tnear scaled by 1 - kBeyond the test passes
+// whenever the exact one does (2^-20 would do).  For that s must not be subnormal (rays with
 // an inverse below kInvMin are traced over the exact boxes).  Where s is infinite
 // the distances are NaN and the axis constrains nothing.  Where s is finite and
 // (origin - o) inv - s / 2 is not, the origin lies 2^15 steps or more outside and
@@ -667,7 +672,7 @@ __device__ __forceinline__ void visit_q(const NodeQ *__restrict__ node, const fl
   const float by = fmaf(-0.5f, sy, (__uint_as_float(A.y) - o.y) * inv.y);
   const float bz = fmaf(-0.5f, sz, (__uint_as_float(A.z) - o.z) * inv.z);
   // (near, far) pairs, the near one scaled
-  constexpr float k = 0.99999905f;  // 1 - 2^-20
+  constexpr float k = 1.0f - kBeyond;
   const f32x2 sx2 = pack2(sx * k, sx), sy2 = pack2(sy * k, sy), sz2 = pack2(sz * k, sz);
   const f32x2 bx2 = pack2(bx * k, bx), by2 = pack2(by * k, by), bz2 = pack2(bz * k, bz);
   const bool gx = __float_as_int(inv.x) < 0, gy = __float_as_int(inv.y) < 0, gz = __float_as_int(inv.z) < 0;
@@ -771,8 +776,8 @@ __device__ __forceinline__ void tri_rec_box(const TriRec *__restrict__ tris, int
 //
 // `near` >= 0: the t that the traversal found to be the closest.  What the exact
 // order finds is decided by the candidates that lie within rounding of it, so the
-// walk only enters boxes that the ray is in there: about as many as the tree is
-// deep.  (Should it find nothing, it starts again without `near`.)  1 M rays on
+// walk only enters boxes that the ray is in there, give or take kAround: about as
+// many as the tree is deep.  (Should it find nothing, it starts again without `near`.)  1 M rays on
 // 65,536 triangles, three of each: 10.9 ms with whole walks, 1.97 with these.
 struct ExactHit {
   int32_t prim;
@@ -791,7 +796,7 @@ __device__ __forceinline__ ExactHit retrace4(const Exact4 &X, const RaySoA &RS, 
   if (root == INT32_MIN) return h;
   bool again;
   do {
-    float best = near >= 0.0f ? fminf(near * (1.0f + kNear), tmax) : tmax;
+    float best = near >= 0.0f ? fminf(near * (1.0f + kAround), tmax) : tmax;
     bool have = false;
     int sp = 0;
     int32_t cur = root < 0 ? ~((~root) << 3) : root;
@@ -814,7 +819,7 @@ __device__ __forceinline__ ExactHit retrace4(const Exact4 &X, const RaySoA &RS, 
           key[k] = ~0u;
           ref[k] = 0;
           if (k < nc) {
-            const float t0 = slab_exact(c[k].lo, c[k].hi, o, inv, best, near * 0.999f);
+            const float t0 = slab_exact(c[k].lo, c[k].hi, o, inv, best, near * (1.0f - kAround));
             if (t0 == t0) {
               key[k] = (__float_as_uint(t0) & 0x7FFFFFFCu) | (uint32_t)k;
               ++nh;
@@ -1165,7 +1170,7 @@ __global__ void __launch_bounds__(256, 4)
           tri_rec_box(tris, prim, lo, hi);
           float t0 = slab_exact(lo, hi, o, ie, 3.402823466e+38f);
           listed = tie == kNone ? !(t0 <= best * (1.0f + kNear)) : tie == kSome ? !(t0 <= best) : true;
-          if (t0 <= best * (1.0f + kNear)) other = kByWalk;
+          if (t0 <= best * (1.0f + 0.5f * kAround)) other = kByWalk;
           if (tie >= 0 && t0 <= best) {
             tri_rec_box(tris, tie, lo, hi);
             t0 = slab_exact(lo, hi, o, ie, 3.402823466e+38f);

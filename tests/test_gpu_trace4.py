@@ -226,6 +226,36 @@ def test_ids_are_those_of_the_walk_over_exact_boxes(ctx, kind, leaf):
     assert torch.equal(b.intersectP(rd), b.intersectP(rl))
 
 
+@pytest.mark.parametrize("leaf", [1, 2])
+@pytest.mark.parametrize("distance", [3.0, 30.0, 300.0])
+def test_rays_at_the_vertices_of_a_mesh(ctx, distance, leaf):
+    """Rays at the vertices of a displaced sphere of 81,920 triangles, half of them
+    off by up to 1e-6: the triangles around a vertex share its distance but for
+    rounding, which also puts some of the distances before their boxes.  The
+    same ids as by the walk over exact boxes (directions 2^104 times as long)."""
+    import fledge_gb300 as F
+    import torch
+    from fledge_gb300 import scenes
+    v, f = scenes.icosphere(6, amplitude=0.05)
+    g = torch.Generator(device="cuda").manual_seed(int(distance))
+    n = 1 << 20
+    p, ind = U.dev(v.astype(np.float32)), U.dev(f.astype(np.int32))
+    o = torch.randn(3, n, device="cuda", generator=g)
+    o = o / o.norm(dim=0) * distance
+    at = p[torch.randint(0, p.shape[0], (n,), device="cuda", generator=g)].T
+    at = at + (torch.rand(3, n, device="cuda", generator=g) - 0.5) * 2e-6 * (torch.arange(n, device="cuda") % 2)
+    d = at - o
+    d = d / d.norm(dim=0)
+    b = F.RadixBVHBuilder(F.InternalTriangleMesh(p, ind), ctx, leaf_size=leaf)
+    b.build()
+    r, rl = (F.Rays.from_soa(torch.cat([o, d * k], 0).contiguous(), tmin=0.0) for k in (1.0, 2.0 ** 104))
+    h, e = b.intersect(r)["prim"], b.intersect(rl)["prim"]
+    ctx.sync()
+    assert (h >= 0).float().mean() > 0.9
+    assert torch.equal(h, e), int((h != e).sum())
+    assert torch.equal(b.intersectP(r), b.intersectP(rl))
+
+
 def test_more_ties_than_the_list_holds(ctx):
     """Over 2^20 rays that all end in a tie: the list overflows and the rays
     are found by their marks.  Equal to tracing them in parts."""
