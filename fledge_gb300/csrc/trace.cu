@@ -520,21 +520,22 @@ __global__ void __launch_bounds__(256)
 //     settles the equal pairs (first_of_two) and traces the others again over
 //     the exact boxes (retrace4), of which those around the hit decide where only
 //     rounding is in question: about one ray per million on random soups.
-//   * A triangle's fp32 t may also lie in front of its own box: by rounding at
-//     vertices and edges, the more the smaller the triangle is for its
-//     distance, and without bound for a grazing one, as N.D goes to 0.  The exact
-//     order may come to such a triangle before another hit whose t lies
-//     between, so boxes up to kBeyond of t beyond the hit are entered too.
-//     Left open are triangles that lie further than that in front of their box:
-//     none in 150 M rays at the vertices of spheres and soups from 3, 30 and 300
-//     sizes away; 34 of 131,072 rays, each through 16 slivers of 1e-7 to 1e-6 of the
-//     distance.
+//   * A triangle's fp32 t may also lie outside of its own box: by rounding at
+//     vertices and edges, the more the smaller the triangle is for its distance
+//     or the direction along an axis, and without bound for a grazing one, as
+//     N.D goes to 0.  The exact order may come to such a triangle before
+//     another hit whose t lies between, so boxes up to kBeyond of t beyond the hit
+//     are entered too.  Left open are triangles that lie further than that in front
+//     of their box: none in 150 M rays at the vertices of spheres and soups from 3,
+//     30 and 300 sizes away, 8 of 2 M where the directions' components along two axes
+//     are 1 to 1e-7, 34 of 131,072 rays through 16 slivers each, of 1e-7 to 1e-6 of the
+//     distance; in no occlusion.
 //   * Any hit: an accepted triangle counts if its own box passes the exact slab
 //     test.  A ray that found only others is traced again over the exact boxes
 //     (k_trace_retry4).
 // ----------------------------------------------------------------------------
 constexpr float kNear = 4.76837158203125e-07f;  // 2^-21
-constexpr float kBeyond = 1.220703125e-04f;     // 2^-13: 2^-20 left 28 of 4.2 M such rays wrong, 2^-14 one
+constexpr float kBeyond = 1.220703125e-04f;     // 2^-13: of 4.2 M such rays 2^-20 left 28 wrong, 2^-14 one
 constexpr float kAround = 9.765625e-04f;        // 2^-10: what retrace4 takes for the surroundings of a hit
 // prim between k_trace4 and the kernels after it: a sorted position (< 2^28) with
 // kPending, -1, or kListed for a listed ray.  A listed ray's u and v hold two
@@ -735,20 +736,27 @@ __device__ __forceinline__ bool pluecker_t2(float3 a, float3 b, float3 c, float3
 }
 
 // The exact slab test of a box against (o, inv), limit lim: tnear, or NaN on
-// a miss or with tfar below `reach` — the same operations as the fp32 wide nodes'
-// visit_node.
+// a miss — the same operations as the fp32 wide nodes' visit_node.  `reach`: where
+// the ray leaves the box enlarged by `slack`.
 __device__ __forceinline__ float slab_exact(const float *lo, const float *hi, const float3 &o, const float3 &inv,
-                                            float lim, float reach = 0.0f) {
+                                            float lim, float slack, float &reach) {
   const float oo[3] = {o.x, o.y, o.z}, ii[3] = {inv.x, inv.y, inv.z};
   float t0 = 0.0f, t1 = fminf(lim, 3.402823466e+38f);
+  reach = __int_as_float(0x7f800000);
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     const bool g = (__float_as_uint(ii[a]) >> 31) != 0u;
     const float tn = ((g ? hi[a] : lo[a]) - oo[a]) * ii[a], tf = ((g ? lo[a] : hi[a]) - oo[a]) * ii[a];
     t0 = fmaxf(tn, t0);
     t1 = fminf(tf, t1);
+    reach = fminf(tf + slack * fabsf(ii[a]), reach);
   }
-  return t0 <= t1 && t1 >= reach ? t0 : __int_as_float(0x7fffffff);
+  return t0 <= t1 ? t0 : __int_as_float(0x7fffffff);
+}
+__device__ __forceinline__ float slab_exact(const float *lo, const float *hi, const float3 &o, const float3 &inv,
+                                            float lim) {
+  float reach;
+  return slab_exact(lo, hi, o, inv, lim, 0.0f, reach);
 }
 
 // The exact-box tree of a 4-wide handle.
@@ -797,6 +805,8 @@ __device__ __forceinline__ ExactHit retrace4(const Exact4 &X, const RaySoA &RS, 
   bool again;
   do {
     float best = near >= 0.0f ? fminf(near * (1.0f + kAround), tmax) : tmax;
+    // a hit may lie that far from its triangle
+    const float slack = fabsf(near) * max3f(fabsf(d.x), fabsf(d.y), fabsf(d.z)) * 3.814697265625e-06f;  // 2^-18
     bool have = false;
     int sp = 0;
     int32_t cur = root < 0 ? ~((~root) << 3) : root;
@@ -819,8 +829,9 @@ __device__ __forceinline__ ExactHit retrace4(const Exact4 &X, const RaySoA &RS, 
           key[k] = ~0u;
           ref[k] = 0;
           if (k < nc) {
-            const float t0 = slab_exact(c[k].lo, c[k].hi, o, inv, best, near * (1.0f - kAround));
-            if (t0 == t0) {
+            float reach;
+            const float t0 = slab_exact(c[k].lo, c[k].hi, o, inv, best, slack, reach);
+            if (t0 == t0 && !(reach < near * (1.0f - kAround))) {
               key[k] = (__float_as_uint(t0) & 0x7FFFFFFCu) | (uint32_t)k;
               ++nh;
             }

@@ -256,6 +256,37 @@ def test_rays_at_the_vertices_of_a_mesh(ctx, distance, leaf):
     assert torch.equal(b.intersectP(r), b.intersectP(rl))
 
 
+@pytest.mark.parametrize("leaf", [1, 2])
+@pytest.mark.parametrize("kind", ["flat", "inside"])
+def test_rays_nearly_along_an_axis_at_the_vertices(ctx, kind, leaf):
+    """Rays at the vertices of a height field whose direction has a component of
+    about 1e-3 along x (`flat`): a triangle hit by rounding beside its box may be
+    one that the ray leaves along that axis well before the hit.  The same ids as by the walk over exact boxes (directions 2^104 times
+    as long)."""
+    import fledge_gb300 as F
+    import torch
+    m, n = 256, 1 << 21
+    g = torch.Generator(device="cuda").manual_seed(17)
+    x, y = torch.meshgrid(torch.arange(m + 1, device="cuda") / m, torch.arange(m + 1, device="cuda") / m, indexing="ij")
+    p = torch.stack([x, y, 0.1 * torch.sin(11 * x) * torch.cos(7 * y)], -1).reshape(-1, 3).contiguous()
+    i = (torch.arange(m, device="cuda")[:, None] * (m + 1) + torch.arange(m, device="cuda")).reshape(-1)
+    f = torch.cat([torch.stack([i, i + m + 1, i + m + 2], 1), torch.stack([i, i + m + 2, i + 1], 1)]).int().contiguous()
+    d = torch.randn(n, 3, device="cuda", generator=g)
+    if kind == "flat":
+        d[:, 0] *= 1e-3
+    d = d / d.norm(dim=1, keepdim=True)
+    back = 0.3 * torch.rand(n, 1, device="cuda", generator=g) if kind == "inside" else 3.0
+    o = p[torch.randint(0, p.shape[0], (n,), device="cuda", generator=g)] - back * d
+    b = F.RadixBVHBuilder(F.InternalTriangleMesh(p, f), ctx, leaf_size=leaf)
+    b.build()
+    r, rl = (F.Rays.from_soa(torch.cat([o.T, d.T * k], 0).contiguous(), tmin=0.0) for k in (1.0, 2.0 ** 104))
+    h, e = b.intersect(r)["prim"], b.intersect(rl)["prim"]
+    ctx.sync()
+    assert (h >= 0).float().mean() > 0.9
+    assert torch.equal(h, e), int((h != e).sum())
+    assert torch.equal(b.intersectP(r), b.intersectP(rl))
+
+
 def test_more_ties_than_the_list_holds(ctx):
     """Over 2^20 rays that all end in a tie: the list overflows and the rays
     are found by their marks.  Equal to tracing them in parts."""
