@@ -470,7 +470,7 @@ static int collapse_levels(flg_ctx ctx, flg_bvh b) {
   Collapse X;
   X.nodes2 = b->d_nodes2;
   X.R = Ranges{b->d_rfirst, b->d_rcount};
-  X.leaf_size = W == 4 ? std::min<int>(b->leaf_size, kLeaf4) : b->leaf_size;
+  X.leaf_size = b->leaf_size;
   X.roots = b->d_queue_init;
   X.n_roots = b->n_wide_roots;
   X.cap = b->wide_cap;

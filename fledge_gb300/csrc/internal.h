@@ -56,15 +56,6 @@ static_assert(sizeof(NodeQ) == 64, "NodeQ layout");
 // mark in a bit that no exponent uses.
 constexpr uint32_t kLoneStep = 255u << 23 | 255u << 15 | 255u << 7 | 1u;
 
-// 4-wide layouts hold leaf ranges of at most this many triangles, whatever
-// the handle's leaf_size: with quantised nodes a visit costs about as much as
-// a triangle test, and ranges of 1 / 2 / 3 / 4 traced 24 batched scenes in
-// 20.7 / 20.5 / 22.0 / 23.8 ms (64 k soup 890 / 913 / 985 / 1061 us, camera
-// rays 243 / 228 / 228 / 236).  The hits stay those of ranges of leaf_size:
-// k_trace4's superset argument does not depend on the ranges, and retrace4 and
-// first_of_two form the exact tree with leaf_size.
-constexpr int kLeaf4 = 2;
-
 // 8-wide node, structure of arrays inside the record (14 16-byte loads per
 // visit).
 template <int W>

@@ -510,6 +510,10 @@ __global__ void __launch_bounds__(256)
 //   * A quantised box contains the exact one with room for every rounding of
 //     visit_q, so the leaves visited are a superset of the exact ones.  (A ray
 //     whose direction leaves no such room is traced over the exact boxes: inv_q.)
+//     The leaf ranges are the exact tree's: in smaller ones, which would be faster
+//     (24 batched scenes in ranges of up to 1 / 2 / 3 / 4: 18.9 / 20.1 / 22.3 / 24.7 ms),
+//     a ray that misses a triangle's own box by rounding, but not its range's,
+//     would not test it.
 //   * Closest hit: a finished ray's winner stands if its own box, which its
 //     leaf range's and every ancestor's box contain, passes the exact slab
 //     test with tnear <= t: then the exact traversal reaches it, whatever it
@@ -2121,10 +2125,10 @@ namespace flg {
 // Staged search of the traversal configuration on a given workload (node
 // width and leaf size, then the kernel, then the block size; single-scene
 // handles also try the ray-sort key).  Options that a layout's kernel does not
-// read are not varied: the 4-wide one has leaf ranges of at most kLeaf4
-// triangles and one kernel, which refills at kRefill4 idle lanes at most.  Every
-// trial is one untimed launch and `reps` launches timed one by one with events;
-// the trial's time is their median.  Leaves the handle at the fastest layout.
+// read are not varied: the 4-wide one has one kernel, which refills at kRefill4
+// idle lanes at most.  Every trial is one untimed launch and `reps` launches timed
+// one by one with events; the trial's time is their median.  Leaves the handle at
+// the fastest layout.
 struct Tuner {
   flg_ctx ctx;
   flg_bvh bvh;
@@ -2186,7 +2190,7 @@ struct Tuner {
     // 1. layout, with the default kernel of each width
     for (int w : {2, 4, 8}) {
       for (int leaf : {1, 2, 3, 4}) {
-        if ((w == 2 && leaf > 1) || (w == 4 && leaf > kLeaf4)) continue;
+        if (w == 2 && leaf > 1) continue;
         rc = flg_bvh_set_width(ctx, bvh, w, leaf);
         if (rc) return rc;
         rc = trial(w, leaf, kernel_opts(w, 2, 8, 64, 256), "layout");

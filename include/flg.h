@@ -257,16 +257,16 @@ FLG_API int flg_trace_closest_noalloc(flg_ctx ctx, flg_bvh bvh, const flg_rays *
 
 /* Autotuner of the traversal (no counterpart in the reference): a staged
  * search on the given workload — (1) node width 2/4/8 with leaf ranges of
- * 1..4 triangles (4-wide: 1..2) under each width's default kernel, (2) on the
- * fastest layout the kernel (8-wide: one ray per thread, persistent, persistent
+ * 1..4 triangles under each width's default kernel, (2) on the fastest
+ * layout the kernel (8-wide: one ray per thread, persistent, persistent
  * while-while; refill threshold 4/8/16; stack depth 32/64.  4-wide, where one
  * kernel has no such options: refill threshold 2/4/6/8), (3) 128- or 256-thread
- * blocks (4-wide: also 64), (4) for single-scene traces the ray-sort key.  Each trial is one
- * untimed and `reps` timed launches; its time is their median.  Leaves the
- * handle laid out at the fastest width and leaf size, returns the fastest
- * options in *best and writes a JSON record of every trial (NUL-terminated)
- * to json_out (FLG_ERR_ARG if json_len is too small).  Synchronous; not
- * capturable.  flg_autotune_trace: single-scene handles, reps = 5. */
+ * blocks (4-wide: also 64), (4) for single-scene traces the ray-sort key.  Each
+ * trial is one untimed and `reps` timed launches; its time is their median.
+ * Leaves the handle laid out at the fastest width and leaf size, returns the
+ * fastest options in *best and writes a JSON record of every trial
+ * (NUL-terminated) to json_out (FLG_ERR_ARG if json_len is too small).
+ * Synchronous; not capturable.  flg_autotune_trace: single-scene handles, reps = 5. */
 FLG_API int flg_autotune_trace(flg_ctx ctx, flg_bvh bvh, const flg_rays *rays, int64_t n,
                                flg_trace_opts *best, int32_t *best_node_width, char *json_out,
                                size_t json_len);

@@ -226,7 +226,7 @@ def test_ids_are_those_of_the_walk_over_exact_boxes(ctx, kind, leaf):
     assert torch.equal(b.intersectP(rd), b.intersectP(rl))
 
 
-@pytest.mark.parametrize("leaf", [1, 2])
+@pytest.mark.parametrize("leaf", [1, 2, 3, 8])
 @pytest.mark.parametrize("distance", [3.0, 30.0, 300.0])
 def test_rays_at_the_vertices_of_a_mesh(ctx, distance, leaf):
     """Rays at the vertices of a displaced sphere of 81,920 triangles, half of them
@@ -256,7 +256,7 @@ def test_rays_at_the_vertices_of_a_mesh(ctx, distance, leaf):
     assert torch.equal(b.intersectP(r), b.intersectP(rl))
 
 
-@pytest.mark.parametrize("leaf", [1, 2])
+@pytest.mark.parametrize("leaf", [1, 2, 3, 8])
 @pytest.mark.parametrize("kind", ["flat", "inside"])
 def test_rays_nearly_along_an_axis_at_the_vertices(ctx, kind, leaf):
     """Rays at the vertices of a height field whose direction has a component of
@@ -418,8 +418,8 @@ def test_a_walk_of_more_than_2_to_22_entries(ctx):
 @pytest.mark.parametrize("scenes", [1, 5])
 def test_the_tuner_tries_nothing_twice(ctx, scenes):
     """Every trial on the 4-wide layout differs from the others in something
-    that its kernel reads: leaf ranges up to 2, refills up to 8 lanes, the block
-    size, the ray sort."""
+    that its kernel reads: leaf ranges, refills up to 8 lanes, the block size, the
+    ray sort."""
     import ctypes as C
     import json
 
@@ -438,7 +438,7 @@ def test_the_tuner_tries_nothing_twice(ctx, scenes):
         ro = np.ascontiguousarray(10 * offs)
         ctx.check(ctx.lib.flg_autotune_trace_batched(ctx.h, b.h, C.byref(r), ro.ctypes.data_as(C.POINTER(C.c_int64)), 3,
                                                      C.byref(best), C.byref(w), C.byref(leaf), buf, len(buf)))
-    four = [(min(t["leaf_size"], 2), min(t["refill_lanes"], 8), t["block_threads"], t["ray_sort"])
+    four = [(t["leaf_size"], min(t["refill_lanes"], 8), t["block_threads"], t["ray_sort"])
             for t in json.loads(buf.value.decode())["trials"] if t["node_width"] == 4]
     assert w.value == 4 and len(four) > 6
     assert len(set(four)) == len(four), four
