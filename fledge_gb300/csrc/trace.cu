@@ -531,15 +531,16 @@ __global__ void __launch_bounds__(256)
 //     another hit whose t lies between, so boxes up to kBeyond of t beyond the hit
 //     are entered too.  Left open are triangles that lie further than that in front
 //     of their box: none in 150 M rays at the vertices of spheres and soups from 3,
-//     30 and 300 sizes away, 8 of 2 M where the directions' components along two axes
-//     are 1 to 1e-7, 34 of 131,072 rays through 16 slivers each, of 1e-7 to 1e-6 of the
-//     distance; in no occlusion.
+//     30 and 300 sizes away, 2 of 2 M where the direction has 1e-3 of its length
+//     along x, 10 of 2 M where two of its components are 1 to 1e-7 of it, 35 of
+//     131,072 rays through 16 slivers each, of 1e-7 to 1e-6 of the distance, none
+//     with slivers ten times as wide; and in all of these no occlusion.
 //   * Any hit: an accepted triangle counts if its own box passes the exact slab
 //     test.  A ray that found only others is traced again over the exact boxes
 //     (k_trace_retry4).
 // ----------------------------------------------------------------------------
 constexpr float kNear = 4.76837158203125e-07f;  // 2^-21
-constexpr float kBeyond = 1.220703125e-04f;     // 2^-13: of 4.2 M such rays 2^-20 left 28 wrong, 2^-14 one
+constexpr float kBeyond = 1.220703125e-04f;     // 2^-13: of 4.2 M rays at vertices 2^-20 left up to 37 open, 2^-14 one
 constexpr float kAround = 9.765625e-04f;        // 2^-10: what retrace4 takes for the surroundings of a hit
 // prim between k_trace4 and the kernels after it: a sorted position (< 2^28) with
 // kPending, -1, or kListed for a listed ray.  A listed ray's u and v hold two
