@@ -834,7 +834,7 @@ def _graph_step(torch, F, ctx, b, pos, rays, hits, topts, dev):
     ctx2.sync()
     ctx2.lib.flg_graph_destroy(g)
     ctx2.close()
-    res["launches_per_step"] = "build (10 kernels) + trace (3), one graph launch when replayed"
+    res["launches_per_step"] = "build (10 kernels) + trace (2), one graph launch when replayed"
     return res
 
 
