@@ -39,13 +39,14 @@ __device__ __forceinline__ int scene_of(const int64_t *__restrict__ tri_off, int
   return prev;
 }
 
-// Ordered float atomics (IEEE order on the sign/magnitude encoding).
+// Ordered float atomics (IEEE order on the sign/magnitude encoding; -0 goes with
+// the negative numbers, as its pattern does).
 __device__ __forceinline__ void atomic_min_f(float *a, float v) {
-  if (v >= 0.0f) atomicMin((int *)a, __float_as_int(v));
+  if (__float_as_int(v) >= 0) atomicMin((int *)a, __float_as_int(v));
   else atomicMax((unsigned int *)a, __float_as_uint(v));
 }
 __device__ __forceinline__ void atomic_max_f(float *a, float v) {
-  if (v >= 0.0f) atomicMax((int *)a, __float_as_int(v));
+  if (__float_as_int(v) >= 0) atomicMax((int *)a, __float_as_int(v));
   else atomicMin((unsigned int *)a, __float_as_uint(v));
 }
 

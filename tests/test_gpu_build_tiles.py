@@ -143,3 +143,26 @@ def test_cluster_sort_edges(ctx, oracle, n):
         if n > 1:
             U.assert_same_topology(b.topology(), oracle.build_bvh(pos))
     ctx.sync()
+
+
+@pytest.mark.parametrize("counts", [[40000], [33000, 40000, 500]])
+def test_scene_bounds_with_negative_zeros(ctx, oracle, counts):
+    """-0 as the extreme of most blocks' triangles, beside a negative minimum and
+    as the largest coordinate of an axis: the bounds, and so the codes, are the
+    oracle's."""
+    import fledge_gb300 as F
+    offs = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+    tri = np.random.default_rng(5).random((int(offs[-1]), 3, 3)).astype(np.float32)
+    tri[::7, 0, 0] = np.float32(-0.0)
+    tri[:, :, 1] = -tri[:, :, 1]
+    tri[::5, 1, 1] = np.float32(-0.0)
+    tri[offs[:-1] + 3, 1, 0] = np.float32(-0.25)
+    pos = tri.reshape(-1, 3)
+    if len(counts) == 1:
+        b, _ = U.gpu_build(ctx, pos)
+    else:
+        b = F.BatchedRadixBVHBuilder(F.InternalTriangleMesh(U.dev(pos)), offs, ctx, node_width=2)
+    for _ in range(3):
+        b.build()
+        for s in range(len(counts)):
+            U.assert_same_topology(b.topology(s), oracle.build_bvh(pos[3 * offs[s]:3 * offs[s + 1]]))
